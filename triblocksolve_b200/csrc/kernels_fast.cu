@@ -255,8 +255,7 @@ int launch_axpy2_f32_f64(cudaStream_t st, const float *c, const float *d, double
  * and the chain's last Gam couples it to the twist cell.  The twist kernel
  * then forms Dinv_tw = (D_m - A_tw Gam_top - C_tw Gam_bot)^-1 and stores
  * Dinv_tw A_tw / Dinv_tw C_tw in the G / Gam slots of the twist position.
- * Dinv is stored column-major like the input blocks; G and Gam row-major
- * (entry (i,j) at 9i+j), the order the Thomas kernel reads them in.  The
+ * All are stored column-major like the input blocks.  The
  * FP32 arrays, when given, are the FP64 results rounded once. */
 __device__ __forceinline__ void gj_invert(double *W, int t, unsigned *status) {
     const int i = t % NV, j = t / NV;
@@ -295,14 +294,13 @@ struct FactorOut {
         if (Dinv) Dinv[p * NB + t] = w;
         if (Dinv32) Dinv32[p * NB + t] = (float)w;
     }
-    /* row-major store of entry (i, j) */
-    __device__ void put_g(size_t p, int i, int j, double v) const {
-        if (G) G[p * NB + NV * i + j] = v;
-        if (G32) G32[p * NB + NV * i + j] = (float)v;
+    __device__ void put_g(size_t p, int t, double v) const {
+        if (G) G[p * NB + t] = v;
+        if (G32) G32[p * NB + t] = (float)v;
     }
-    __device__ void put_gam(size_t p, int i, int j, double v) const {
-        if (Gam) Gam[p * NB + NV * i + j] = v;
-        if (Gam32) Gam32[p * NB + NV * i + j] = (float)v;
+    __device__ void put_gam(size_t p, int t, double v) const {
+        if (Gam) Gam[p * NB + t] = v;
+        if (Gam32) Gam32[p * NB + t] = (float)v;
     }
 };
 
@@ -407,7 +405,7 @@ __global__ void __launch_bounds__(32) fast_factor_kernel(
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             out.put_dinv(cs, r0 + k + NV * jj, w[k]);
-            out.put_g(cs, r0 + k, jj, 0.0);
+            out.put_g(cs, r0 + k + NV * jj, 0.0);
             sM[r0 + k + NV * jj] = w[k];
         }
     }
@@ -441,7 +439,7 @@ __global__ void __launch_bounds__(32) fast_factor_kernel(
         if (act) {
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                out.put_gam(p - 1, r0 + k, jj, gm[k]);
+                out.put_gam(p - 1, r0 + k + NV * jj, gm[k]);
                 sG[r0 + k + NV * jj] = gm[k];
             }
         }
@@ -471,7 +469,7 @@ __global__ void __launch_bounds__(32) fast_factor_kernel(
                 double acc = 0.0;
 #pragma unroll
                 for (int q = 0; q < NV; ++q) acc += sM[r0 + k + NV * q] * sA[q + NV * jj];
-                out.put_g(p, r0 + k, jj, acc);
+                out.put_g(p, r0 + k + NV * jj, acc);
             }
         }
         __syncwarp(); /* sA and sC are rewritten by the next cell */
@@ -491,7 +489,7 @@ __global__ void __launch_bounds__(32) fast_factor_kernel(
                 double acc = 0.0;
 #pragma unroll
                 for (int q = 0; q < NV; ++q) acc += sM[r0 + k + NV * q] * sC[q + NV * jj];
-                out.put_gam(cs + len - 1, r0 + k, jj, acc);
+                out.put_gam(cs + len - 1, r0 + k + NV * jj, acc);
                 gamlast[((size_t)l * 2 + chain) * NB + r0 + k + NV * jj] = acc; /* column-major, FP64 */
             }
         }
@@ -540,8 +538,8 @@ __global__ void __launch_bounds__(128) fast_twist_kernel(
             gc += sW[i + NV * q] * sC[q + NV * j];
         }
         out.put_dinv(ptw, t, sW[t]);
-        out.put_g(ptw, i, j, ga);
-        out.put_gam(ptw, i, j, gc);
+        out.put_g(ptw, t, ga);
+        out.put_gam(ptw, t, gc);
     }
 }
 
@@ -942,22 +940,34 @@ template int launch_fast_resid<float>(cudaStream_t, const FastLayout &, int, con
 /* =========================================================== line Thomas
  * One warp per line, twisted: lanes 0..8 run the top chain and lanes
  * 16..24 the bottom chain of the line with the same instruction stream, so
- * a line of n cells takes n+1 dependent steps instead of 2n.  Lane 0
- * streams "jobs" through an NS-stage bulk-copy ring, each stage holding one
- * chunk of P cells per chain: jobs 0..nf-1 forward chunks (G rows and b),
- * jobs nf..2nf-1 backward chunks in reverse (Gam rows).  G and Gam are
- * row-major; lane i owns row i and holds the row of the NEXT cell in
- * registers while the current cell's dot product runs.  The previous
- * cell's 9-vector is published through shared memory in two copies (at
- * offsets 0 and 11), so that every lane reads it with the 16-byte
- * alignment of its row.  Chain forward:  y_s = b_s - G_s y_{s-1};  twist:
- * x_m = b_m - G_tw y_top - Gam_tw y_bot;  chain backward:  x_s = y_s -
- * Gam_s x_{s+1} (s+1 toward the twist).
- * YS: the line's y and x live in shared memory, and dU / U are written with
- * coalesced 16-byte accesses after the line is solved; otherwise y goes to
+ * a line of n cells takes n+1 dependent steps instead of 2n.  Lane 0 (or a
+ * copy warp) streams "jobs" through an NS-stage bulk-copy ring, each stage
+ * holding one chunk of P cells per chain: jobs 0..nf-1 forward chunks (G
+ * blocks and b), jobs nf..2nf-1 backward chunks in reverse (Gam blocks).
+ * Chain forward:  y_s = b_s - G_s y_{s-1};  twist:  x_m = b_m - G_tw y_top
+ * - Gam_tw y_bot;  chain backward:  x_s = y_s - Gam_s x_{s+1} (s+1 toward
+ * the twist).
+ *
+ * What bounds it where few lines share an SM is the step: publish the
+ * 9-vector in shared memory, read it back, a 9-term dot product.  On a warp
+ * alone, rows held in registers, that is 86 cycles; so everything else is
+ * kept off the chain.  Lane i owns row i; the row of the NEXT cell is read
+ * into registers behind the current step's vector reads, across chunk
+ * boundaries too: the next chunk's barrier is tested early in a chunk and
+ * the result looked at a few steps later (testing it between chunks and
+ * reading the row after it cost about 300 cycles per 8-cell chunk).  The
+ * blocks are column-major, so that the nine lanes read a column of nine
+ * neighbouring words: no bank conflicts and one copy of the vector (with
+ * row-major blocks: two copies, lane-dependent offsets, 122 cycles a step
+ * against 106; rows as aligned pairs of columns: 111).  Two partial sums,
+ * since the vector's words arrive one after the other: the last one is two
+ * operations from the result (three sums: 115 cycles).
+ * YS: the line's y and x live in shared memory, and dU / U are written after
+ * the line is solved: dU by one bulk copy, and in FP64 U += dU by one bulk
+ * add (the L2 adds, so the warp does not wait for U); otherwise y goes to
  * global memory (read back one chunk ahead) and dU / U per step, U read
  * one chunk ahead with y (one-warp form) or staged behind the backward
- * chunk's Gam rows by the copy warp (warp-specialised form).
+ * chunk's Gam blocks by the copy warp (warp-specialised form).
  *   accumulate = 0:  U = dU
  *   accumulate = 1:  U += dU (the FP64 sweeps of a context; U read from a
  *                    second buffer Uin when one is given: line partitions)
@@ -976,120 +986,133 @@ __host__ __device__ inline uint32_t thomas_stage_bytes() {
     return 2 * thomas_half_bytes<T>();
 }
 
-/* Lane constants for rows whose start parity is (q + i) & 1: pairs start at
- * row+par, the single element is row[8] (par 0) or row[0] (par 1); the
- * broadcast vector is read from copy A (offset 0) or copy B (offset 10,
- * holding y_j at 11+j) so that the pairs line up.  The same scheme serves
- * FP64 (16-byte pairs) and FP32 (8-byte pairs). */
-struct LaneOff {
-    int row;
-    int rp[2], rs[2], vp[2], vs[2];
-};
+/* The vector a step reads and the row it multiplies.
+ * FP64: lane i's row in column order, and one copy of the vector read as
+ * four pairs and a single (two partial sums, see above).
+ * FP32: the vector in two copies (y_j at j and at 11 + j), so that a lane
+ * whose row number and cell have different parity starts its pairs at
+ * column 1; the order of the sum by lane is kept as it was first written,
+ * since the outer refinement's history shows a change of FP32 rounding. */
+template <typename T> struct StepVec;
 
-__device__ __forceinline__ LaneOff lane_offsets(int i) {
-    LaneOff o;
-    o.row = NV * i;
-    for (int odd = 0; odd < 2; ++odd) {
-        const int par = (i + odd) & 1;
-        o.rp[odd] = NV * i + par;
-        o.rs[odd] = NV * i + (par ? 0 : 8);
-        o.vp[odd] = par ? 12 : 0;
-        o.vs[odd] = par ? 0 : 8;
-    }
-    return o;
-}
-
-struct RowD {
-    double2 r0, r1, r2, r3;
+template <>
+struct StepVec<double> {
+    static constexpr int BUF = 10; /* words of one buffer */
+    double2 p[4];
     double s;
+    __device__ __forceinline__ void load(const double *v, int, int) {
+        const double2 *q = reinterpret_cast<const double2 *>(v);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) p[c] = q[c];
+        s = v[8];
+    }
+    static __device__ __forceinline__ void put(double *buf, int i, double y) { buf[i] = y; }
 };
-struct RowF {
-    float2 r0, r1, r2, r3;
+
+template <>
+struct StepVec<float> {
+    static constexpr int BUF = 20;
+    float2 p[4];
     float s;
+    __device__ __forceinline__ void load(const float *v, int i, int odd) {
+        const int par = (i + odd) & 1;
+        const float2 *q = reinterpret_cast<const float2 *>(v + (par ? 12 : 0));
+#pragma unroll
+        for (int c = 0; c < 4; ++c) p[c] = q[c];
+        s = v[par ? 0 : 8];
+    }
+    static __device__ __forceinline__ void put(float *buf, int i, float y) {
+        buf[i] = y;
+        buf[11 + i] = y;
+    }
 };
-template <typename T> struct RowOf;
-template <> struct RowOf<double> { using type = RowD; };
-template <> struct RowOf<float> { using type = RowF; };
 
-__device__ __forceinline__ void load_row(RowD &R, const double *rowbase, const LaneOff &o, int odd) {
-    const double2 *r = reinterpret_cast<const double2 *>(rowbase + o.rp[odd]);
-    R.r0 = r[0];
-    R.r1 = r[1];
-    R.r2 = r[2];
-    R.r3 = r[3];
-    R.s = rowbase[o.rs[odd]];
+/* row i of a block, in the order StepVec gives the vector: FP64 columns
+ * 0..8; FP32 the single's column, then the pairs' */
+template <typename T>
+struct Row {
+    T r[NV];
+};
+
+__device__ __forceinline__ void load_row(Row<double> &R, const double *blk, int i, int) {
+#pragma unroll
+    for (int j = 0; j < NV; ++j) R.r[j] = blk[NV * j + i];
 }
 
-__device__ __forceinline__ void load_row(RowF &R, const float *rowbase, const LaneOff &o, int odd) {
-    const float2 *r = reinterpret_cast<const float2 *>(rowbase + o.rp[odd]);
-    R.r0 = r[0];
-    R.r1 = r[1];
-    R.r2 = r[2];
-    R.r3 = r[3];
-    R.s = rowbase[o.rs[odd]];
+__device__ __forceinline__ void load_row(Row<float> &R, const float *blk, int i, int odd) {
+    const int par = (i + odd) & 1;
+    const float *q = blk + i - (par ? 0 : NV);
+    R.r[0] = blk[par ? i : 8 * NV + i];
+#pragma unroll
+    for (int j = 1; j < NV; ++j) R.r[j] = q[NV * j];
 }
 
-/* init - row . vec, vec from the broadcast buffer `cur` */
-__device__ __forceinline__ double row_dot(const RowD &R, const double *cur, const LaneOff &o,
-                                          int odd, double init) {
-    const double2 *v = reinterpret_cast<const double2 *>(cur + o.vp[odd]);
-    const double2 v0 = v[0], v1 = v[1], v2 = v[2], v3 = v[3];
-    const double w = cur[o.vs[odd]];
-    double a0 = init - R.s * w;
-    double a1 = R.r0.x * v0.x;
-    double a2 = R.r0.y * v0.y;
-    a0 -= R.r1.x * v1.x;
-    a1 += R.r1.y * v1.y;
-    a2 += R.r2.x * v2.x;
-    a0 -= R.r2.y * v2.y;
-    a1 += R.r3.x * v3.x;
-    a2 += R.r3.y * v3.y;
+/* init - row . vec */
+__device__ __forceinline__ double row_dot(const Row<double> &R, const StepVec<double> &V, double init) {
+    double a0 = init - R.r[0] * V.p[0].x;
+    double a1 = R.r[1] * V.p[0].y;
+#pragma unroll
+    for (int c = 1; c < 4; ++c) {
+        a0 -= R.r[2 * c] * V.p[c].x;
+        a1 += R.r[2 * c + 1] * V.p[c].y;
+    }
+    a0 -= R.r[8] * V.s;
+    return a0 - a1;
+}
+
+__device__ __forceinline__ float row_dot(const Row<float> &R, const StepVec<float> &V, float init) {
+    float a0 = init - R.r[0] * V.s;
+    float a1 = R.r[1] * V.p[0].x;
+    float a2 = R.r[2] * V.p[0].y;
+    a0 -= R.r[3] * V.p[1].x;
+    a1 += R.r[4] * V.p[1].y;
+    a2 += R.r[5] * V.p[2].x;
+    a0 -= R.r[6] * V.p[2].y;
+    a1 += R.r[7] * V.p[3].x;
+    a2 += R.r[8] * V.p[3].y;
     return a0 - (a1 + a2);
 }
 
-__device__ __forceinline__ float row_dot(const RowF &R, const float *cur, const LaneOff &o,
-                                         int odd, float init) {
-    const float2 *v = reinterpret_cast<const float2 *>(cur + o.vp[odd]);
-    const float2 v0 = v[0], v1 = v[1], v2 = v[2], v3 = v[3];
-    const float w = cur[o.vs[odd]];
-    float a0 = init - R.s * w;
-    float a1 = R.r0.x * v0.x;
-    float a2 = R.r0.y * v0.y;
-    a0 -= R.r1.x * v1.x;
-    a1 += R.r1.y * v1.y;
-    a2 += R.r2.x * v2.x;
-    a0 -= R.r2.y * v2.y;
-    a1 += R.r3.x * v3.x;
-    a2 += R.r3.y * v3.y;
-    return a0 - (a1 + a2);
-}
+/* words of the broadcast vectors: 2 halves x 2 alternating buffers */
+template <typename T>
+constexpr int BCAST = 4 * StepVec<T>::BUF;
 
 /* Forward steps kbase..kbase+P-1 of this half's chain (length len, first
- * position cpos relative to the line start).  CHECK: some steps of the
- * warp may lie beyond one chain's end; those compute but write nothing. */
-template <typename T, int P, bool CHECK, bool YS>
-__device__ __forceinline__ void fwd_chunk(const T *sG, const T *sB, T *bc, T *ys, T *yg, int kbase,
-                                          int len, int cpos, int i, const LaneOff &o,
-                                          uint64_t ypol) {
-    typename RowOf<T>::type cur_row, next_row;
-    load_row(cur_row, sG, o, 0);
-    T cur_b = sB[i];
+ * position cpos relative to the line start), the chunk's blocks at sG and
+ * its b behind them; `row` / `bi` hold the first cell's row and b, and are
+ * left holding those of the next chunk, whose stage next() gives (null:
+ * none; probe() has asked for it).  CHECK: some steps of the warp may lie
+ * beyond one chain's end; those compute but write nothing. */
+template <typename T, int P, bool CHECK, bool YS, typename Probe, typename Next>
+__device__ __forceinline__ void fwd_chunk(const T *sG, Row<T> &row, T &bi, T *bc, T *ys, T *yg,
+                                          int kbase, int len, int cpos, int i, uint64_t ypol,
+                                          Probe &&probe, Next &&next) {
+    constexpr int VB = StepVec<T>::BUF;
+    const T *sB = sG + P * NB;
+    const T *sN = sG;
 #pragma unroll
     for (int q = 0; q < P; ++q) {
-        const int odd = q & 1;
-        T next_b = T(0);
+        Row<T> nrow;
+        StepVec<T> v;
+        T nb = T(0);
+        v.load(bc + (q & 1) * VB, i, q & 1);
         if (q + 1 < P) {
-            load_row(next_row, sG + (q + 1) * NB, o, odd ^ 1);
-            next_b = sB[(q + 1) * NV + i];
+            load_row(nrow, sG + (q + 1) * NB, i, (q + 1) & 1);
+            nb = sB[(q + 1) * NV + i];
+        } else { /* no next chunk: some cell of this one, not used */
+            load_row(nrow, sN, i, 0);
+            nb = sN[P * NB + i];
         }
-        const T *cur = bc + odd * 20;
-        T *nxt = bc + (odd ^ 1) * 20;
-        const T yi = row_dot(cur_row, cur, o, odd, cur_b);
+        if (q == 1) probe();
+        if (q == P - 3) {
+            const T *n = next();
+            if (n) sN = n;
+        }
+        const T yi = row_dot(row, v, bi);
         /* lanes 9..15 of a half compute row 8 from the same inputs as lane
          * 8 and store the same value to the same address: no divergence */
         if (!CHECK || kbase + q < len) {
-            nxt[i] = yi;
-            nxt[11 + i] = yi;
+            StepVec<T>::put(bc + ((q & 1) ^ 1) * VB, i, yi);
             const int pos = cpos + kbase + q;
             if (YS)
                 ys[pos * NV + i] = yi;
@@ -1097,34 +1120,42 @@ __device__ __forceinline__ void fwd_chunk(const T *sG, const T *sB, T *bc, T *ys
                 st_hint(yg + (size_t)pos * NV + i, yi, ypol);
         }
         __syncwarp();
-        cur_row = next_row;
-        cur_b = next_b;
+        row = nrow;
+        bi = nb;
     }
 }
 
-/* uv: U of the chunk's cells read ahead in registers, or sU (when set):
- * the chunk's U staged behind its Gam rows */
-template <typename T, int P, bool CHECK, bool YS>
-__device__ __forceinline__ void bwd_chunk(const T *sG, T *bc, T *ys, const T *yv, const T *uv,
-                                          T *dUl, T *Ul, int kbase, int len, int cpos, int i,
-                                          const LaneOff &o, const T *sU = nullptr) {
-    typename RowOf<T>::type cur_row, next_row;
-    load_row(cur_row, sG + (P - 1) * NB, o, (P - 1) & 1);
+/* Backward steps kbase+P-1..kbase, `row` holding the row of the first of
+ * them (and left holding the next chunk's).  YS: y and x in ys, `yk` the y
+ * of the first step, left holding the next chunk's; otherwise the chunk's
+ * y in yv.  uv: U of the chunk's cells read ahead in registers, or sU (when
+ * set): the chunk's U staged behind its Gam blocks */
+template <typename T, int P, bool CHECK, bool YS, typename Probe, typename Next>
+__device__ __forceinline__ void bwd_chunk(const T *sG, Row<T> &row, T &yk, T *bc, T *ys, const T *yv,
+                                          const T *uv, T *dUl, T *Ul, int kbase, int len, int cpos,
+                                          int i, const T *sU, Probe &&probe, Next &&next) {
+    constexpr int VB = StepVec<T>::BUF;
+    const T *sN = sG;
 #pragma unroll
     for (int q = P - 1; q >= 0; --q) {
-        const int odd = q & 1;
-        if (q > 0) load_row(next_row, sG + (q - 1) * NB, o, odd ^ 1);
         const int f = (P - 1 - q) & 1; /* buffer alternates per step */
-        const T *cur = bc + f * 20;
-        T *nxt = bc + (f ^ 1) * 20;
-        const bool valid = !CHECK || (kbase + q >= 0 && kbase + q < len);
-        const int pos = cpos + kbase + q;
-        T yk = T(0);
-        if (valid) yk = YS ? ys[pos * NV + i] : yv[q];
-        const T d = row_dot(cur_row, cur, o, odd, yk);
+        Row<T> nrow;
+        StepVec<T> v;
+        v.load(bc + f * VB, i, q & 1);
+        load_row(nrow, q > 0 ? sG + (q - 1) * NB : sN + (P - 1) * NB, i, (q + P - 1) & 1);
+        if (q == P - 2) probe();
+        if (q == 2) {
+            const T *n = next();
+            if (n) sN = n;
+        }
+        const int k = kbase + q;
+        const bool valid = !CHECK || (k >= 0 && k < len);
+        const int pos = cpos + k;
+        T nyk = T(0);
+        if (YS && ((CHECK || q == 0) ? (k >= 1 && k - 1 < len) : true)) nyk = ys[(pos - 1) * NV + i];
+        const T d = row_dot(row, v, YS ? yk : (valid ? yv[q] : T(0)));
         if (valid) { /* lanes 9..15 repeat lane 8's row, value and address */
-            nxt[i] = d;
-            nxt[11 + i] = d;
+            StepVec<T>::put(bc + (f ^ 1) * VB, i, d);
             if (YS) {
                 ys[pos * NV + i] = d;
             } else {
@@ -1133,7 +1164,8 @@ __device__ __forceinline__ void bwd_chunk(const T *sG, T *bc, T *ys, const T *yv
             }
         }
         __syncwarp();
-        cur_row = next_row;
+        row = nrow;
+        yk = nyk;
     }
 }
 
@@ -1166,13 +1198,12 @@ __device__ __forceinline__ bool thomas_line(
     const uint32_t stage = 2 * P * (NB + NV) * sizeof(T);
     const uint32_t half = P * (NB + NV) * sizeof(T);
     unsigned char *st0 = smem + thomas_hdr<WS>();
-    /* broadcast: 2 halves x 2 alternating buffers x [copy A: 10][copy B: 10] */
     T *bcall = reinterpret_cast<T *>(st0 + (size_t)NS * stage);
-    T *ys = bcall + 80;
+    constexpr int VB = StepVec<T>::BUF;
+    T *ys = bcall + BCAST<T>;
     const int lane = threadIdx.x & 31;
     const int h = lane >> 4, li = lane & 15;
     const int i = li < NV ? li : NV - 1;
-    const LaneOff off = lane_offsets(i);
     const int nb = n - 1 - m;
     const int len = h ? nb : m;      /* this half's chain length */
     const int cpos = h ? m : 0;      /* its first position, relative to ps */
@@ -1180,21 +1211,20 @@ __device__ __forceinline__ bool thomas_line(
     const int nch = h ? nchB : nchT;
     const int nf = nchT > nchB ? nchT : nchB;
     const int njobs = 2 * nf;
-    T *bc = bcall + h * 40;
+    T *bc = bcall + h * 2 * VB;
     T *yl = y + (size_t)ps * NV;
     T *dUl = dU + (size_t)ps * NV;
     T *Ul = U ? U + (size_t)ps * NV : nullptr;
     const T *Uil = Uin ? Uin + (size_t)ps * NV : Ul;
-    auto parity = [&](int job) { return ((pbase >> (job % NS)) ^ (uint32_t)(job / NS)) & 1u; };
 
     const bool producer = WS && (threadIdx.x >> 5) == 1;
     /* warp-specialised form: the copy warp also stages U behind the
-     * backward chunks' Gam rows (where the forward stages hold b), so the
+     * backward chunks' Gam blocks (where the forward stages hold b), so the
      * chain warp reads it from shared memory */
     const bool stage_u = WS && !YS && accumulate == 1 && Ul != nullptr;
     __syncwarp(); /* the previous line's readers of the stages are done */
     if (!producer)
-        for (int t = lane; t < 80; t += 32) bcall[t] = T(0);
+        for (int t = lane; t < BCAST<T>; t += 32) bcall[t] = T(0);
     __syncwarp();
 
     /* copy size of chunk c of a chain of length ln, rounded up to 4 cells
@@ -1234,87 +1264,133 @@ __device__ __forceinline__ bool thomas_line(
             }
         }
     };
+    /* Each full barrier completes one phase per job landed in its stage,
+     * each empty barrier one per job consumed from it: `pbase` gives the
+     * parity of the first of them (carried across lines by a persistent
+     * CTA), RingPos the rest, without divisions */
+    struct RingPos {
+        int s = 0;
+        uint32_t wrap = 0;
+        __device__ void next(int NS) {
+            if (++s == NS) {
+                s = 0;
+                wrap ^= 1u;
+            }
+        }
+    };
+    auto parity = [&](const RingPos &r) { return ((pbase >> r.s) ^ r.wrap) & 1u; };
+    /* after the line, every job was waited for: barrier s completed one
+     * phase per job j = s, s+NS, ... below njobs */
+    auto close_phases = [&]() {
+        for (int s = 0; s < NS && s < njobs; ++s) {
+            const int cnt = (njobs - 1 - s) / NS + 1;
+            pbase ^= (uint32_t)(cnt & 1) << s;
+        }
+    };
     if (producer) {
-        /* every job as soon as the consumer has released its stage.  Each
-         * empty barrier completes one phase per job consumed from its stage,
-         * as each full barrier does per job landed, so the parity bits of
-         * `pbase` serve both (a persistent CTA carries them across lines);
-         * job j >= NS waits for the consumption of job j - NS */
+        /* every job as soon as the consumer has released its stage: job
+         * j >= NS waits for the consumption of job j - NS */
         if (lane == 0) {
+            RingPos r, e; /* e: the consumed job's place, NS jobs behind */
             for (int job = 0; job < njobs; ++job) {
                 if (*ws_abort) break;
-                const int s = job % NS;
-                if (job >= NS && !mbar_wait(&empty[s], parity(job - NS))) {
-                    atomicOr(status, ST_TIMEOUT);
-                    break;
+                if (job >= NS) {
+                    if (!mbar_wait(&empty[e.s], parity(e))) {
+                        atomicOr(status, ST_TIMEOUT);
+                        break;
+                    }
+                    e.next(NS);
                 }
-                issue(job, s);
+                issue(job, r.s);
+                r.next(NS);
                 *ws_issued = job + 1;
             }
         }
         __syncwarp();
         __syncthreads(); /* meets the consumer's */
-        for (int s = 0; s < NS && s < njobs; ++s) {
-            const int cnt = (njobs - 1 - s) / NS + 1;
-            pbase ^= (uint32_t)(cnt & 1) << s;
-        }
+        close_phases();
         return true;
     }
     int issued = 0;
     if (!WS && lane == 0) {
         for (; issued < NS && issued < njobs; ++issued) issue(issued, issued);
     }
-    int consumed = 0;
+    int consumed = 0; /* jobs waited for */
     bool timed_out = false;
     const int both_full = (m < nb ? m : nb) / P; /* jobs where both chains run P steps */
     /* y, written by the forward chains and read once by the backward ones */
     const uint64_t ypol_last = YS ? 0ull : policy_evict_last();
     const uint64_t ypol_first = YS ? 0ull : policy_evict_first();
 
-    /* ---------------- forward */
-    for (int c = 0; c < nf; ++c) {
-        const int s = c % NS;
-        const bool ok = mbar_wait(&bars[s], parity(c));
-        if (__any_sync(FULL, !ok)) {
-            timed_out = true;
-            break;
+    RingPos rd; /* the next job to wait for */
+    bool landed = false;
+    auto probe = [&]() { landed = mbar_test(&bars[rd.s], parity(rd)); };
+    /* the next job's stage (this half's part of it), waited for when probe()
+     * did not find it landed; null when the wait ran out of time */
+    auto take = [&]() -> const T * {
+        const T *p = reinterpret_cast<const T *>(st0 + (size_t)rd.s * stage + h * half);
+        if (__any_sync(FULL, !landed)) {
+            if (__any_sync(FULL, !mbar_wait(&bars[rd.s], parity(rd)))) {
+                timed_out = true;
+                return nullptr;
+            }
         }
         ++consumed;
-        const T *sG = reinterpret_cast<const T *>(st0 + (size_t)s * stage + h * half);
-        const T *sB = sG + P * NB;
-        if (c < both_full)
-            fwd_chunk<T, P, false, YS>(sG, sB, bc, ys, yl, c * P, len, cpos, i, off, ypol_last);
-        else
-            fwd_chunk<T, P, true, YS>(sG, sB, bc, ys, yl, c * P, len, cpos, i, off, ypol_last);
-        __syncwarp();
+        rd.next(NS);
+        return p;
+    };
+    /* the stage of the chunk just finished may be refilled */
+    int rel = 0;
+    auto release = [&]() {
         if (WS) {
-            if (lane == 0) mbar_arrive(&empty[s]);
+            mbar_arrive_if(&empty[rel], lane == 0);
         } else if (lane == 0 && issued < njobs) {
-            issue(issued, s);
+            issue(issued, rel);
             ++issued;
         }
+        if (++rel == NS) rel = 0;
+    };
+
+    /* ---------------- forward */
+    const T *sG = nullptr, *sN = nullptr;
+    Row<T> row;
+    T bi = T(0);
+    if (nf > 0) {
+        sG = take();
+        if (sG) {
+            load_row(row, sG, i, 0);
+            bi = sG[P * NB + i];
+        }
+    }
+    for (int c = 0; c < nf && !timed_out; ++c) {
+        auto next = [&]() -> const T * { return sN = (c + 1 < nf ? take() : nullptr); };
+        if (c < both_full)
+            fwd_chunk<T, P, false, YS>(sG, row, bi, bc, ys, yl, c * P, len, cpos, i, ypol_last, probe,
+                                       next);
+        else
+            fwd_chunk<T, P, true, YS>(sG, row, bi, bc, ys, yl, c * P, len, cpos, i, ypol_last, probe,
+                                      next);
+        release();
+        sG = sN;
     }
 
     if (!timed_out) {
         /* ---------------- twist: x_m = b_m - G_tw y_top - Gam_tw y_bot */
         const int ptw = n - 1; /* relative to ps */
-        const T *ytop = bcall + 0 * 40 + (m & 1) * 20;
-        const T *ybot = bcall + 1 * 40 + (nb & 1) * 20;
+        const T *ytop = bcall + (m & 1) * VB;
+        const T *ybot = bcall + (2 + (nb & 1)) * VB;
         T xm = T(0);
         if (lane < NV) {
-            const T *gr = G + (size_t)(ps + ptw) * NB + NV * lane;
-            const T *cr = Gam + (size_t)(ps + ptw) * NB + NV * lane;
+            const T *gr = G + (size_t)(ps + ptw) * NB + lane;
+            const T *cr = Gam + (size_t)(ps + ptw) * NB + lane;
             T acc = b[(size_t)(ps + ptw) * NV + lane];
 #pragma unroll
-            for (int j = 0; j < NV; ++j) acc -= gr[j] * ytop[j] + cr[j] * ybot[j];
+            for (int j = 0; j < NV; ++j) acc -= gr[NV * j] * ytop[j] + cr[NV * j] * ybot[j];
             xm = acc;
         }
         __syncwarp();
         if (lane < NV) {
-            for (int t = 0; t < 4; ++t) {
-                bcall[t * 20 + lane] = xm;
-                bcall[t * 20 + 11 + lane] = xm;
-            }
+            for (int t = 0; t < 4; ++t) StepVec<T>::put(bcall + t * VB, lane, xm);
             if (YS)
                 ys[ptw * NV + lane] = xm;
             else {
@@ -1340,34 +1416,30 @@ __device__ __forceinline__ bool thomas_line(
             }
         };
         if (!YS) load_chunk(nch - 1, yv, uv);
-        for (int jb = 0; jb < nf; ++jb) {
-            const int job = nf + jb;
+        T yk = T(0);
+        if (nf > 0) {
+            probe();
+            sG = take();
+            if (sG) load_row(row, sG + (P - 1) * NB, i, (P - 1) & 1);
+            const int k = nch * P - 1;
+            if (YS && k >= 0 && k < len) yk = ys[(cpos + k) * NV + i];
+        }
+        for (int jb = 0; jb < nf && !timed_out; ++jb) {
             const int c = nch - 1 - jb; /* this half's chunk (may be < 0) */
             if (!YS) load_chunk(c - 1, nyv, nuv);
-            const int s = job % NS;
-            const bool ok = mbar_wait(&bars[s], parity(job));
-            if (__any_sync(FULL, !ok)) {
-                timed_out = true;
-                break;
-            }
-            ++consumed;
-            const T *sG = reinterpret_cast<const T *>(st0 + (size_t)s * stage + h * half);
             const bool full = (nchT - 1 - jb) * P + P <= m && (nchB - 1 - jb) * P + P <= nb &&
                               nchT - 1 - jb >= 0 && nchB - 1 - jb >= 0;
             const T *sU = stage_u ? sG + P * NB : nullptr;
+            T *Uw = accumulate < 2 ? Ul : nullptr;
+            auto next = [&]() -> const T * { return sN = (jb + 1 < nf ? take() : nullptr); };
             if (full)
-                bwd_chunk<T, P, false, YS>(sG, bc, ys, yv, uv, dUl, accumulate < 2 ? Ul : nullptr,
-                                           c * P, len, cpos, i, off, sU);
+                bwd_chunk<T, P, false, YS>(sG, row, yk, bc, ys, yv, uv, dUl, Uw, c * P, len, cpos, i, sU,
+                                           probe, next);
             else
-                bwd_chunk<T, P, true, YS>(sG, bc, ys, yv, uv, dUl, accumulate < 2 ? Ul : nullptr,
-                                          c * P, len, cpos, i, off, sU);
-            __syncwarp();
-            if (WS) {
-                if (lane == 0) mbar_arrive(&empty[s]);
-            } else if (lane == 0 && issued < njobs) {
-                issue(issued, s);
-                ++issued;
-            }
+                bwd_chunk<T, P, true, YS>(sG, row, yk, bc, ys, yv, uv, dUl, Uw, c * P, len, cpos, i, sU,
+                                          probe, next);
+            release();
+            sG = sN;
             if (!YS) {
 #pragma unroll
                 for (int q = 0; q < P; ++q) {
@@ -1377,11 +1449,24 @@ __device__ __forceinline__ bool thomas_line(
             }
         }
         if (YS && !timed_out) {
-            /* dU = x (and U = x or U += x) for the line's n cells; the U loads
-             * of a batch are issued together so that their latencies overlap */
-            const int nv = n * NV;
+            /* dU = x (and U = x or U += x) for the line's n cells.  The whole
+             * groups of 4 cells (16-byte multiples) of dU go by one bulk
+             * copy, and in FP64 those of U by one bulk add (U + x rounded
+             * once, as the loop would); what is left, and the forms that
+             * read another buffer, by the loop, whose U loads of a batch are
+             * issued together so that their latencies overlap */
+            const int nbulk = (n & ~3) * NV, nv = n * NV;
+            const bool ub = accumulate == 0 || (accumulate == 1 && sizeof(T) == 8 && !Uin);
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0 && nbulk > 0) {
+                bulk_s2g(dUl, ys, nbulk * sizeof(T));
+                if (accumulate == 0) bulk_s2g(Ul, ys, nbulk * sizeof(T));
+                if (accumulate == 1 && ub) bulk_add_s2g(Ul, ys, nbulk * sizeof(T));
+                bulk_s2g_commit();
+            }
             constexpr int B = 8;
-            for (int t0 = lane; t0 < nv; t0 += 32 * B) {
+            for (int t0 = (accumulate < 2 && !ub ? 0 : nbulk) + lane; t0 < nv; t0 += 32 * B) {
                 T u[B];
 #pragma unroll
                 for (int k = 0; k < B; ++k) {
@@ -1393,11 +1478,13 @@ __device__ __forceinline__ bool thomas_line(
                     const int t = t0 + 32 * k;
                     if (t < nv) {
                         const T x = ys[t];
-                        dUl[t] = x;
+                        if (t >= nbulk) dUl[t] = x;
                         if (accumulate < 2) Ul[t] = u[k] + x;
                     }
                 }
             }
+            if (lane == 0 && nbulk > 0) bulk_s2g_wait_read(); /* before the CTA's memory goes */
+            __syncwarp();
         }
     }
     if (timed_out) {
@@ -1411,19 +1498,17 @@ __device__ __forceinline__ bool thomas_line(
         }
         if (lane == 0) {
             atomicOr(status, ST_TIMEOUT);
-            for (int job = consumed; job < issued; ++job)
-                mbar_wait(&bars[job % NS], parity(job), 1LL << 28);
+            RingPos r = rd;
+            for (int job = consumed; job < issued; ++job) {
+                mbar_wait(&bars[r.s], parity(r), 1LL << 28);
+                r.next(NS);
+            }
         }
         __syncwarp();
         return false;
     }
     if (WS) __syncthreads(); /* meets the producer's */
-    /* every job was waited for: barrier s completed one phase per job
-     * j = s, s+NS, ... below njobs */
-    for (int s = 0; s < NS && s < njobs; ++s) {
-        const int cnt = (njobs - 1 - s) / NS + 1;
-        pbase ^= (uint32_t)(cnt & 1) << s;
-    }
+    close_phases();
     return true;
 }
 
@@ -1602,7 +1687,7 @@ static ThomasCfg thomas_cfg(const FastLayout &L) {
     const int per_sm = (L.nline + nsm - 1) / nsm;
     const long long budget = (long long)smem_sm / (per_sm > 0 ? per_sm : 1) - reserved;
     const size_t ys_bytes = (size_t)((L.max_len + 3) & ~3) * NV * sizeof(T);
-    const size_t fixed = thomas_hdr<WS>() + 80 * sizeof(T);
+    const size_t fixed = thomas_hdr<WS>() + BCAST<T> * sizeof(T);
     ThomasCfg c;
     c.ys = (long long)(fixed + ys_bytes + 3 * sb) <= budget;
     long long left = budget - (long long)fixed - (c.ys ? (long long)ys_bytes : 0);
@@ -2151,7 +2236,7 @@ static int sm_count() {
 template <typename T>
 size_t thomas_batch_smem(int stages, int warps) {
     return (warps == 2 ? thomas_hdr<true>() : thomas_hdr<false>()) +
-           (size_t)stages * 2 * THOMAS_P * (NB + NV) * sizeof(T) + 80 * sizeof(T);
+           (size_t)stages * 2 * THOMAS_P * (NB + NV) * sizeof(T) + BCAST<T> * sizeof(T);
 }
 
 template <typename T>
@@ -2706,35 +2791,35 @@ constexpr int MULTI_RPW = 2;
 template <int P, bool CHECK>
 __device__ __forceinline__ void fwd_chunk_m(const double *sG, const double *const *sB,
                                             double *const *bc, double *const *yg, int nown,
-                                            int kbase, int len, int cpos, int i,
-                                            const LaneOff &o) {
-    RowD cur_row, next_row;
-    load_row(cur_row, sG, o, 0);
+                                            int kbase, int len, int cpos, int i) {
+    Row<double> cur_row, next_row;
+    load_row(cur_row, sG, i, 0);
     double cur_b[MULTI_RPW], next_b[MULTI_RPW];
 #pragma unroll
     for (int j = 0; j < MULTI_RPW; ++j) cur_b[j] = sB[j][i];
 #pragma unroll
     for (int q = 0; q < P; ++q) {
-        const int odd = q & 1;
+        StepVec<double> v[MULTI_RPW];
 #pragma unroll
-        for (int j = 0; j < MULTI_RPW; ++j) next_b[j] = 0.0;
+        for (int j = 0; j < MULTI_RPW; ++j) {
+            v[j].load(bc[j] + (q & 1) * 10, i, 0);
+            next_b[j] = 0.0;
+        }
         if (q + 1 < P) {
-            load_row(next_row, sG + (q + 1) * NB, o, odd ^ 1);
+            load_row(next_row, sG + (q + 1) * NB, i, 0);
 #pragma unroll
             for (int j = 0; j < MULTI_RPW; ++j) next_b[j] = sB[j][(q + 1) * NV + i];
         }
         double yi[MULTI_RPW];
 #pragma unroll
-        for (int j = 0; j < MULTI_RPW; ++j) yi[j] = row_dot(cur_row, bc[j] + odd * 20, o, odd, cur_b[j]);
+        for (int j = 0; j < MULTI_RPW; ++j) yi[j] = row_dot(cur_row, v[j], cur_b[j]);
         /* lanes 9..15 repeat lane 8's row, value and address: no divergence */
         if (!CHECK || kbase + q < len) {
             const int pos = cpos + kbase + q;
 #pragma unroll
             for (int j = 0; j < MULTI_RPW; ++j) {
                 if (j < nown) {
-                    double *nxt = bc[j] + (odd ^ 1) * 20;
-                    nxt[i] = yi[j];
-                    nxt[11 + i] = yi[j];
+                    bc[j][((q & 1) ^ 1) * 10 + i] = yi[j];
                     yg[j][(size_t)pos * NV + i] = yi[j];
                 }
             }
@@ -2749,28 +2834,26 @@ __device__ __forceinline__ void fwd_chunk_m(const double *sG, const double *cons
 template <int P, bool CHECK>
 __device__ __forceinline__ void bwd_chunk_m(const double *sG, double *const *bc,
                                             const double (*yv)[P], double *const *dUl, int nown,
-                                            int kbase, int len, int cpos, int i,
-                                            const LaneOff &o) {
-    RowD cur_row, next_row;
-    load_row(cur_row, sG + (P - 1) * NB, o, (P - 1) & 1);
+                                            int kbase, int len, int cpos, int i) {
+    Row<double> cur_row, next_row;
+    load_row(cur_row, sG + (P - 1) * NB, i, 0);
 #pragma unroll
     for (int q = P - 1; q >= 0; --q) {
-        const int odd = q & 1;
-        if (q > 0) load_row(next_row, sG + (q - 1) * NB, o, odd ^ 1);
         const int f = (P - 1 - q) & 1;
+        StepVec<double> v[MULTI_RPW];
+#pragma unroll
+        for (int j = 0; j < MULTI_RPW; ++j) v[j].load(bc[j] + f * 10, i, 0);
+        if (q > 0) load_row(next_row, sG + (q - 1) * NB, i, 0);
         const bool valid = !CHECK || (kbase + q >= 0 && kbase + q < len);
         const int pos = cpos + kbase + q;
         double d[MULTI_RPW];
 #pragma unroll
-        for (int j = 0; j < MULTI_RPW; ++j)
-            d[j] = row_dot(cur_row, bc[j] + f * 20, o, odd, valid ? yv[j][q] : 0.0);
+        for (int j = 0; j < MULTI_RPW; ++j) d[j] = row_dot(cur_row, v[j], valid ? yv[j][q] : 0.0);
         if (valid) { /* lanes 9..15 repeat lane 8's row, value and address */
 #pragma unroll
             for (int j = 0; j < MULTI_RPW; ++j) {
                 if (j < nown) {
-                    double *nxt = bc[j] + (f ^ 1) * 20;
-                    nxt[i] = d[j];
-                    nxt[11 + i] = d[j];
+                    bc[j][(f ^ 1) * 10 + i] = d[j];
                     dUl[j][(size_t)pos * NV + i] = d[j];
                 }
             }
@@ -2832,11 +2915,10 @@ __device__ __forceinline__ void multi_thomas_line(const MultiLine &S, int l, int
     const uint32_t halfb = P * (NB + nr * NV) * sizeof(T);
     const uint32_t stage = 2 * halfb;
     unsigned char *st0 = smem + 128;
-    T *bcw = reinterpret_cast<T *>(st0 + (size_t)NS * stage) + w * MULTI_RPW * 80;
+    T *bcw = reinterpret_cast<T *>(st0 + (size_t)NS * stage) + w * MULTI_RPW * BCAST<T>;
     const int ps = line_start[l], n = line_len[l], m = line_twist[l];
     const int h = lane >> 4, li = lane & 15;
     const int i = li < NV ? li : NV - 1;
-    const LaneOff off = lane_offsets(i);
     const int nb = n - 1 - m;
     const int len = h ? nb : m;
     const int cpos = h ? m : 0;
@@ -2854,13 +2936,13 @@ __device__ __forceinline__ void multi_thomas_line(const MultiLine &S, int l, int
         const int jj = j < nown ? j : 0;
         slot[j] = mine ? k0 + jj : 0;
         const int rr = mine ? rid[k0 + jj] : 0;
-        bc[j] = bcw + j * 80 + h * 40;
+        bc[j] = bcw + j * BCAST<T> + h * 20;
         yl[j] = syp[rr] + (size_t)ps * NV;
         dUl[j] = sdp[rr] + (size_t)ps * NV;
         bg[j] = sbp[rr] + (size_t)ps * NV;
     }
     const uint64_t pol = tid == 0 ? policy_evict_first() : 0;
-    for (int t = lane; t < MULTI_RPW * 80; t += 32) bcw[t] = T(0);
+    for (int t = lane; t < MULTI_RPW * BCAST<T>; t += 32) bcw[t] = T(0);
     __syncwarp();
 
     auto cells = [&](int ln, int c) { return ((min(P, ln - c * P) + 3) & ~3); };
@@ -2915,9 +2997,9 @@ __device__ __forceinline__ void multi_thomas_line(const MultiLine &S, int l, int
 #pragma unroll
             for (int j = 0; j < MULTI_RPW; ++j) sB[j] = sG + P * NB + slot[j] * P * NV;
             if (c < both_full)
-                fwd_chunk_m<P, false>(sG, sB, bc, yl, nown, c * P, len, cpos, i, off);
+                fwd_chunk_m<P, false>(sG, sB, bc, yl, nown, c * P, len, cpos, i);
             else
-                fwd_chunk_m<P, true>(sG, sB, bc, yl, nown, c * P, len, cpos, i, off);
+                fwd_chunk_m<P, true>(sG, sB, bc, yl, nown, c * P, len, cpos, i);
             __syncwarp();
         }
         if (__syncthreads_or(!ok)) {
@@ -2938,16 +3020,16 @@ __device__ __forceinline__ void multi_thomas_line(const MultiLine &S, int l, int
 #pragma unroll
         for (int j = 0; j < MULTI_RPW; ++j) xm[j] = T(0);
         if (mine && lane < NV) {
-            const T *gr = G + (size_t)(ps + ptw) * NB + NV * lane;
-            const T *cr = Gam + (size_t)(ps + ptw) * NB + NV * lane;
+            const T *gr = G + (size_t)(ps + ptw) * NB + lane;
+            const T *cr = Gam + (size_t)(ps + ptw) * NB + lane;
 #pragma unroll
             for (int j = 0; j < MULTI_RPW; ++j) {
-                const T *base = bcw + j * 80;
-                const T *ytop = base + 0 * 40 + (m & 1) * 20;
-                const T *ybot = base + 1 * 40 + (nb & 1) * 20;
+                const T *base = bcw + j * BCAST<T>;
+                const T *ytop = base + (m & 1) * 10;
+                const T *ybot = base + 20 + (nb & 1) * 10;
                 T acc = bg[j][(size_t)ptw * NV + lane];
 #pragma unroll
-                for (int jj = 0; jj < NV; ++jj) acc -= gr[jj] * ytop[jj] + cr[jj] * ybot[jj];
+                for (int jj = 0; jj < NV; ++jj) acc -= gr[NV * jj] * ytop[jj] + cr[NV * jj] * ybot[jj];
                 xm[j] = acc;
             }
         }
@@ -2956,11 +3038,8 @@ __device__ __forceinline__ void multi_thomas_line(const MultiLine &S, int l, int
 #pragma unroll
             for (int j = 0; j < MULTI_RPW; ++j) {
                 if (j < nown) {
-                    T *base = bcw + j * 80;
-                    for (int t = 0; t < 4; ++t) {
-                        base[t * 20 + lane] = xm[j];
-                        base[t * 20 + 11 + lane] = xm[j];
-                    }
+                    T *base = bcw + j * BCAST<T>;
+                    for (int t = 0; t < 4; ++t) base[t * 10 + lane] = xm[j];
                     dUl[j][(size_t)ptw * NV + lane] = xm[j];
                 }
             }
@@ -2992,9 +3071,9 @@ __device__ __forceinline__ void multi_thomas_line(const MultiLine &S, int l, int
                 const bool full = (nchT - 1 - jb) * P + P <= m && (nchB - 1 - jb) * P + P <= nb &&
                                   nchT - 1 - jb >= 0 && nchB - 1 - jb >= 0;
                 if (full)
-                    bwd_chunk_m<P, false>(sG, bc, yv, dUl, nown, c * P, len, cpos, i, off);
+                    bwd_chunk_m<P, false>(sG, bc, yv, dUl, nown, c * P, len, cpos, i);
                 else
-                    bwd_chunk_m<P, true>(sG, bc, yv, dUl, nown, c * P, len, cpos, i, off);
+                    bwd_chunk_m<P, true>(sG, bc, yv, dUl, nown, c * P, len, cpos, i);
                 __syncwarp();
             }
             if (__syncthreads_or(!ok)) {
@@ -3045,7 +3124,7 @@ static size_t multi_thomas_stage(int nr) {
 
 static size_t multi_thomas_smem(int nr, int NS) {
     return 128 + (size_t)NS * multi_thomas_stage(nr) +
-           (size_t)multi_thomas_warps(nr) * MULTI_RPW * 80 * sizeof(double);
+           (size_t)multi_thomas_warps(nr) * MULTI_RPW * BCAST<double> * sizeof(double);
 }
 
 /* ring depth: the shared memory each of the SM's resident lines may use,

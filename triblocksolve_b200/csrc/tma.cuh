@@ -52,6 +52,29 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
+/* the same by the lanes with `on` set, without a branch */
+__device__ __forceinline__ void mbar_arrive_if(uint64_t *bar, bool on) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(smem_u32(bar)),
+        "r"((unsigned)on)
+        : "memory");
+}
+
+/* whether phase `parity` of `bar` has completed; does not wait */
+__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 /* Wait for phase `parity` of `bar` to complete; false after ~budget cycles. */
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity,
                                           long long budget = (1LL << 31)) {
@@ -112,6 +135,32 @@ __device__ __forceinline__ void bulk_g2s_hint(void *dst, const void *src, uint32
         "[%0], [%1], %2, [%3], %4;" ::"r"(smem_u32(dst)),
         "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(pol)
         : "memory");
+}
+
+/* makes this thread's writes to shared memory visible to the bulk copies
+ * that are issued after the next barrier */
+__device__ __forceinline__ void fence_async_smem() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+/* bulk copy / bulk FP64 add, this CTA's shared memory -> global (addresses
+ * and size multiples of 16 bytes), in the issuing thread's open group */
+__device__ __forceinline__ void bulk_s2g(void *dst, const void *src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+                 "r"(smem_u32(src)), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_add_s2g(void *dst, const void *src, uint32_t bytes) {
+    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], %2;" ::"l"(dst),
+                 "r"(smem_u32(src)), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_s2g_commit() {
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+/* the shared memory of this thread's committed groups has been read */
+__device__ __forceinline__ void bulk_s2g_wait_read() {
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
 }  // namespace tbs
