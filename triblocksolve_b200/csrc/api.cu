@@ -421,7 +421,7 @@ static int build_layout(tbs_ctx *ctx) {
     DA(L.xnbr, (size_t)np16 * std::max(nx, 1));
     DA(L.xsrcf, (size_t)np16 * nxfa);
     DA(L.xnbrf, (size_t)np16 * nxfa);
-    DA(ctx->d_gamlast, (size_t)nline * 2 * ctx->nvar * ctx->nvar);
+    if (ctx->nvar != 9) DA(ctx->d_gamlast, (size_t)nline * 2 * ctx->nvar * ctx->nvar);
     cudaStream_t st = ctx->stream;
     CK(cudaMemcpyAsync(L.line_start, start.data(), nline * sizeof(int), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(L.line_len, len.data(), nline * sizeof(int), cudaMemcpyHostToDevice, st));
@@ -1000,12 +1000,11 @@ static int run_factor(tbs_ctx *ctx, int algo) {
     if (algo == TBS_ALGO_FP64) {
         RUN("fast_factor", launch_fast_factor(st, L, ctx->d_jacD, ctx->d_O1, ctx->d_O2, ctx->d_Dinv,
                                               ctx->d_G, ctx->d_Gam, nullptr, nullptr, nullptr,
-                                              ctx->d_gamlast, ctx->d_status));
-        RUN("fast_xlayout", launch_fast_xlayout(st, L, ctx->d_O1, ctx->d_O2, ctx->d_X, nullptr));
+                                              ctx->d_X, ctx->d_status));
     } else {
         RUN("fast_factor", launch_fast_factor(st, L, ctx->d_jacD, ctx->d_O1, ctx->d_O2, ctx->d_Dinv,
                                               nullptr, nullptr, ctx->d_Dinv32, ctx->d_G32,
-                                              ctx->d_Gam32, ctx->d_gamlast, ctx->d_status));
+                                              ctx->d_Gam32, nullptr, ctx->d_status));
         RUN("fast_dx", launch_fast_dx(st, L, ctx->d_Dinv, ctx->d_O1, ctx->d_O2, ctx->d_X32));
         if (fullpos_ok(ctx)) {
             CKL(fullpos_prepare(L));

@@ -61,7 +61,7 @@ struct tbs_ctx {
     /* ---- line-ordered layout (FP64 / MIXED) ---- */
     tbs::FastLayout L{};
     bool layout_ok = false;
-    double *d_gamlast = nullptr; /* per line and chain: last Gam toward the twist, FP64 */
+    double *d_gamlast = nullptr; /* per line and chain: last Gam toward the twist (block sizes other than 9) */
     long long n_xslots_real = 0;
     long long n_fslots_real = 0; /* interior face slots of all cells */
     double *d_Dinv = nullptr, *d_G = nullptr, *d_Gam = nullptr, *d_X = nullptr;

@@ -26,6 +26,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 
 namespace tbs {
@@ -242,67 +243,93 @@ int launch_axpy2_f32_f64(cudaStream_t st, const float *c, const float *d, double
  * Twisted block Thomas.  Each line is split into a top chain (cells
  * 0..m-1, eliminated downward as in src/okl/lineLU_v2.okl:58-182), a
  * bottom chain (cells n-1 down to m+1, the same elimination run upward) and
- * the twist cell m.  One warp per chain (grid = 2 x lines); lane j < 9 owns
- * column j of each 9x9 block.  For
- * chain step s >= 1 with A = block(row c_s, col c_{s-1}) and C =
- * block(row c_{s-1}, col c_s), both from the in-line face between them
- * (picked as in lineLU_v2.okl:116-117):
+ * the twist cell m.  For chain step s >= 1 with A = block(row c_s, col
+ * c_{s-1}) and C = block(row c_{s-1}, col c_s), both from the in-line face
+ * between them (picked as in lineLU_v2.okl:116-117):
  *   Gam_{s-1} = Dinv_{s-1} C
  *   W         = D_s - A Gam_{s-1}          (block-Thomas pivot)
  *   Dinv_s    = W^-1   (in-place Gauss-Jordan, no pivoting, as the
  *                        reference's LU has none: lineLU_v2.okl:17-27)
  *   G_s       = Dinv_s A
- * and the chain's last Gam couples it to the twist cell.  The twist kernel
- * then forms Dinv_tw = (D_m - A_tw Gam_top - C_tw Gam_bot)^-1 and stores
- * Dinv_tw A_tw / Dinv_tw C_tw in the G / Gam slots of the twist position.
- * All are stored column-major like the input blocks.  The
- * FP32 arrays, when given, are the FP64 results rounded once. */
-__device__ __forceinline__ void gj_invert(double *W, int t, unsigned *status) {
-    const int i = t % NV, j = t / NV;
-#pragma unroll 1
-    for (int p = 0; p < NV; ++p) {
-        double wpp = 0.0, wip = 0.0, wpj = 0.0, wij = 0.0;
-        if (t < NB) {
-            wpp = W[p * (NV + 1)];
-            wip = W[i + NV * p];
-            wpj = W[p + NV * j];
-            wij = W[t];
-        }
-        __syncthreads();
-        if (t < NB) {
-            const double r = 1.0 / wpp;
-            double v;
-            if (i == p && j == p)
-                v = r;
-            else if (i == p)
-                v = wpj * r;
-            else if (j == p)
-                v = -wip * r;
-            else
-                v = wij - wip * (wpj * r);
-            W[t] = v;
-        }
-        if (t == 0 && !(fabs(wpp) > 0.0 && isfinite(wpp))) atomicOr(status, ST_PIVOT);
-        __syncthreads();
-    }
-}
+ * and the chain's last Gam couples it to the twist cell, for which
+ *   Dinv_tw = (D_m - A_tw Gam_top - C_tw Gam_bot)^-1
+ * and Dinv_tw A_tw / Dinv_tw C_tw go in the G / Gam slots of the twist
+ * position.  All are stored column-major like the input blocks.  The FP32
+ * arrays, when given, are the FP64 results rounded once.
+ *
+ * What bounds it is the step along the chain (nine dependent pivots and two
+ * products; a warp issues an FP64 operation every 4 cycles at best and a
+ * reciprocal takes about 70) where lines are few, and the shuffles and
+ * shared-memory reads of all the chains of an SM where they are many; the
+ * bytes (six blocks a cell) come last.  So a warp runs three chains, nine
+ * lanes each, a lane holding a 3x3 tile of its block: 54 reads for the 81
+ * multiply-adds of three products and 14 shuffles for three pivots, where 27
+ * lanes per chain took 108 and 48.  A CTA takes three lines: one such warp
+ * for their top chains, one for the bottom chains, and beside each a helper
+ * warp that copies the coming cells' blocks into shared memory, forms G (no
+ * step waits for it) and writes the results, so that the chain warps run
+ * nothing but the chain.
+ * Few lines (at most two per SM) leave the SM's pipes idle and the step's
+ * latency counts alone; there 27 lanes per chain are faster (27 multiply-adds
+ * a product, 98 cycles a pivot against 122), one CTA per line:
+ * fast_factor_few_kernel.  Measured (us; few / this / a warp per chain doing
+ * everything, the form before): 100 lines of 256 cells 157 / 204 / 218, 290 of
+ * 256 195 / 201 / 229, 440 of 256 239 / 201 / 261, 600 of 640 876 / 758 / 789,
+ * 1200 of 1280 3,060 / 2,260 / 2,810.
+ */
 
 struct FactorOut {
     double *Dinv, *G, *Gam;
     float *Dinv32, *G32, *Gam32;
-    __device__ void put_dinv(size_t p, int t, double w) const {
-        if (Dinv) Dinv[p * NB + t] = w;
-        if (Dinv32) Dinv32[p * NB + t] = (float)w;
+    __device__ void put_dinv(size_t q, double v) const {
+        if (Dinv) Dinv[q] = v;
+        if (Dinv32) Dinv32[q] = (float)v;
     }
-    __device__ void put_g(size_t p, int t, double v) const {
-        if (G) G[p * NB + t] = v;
-        if (G32) G32[p * NB + t] = (float)v;
+    __device__ void put_g(size_t q, double v) const {
+        if (G) G[q] = v;
+        if (G32) G32[q] = (float)v;
     }
-    __device__ void put_gam(size_t p, int t, double v) const {
-        if (Gam) Gam[p * NB + t] = v;
-        if (Gam32) Gam32[p * NB + t] = (float)v;
+    __device__ void put_gam(size_t q, double v) const {
+        if (Gam) Gam[q] = v;
+        if (Gam32) Gam32[q] = (float)v;
     }
 };
+
+/* X[q] = cross-line block of slot q = s*np16 + p (slot-major), or zeros: work
+ * that needs nothing of the factorization, done by CTAs behind its own in the
+ * same launch.  A chain leaves most of the memory system idle, so the copy
+ * (235 us by itself at 600x640, 15 at 120x128) runs under it. */
+struct XCopy {
+    const int *xsrc;
+    double *X; /* null: no copy */
+    long long nslots;
+    int first; /* the first CTA that copies */
+};
+
+/* a warp's share: four blocks at a time, their loads before their stores */
+__device__ __forceinline__ void xcopy_part(const XCopy &xc, const double *__restrict__ O1,
+                                           const double *__restrict__ O2) {
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const long long warps = (long long)(gridDim.x - xc.first) * nw;
+    const long long w = (long long)(blockIdx.x - xc.first) * nw + (threadIdx.x >> 5);
+    for (long long q0 = 4 * w; q0 < xc.nslots; q0 += 4 * warps) {
+        double v[4][3];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int src = q0 + k < xc.nslots ? xc.xsrc[q0 + k] : -1;
+            const double *x = ((src & 1) ? O2 : O1) + (size_t)(src >> 1) * NB + lane;
+#pragma unroll
+            for (int r = 0; r < 3; ++r) v[k][r] = (src >= 0 && lane + 32 * r < NB) ? __ldcs(x + 32 * r) : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            double *d = xc.X + (q0 + k) * NB + lane;
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+                if (q0 + k < xc.nslots && lane + 32 * r < NB) d[32 * r] = v[k][r];
+        }
+    }
+}
 
 /* In-place Gauss-Jordan inverse of a 9x9 block distributed by columns:
  * lane j < 9 holds column j in w[0..8].  Pivot column p is broadcast with
@@ -325,233 +352,670 @@ __device__ __forceinline__ void gj_invert_cols(double (&w)[NV], int j, unsigned 
     }
 }
 
+/* 1 / d, correctly rounded, by Newton's iteration and Markstein's last step
+ * (P. Markstein, IBM J. Res. Dev. 34 (1990) 111-119) from the hardware's
+ * approximation: about 70 cycles, and no branch in the usual range. */
+__device__ __forceinline__ double rcp_chain(double d) {
+    double x;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+    double e = fma(-d, x, 1.0);
+    x = fma(x, fma(e, e, e), x);
+    e = fma(-d, x, 1.0);
+    return fma(x, e, x);
+}
+
 /* Gauss-Jordan inverse of a 9x9 block held by 27 lanes: lane j + 9g
  * (column j, row group g) holds rows 3g..3g+2 of column j in w[0..2].  For
  * pivot p, the pivot column's entries of this lane's rows come from lane
- * p + 9g, the pivot row's entry of this column and the pivot from the lanes
- * of row group p / 3 (their w[p % 3]).  Each entry is updated with the
- * operations of gj_invert_cols; no pivoting, as the reference's LU has none. */
-__device__ __forceinline__ void gj_invert_27(double (&w)[3], int j, int g, unsigned *status) {
+ * p + 9g, the pivot row's entry of this column from row group p / 3, and
+ * the three entries that make the next pivot from their lanes; all lanes
+ * then know the next pivot two operations after the reciprocal of this one.
+ * Each entry is updated with the operations of gj_invert_cols (the pivot
+ * column as 0 - column * r); no pivoting, as the reference's LU has none.
+ * No branch stands in the chain: a pivot outside 2^-1000 .. 2^1000, where
+ * rcp_chain does not hold, is noted, and the block is then done again with
+ * the general reciprocal.  Returns whether a pivot was zero or not finite. */
+template <bool GENERAL>
+__device__ __forceinline__ bool gj_pass_27(double (&w)[3], int j, int g) {
+    bool bad = false;
+    double piv = __shfl_sync(FULL, w[0], 0);
 #pragma unroll
     for (int p = 0; p < NV; ++p) {
         const int pg = p / 3, pr = p % 3;
+        const int n = p + 1 < NV ? p + 1 : p, ng = n / 3, nr = n % 3;
+        const double dn = __shfl_sync(FULL, w[nr], n + 9 * ng);
+        const double cn = __shfl_sync(FULL, w[nr], p + 9 * ng);
+        const double rn = __shfl_sync(FULL, w[pr], n + 9 * pg);
         double colp[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) colp[k] = __shfl_sync(FULL, w[k], p + 9 * g);
-        const double rowp = __shfl_sync(FULL, w[pr], j + 9 * pg);
-        const double piv = __shfl_sync(FULL, w[pr], p + 9 * pg);
-        if (threadIdx.x == 0 && !(fabs(piv) > 0.0 && isfinite(piv))) atomicOr(status, ST_PIVOT);
-        const double r = __drcp_rn(piv);
-        const bool isp = (j == p);
-        const double t = rowp * r;
+        double t = __shfl_sync(FULL, w[pr], j + 9 * pg);
+        if (j == p) {
+            t = 1.0;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) w[k] = 0.0;
+        }
+        if (GENERAL)
+            bad |= !(fabs(piv) > 0.0 && isfinite(piv));
+        else
+            bad |= (unsigned)((__double2hiint(piv) & 0x7fffffff) - 0x01700000) >= 0x7d000000u;
+        const double r = GENERAL ? __drcp_rn(piv) : rcp_chain(piv);
+        piv = dn - cn * (rn * r);
+        t *= r;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) w[k] -= colp[k] * t;
+        if (g == pg) w[pr] = t;
+    }
+    return bad;
+}
+
+__device__ __noinline__ bool gj_general_27(double &a, double &b, double &c, int j, int g) {
+    double w[3] = {a, b, c};
+    const bool bad = gj_pass_27<true>(w, j, g);
+    a = w[0];
+    b = w[1];
+    c = w[2];
+    return bad;
+}
+
+__device__ __forceinline__ bool gj_invert_27(double (&w)[3], int j, int g) {
+    double a = w[0], b = w[1], c = w[2];
+    if (!gj_pass_27<false>(w, j, g)) return false; /* the pivots are the same in every lane */
+    const bool bad = gj_general_27(a, b, c, j, g);
+    w[0] = a;
+    w[1] = b;
+    w[2] = c;
+    return bad;
+}
+
+/* the lane's three entries of c +- x y, x and y 9x9 blocks in shared memory
+ * (r0 = 3g), the sum over q = 0..8 in order */
+template <bool NEG>
+__device__ __forceinline__ void product_27(double (&c)[3], const double *x, const double *y, int j, int r0) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+        const double v = y[q + NV * j];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            if (3 * g + k != p)
-                w[k] = isp ? -colp[k] * r : w[k] - colp[k] * t;
+            if (NEG)
+                c[k] -= x[r0 + k + NV * q] * v;
             else
-                w[k] = isp ? r : t;
+                c[k] += x[r0 + k + NV * q] * v;
         }
     }
 }
 
-/* One warp per chain (grid = 2 x lines).  Lane j + 9g (27 lanes) owns rows
- * 3g..3g+2 of column j of every block, so 27 lanes share each product and
- * each pivot step; lanes 27..31 repeat lanes 18..22 and store nothing.  The
- * blocks every lane needs whole (Dinv_{s-1}, C, A, Gam_{s-1}, Dinv_s) are
- * published in shared memory.  Per entry the products add q = 0..8 in
- * order, as the column-per-lane form did. */
-__global__ void __launch_bounds__(32) fast_factor_kernel(
+__device__ __forceinline__ void entries_27(double (&c)[3], const double *x, int j, int r0) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) c[k] = x[r0 + k + NV * j];
+}
+
+__device__ __forceinline__ void put_27(const double (&c)[3], double *x, int j, int r0) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) x[r0 + k + NV * j] = c[k];
+}
+
+/* shared memory of one chain: FEW_STAGES cells (A, C, D), two Dinv, two Gam
+ * and the helper's G */
+constexpr int FEW_STAGES = 6;
+constexpr int FEW_WORDS = (3 * FEW_STAGES + 5) * NB;
+
+/* The factorization of few lines (at most two per SM): one CTA per line,
+ * warps 0 / 1 on its top / bottom chain, warp 2 helping both; the three meet
+ * once per cell.  In step s a chain warp eliminates cell s (Gam_{s-1},
+ * Dinv_s), the helper starts the copies of cell s + 4, forms and writes
+ * G_{s-1}, Dinv_{s-1} and Gam_{s-2}, and waits for cell s + 1. */
+__global__ void __launch_bounds__(96) fast_factor_few_kernel(
     int nline, const int *__restrict__ line_start, const int *__restrict__ line_len,
     const int *__restrict__ line_twist, const int *__restrict__ fsrc,
     const double *__restrict__ jacD, const double *__restrict__ O1, const double *__restrict__ O2,
-    FactorOut out, double *__restrict__ gamlast, unsigned *status) {
-    const int l = blockIdx.x >> 1, chain = blockIdx.x & 1;
-    if (l >= nline) return;
-    const int lane = threadIdx.x;
-    const bool act = lane < 27;
-    const int jj = act ? lane % 9 : lane - 27; /* column */
-    const int gg = act ? lane / 9 : 2;         /* row group: rows 3gg .. 3gg+2 */
-    const int r0 = 3 * gg;
-    __shared__ double sM[NB], sA[NB], sC[NB], sG[NB];
-    const int ps = line_start[l], n = line_len[l], m = line_twist[l];
-    const int len = chain ? n - 1 - m : m;
-    const int cs = ps + (chain ? m : 0);
-    const int ptw = ps + n - 1;
-    if (len == 0) {
-        for (int t = lane; t < NB; t += 32) gamlast[((size_t)l * 2 + chain) * NB + t] = 0.0;
+    FactorOut out, XCopy xc, unsigned *status) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    constexpr int stages = FEW_STAGES, ahead = stages - 2;
+    const int line = blockIdx.x;
+    if (line >= nline) {
+        xcopy_part(xc, O1, O2);
         return;
     }
-    double w[3], an[3], cn[3], dn[3];
-    {
-        const double *D0 = jacD + (size_t)fsrc[5 * cs] * NB + NV * jj + r0;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ps = line_start[line], n = line_len[line], m = line_twist[line];
+    const int ptw = ps + n - 1;
+    const int lens[2] = {m, n - 1 - m};
+    const int maxlen = max(lens[0], lens[1]);
+    auto base = [&](int chain) { return reinterpret_cast<double *>(smem) + chain * FEW_WORDS; };
+    /* block `which` (0: A, 1: C, 2: D) of a cell's slot; the last Dinv, Gam */
+    auto blk = [&](int chain, int slot, int which) { return base(chain) + (slot * 3 + which) * NB; };
+    auto sM = [&](int chain, int s) { return base(chain) + (3 * stages + (s & 1)) * NB; };
+    auto sGm = [&](int chain, int s) { return base(chain) + (3 * stages + 2 + (s & 1)) * NB; };
+    auto turn = [&](int slot) { return slot + 1 == stages ? 0 : slot + 1; };
+    /* lanes 27..31 repeat lanes 18..22 and store nothing */
+    const bool act = lane < 27;
+    const int j = act ? lane % 9 : lane - 27;
+    const int g = act ? lane / 9 : 2, r0 = 3 * g;
+
+    if (warp == 2) {
+        /* the layout's row of a chain's cell c, entry `lane` of five (loaded in
+         * one step, used in the next).  The cell after a chain's last (c ==
+         * len) has C alone, which couples the chain to the twist; after the
+         * longer chain's, the top slot takes the twist cell's own blocks (the
+         * CTA's last phase). */
+        auto row = [&](int chain, int c) {
+            const int p = c < lens[chain] ? ps + (chain ? m : 0) + c : ptw;
+            return lane < 5 ? fsrc[5 * p + lane] : 0;
+        };
+        auto copy = [&](int chain, int c, int slot, int v) {
+            const int len = lens[chain];
+            const int e = __shfl_sync(FULL, v, 0);
+            const int f1 = __shfl_sync(FULL, v, 1), s1 = __shfl_sync(FULL, v, 2);
+            const int f2 = __shfl_sync(FULL, v, 3), s2 = __shfl_sync(FULL, v, 4);
+            const bool twist = c == maxlen + 1 && chain == 0;
+            const double *q[3] = {nullptr, nullptr, nullptr};
+            if (c < len || twist) q[2] = jacD + (size_t)e * NB;
+            if (twist) {
+                if (f1 >= 0) q[0] = (s1 ? O2 : O1) + (size_t)f1 * NB;
+                if (f2 >= 0) q[1] = (s2 ? O2 : O1) + (size_t)f2 * NB;
+            } else if (c < len && c > 0) {
+                q[0] = (s1 ? O2 : O1) + (size_t)f1 * NB;
+                q[1] = (s1 ? O1 : O2) + (size_t)f1 * NB;
+            } else if (c == len && len > 0) {
+                q[1] = ((chain ? s2 : s1) ? O1 : O2) + (size_t)(chain ? f2 : f1) * NB;
+            }
+            double *d = blk(chain, slot, 0) + lane;
 #pragma unroll
-        for (int k = 0; k < 3; ++k) w[k] = D0[k];
+            for (int which = 0; which < 3; ++which, d += NB) {
+                if (q[which]) {
+                    const double *x = q[which] + lane;
+                    cp_async8(d, x);
+                    cp_async8(d + 32, x + 32);
+                    if (lane < NB - 64) cp_async8(d + 64, x + 64);
+                } else if (twist) { /* a line's end without a neighbour */
+                    d[0] = d[32] = 0.0;
+                    if (lane < NB - 64) d[64] = 0.0;
+                }
+            }
+        };
+        for (int c = 0; c < ahead; ++c) {
+            const int v0 = row(0, c), v1 = row(1, c);
+            copy(0, c, c, v0);
+            copy(1, c, c, v1);
+            cp_async_commit();
+        }
+        int v0 = row(0, ahead), v1 = row(1, ahead);
+        int into = ahead, done = stages - 1; /* slots of cells s + ahead and s - 1 */
+        cp_async_wait<ahead - 1>(); /* cell 0 has landed */
+        __syncthreads();
+        for (int s = 0; s <= maxlen + 2; ++s) {
+            copy(0, s + ahead, into, v0);
+            copy(1, s + ahead, into, v1);
+            cp_async_commit();
+            into = turn(into);
+            v0 = row(0, s + ahead + 1);
+            v1 = row(1, s + ahead + 1);
+            const int c = s - 1; /* the cell whose Dinv is done; Gam's is c - 1 */
+            /* both chains' products side by side; what lies beyond a chain's
+             * cells is not written out */
+            double gt[2][3];
+#pragma unroll
+            for (int chain = 0; chain < 2; ++chain) {
+                gt[chain][0] = gt[chain][1] = gt[chain][2] = 0.0;
+                product_27<false>(gt[chain], sM(chain, c), blk(chain, done, 0), j, r0);
+            }
+#pragma unroll
+            for (int chain = 0; chain < 2; ++chain) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+                    if (c == 0) gt[chain][k] = 0.0;
+                if (act) put_27(gt[chain], base(chain) + (3 * stages + 4) * NB, j, r0);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int chain = 0; chain < 2; ++chain) {
+                const int len = lens[chain];
+                const size_t q = (size_t)(ps + (chain ? m : 0) + c) * NB;
+                const double *go = base(chain) + (3 * stages + 4) * NB, *di = sM(chain, c);
+                if (c >= 0 && c < len) {
+#pragma unroll
+                    for (int r = 0; r < 3; ++r) {
+                        const int e = lane + 32 * r;
+                        if (e < NB) {
+                            out.put_dinv(q + e, di[e]);
+                            out.put_g(q + e, go[e]);
+                        }
+                    }
+                }
+                if (c >= 1 && c - 1 < len) {
+                    const double *gm = sGm(chain, c);
+#pragma unroll
+                    for (int r = 0; r < 3; ++r) {
+                        const int e = lane + 32 * r;
+                        if (e < NB) out.put_gam(q - NB + e, gm[e]);
+                    }
+                }
+            }
+            __syncwarp();
+            done = turn(done);
+            cp_async_wait<ahead - 1>(); /* cell s + 1 */
+            __syncthreads();
+        }
+        cp_async_wait<0>();
+        __syncthreads(); /* the twist's blocks for warp 0 */
+        return;
     }
-    auto fetch = [&](int p) {
-        const int e = fsrc[5 * p], f = fsrc[5 * p + 1], side = fsrc[5 * p + 2];
-        const double *Ap = (side ? O2 : O1) + (size_t)f * NB + NV * jj + r0;
-        const double *Cp = (side ? O1 : O2) + (size_t)f * NB + NV * jj + r0;
-        const double *Dp = jacD + (size_t)e * NB + NV * jj + r0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            an[k] = Ap[k];
-            cn[k] = Cp[k];
-            dn[k] = Dp[k];
+
+    const int len = lens[warp];
+    bool bad = false;
+    int slot = 0; /* of cell s */
+    __syncthreads();
+    for (int s = 0; s <= maxlen + 2; ++s) {
+        if (s <= len) {
+            if (s > 0) {
+                double gm[3] = {0.0, 0.0, 0.0};
+                product_27<false>(gm, sM(warp, s - 1), blk(warp, slot, 1), j, r0);
+                if (act) put_27(gm, sGm(warp, s), j, r0);
+                __syncwarp();
+            }
+            if (s < len) {
+                double w[3];
+                entries_27(w, blk(warp, slot, 2), j, r0);
+                if (s > 0) product_27<true>(w, blk(warp, slot, 0), sGm(warp, s), j, r0);
+                bad = gj_invert_27(w, j, g) || bad;
+                if (act) put_27(w, sM(warp, s), j, r0);
+                __syncwarp();
+            }
         }
-    };
-    if (len > 1) fetch(cs + 1);
-    gj_invert_27(w, jj, gg, status);
-    if (act) {
+        slot = turn(slot);
+        __syncthreads();
+    }
+    __syncthreads(); /* the twist's blocks have landed */
+    /* ---------------- the twist cell: warp 0, the chains' last Gam where their
+     * step s = len left it */
+    if (warp == 0) {
+        const int tw = (maxlen + 1) % stages;
+        const double *A = blk(0, tw, 0), *C = blk(0, tw, 1);
+        double w[3];
+        entries_27(w, blk(0, tw, 2), j, r0);
+        if (lens[0] > 0) product_27<true>(w, A, sGm(0, lens[0]), j, r0);
+        if (lens[1] > 0) product_27<true>(w, C, sGm(1, lens[1]), j, r0);
+        bad = gj_invert_27(w, j, g) || bad;
+        double *inv = sM(0, 0);
+        if (act) put_27(w, inv, j, r0);
+        __syncwarp();
+        double ga[3] = {0.0, 0.0, 0.0}, gc[3] = {0.0, 0.0, 0.0};
+        product_27<false>(ga, inv, A, j, r0);
+        product_27<false>(gc, inv, C, j, r0);
+        if (act) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            out.put_dinv(cs, r0 + k + NV * jj, w[k]);
-            out.put_g(cs, r0 + k + NV * jj, 0.0);
-            sM[r0 + k + NV * jj] = w[k];
+            for (int k = 0; k < 3; ++k) {
+                const size_t q = (size_t)ptw * NB + r0 + k + NV * j;
+                out.put_dinv(q, w[k]);
+                out.put_g(q, ga[k]);
+                out.put_gam(q, gc[k]);
+            }
         }
     }
-    for (int s = 1; s < len; ++s) {
-        const int p = cs + s;
-        double a[3], c[3], d[3];
+    if (bad && lane == 0) atomicOr(status, ST_PIVOT);
+}
+
+/* Gauss-Jordan inverse of three 9x9 blocks by 27 lanes: lane (a, b) of the
+ * nine from `base` holds rows 3a..3a+2, columns 3b..3b+2 of its block.  For
+ * pivot p each lane takes the pivot, the pivot column's entries of its rows
+ * and the pivot row's of its columns.  Each entry is updated with the
+ * operations of gj_invert_cols (the pivot column as 0 - column * r); no
+ * pivoting, as the reference's LU has none.  No branch stands in the chain: a
+ * pivot outside 2^-1000 .. 2^1000, where rcp_chain does not hold, is noted,
+ * and the blocks are then done again with the general reciprocal.  Returns
+ * whether a pivot of the lane's block was zero or not finite. */
+template <bool GENERAL>
+__device__ __forceinline__ bool gj_pass(double (&w)[3][3], int a, int b, int base) {
+    bool bad = false;
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            a[k] = an[k];
-            c[k] = cn[k];
-            d[k] = dn[k];
+    for (int p = 0; p < NV; ++p) {
+        const int pa = p / 3, pk = p % 3;
+        const double piv = __shfl_sync(FULL, w[pk][pk], base + 4 * pa);
+        double colp[3], t[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) colp[k] = __shfl_sync(FULL, w[k][pk], base + 3 * a + pa);
+#pragma unroll
+        for (int l = 0; l < 3; ++l) t[l] = __shfl_sync(FULL, w[pk][l], base + 3 * pa + b);
+        if (GENERAL)
+            bad |= !(fabs(piv) > 0.0 && isfinite(piv));
+        else
+            bad |= (unsigned)((__double2hiint(piv) & 0x7fffffff) - 0x01700000) >= 0x7d000000u;
+        const double r = GENERAL ? __drcp_rn(piv) : rcp_chain(piv);
+        if (b == pa) {
+            t[pk] = 1.0;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) w[k][pk] = 0.0;
         }
-        if (s + 1 < len) fetch(p + 1);
-        if (act) {
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                sC[r0 + k + NV * jj] = c[k];
-                sA[r0 + k + NV * jj] = a[k];
-            }
+        for (int l = 0; l < 3; ++l) t[l] *= r;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int l = 0; l < 3; ++l) w[k][l] -= colp[k] * t[l];
+        if (a == pa) {
+#pragma unroll
+            for (int l = 0; l < 3; ++l) w[pk][l] = t[l];
         }
-        __syncwarp();
-        /* Gam_{s-1}(:, j) = Dinv_{s-1} C(:, j) */
-        double gm[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            double acc = 0.0;
-#pragma unroll
-            for (int q = 0; q < NV; ++q) acc += sM[r0 + k + NV * q] * sC[q + NV * jj];
-            gm[k] = acc;
-        }
-        if (act) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                out.put_gam(p - 1, r0 + k + NV * jj, gm[k]);
-                sG[r0 + k + NV * jj] = gm[k];
-            }
-        }
-        __syncwarp();
-        /* W(:, j) = D(:, j) - A Gam_{s-1}(:, j) */
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            double acc = d[k];
-#pragma unroll
-            for (int q = 0; q < NV; ++q) acc -= sA[r0 + k + NV * q] * sG[q + NV * jj];
-            w[k] = acc;
-        }
-        gj_invert_27(w, jj, gg, status);
-        __syncwarp(); /* every lane has read Dinv_{s-1} */
-        if (act) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                out.put_dinv(p, r0 + k + NV * jj, w[k]);
-                sM[r0 + k + NV * jj] = w[k];
-            }
-        }
-        __syncwarp();
-        /* G_s(:, j) = Dinv_s A(:, j) */
-        if (act) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                double acc = 0.0;
-#pragma unroll
-                for (int q = 0; q < NV; ++q) acc += sM[r0 + k + NV * q] * sA[q + NV * jj];
-                out.put_g(p, r0 + k + NV * jj, acc);
-            }
-        }
-        __syncwarp(); /* sA and sC are rewritten by the next cell */
     }
-    /* coupling of the chain's last cell to the twist: Gam = Dinv_last block(row last, col m) */
-    {
-        const int f = fsrc[5 * ptw + (chain ? 3 : 1)], side = fsrc[5 * ptw + (chain ? 4 : 2)];
-        const double *Cp = (side ? O1 : O2) + (size_t)f * NB + NV * jj + r0;
-        if (act) {
+    return bad;
+}
+
+/* a block's tiles through memory, out of line: x[9] per lane */
+__device__ __noinline__ bool gj_general(double *x, int a, int b, int base) {
+    double w[3][3];
 #pragma unroll
-            for (int k = 0; k < 3; ++k) sC[r0 + k + NV * jj] = Cp[k];
+    for (int k = 0; k < 9; ++k) w[k / 3][k % 3] = x[k];
+    const bool bad = gj_pass<true>(w, a, b, base);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) x[k] = w[k / 3][k % 3];
+    return bad;
+}
+
+/* W from the lane's tile in shared memory form: `again` rebuilds the tile
+ * (the general pass starts from the block itself); `use`: the lane's chain
+ * has a block here (the lanes of the others take part in the shuffles) */
+template <typename Build>
+__device__ __forceinline__ bool gj_invert_tile(double (&w)[3][3], int a, int b, int base, bool use,
+                                               Build &&again) {
+    const bool odd = gj_pass<false>(w, a, b, base);
+    if (!__any_sync(FULL, use && odd)) return false;
+    again(w);
+    double x[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) x[k] = w[k / 3][k % 3];
+    const bool bad = gj_general(x, a, b, base);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) w[k / 3][k % 3] = x[k];
+    return use && bad;
+}
+
+/* lane (a, b)'s 3x3 tile of c +- x y; x and y are 9x9 blocks in shared
+ * memory, the sum over q = 0..8 in order */
+template <bool NEG>
+__device__ __forceinline__ void tile_product(double (&c)[3][3], const double *x, const double *y, int a,
+                                             int b) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+        double r[3], s[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            r[k] = x[3 * a + k + NV * q];
+            s[k] = y[q + NV * (3 * b + k)];
         }
-        __syncwarp();
-        if (act) {
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                double acc = 0.0;
+        for (int k = 0; k < 3; ++k)
 #pragma unroll
-                for (int q = 0; q < NV; ++q) acc += sM[r0 + k + NV * q] * sC[q + NV * jj];
-                out.put_gam(cs + len - 1, r0 + k + NV * jj, acc);
-                gamlast[((size_t)l * 2 + chain) * NB + r0 + k + NV * jj] = acc; /* column-major, FP64 */
+            for (int l = 0; l < 3; ++l) {
+                if (NEG)
+                    c[k][l] -= r[k] * s[l];
+                else
+                    c[k][l] += r[k] * s[l];
             }
-        }
     }
 }
 
-__global__ void __launch_bounds__(128) fast_twist_kernel(
-    int nline, const int *__restrict__ line_start, const int *__restrict__ line_len,
+__device__ __forceinline__ void tile_zero(double (&c)[3][3]) {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) c[k / 3][k % 3] = 0.0;
+}
+
+__device__ __forceinline__ void tile_load(double (&c)[3][3], const double *x, int a, int b) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int l = 0; l < 3; ++l) c[k][l] = x[3 * a + k + NV * (3 * b + l)];
+}
+
+__device__ __forceinline__ void tile_store(const double (&c)[3][3], double *x, int a, int b) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int l = 0; l < 3; ++l) x[3 * a + k + NV * (3 * b + l)] = c[k][l];
+}
+
+/* blocks of a group of three lie FB words apart (81 and 8 of padding), so
+ * that the nine rows (or columns) that the 27 lanes read at once lie in
+ * different banks */
+constexpr int FB = NB + 8;
+/* shared memory of three chains: `stages` cells (A, C, D), two Dinv, two Gam
+ * and the helper's G */
+__host__ __device__ constexpr int fac_pair_words(int stages) { return (3 * stages + 5) * 3 * FB; }
+
+/* CTA: lines 3 * blockIdx.x + g, g = 0..2; warps 0 / 1 run their top / bottom
+ * chains, warps 2 / 3 help them; a pair of warps meets at its own barrier
+ * once per cell.  In step s the chain warp eliminates cell s (Gam_{s-1},
+ * Dinv_s), the helper starts the copies of cell s + stages - 2, forms and
+ * writes G_{s-1}, Dinv_{s-1} and Gam_{s-2}, and waits for cell s + 1. */
+__global__ void __launch_bounds__(128, 3) fast_factor_kernel(
+    int nline, int stages, int nsm, const int *__restrict__ line_start, const int *__restrict__ line_len,
     const int *__restrict__ line_twist, const int *__restrict__ fsrc,
     const double *__restrict__ jacD, const double *__restrict__ O1, const double *__restrict__ O2,
-    FactorOut out, const double *__restrict__ gamlast, unsigned *status) {
-    const int l = blockIdx.x;
-    if (l >= nline) return;
-    const int t = threadIdx.x;
-    const bool act = t < NB;
-    const int i = t % NV, j = t / NV;
-    __shared__ double sW[NB], sA[NB], sC[NB], sGt[NB], sGb[NB];
-    const int ps = line_start[l], n = line_len[l];
+    FactorOut out, XCopy xc, unsigned *status) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    if ((int)blockIdx.x * 3 >= nline) {
+        xcopy_part(xc, O1, O2);
+        return;
+    }
+    /* a warp's scheduler goes by its number in the CTA: every other CTA of an
+     * SM (they come round every nsm) has its chain warps on the schedulers
+     * where the others' helpers are */
+    const int warp = (threadIdx.x >> 5) ^ ((blockIdx.x / nsm & 1) << 1), lane = threadIdx.x & 31;
+    const int chain = warp & 1; /* 0: top, 1: bottom */
+    /* lanes 27..31 repeat lanes 18..22 and write nothing */
+    const bool lact = lane < 27;
+    const int ln = lact ? lane : lane - 9;
+    const int g = ln / 9, l9 = ln % 9, a = l9 / 3, b = l9 % 3;
+    const int line = 3 * blockIdx.x + g;
+    const bool have = line < nline, act = lact && have;
+    const int lc = have ? line : nline - 1;
+    const int ps = line_start[lc], n = line_len[lc], m = line_twist[lc];
     const int ptw = ps + n - 1;
-    if (act) {
-        const int e = fsrc[5 * ptw];
-        const int fa = fsrc[5 * ptw + 1], sa = fsrc[5 * ptw + 2];
-        const int fb = fsrc[5 * ptw + 3], sb = fsrc[5 * ptw + 4];
-        sW[t] = jacD[(size_t)e * NB + t];
-        sA[t] = fa >= 0 ? (sa ? O2 : O1)[(size_t)fa * NB + t] : 0.0;
-        sC[t] = fb >= 0 ? (sb ? O2 : O1)[(size_t)fb * NB + t] : 0.0;
-        sGt[t] = gamlast[((size_t)l * 2 + 0) * NB + t];
-        sGb[t] = gamlast[((size_t)l * 2 + 1) * NB + t];
-    }
-    __syncthreads();
-    if (act) {
-        double w = sW[t];
+    const int len = have ? (chain ? n - 1 - m : m) : 0;
+    const int cs = ps + (chain ? m : 0);
+    int maxlen = len;
 #pragma unroll
-        for (int q = 0; q < NV; ++q) w -= sA[i + NV * q] * sGt[q + NV * j];
+    for (int k = 0; k < 3; ++k) maxlen = max(maxlen, __shfl_sync(FULL, len, 9 * k));
+    double *pair = reinterpret_cast<double *>(smem) + chain * fac_pair_words(stages) + g * FB;
+    /* block `which` (0: A, 1: C, 2: D) of a cell's slot; the last Dinv, Gam */
+    auto blk = [&](int slot, int which) { return pair + (slot * 3 + which) * 3 * FB; };
+    auto sM = [&](int s) { return pair + (3 * stages + (s & 1)) * 3 * FB; };
+    auto sGm = [&](int s) { return pair + (3 * stages + 2 + (s & 1)) * 3 * FB; };
+    auto turn = [&](int slot) { return slot + 1 == stages ? 0 : slot + 1; };
+    auto meet = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + chain) : "memory"); };
+
+    if (warp >= 2) {
+        const int ahead = stages - 2;
+        double *sGo = pair + (3 * stages + 4) * 3 * FB;
+        /* the layout's row of the chain's cell c (loaded in one step, used in
+         * the next).  The cell after a chain's last (c == len) has C alone,
+         * which couples the chain to the twist; after the longest chain's, the
+         * top slots take the twist cells' own blocks (the CTA's last phase). */
+        struct Src {
+            int e, f1, s1, f2, s2;
+        };
+        auto row = [&](int c) {
+            const int *q = fsrc + 5 * (c < len ? cs + c : ptw);
+            return Src{q[0], q[1], q[2], q[3], q[4]};
+        };
+        auto copy = [&](int c, int slot, const Src &r) {
+            const bool twist = c == maxlen + 1 && chain == 0 && have;
+            const double *q[3] = {nullptr, nullptr, nullptr};
+            if (c < len || twist) q[2] = jacD + (size_t)r.e * NB;
+            if (twist) {
+                if (r.f1 >= 0) q[0] = (r.s1 ? O2 : O1) + (size_t)r.f1 * NB;
+                if (r.f2 >= 0) q[1] = (r.s2 ? O2 : O1) + (size_t)r.f2 * NB;
+            } else if (c < len && c > 0) {
+                q[0] = (r.s1 ? O2 : O1) + (size_t)r.f1 * NB;
+                q[1] = (r.s1 ? O1 : O2) + (size_t)r.f1 * NB;
+            } else if (c == len && len > 0) {
+                q[1] = ((chain ? r.s2 : r.s1) ? O1 : O2) + (size_t)(chain ? r.f2 : r.f1) * NB;
+            }
+            if (lact) {
 #pragma unroll
-        for (int q = 0; q < NV; ++q) w -= sC[i + NV * q] * sGb[q + NV * j];
-        sW[t] = w; /* only this thread reads or writes sW[t] in this phase */
-    }
-    __syncthreads();
-    gj_invert(sW, t, status);
-    if (act) {
-        double ga = 0.0, gc = 0.0;
+                for (int which = 0; which < 3; ++which) {
+                    double *d = blk(slot, which) + l9;
+                    if (q[which]) {
 #pragma unroll
-        for (int q = 0; q < NV; ++q) {
-            ga += sW[i + NV * q] * sA[q + NV * j];
-            gc += sW[i + NV * q] * sC[q + NV * j];
+                        for (int k = 0; k < NV; ++k) cp_async8(d + NV * k, q[which] + l9 + NV * k);
+                    } else if (twist) { /* a line's end without a neighbour */
+#pragma unroll
+                        for (int k = 0; k < NV; ++k) d[NV * k] = 0.0;
+                    }
+                }
+            }
+            cp_async_commit();
+        };
+        auto wait_next = [&]() { /* all but the newest ahead - 1 cells */
+            if (ahead == 4)
+                cp_async_wait<3>();
+            else
+                cp_async_wait<1>();
+        };
+        for (int c = 0; c < ahead; ++c) copy(c, c, row(c));
+        Src nxt = row(ahead);
+        int into = ahead, done = stages - 1; /* slots of cells s + ahead and s - 1 */
+        wait_next();
+        meet();
+        for (int s = 0; s <= maxlen + 2; ++s) {
+            copy(s + ahead, into, nxt);
+            into = turn(into);
+            nxt = row(s + ahead + 1);
+            const int c = s - 1; /* the cell whose Dinv is done; Gam's is c - 1 */
+            double gt[3][3];
+            tile_zero(gt);
+            if (c > 0) tile_product<false>(gt, sM(c), blk(done, 0), a, b);
+            if (lact) tile_store(gt, sGo, a, b);
+            __syncwarp();
+            if (act && c >= 0 && c < len) {
+                const size_t q = (size_t)(cs + c) * NB + l9;
+                const double *di = sM(c) + l9, *go = sGo + l9;
+#pragma unroll
+                for (int k = 0; k < NV; ++k) {
+                    out.put_dinv(q + NV * k, di[NV * k]);
+                    out.put_g(q + NV * k, go[NV * k]);
+                }
+            }
+            if (act && c >= 1 && c - 1 < len) {
+                const size_t q = (size_t)(cs + c - 1) * NB + l9;
+                const double *gm = sGm(c) + l9;
+#pragma unroll
+                for (int k = 0; k < NV; ++k) out.put_gam(q + NV * k, gm[NV * k]);
+            }
+            __syncwarp();
+            done = turn(done);
+            wait_next();
+            meet();
         }
-        out.put_dinv(ptw, t, sW[t]);
-        out.put_g(ptw, t, ga);
-        out.put_gam(ptw, t, gc);
+        cp_async_wait<0>();
+        __syncthreads(); /* the twists' blocks for warp 0 */
+        return;
     }
+
+    bool bad = false;
+    int slot = 0; /* of cell s */
+    meet();
+    for (int s = 0; s <= maxlen + 2; ++s) {
+        if (s <= maxlen) {
+            if (s > 0) {
+                double gm[3][3];
+                tile_zero(gm);
+                tile_product<false>(gm, sM(s - 1), blk(slot, 1), a, b);
+                if (lact && s <= len) tile_store(gm, sGm(s), a, b);
+                __syncwarp();
+            }
+            double w[3][3];
+            auto pivot = [&](double(&x)[3][3]) {
+                tile_load(x, blk(slot, 2), a, b);
+                if (s > 0) tile_product<true>(x, blk(slot, 0), sGm(s), a, b);
+            };
+            pivot(w);
+            bad = gj_invert_tile(w, a, b, 9 * g, have && s < len, pivot) || bad;
+            if (lact && s < len) tile_store(w, sM(s), a, b);
+            __syncwarp();
+        }
+        slot = turn(slot);
+        meet();
+    }
+    __syncthreads(); /* both chains are done, the twists' blocks have landed */
+    /* ---------------- the twist cells: warp 0, the chains' last Gam where
+     * their step s = len left it */
+    if (warp == 0) {
+        const int tw = (maxlen + 1) % stages, lenb = have ? n - 1 - m : 0;
+        const double *A = blk(tw, 0), *C = blk(tw, 1), *gt = sGm(len);
+        const double *gb = pair + fac_pair_words(stages) + (3 * stages + 2 + (lenb & 1)) * 3 * FB;
+        double w[3][3];
+        auto pivot = [&](double(&x)[3][3]) {
+            tile_load(x, blk(tw, 2), a, b);
+            if (len > 0) tile_product<true>(x, A, gt, a, b);
+            if (lenb > 0) tile_product<true>(x, C, gb, a, b);
+        };
+        pivot(w);
+        __syncwarp();
+        bad = gj_invert_tile(w, a, b, 9 * g, have, pivot) || bad;
+        double *inv = pair + (3 * stages + 4) * 3 * FB; /* the helper is done with it */
+        if (lact) tile_store(w, inv, a, b);
+        __syncwarp();
+        double ga[3][3], gc[3][3];
+        tile_zero(ga);
+        tile_zero(gc);
+        tile_product<false>(ga, inv, A, a, b);
+        tile_product<false>(gc, inv, C, a, b);
+        if (act) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+#pragma unroll
+                for (int l = 0; l < 3; ++l) {
+                    const size_t q = (size_t)ptw * NB + 3 * a + k + NV * (3 * b + l);
+                    out.put_dinv(q, w[k][l]);
+                    out.put_g(q, ga[k][l]);
+                    out.put_gam(q, gc[k][l]);
+                }
+        }
+    }
+    if (bad && act) atomicOr(status, ST_PIVOT);
 }
+
+/* cells in shared memory per pair of warps: six (copies four steps ahead)
+ * where the CTAs of three lines are at most two per SM, else four, which
+ * keeps three CTAs resident */
+static int fac_stages(const FastLayout &L, int nsm) { return (L.nline + 2) / 3 <= 2 * nsm ? 6 : 4; }
 
 int launch_fast_factor(cudaStream_t st, const FastLayout &L, const double *jacD, const double *O1,
                        const double *O2, double *Dinv, double *G, double *Gam, float *Dinv32,
-                       float *G32, float *Gam32, double *gamlast, unsigned *status) {
+                       float *G32, float *Gam32, double *X, unsigned *status) {
     if (L.nv != NV) return (int)cudaErrorInvalidValue;
     FactorOut out{Dinv, G, Gam, Dinv32, G32, Gam32};
-    fast_factor_kernel<<<2 * L.nline, 32, 0, st>>>(L.nline, L.line_start, L.line_len, L.line_twist,
-                                                   L.fsrc, jacD, O1, O2, out, gamlast, status);
-    fast_twist_kernel<<<L.nline, 128, 0, st>>>(L.nline, L.line_start, L.line_len, L.line_twist,
-                                               L.fsrc, jacD, O1, O2, out, gamlast, status);
+    XCopy xc{L.xsrc, X, (long long)L.np16 * L.nx, 0};
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (nsm < 1) nsm = 148;
+    /* CTAs that copy, each with at least a few blocks.  While the
+     * factorization's CTAs are at most one per SM: one per SM, so that all are
+     * resident at once and the chains stay spread over the SMs (360x384: 307
+     * us with 148, 329 with 74, 458 with 296, which fills the SMs and puts two
+     * factorizing CTAs on one; 120x128: 88, 89, 105).  Else four per SM, which
+     * take their places as they come free (600x640: 758 us with 592, 864 with
+     * 148; 1200x640: 1,420 and 1,890). */
+    const bool few = L.nline <= 2 * nsm;
+    const int nfac = (L.nline + 2) / 3;
+    const int most = few || nfac <= nsm ? nsm : 4 * nsm;
+    const int copiers = X ? (int)std::min<long long>(most, (xc.nslots + 63) / 64) : 0;
+    if (few) {
+        xc.first = L.nline;
+        fast_factor_few_kernel<<<L.nline + copiers, 96, 2 * FEW_WORDS * sizeof(double), st>>>(
+            L.nline, L.line_start, L.line_len, L.line_twist, L.fsrc, jacD, O1, O2, out, xc, status);
+        return (int)cudaGetLastError();
+    }
+    const int stages = fac_stages(L, nsm);
+    const size_t smem = 2 * (size_t)fac_pair_words(stages) * sizeof(double);
+    const int rc = smem_raise((const void *)fast_factor_kernel, smem);
+    if (rc) return rc;
+    xc.first = nfac;
+    fast_factor_kernel<<<xc.first + copiers, 128, smem, st>>>(L.nline, stages, nsm, L.line_start, L.line_len,
+                                                              L.line_twist, L.fsrc, jacD, O1, O2, out, xc,
+                                                              status);
     return (int)cudaGetLastError();
 }
 
@@ -592,33 +1056,6 @@ int launch_fast_dx(cudaStream_t st, const FastLayout &L, const double *Dinv, con
     const long long nslots = (long long)L.np16 * L.nx;
     if (nslots == 0) return 0;
     fast_dx_kernel<<<grid_for(nslots * 32, 256), 256, 0, st>>>(nslots, L.np16, L.xsrc, Dinv, O1, O2, DX);
-    return (int)cudaGetLastError();
-}
-
-/* X[q] = cross-line block of slot q = s*np16 + p (slot-major), or zeros;
- * one warp per slot */
-__global__ void fast_xlayout_kernel(long long nslots, const int *__restrict__ xsrc,
-                                    const double *__restrict__ O1, const double *__restrict__ O2,
-                                    double *__restrict__ X, float *__restrict__ X32) {
-    const int lane = threadIdx.x & 31;
-    const long long w0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long q = w0; q < nslots; q += nw) {
-        const int src = xsrc[q];
-        for (int tt = lane; tt < NB; tt += 32) {
-            double v = 0.0;
-            if (src >= 0) v = ((src & 1) ? O2 : O1)[(size_t)(src >> 1) * NB + tt];
-            if (X) X[q * NB + tt] = v;
-            if (X32) X32[q * NB + tt] = (float)v;
-        }
-    }
-}
-
-int launch_fast_xlayout(cudaStream_t st, const FastLayout &L, const double *O1, const double *O2,
-                        double *X, float *X32) {
-    const long long nslots = (long long)L.np16 * L.nx;
-    if (nslots == 0) return 0;
-    fast_xlayout_kernel<<<grid_for(nslots * 32, 256), 256, 0, st>>>(nslots, L.xsrc, O1, O2, X, X32);
     return (int)cudaGetLastError();
 }
 

@@ -160,13 +160,11 @@ int launch_permute_to_elem(cudaStream_t st, int nv, int nelem, const int *pos_of
 int launch_permute_f32_to_elem(cudaStream_t st, int nv, int nelem, const int *pos_of_elem,
                                const float *src_pos, double *dst_elem);
 
-/* fast FP64 / FP32 kernels (kernels_fast.cu) */
+/* fast FP64 / FP32 kernels (kernels_fast.cu); X (may be null): the cross-line
+ * blocks by position, copied in the same launch */
 int launch_fast_factor(cudaStream_t st, const FastLayout &L, const double *jacD,
                        const double *O1, const double *O2, double *Dinv, double *G, double *Gam,
-                       float *Dinv32, float *G32, float *Gam32, double *gamlast,
-                       unsigned *status);
-int launch_fast_xlayout(cudaStream_t st, const FastLayout &L, const double *O1, const double *O2,
-                        double *X, float *X32);
+                       float *Dinv32, float *G32, float *Gam32, double *X, unsigned *status);
 /* DX = Dinv X per cross-line slot, FP32 (TBS_ALGO_MIXED inner sweeps) */
 int launch_fast_dx(cudaStream_t st, const FastLayout &L, const double *Dinv, const double *O1,
                    const double *O2, float *DX);

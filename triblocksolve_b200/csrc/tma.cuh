@@ -137,6 +137,18 @@ __device__ __forceinline__ void bulk_g2s_hint(void *dst, const void *src, uint32
         : "memory");
 }
 
+/* 8-byte asynchronous copies global -> shared memory, in groups of the
+ * issuing thread */
+__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+/* all but the newest N groups have landed */
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 /* makes this thread's writes to shared memory visible to the bulk copies
  * that are issued after the next barrier */
 __device__ __forceinline__ void fence_async_smem() {
