@@ -970,13 +970,10 @@ static int run_factor(tbs_ctx *ctx, int algo) {
         CKL(copy_words(st, ctx->d_jacD, ctx->d_DLU, nb * sizeof(double)));
         CK(cudaMemsetAsync(ctx->d_DinvC, 0, nb * sizeof(double), st));
         CK(cudaMemsetAsync(ctx->d_A, 0, nb * sizeof(double), st));
-        RUN("ref_assemble_A", launch_ref_assemble_A(st, nv, ctx->nline, ctx->d_fc, ctx->d_linesize,
-                                                    ctx->d_linepoint, ctx->d_lines, ctx->d_lineface,
-                                                    ctx->d_O1, ctx->d_O2, ctx->d_A));
         RUN("ref_line_lu", launch_ref_line_lu(st, nv, ctx->nline, ctx->d_fc, ctx->d_linesize,
                                               ctx->d_linepoint, ctx->d_lines, ctx->d_lineface,
                                               ctx->d_DLU, ctx->d_O1, ctx->d_O2, ctx->d_DinvC,
-                                              ctx->d_status));
+                                              ctx->d_A, ctx->d_status));
         return TBS_OK;
     }
     const FastLayout &L = ctx->L;

@@ -18,6 +18,7 @@
  * summed from 0.0 in ascending j as in the OKL loops.
  */
 #include "tbs_internal.hxx"
+#include "tma.cuh"
 
 #include <cuda_runtime.h>
 
@@ -53,9 +54,7 @@ __device__ __forceinline__ void solve_lu_lane(const double *A, const double *b, 
 /* In-place no-pivot Doolittle on a shared-memory block, rows over lanes.
  * Row j is final when step j starts and only rows i > j change in it, so
  * lane i applying its own row's updates reproduces lineLU_v2.okl:17-27. */
-template <int NV>
-__device__ __forceinline__ void lu_rows(double *A, int lane, int nv_rt, unsigned *status) {
-    const int nv = NV ? NV : nv_rt;
+__device__ __forceinline__ void lu_rows(double *A, int lane, int nv, unsigned *status) {
     for (int j = 0; j < nv; ++j) {
         __syncwarp();
         const double ajj = A[MIDX(j, j, nv)];
@@ -70,13 +69,11 @@ __device__ __forceinline__ void lu_rows(double *A, int lane, int nv_rt, unsigned
     __syncwarp();
 }
 
-template <int NV>
 __global__ void __launch_bounds__(32) ref_line_lu_kernel(
-    int nv_rt, int nline, const int *__restrict__ fc, const int *__restrict__ linesize,
+    int nv, int nline, const int *__restrict__ fc, const int *__restrict__ linesize,
     const int *__restrict__ linepoint, const int *__restrict__ lines,
     const int *__restrict__ lineface, double *__restrict__ Dia, const double *__restrict__ O1,
     const double *__restrict__ O2, double *__restrict__ DinvC, unsigned *status) {
-    const int nv = NV ? NV : nv_rt;
     const int l = blockIdx.x;
     if (l >= nline) return;
     const int lane = threadIdx.x;
@@ -93,7 +90,7 @@ __global__ void __launch_bounds__(32) ref_line_lu_kernel(
     int e = lines[m0];
     if (lane < nv)
         for (int j = 0; j < nv; ++j) sDe[MIDX(lane, j, nv)] = Dia[MIDX(lane, j, nv) + bs * e];
-    lu_rows<NV>(sDe, lane, nv, status);
+    lu_rows(sDe, lane, nv, status);
     if (lane < nv)
         for (int j = 0; j < nv; ++j) Dia[MIDX(lane, j, nv) + bs * e] = sDe[MIDX(lane, j, nv)];
 
@@ -123,7 +120,7 @@ __global__ void __launch_bounds__(32) ref_line_lu_kernel(
         }
         __syncwarp();
         /* Gamma(:,i) = D'_{k-1}^-1 C(:,i)  (lineLU_v2.okl:142-144) */
-        if (lane < nv) solve_lu_lane<NV>(sDl, &sC[MIDX(0, lane, nv)], &sGamma[MIDX(0, lane, nv)], nv);
+        if (lane < nv) solve_lu_lane<0>(sDl, &sC[MIDX(0, lane, nv)], &sGamma[MIDX(0, lane, nv)], nv);
         __syncwarp();
         /* D_k - A_k Gamma  (lineLU_v2.okl:147-161) */
         if (lane < nv) {
@@ -133,7 +130,7 @@ __global__ void __launch_bounds__(32) ref_line_lu_kernel(
                 sDe[MIDX(lane, kk, nv)] -= tot;
             }
         }
-        lu_rows<NV>(sDe, lane, nv, status);
+        lu_rows(sDe, lane, nv, status);
         if (lane < nv) {
             for (int j = 0; j < nv; ++j) {
                 Dia[MIDX(lane, j, nv) + bs * e] = sDe[MIDX(lane, j, nv)];
@@ -143,23 +140,275 @@ __global__ void __launch_bounds__(32) ref_line_lu_kernel(
     }
 }
 
-int launch_ref_line_lu(cudaStream_t st, int nv, int nline, const int *fc, const int *linesize,
-                       const int *linepoint, const int *lines, const int *lineface, double *DLU,
-                       const double *O1, const double *O2, double *DinvC, unsigned *status) {
-    if (nv < 1 || nv > REF_MAXNV) return (int)cudaErrorInvalidValue;
-    const size_t smem = 5 * (size_t)nv * nv * sizeof(double);
-    if (nv == 9) {
-        ref_line_lu_kernel<9><<<nline, 32, smem, st>>>(nv, nline, fc, linesize, linepoint, lines,
-                                                       lineface, DLU, O1, O2, DinvC, status);
-    } else {
-        if (smem > 48 * 1024) {
-            const int e = smem_raise((const void *)ref_line_lu_kernel<0>, smem);
-            if (e != 0) return e;
-        }
-        ref_line_lu_kernel<0><<<nline, 32, smem, st>>>(nv, nline, fc, linesize, linepoint, lines,
-                                                       lineface, DLU, O1, O2, DinvC, status);
+/* ------------------------------------------------- block size 9, quickly
+ * The same scalars, each by the same sequence of roundings, with the chain
+ * kept short: solveLU's divisions by a diagonal whose reciprocal is known
+ * beforehand, every lane of a warp computing the whole vector (no exchange
+ * inside a triangular solve), a second warp copying the coming cells' blocks
+ * into shared memory. */
+
+/* RN(1 / d) by Newton's iteration and Markstein's last step (P. Markstein,
+ * IBM J. Res. Dev. 34 (1990) 111-119); d within 2^-500 .. 2^500 and its
+ * significand not all ones (the theorem's exception): ref_plain_divisor */
+__device__ __forceinline__ double ref_rcp(double d) {
+    double x;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+    double e = fma(-d, x, 1.0);
+    x = fma(x, fma(e, e, e), x);
+    e = fma(-d, x, 1.0);
+    return fma(x, e, x);
+}
+
+/* |v| within 2^-e .. 2^e (not zero, not infinite, a number) */
+__device__ __forceinline__ bool ref_within(double v, int e) {
+    return (unsigned)((__double2hiint(v) & 0x7fffffff) - ((1023 - e) << 20)) < (unsigned)(2 * e) << 20;
+}
+
+/* a divisor left to the general division */
+__device__ __forceinline__ bool ref_plain_divisor(double d) {
+    return !ref_within(d, 500) || ((__double2hiint(d) & 0xfffff) == 0xfffff && __double2loint(d) == -1);
+}
+
+/* RN(n / d) from r = RN(1 / d) and rl, the rest of 1 / d to twice the
+ * precision: q is within an ulp, the remainder exact and the last step
+ * rounds correctly (Markstein, as above).  Holds for |d| within 2^-500 ..
+ * 2^500 and |n| within 2^-400 .. 2^400; the caller checks both. */
+__device__ __forceinline__ double ref_div(double n, double d, double r, double rl) {
+    const double q = fma(n, r, n * rl);
+    return fma(fma(-q, d, n), r, q);
+}
+
+constexpr int RC = 4;                        /* cells of one copy job */
+constexpr int RS = 3;                        /* jobs in shared memory */
+constexpr int RCELL = 81 + 81 + 9 + 9 + 9 + 1; /* D', A, R, 1/U_ii (r, rl), flag */
+
+/* x = (LU)^-1 s, all of it in every lane; D: the block in shared memory
+ * (column-major), rc: r and rl of its diagonal.  The sums start from 0.0 and
+ * take j in ascending order, as solveLU's: forward by columns (each row's
+ * terms still come in order), backward by rows, from products formed as the
+ * x_j come.  A first term is rounded once by fma(a, b, 0.0) (0.0 + a*b).
+ * plain: the diagonal or a numerator may be out of ref_div's range (decided by
+ * the caller), so divide. */
+__device__ __forceinline__ bool ref_solve9(const double *D, const double *rc, const double (&s)[9],
+                                           double (&x)[9]) {
+    double tot[9], y[9];
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+        y[j] = j == 0 ? s[0] - 0.0 : s[j] - tot[j];
+#pragma unroll
+        for (int i = j + 1; i < 9; ++i)
+            tot[i] = j == 0 ? fma(D[i], y[0], 0.0) : tot[i] + D[i + 9 * j] * y[j];
     }
-    return (int)cudaGetLastError();
+    double p[9][9];
+    bool ok = true;
+#pragma unroll
+    for (int i = 8; i >= 0; --i) {
+        double t = 0.0;
+#pragma unroll
+        for (int j = i + 1; j < 9; ++j) t = j == i + 1 ? p[i][j] : t + p[i][j];
+        const double n = y[i] - t;
+        ok = ok && ref_within(n, 400);
+        x[i] = ref_div(n, D[10 * i], rc[i], rc[9 + i]);
+#pragma unroll
+        for (int k = 0; k < i; ++k) p[k][i] = k + 1 == i ? fma(D[k + 9 * i], x[i], 0.0) : D[k + 9 * i] * x[i];
+    }
+    return ok;
+}
+
+/* In-place no-pivot Doolittle (lineLU_v2.okl:17-27) of a block held by 27
+ * lanes, lane i + 9g row i, columns 3g..3g+2.  Step j: l_ij = a_ij * (1/a_jj),
+ * a_ik -= l_ij a_jk, each operation rounded by itself; every lane forms the
+ * next pivot from three entries fetched while this one's reciprocal is on its
+ * way.  rc[0..8], rc[9..17]: r and rl of the diagonal (ref_div), rc[18]: not 0
+ * when a pivot is not for ref_div (and, unless PLAIN, the result not valid).
+ * Returns whether a pivot was zero or not finite (PLAIN) or has to be done by
+ * the general division. */
+template <bool PLAIN>
+__device__ __forceinline__ bool ref_lu27(double (&w)[3], int i, int g, bool first, double *rc) {
+    bool odd = false, bad = false;
+    double a = __shfl_sync(0xffffffffu, w[0], 0);
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+        const int jg = j / 3, jk = j % 3, n = j < 8 ? j + 1 : j, ng = n / 3, nk = n % 3;
+        const double dn = __shfl_sync(0xffffffffu, w[nk], n + 9 * ng);
+        const double cn = __shfl_sync(0xffffffffu, w[jk], n + 9 * jg);
+        const double rn = __shfl_sync(0xffffffffu, w[nk], j + 9 * ng);
+        double l = __shfl_sync(0xffffffffu, w[jk], i + 9 * jg);
+        double u[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) u[k] = __shfl_sync(0xffffffffu, w[k], j + 9 * g);
+        if (PLAIN) bad |= !(fabs(a) > 0.0 && isfinite(a));
+        odd |= ref_plain_divisor(a);
+        const double r = PLAIN ? 1.0 / a : ref_rcp(a);
+        if (first && i == j) {
+            rc[j] = r;
+            rc[9 + j] = fma(-a, r, 1.0) * r;
+        }
+        l = l * r;
+        a = dn - (cn * r) * rn;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int c = 3 * g + k;
+            const double v = w[k] - l * u[k];
+            if (i > j) w[k] = c > j ? v : (c == j ? l : w[k]);
+        }
+    }
+    if (first && i == 0) rc[18] = odd ? 1.0 : 0.0;
+    return PLAIN ? bad : odd;
+}
+
+__device__ __noinline__ bool ref_lu27_plain(double *v, int i, int g, bool first, double *rc) {
+    double w[3] = {v[0], v[1], v[2]};
+    const bool bad = ref_lu27<true>(w, i, g, first, rc);
+    v[0] = w[0];
+    v[1] = w[1];
+    v[2] = w[2];
+    return bad;
+}
+
+constexpr int LS = 4;                /* cells in shared memory */
+constexpr int LCELL = 3 * 81;        /* D, A, C */
+
+/* ref_line_lu_kernel for block size 9, and the packing of the lower blocks
+ * (ref_assemble_A_kernel): one CTA of two warps per line, warp 0 on the chain
+ * (Gamma: a column per lane; D - A Gamma and the LU: 27 lanes), warp 1 copying
+ * the cells two steps ahead into shared memory and writing D', D'^-1 C and A
+ * out.  ref_line_lu_kernel, which loads as it goes and divides 18 times a
+ * cell, took 9,900 cycles a cell; 360x384: 1,960 us and 95 for the packing,
+ * 720 together here. */
+__global__ void __launch_bounds__(64) ref_line_lu9_kernel(
+    int nline, const int *__restrict__ fc, const int *__restrict__ linesize,
+    const int *__restrict__ linepoint, const int *__restrict__ lines,
+    const int *__restrict__ lineface, double *Dia, const double *__restrict__ O1,
+    const double *__restrict__ O2, double *__restrict__ DinvC, double *__restrict__ Aout,
+    unsigned *status) {
+    __shared__ __align__(16) double stage[LS][LCELL];
+    __shared__ __align__(16) double sL[2][81], sG[2][81], rc[19];
+    const int l = blockIdx.x;
+    if (l >= nline) return;
+    const int lane = threadIdx.x & 31;
+    const int n = linesize[l], m0 = linepoint[l];
+    if (threadIdx.x >= 32) {
+        auto elem = [&](int c) { return c >= 0 && c < n ? lines[m0 + c] : 0; };
+        auto face = [&](int c) { return c >= 1 && c < n ? lineface[m0 + c] : 0; };
+        auto first = [&](int c, int f) { return c >= 1 && c < n ? fc[2 * f] : 0; };
+        /* copies of cell c (element e, face f, whose first element is e1) */
+        auto copy = [&](int c, int e, int f, int e1) {
+            if (c < n) {
+                const double *pD = Dia + 81 * (size_t)e;
+                const double *pA = (e == e1 ? O2 : O1) + 81 * (size_t)f;
+                const double *pC = (e == e1 ? O1 : O2) + 81 * (size_t)f;
+                double *d = stage[c % LS];
+#pragma unroll
+                for (int r = 0; r < 3; ++r) {
+                    const int t = lane + 32 * r;
+                    if (t < 81) {
+                        cp_async8(d + t, pD + t);
+                        if (c > 0) {
+                            cp_async8(d + 81 + t, pA + t);
+                            cp_async8(d + 162 + t, pC + t);
+                        }
+                    }
+                }
+            }
+            cp_async_commit();
+        };
+        auto put = [&](double *dst, const double *src) {
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                const int t = lane + 32 * r;
+                if (t < 81) dst[t] = src[t];
+            }
+        };
+        int ep2 = 0, ep1 = 0, e0 = elem(0), e1 = elem(1), e2 = elem(2), e3 = elem(3);
+        int f2 = face(2), f3 = face(3), a2;
+        {
+            const int f1 = face(1);
+            copy(0, e0, 0, 0);
+            copy(1, e1, f1, first(1, f1));
+        }
+        a2 = first(2, f2);
+        cp_async_wait<1>();
+        __syncthreads();
+        for (int s = 0; s <= n + 1; ++s) {
+            copy(s + 2, e2, f2, a2);
+            const int en = elem(s + 4), fn = face(s + 4), an = first(s + 3, f3);
+            if (s >= 1 && s < n) put(Aout + 81 * (size_t)e0, stage[s % LS] + 81);
+            if (s >= 1 && s - 1 < n) put(Dia + 81 * (size_t)ep1, sL[(s - 1) & 1]);
+            if (s >= 2 && s - 1 < n) put(DinvC + 81 * (size_t)ep2, sG[(s - 1) & 1]);
+            ep2 = ep1;
+            ep1 = e0;
+            e0 = e1;
+            e1 = e2;
+            e2 = e3;
+            e3 = en;
+            f2 = f3;
+            f3 = fn;
+            a2 = an;
+            cp_async_wait<1>();
+            __syncthreads();
+        }
+        cp_async_wait<0>();
+        return;
+    }
+    /* lanes 27..31 repeat lanes 18..22 and store nothing */
+    const bool act = lane < 27;
+    const int ln = act ? lane : lane - 9;
+    const int i = ln % 9, g = ln / 9;
+    const int col = lane < 9 ? lane : 8;
+    bool bad = false;
+    __syncthreads();
+    for (int s = 0; s <= n + 1; ++s) {
+        if (s < n) {
+            const double *D = stage[s % LS], *A = D + 81, *C = D + 162;
+            double w[3];
+            if (s > 0) {
+                /* Gamma(:, col) = D'_{s-1}^-1 C(:, col) (lineLU_v2.okl:142-144) */
+                double v[9], x[9];
+#pragma unroll
+                for (int k = 0; k < 9; ++k) v[k] = C[k + 9 * col];
+                const double *L = sL[(s - 1) & 1];
+                const bool ok = ref_solve9(L, rc, v, x);
+                if (!ok || rc[18] != 0.0) solve_lu_lane<9>(L, v, x, 9);
+                if (lane < 9) {
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) sG[s & 1][k + 9 * col] = x[k];
+                }
+                __syncwarp();
+            }
+            /* D_s - A Gamma (lineLU_v2.okl:147-161) */
+            auto pivot = [&]() {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const int c = 3 * g + k;
+                    w[k] = D[i + 9 * c];
+                    if (s > 0) {
+                        const double *G = sG[s & 1] + 9 * c;
+                        double tot = fma(A[i], G[0], 0.0);
+#pragma unroll
+                        for (int j = 1; j < 9; ++j) tot += A[i + 9 * j] * G[j];
+                        w[k] = w[k] - tot;
+                    }
+                }
+            };
+            pivot();
+            if (ref_lu27<false>(w, i, g, act && g == 0, rc)) { /* the same in every lane */
+                pivot();
+                double v[3] = {w[0], w[1], w[2]};
+                __syncwarp();
+                bad = ref_lu27_plain(v, i, g, act && g == 0, rc) || bad;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) w[k] = v[k];
+            }
+            if (act) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) sL[s & 1][i + 9 * (3 * g + k)] = w[k];
+            }
+            __syncwarp();
+        }
+        __syncthreads();
+    }
+    if (bad && lane == 0) atomicOr(status, ST_PIVOT);
 }
 
 /* Jacobian.cxx:76-117: A[e] = (e == fc[2f]) ? O2[f] : O1[f], f = lineface[m],
@@ -184,24 +433,196 @@ __global__ void ref_assemble_A_kernel(int nv, int nline, const int *__restrict__
     }
 }
 
-int launch_ref_assemble_A(cudaStream_t st, int nv, int nline, const int *fc, const int *linesize,
-                          const int *linepoint, const int *lines, const int *lineface,
-                          const double *O1, const double *O2, double *A) {
+/* the line factorization (DLU in place, DinvC) and the packed lower blocks */
+int launch_ref_line_lu(cudaStream_t st, int nv, int nline, const int *fc, const int *linesize,
+                       const int *linepoint, const int *lines, const int *lineface, double *DLU,
+                       const double *O1, const double *O2, double *DinvC, double *A, unsigned *status) {
+    if (nv < 1 || nv > REF_MAXNV) return (int)cudaErrorInvalidValue;
+    if (nv == 9) {
+        ref_line_lu9_kernel<<<nline, 64, 0, st>>>(nline, fc, linesize, linepoint, lines, lineface, DLU, O1,
+                                                  O2, DinvC, A, status);
+        return (int)cudaGetLastError();
+    }
+    const size_t smem = 5 * (size_t)nv * nv * sizeof(double);
+    if (smem > 48 * 1024) {
+        const int e = smem_raise((const void *)ref_line_lu_kernel, smem);
+        if (e != 0) return e;
+    }
     ref_assemble_A_kernel<<<nline, dim3(32, 8), 0, st>>>(nv, nline, fc, linesize, linepoint, lines,
                                                          lineface, O1, O2, A);
+    ref_line_lu_kernel<<<nline, 32, smem, st>>>(nv, nline, fc, linesize, linepoint, lines, lineface, DLU,
+                                                O1, O2, DinvC, status);
     return (int)cudaGetLastError();
 }
 
-/* linesmoothLU_TriBlock_v3.okl:92-226.  Lane 0 runs solveLU as the
+/* ref_solve_du_kernel for block size 9: one CTA of two warps per line.
+ * What bounds it is the dependent chain of a cell -- 9 multiply-adds and
+ * subtractions forward, 28 additions, 9 subtractions and 9 divisions
+ * backward, in solveLU's order -- about 1,100 cycles; lane 0 solving alone
+ * and loading what it needs as it goes (ref_solve_du_kernel) took 5,300.
+ * 360x384: 1,053 -> 382 us. */
+__global__ void __launch_bounds__(64) ref_solve_du9_kernel(
+    int nline, const int *__restrict__ linesize, const int *__restrict__ linepoint,
+    const int *__restrict__ lines, const double *__restrict__ Dia, const double *__restrict__ DinvC,
+    const double *__restrict__ A, double *__restrict__ dU, const double *__restrict__ R) {
+    __shared__ __align__(16) double stage[RS][RC][RCELL];
+    __shared__ __align__(16) double vec[2][10];
+    const int l = blockIdx.x;
+    if (l >= nline) return;
+    const int lane = threadIdx.x & 31;
+    const int n = linesize[l], m0 = linepoint[l];
+    const int nf = (n + RC - 1) / RC, nb = (n - 1 + RC - 1) / RC, njobs = nf + nb;
+    /* forward job c: cells 4c..; backward job c: cells n-2-4c, n-3-4c, .. */
+    auto cell = [&](int job, int q) { return job < nf ? job * RC + q : n - 2 - ((job - nf) * RC + q); };
+    auto valid = [&](int job, int q) {
+        const int k = cell(job, q);
+        return job < njobs && k >= 0 && k < (job < nf ? n : n - 1);
+    };
+    if (threadIdx.x >= 32) {
+        auto index = [&](int job) { return lane < RC && valid(job, lane) ? lines[m0 + cell(job, lane)] : 0; };
+        auto copy = [&](int job, int es) {
+#pragma unroll
+            for (int q = 0; q < RC; ++q) {
+                const size_t e = __shfl_sync(0xffffffffu, es, q);
+                if (!valid(job, q)) continue;
+                double *d = stage[job % RS][q];
+                const double *b0 = (job < nf ? Dia : DinvC) + 81 * e, *b1 = A + 81 * e;
+#pragma unroll
+                for (int r = 0; r < 3; ++r) {
+                    const int t = lane + 32 * r;
+                    if (t < 81) {
+                        cp_async8(d + t, b0 + t);
+                        if (job < nf) cp_async8(d + 81 + t, b1 + t);
+                    }
+                }
+                if (job < nf && lane < 9) cp_async8(d + 162 + lane, R + 9 * e + lane);
+            }
+            cp_async_commit();
+        };
+        /* the reciprocals of a landed forward job's diagonals */
+        auto recips = [&](int job) {
+            __syncwarp();
+            if (job >= nf) return;
+            if (lane < RC) stage[job % RS][lane][189] = 0.0;
+            __syncwarp();
+            for (int t = lane; t < 9 * RC; t += 32) {
+                const int q = t / 9, i = t % 9;
+                double *d = stage[job % RS][q];
+                const double u = d[10 * i], r = ref_rcp(u);
+                d[171 + i] = r;
+                d[180 + i] = fma(-u, r, 1.0) * r;
+                if (ref_plain_divisor(u)) d[189] = 1.0;
+            }
+        };
+        copy(0, index(0));
+        copy(1, index(1));
+        int es = index(2);
+        cp_async_wait<1>();
+        recips(0);
+        __syncthreads();
+        for (int job = 0; job < njobs; ++job) {
+            copy(job + 2, es);
+            es = index(job + 3);
+            cp_async_wait<1>();
+            recips(job + 1);
+            __syncthreads();
+        }
+        cp_async_wait<0>();
+        return;
+    }
+    const int i = lane < 9 ? lane : 8;
+    double x[9];
+    __syncthreads();
+    for (int job = 0; job < nf; ++job) {
+        int es[RC];
+#pragma unroll
+        for (int q = 0; q < RC; ++q) es[q] = valid(job, q) ? lines[m0 + cell(job, q)] : 0;
+#pragma unroll 1
+        for (int q = 0; q < RC; ++q) {
+            if (!valid(job, q)) break;
+            const double *d = stage[job % RS][q];
+            /* lane i: s_i = -R_i - (A dU_{k-1})_i */
+            double si = -d[162 + i];
+            if (job > 0 || q > 0) {
+                double tot = fma(d[81 + i], x[0], 0.0);
+#pragma unroll
+                for (int j = 1; j < 9; ++j) tot += d[81 + i + 9 * j] * x[j];
+                si = si - tot;
+            }
+            double s[9];
+#pragma unroll
+            for (int j = 0; j < 9; ++j) s[j] = __shfl_sync(0xffffffffu, si, j);
+            const bool ok = ref_solve9(d, d + 171, s, x);
+            if (!ok || d[189] != 0.0) solve_lu_lane<9>(d, s, x, 9); /* the same in every lane */
+            double mine = x[0];
+#pragma unroll
+            for (int j = 1; j < 9; ++j) mine = i == j ? x[j] : mine;
+            const int e = q == 0 ? es[0] : q == 1 ? es[1] : q == 2 ? es[2] : es[3];
+            if (lane < 9) dU[9 * (size_t)e + i] = mine;
+        }
+        __syncthreads();
+    }
+    /* back substitution: dU_k -= DinvC_k dU_{k+1}, the vector through shared
+     * memory (lanes 9.. repeat lane 8); a job's dU is read (by the lanes that
+     * wrote it) one job ahead */
+    {
+        double mine = x[0];
+#pragma unroll
+        for (int j = 1; j < 9; ++j) mine = i == j ? x[j] : mine;
+        vec[0][i] = mine;
+        __syncwarp();
+    }
+    double u[RC], nu[RC];
+    int es[RC], ns[RC];
+    auto fetch = [&](int job, double *v, int *ee) {
+#pragma unroll
+        for (int q = 0; q < RC; ++q) {
+            ee[q] = valid(job, q) ? lines[m0 + cell(job, q)] : 0;
+            v[q] = valid(job, q) ? dU[9 * (size_t)ee[q] + i] : 0.0;
+        }
+    };
+    if (nb > 0) fetch(nf, u, es);
+    for (int job = nf; job < njobs; ++job) {
+        fetch(job + 1, nu, ns);
+#pragma unroll
+        for (int q = 0; q < RC; ++q) {
+            if (valid(job, q)) {
+                const double *d = stage[job % RS][q];
+                const double2 *v = reinterpret_cast<const double2 *>(vec[q & 1]);
+                const double2 v0 = v[0], v1 = v[1], v2 = v[2], v3 = v[3];
+                const double v8 = vec[q & 1][8];
+                double tot = fma(d[i], v0.x, 0.0);
+                tot += d[i + 9] * v0.y;
+                tot += d[i + 18] * v1.x;
+                tot += d[i + 27] * v1.y;
+                tot += d[i + 36] * v2.x;
+                tot += d[i + 45] * v2.y;
+                tot += d[i + 54] * v3.x;
+                tot += d[i + 63] * v3.y;
+                tot += d[i + 72] * v8;
+                const double mine = u[q] - tot;
+                vec[(q & 1) ^ 1][i] = mine;
+                if (lane < 9) dU[9 * (size_t)es[q] + i] = mine;
+                __syncwarp();
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < RC; ++q) {
+            u[q] = nu[q];
+            es[q] = ns[q];
+        }
+        __syncthreads();
+    }
+}
+
+/* linesmoothLU_TriBlock_v3.okl:92-226, any block size.  Lane 0 runs solveLU as the
  * reference does (its `if(i==0)` guard, :154/:192); the other lanes do the
  * row-parallel matvecs and prefetch the next cell's blocks meanwhile. */
-template <int NV>
 __global__ void __launch_bounds__(32) ref_solve_du_kernel(
-    int nv_rt, int nline, const int *__restrict__ linesize, const int *__restrict__ linepoint,
+    int nv, int nline, const int *__restrict__ linesize, const int *__restrict__ linepoint,
     const int *__restrict__ lines, const double *__restrict__ Dia,
     const double *__restrict__ DinvC, const double *__restrict__ A, double *__restrict__ dU,
     const double *__restrict__ R) {
-    const int nv = NV ? NV : nv_rt;
     const int l = blockIdx.x;
     if (l >= nline) return;
     const int lane = threadIdx.x;
@@ -220,7 +641,7 @@ __global__ void __launch_bounds__(32) ref_solve_du_kernel(
         for (int j = 0; j < nv; ++j) sDia[MIDX(lane, j, nv)] = Dia[MIDX(lane, j, nv) + bs * e];
     }
     __syncwarp();
-    if (lane == 0) solve_lu_lane<NV>(sDia, sS, sdU, nv);
+    if (lane == 0) solve_lu_lane<0>(sDia, sS, sdU, nv);
     __syncwarp();
     if (lane < nv) dU[lane + (size_t)nv * e] = sdU[lane];
 
@@ -240,7 +661,7 @@ __global__ void __launch_bounds__(32) ref_solve_du_kernel(
             sS[lane] = -R[lane + (size_t)nv * e] - tot;
         }
         __syncwarp();
-        if (lane == 0) solve_lu_lane<NV>(sDia, sS, sdU, nv);
+        if (lane == 0) solve_lu_lane<0>(sDia, sS, sdU, nv);
         __syncwarp();
         if (lane < nv) dU[lane + (size_t)nv * e] = sdU[lane];
     }
@@ -267,10 +688,9 @@ int launch_ref_solve_du(cudaStream_t st, int nv, int nline, const int *linesize,
     if (nv < 1 || nv > REF_MAXNV) return (int)cudaErrorInvalidValue;
     const size_t smem = (2 * (size_t)nv * nv + 2 * REF_MAXNV) * sizeof(double);
     if (nv == 9) {
-        ref_solve_du_kernel<9><<<nline, 32, smem, st>>>(nv, nline, linesize, linepoint, lines, DLU,
-                                                        DinvC, A, dU, R);
+        ref_solve_du9_kernel<<<nline, 64, 0, st>>>(nline, linesize, linepoint, lines, DLU, DinvC, A, dU, R);
     } else {
-        ref_solve_du_kernel<0><<<nline, 32, smem, st>>>(nv, nline, linesize, linepoint, lines, DLU,
+        ref_solve_du_kernel<<<nline, 32, smem, st>>>(nv, nline, linesize, linepoint, lines, DLU,
                                                         DinvC, A, dU, R);
     }
     return (int)cudaGetLastError();

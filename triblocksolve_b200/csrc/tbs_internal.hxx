@@ -131,10 +131,8 @@ int smem_raise(const void *fn, size_t need);
 /* reference-order kernels (kernels_ref.cu, built with -fmad=false) */
 int launch_ref_line_lu(cudaStream_t st, int nv, int nline, const int *fc, const int *linesize,
                        const int *linepoint, const int *lines, const int *lineface, double *DLU,
-                       const double *O1, const double *O2, double *DinvC, unsigned *status);
-int launch_ref_assemble_A(cudaStream_t st, int nv, int nline, const int *fc, const int *linesize,
-                          const int *linepoint, const int *lines, const int *lineface,
-                          const double *O1, const double *O2, double *A);
+                       const double *O1, const double *O2, double *DinvC, double *A,
+                       unsigned *status);
 int launch_ref_solve_du(cudaStream_t st, int nv, int nline, const int *linesize,
                         const int *linepoint, const int *lines, const double *DLU,
                         const double *DinvC, const double *A, double *dU, const double *R);
