@@ -149,6 +149,7 @@ static void drop_mesh(tbs_ctx *ctx) {
     ctx->d_status = nullptr;
     ctx->d_ktimer = nullptr;
     ctx->d_counter = nullptr;
+    ctx->d_meet = nullptr;
     ctx->npart_cap = 0;
     ctx->hist_cap = 0;
     ctx->have_mesh = ctx->have_jac = ctx->factored = false;
@@ -448,6 +449,7 @@ static int status_error(tbs_ctx *ctx, unsigned s) {
     if (s) {
         CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(unsigned), ctx->stream));
         if (ctx->d_counter) CK(cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned), ctx->stream));
+        if (ctx->d_meet) CK(cudaMemsetAsync(ctx->d_meet, 0, SMALL_MEET_WORDS * sizeof(unsigned), ctx->stream));
         if (s & ST_PIVOT)
             return ctx_fail(ctx, TBS_ERR_NUMERIC,
                             "zero or non-finite pivot in the no-pivot block factorization");
@@ -829,6 +831,21 @@ static int add_conditional(tbs_ctx *ctx, cudaGraph_t g, cudaGraphConditionalHand
     return TBS_OK;
 }
 
+/* Few lines (TBS_ALGO_FP64, block size 9): the loop's body is all the sweeps,
+ * one cooperative launch, so the loop goes round again only after a failed
+ * check. */
+static bool small_solve(const tbs_ctx *ctx) {
+    return ctx->algo == TBS_ALGO_FP64 && ctx->nvar == 9 && small_sweeps_grid(ctx->L) > 0;
+}
+
+static int body_small(tbs_ctx *ctx, CondCtl cc) {
+    NormSink ns = sink(ctx, 0, cc);
+    ns.timer = ctx->d_ktimer;
+    CKL(launch_small_sweeps(ctx->stream, ctx->L, ctx->d_G, ctx->d_Gam, ctx->d_Dinv, ctx->d_X, ctx->d_b, ctx->d_y,
+                            ctx->d_dUp, ctx->d_Up, ns, ctx->d_meet, ctx->d_status));
+    return TBS_OK;
+}
+
 /* Graph: prime (records ||R_0||, sets the condition) -> while (cond) { sweep }.
  * TBS_ALGO_MIXED with its own inner sweep count for the first outer step:
  * prime -> if (cond) { first step } -> while (cond) { step }, the prime
@@ -845,6 +862,7 @@ static int build_graph(tbs_ctx *ctx) {
     CK(cudaGraphConditionalHandleCreate(&hw, g, 0, cudaGraphCondAssignDefault));
     if (sched) CK(cudaGraphConditionalHandleCreate(&hf, g, 0, cudaGraphCondAssignDefault));
     const bool chk = checks_solve(ctx);
+    const bool small = small_solve(ctx); /* outside capture: it raises a shared-memory limit */
     cudaGraphConditionalHandle hc = 0, hr = 0;
     if (chk) {
         CK(cudaGraphConditionalHandleCreate(&hc, g, 0, cudaGraphCondAssignDefault));
@@ -869,7 +887,7 @@ static int build_graph(tbs_ctx *ctx) {
     cudaGraph_t checkg = nullptr;
     if (rc == TBS_OK)
         rc = capture_into(ctx, bodyg, [&]() {
-            int r = body(ctx, loop, ctx->inner_sweeps);
+            int r = small ? body_small(ctx, loop) : body(ctx, loop, ctx->inner_sweeps);
             if (r == TBS_OK && chk) r = add_conditional(ctx, bodyg, hc, cudaGraphCondTypeIf, &checkg);
             return r;
         });
@@ -908,6 +926,7 @@ static int alloc_algo(tbs_ctx *ctx, int algo) {
     const int npmax = std::max({ref_line_res_partials(ctx->nelem) * 8, fast_resid_grid(ctx->L.np16),
                                 full_resid_blocks(ctx->nelem), 1024});
     DA(ctx->d_counter, 1);
+    DA(ctx->d_meet, SMALL_MEET_WORDS);
     if (ctx->npart_cap < npmax) {
         dfree(ctx, &ctx->d_partials);
         dfree(ctx, &ctx->d_partials2);

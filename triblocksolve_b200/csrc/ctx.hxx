@@ -97,6 +97,7 @@ struct tbs_ctx {
     unsigned *h_status = nullptr; /* pinned, mapped */
     unsigned *h_status_dev = nullptr;
     unsigned *d_counter = nullptr; /* last-CTA ticket of the fused norm */
+    unsigned *d_meet = nullptr;    /* arrivals of the launch of all sweeps */
     int algo = -1;
 
     /* ---- graph cache ---- */

@@ -28,6 +28,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 namespace tbs {
 
@@ -1617,14 +1618,26 @@ __device__ __forceinline__ void bwd_chunk(const T *sG, Row<T> &row, T &yk, T *bc
 template <bool WS>
 __host__ __device__ constexpr int thomas_hdr() { return WS ? 256 : 128; }
 
+/* the two warps of a warp-specialised line solve (the CTA may hold more) */
+__device__ __forceinline__ void ws_meet() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
+
 /* accumulate = 1 reads U from Uin when it is set (a second buffer: the
- * previous U stays intact), else from U itself */
-template <typename T, int P, bool YS, bool WS = false>
+ * previous U stays intact), else from U itself.  drain (YS): dU has been
+ * written when the call returns, not only read from shared memory (for kernels
+ * that go on to read it), U before the next call writes it.  b and U are read
+ * past the L1, which may hold an earlier sweep's. */
+/* PH 0: the whole line.  The other phases split it (WS; the copy warp's lane
+ * 0 acts in all but the third): PH_BLOCKS starts the copies of the first jobs'
+ * blocks, while others still write b; PH_VECS those of their b; PH_RUN is the
+ * line after both; PH_DROP waits for the copies when no line follows. */
+enum { PH_ALL = 0, PH_BLOCKS, PH_VECS, PH_RUN, PH_DROP };
+
+template <typename T, int P, bool YS, bool WS = false, int PH = PH_ALL>
 __device__ __forceinline__ bool thomas_line(
     int NS, int accumulate, int ps, int n, int m, const T *__restrict__ G,
     const T *__restrict__ Gam, const T *__restrict__ b, T *__restrict__ y, T *__restrict__ dU,
     T *__restrict__ U, unsigned *status, unsigned char *smem, uint32_t &pbase, uint64_t pol,
-    const T *__restrict__ Uin = nullptr) {
+    const T *__restrict__ Uin = nullptr, bool drain = false) {
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
     /* WS (warp-specialised CTA of two warps): bars[0..NS) complete when a
      * stage's copies have landed, bars[8..8+NS) when warp 0 has consumed
@@ -1660,14 +1673,14 @@ __device__ __forceinline__ bool thomas_line(
      * chain warp reads it from shared memory */
     const bool stage_u = WS && !YS && accumulate == 1 && Ul != nullptr;
     __syncwarp(); /* the previous line's readers of the stages are done */
-    if (!producer)
+    if (!producer && (PH == PH_ALL || PH == PH_RUN))
         for (int t = lane; t < BCAST<T>; t += 32) bcall[t] = T(0);
     __syncwarp();
 
     /* copy size of chunk c of a chain of length ln, rounded up to 4 cells
      * (16-byte multiple); the extra cells stay inside the line's range */
     auto cells = [&](int ln, int c) { return ((min(P, ln - c * P) + 3) & ~3); };
-    auto issue = [&](int job, int s) {
+    auto issue = [&](int job, int s, bool blocks = true, bool vecs = true) {
         unsigned char *base = st0 + (size_t)s * stage;
         uint32_t bytes = 0;
         if (job < nf) {
@@ -1679,7 +1692,7 @@ __device__ __forceinline__ bool thomas_line(
             if (nchT - 1 - jb >= 0) bytes += cells(m, nchT - 1 - jb) * bw * sizeof(T);
             if (nchB - 1 - jb >= 0) bytes += cells(nb, nchB - 1 - jb) * bw * sizeof(T);
         }
-        mbar_arrive_expect_tx(&bars[s], bytes);
+        if (blocks) mbar_arrive_expect_tx(&bars[s], bytes);
         for (int hh = 0; hh < 2; ++hh) {
             const int ln = hh ? nb : m, nc = hh ? nchB : nchT, cp = hh ? m : 0;
             unsigned char *hb = base + hh * half;
@@ -1687,10 +1700,12 @@ __device__ __forceinline__ bool thomas_line(
                 const int c = job;
                 if (c >= nc) continue;
                 const int cnt = cells(ln, c);
-                bulk_g2s_hint(hb, G + (size_t)(ps + cp + c * P) * NB, cnt * NB * sizeof(T), &bars[s], pol);
-                bulk_g2s(hb + P * NB * sizeof(T), b + (size_t)(ps + cp + c * P) * NV, cnt * NV * sizeof(T),
-                         &bars[s]);
-            } else {
+                if (blocks)
+                    bulk_g2s_hint(hb, G + (size_t)(ps + cp + c * P) * NB, cnt * NB * sizeof(T), &bars[s], pol);
+                if (vecs)
+                    bulk_g2s(hb + P * NB * sizeof(T), b + (size_t)(ps + cp + c * P) * NV, cnt * NV * sizeof(T),
+                             &bars[s]);
+            } else if (blocks) {
                 const int c = nc - 1 - (job - nf);
                 if (c < 0) continue;
                 const int cnt = cells(ln, c);
@@ -1727,6 +1742,16 @@ __device__ __forceinline__ bool thomas_line(
     if (producer) {
         /* every job as soon as the consumer has released its stage: job
          * j >= NS waits for the consumption of job j - NS */
+        if (PH == PH_BLOCKS || PH == PH_VECS || PH == PH_DROP) {
+            if (lane == 0)
+                for (int job = 0; job < NS && job < njobs; ++job) {
+                    if (PH == PH_DROP)
+                        mbar_wait(&bars[job], (pbase >> job) & 1u, 1LL << 28);
+                    else
+                        issue(job, job, PH == PH_BLOCKS, PH == PH_VECS);
+                }
+            return true;
+        }
         if (lane == 0) {
             RingPos r, e; /* e: the consumed job's place, NS jobs behind */
             for (int job = 0; job < njobs; ++job) {
@@ -1738,13 +1763,13 @@ __device__ __forceinline__ bool thomas_line(
                     }
                     e.next(NS);
                 }
-                issue(job, r.s);
+                if (PH == PH_ALL || job >= NS) issue(job, r.s);
                 r.next(NS);
                 *ws_issued = job + 1;
             }
         }
         __syncwarp();
-        __syncthreads(); /* meets the consumer's */
+        ws_meet();
         close_phases();
         return true;
     }
@@ -1820,7 +1845,7 @@ __device__ __forceinline__ bool thomas_line(
         if (lane < NV) {
             const T *gr = G + (size_t)(ps + ptw) * NB + lane;
             const T *cr = Gam + (size_t)(ps + ptw) * NB + lane;
-            T acc = b[(size_t)(ps + ptw) * NV + lane];
+            T acc = __ldcg(b + (size_t)(ps + ptw) * NV + lane);
 #pragma unroll
             for (int j = 0; j < NV; ++j) acc -= gr[NV * j] * ytop[j] + cr[NV * j] * ybot[j];
             xm = acc;
@@ -1898,6 +1923,11 @@ __device__ __forceinline__ bool thomas_line(
             __syncwarp();
             if (lane == 0 && nbulk > 0) {
                 bulk_s2g(dUl, ys, nbulk * sizeof(T));
+                if (drain) {
+                    bulk_s2g_commit();
+                    /* an earlier line's add to U is complete: the older group */
+                    bulk_s2g_wait_but<1>();
+                }
                 if (accumulate == 0) bulk_s2g(Ul, ys, nbulk * sizeof(T));
                 if (accumulate == 1 && ub) bulk_add_s2g(Ul, ys, nbulk * sizeof(T));
                 bulk_s2g_commit();
@@ -1908,7 +1938,7 @@ __device__ __forceinline__ bool thomas_line(
 #pragma unroll
                 for (int k = 0; k < B; ++k) {
                     const int t = t0 + 32 * k;
-                    u[k] = (accumulate == 1 && t < nv) ? Uil[t] : T(0);
+                    u[k] = (accumulate == 1 && t < nv) ? __ldcg(Uil + t) : T(0);
                 }
 #pragma unroll
                 for (int k = 0; k < B; ++k) {
@@ -1920,7 +1950,10 @@ __device__ __forceinline__ bool thomas_line(
                     }
                 }
             }
-            if (lane == 0 && nbulk > 0) bulk_s2g_wait_read(); /* before the CTA's memory goes */
+            if (lane == 0 && nbulk > 0) {
+                if (drain) bulk_s2g_wait_but<1>(); /* dU */
+                bulk_s2g_wait_read(); /* before the CTA's memory goes */
+            }
             __syncwarp();
         }
     }
@@ -1930,7 +1963,7 @@ __device__ __forceinline__ bool thomas_line(
              * the copies it issued */
             if (lane == 0) *ws_abort = 1;
             __syncwarp();
-            __syncthreads();
+            ws_meet();
             issued = *ws_issued;
         }
         if (lane == 0) {
@@ -1944,7 +1977,7 @@ __device__ __forceinline__ bool thomas_line(
         __syncwarp();
         return false;
     }
-    if (WS) __syncthreads(); /* meets the producer's */
+    if (WS) ws_meet();
     close_phases();
     return true;
 }
@@ -2229,6 +2262,353 @@ int fast_prepare(const FastLayout &L) {
     if (!rc) rc = set_smem(thomas_fn<double, true>(w64.ys), w64.smem);
     if (!rc) rc = set_smem(thomas_fn<float, true>(w32.ys), w32.smem);
     return rc;
+}
+
+/* ==================================================== many sweeps, one launch
+ * TBS_ALGO_FP64 sweeps of a system of few lines as one cooperative launch: a
+ * CTA per line (and more, to share the tiles), per sweep
+ *   line solves (warps 0 and 1, thomas_line's warp-specialised form)
+ *   -- all CTAs meet --
+ *   residual tiles (mode 1 of fast_resid_body: same operations and order),
+ *   each CTA's first tiles' blocks copied before the meeting
+ *   -- all CTAs meet --
+ *   every CTA adds the tiles' partials (finalize_total's order) and decides
+ * until the tolerance, the sweep limit or a norm that is not finite.  The
+ * results, the history and the decisions are those of the launches per sweep,
+ * bit for bit.
+ * What it saves is what bounds a small system: two launches' start and end
+ * and the graph's loop and condition nodes, about 11 us a sweep, against two
+ * meetings of 1.2 us (60x64: 28 us a sweep before).  Vectors that other CTAs
+ * wrote are read past the L1; what bulk copies read or wrote is fenced from
+ * the ordinary accesses. */
+constexpr int SMALL_THREADS = RES_THREADS_FAST;
+constexpr int SMALL_NS = 6;   /* ring stages of the line solve; two residual tiles lie in the ring */
+constexpr int SMALL_HDR = 256;
+constexpr int MEETS = 8, MEET_STRIDE = SMALL_MEET_WORDS / (MEETS + 1);
+
+struct SmallSweeps {
+    int nline, nx, np16, max_len;
+    const int *line_start, *line_len, *line_twist, *xnbr;
+    const double *G, *Gam, *Dinv, *X;
+    double *b, *y, *dU, *U, *partials, *hist;
+    SolveState *state;
+    unsigned *meet; /* MEETS counts of arrivals, one of CTAs that are done; zero between launches */
+    unsigned *status;
+    unsigned long long *timer;
+    unsigned long long loop, check; /* condition handles */
+    int use_check;
+    int keep; /* the blocks fit in the L2 and are read to stay there */
+};
+
+static size_t small_smem(const FastLayout &L) {
+    return SMALL_HDR + SMALL_NS * (size_t)thomas_stage_bytes<double>() + BCAST<double> * sizeof(double) +
+           (size_t)((L.max_len + 3) & ~3) * NV * sizeof(double) +
+           (size_t)(L.nx + 2) * RES_TILE * NV * sizeof(double);
+}
+
+/* tiles whose blocks fit in the ring at once */
+__host__ __device__ inline int small_bufs(int nx) {
+    return (int)(SMALL_NS * 2 * THOMAS_P * (NB + NV) * sizeof(double)) / ((1 + nx) * RES_TILE * NB * 8) >= 2 ? 2 : 1;
+}
+
+__global__ void __launch_bounds__(SMALL_THREADS, 2) small_sweeps_kernel(SmallSweeps A) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int nx = A.nx, np16 = A.np16, ntiles = np16 / RES_TILE, nbuf = small_bufs(nx);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
+    uint64_t *rbar = bars + 18; /* behind thomas_line's two counters */
+    volatile int *s_ok = reinterpret_cast<volatile int *>(smem + 160);
+    double *red = reinterpret_cast<double *>(smem + 168); /* one per warp, then the norm */
+    unsigned char *ring = smem + SMALL_HDR;
+    double *aux = reinterpret_cast<double *>(ring + SMALL_NS * thomas_stage_bytes<double>()) + BCAST<double> +
+                  ((A.max_len + 3) & ~3) * NV;
+    double *sg = aux, *sr = aux + nx * RES_TILE * NV, *sb = sr + RES_TILE * NV;
+    if (tid == 0) {
+        for (int s = 0; s < SMALL_NS; ++s) {
+            mbar_init(&bars[s], 1);
+            mbar_init(&bars[8 + s], 1);
+        }
+        mbar_init(&rbar[0], 1);
+        mbar_init(&rbar[1], 1);
+        int *cnt = reinterpret_cast<int *>(smem + 128);
+        cnt[0] = 0;
+        cnt[1] = 0;
+        mbar_fence_init();
+    }
+    __syncthreads();
+    const SolveState *S = A.state;
+    const double norm0 = S->norm0, tol = S->tol;
+    const int max_sweeps = S->max_sweeps, hist_cap = S->hist_cap;
+    int sw = S->sweep;
+    double nrm = 0.0;
+    bool met = false, ok = true;
+    const bool mine = (int)blockIdx.x < A.nline;
+    const int ls = mine ? A.line_start[blockIdx.x] : 0, ll = mine ? A.line_len[blockIdx.x] : 0,
+              lt = mine ? A.line_twist[blockIdx.x] : 0;
+    const uint64_t pol = A.keep ? policy_evict_last() : policy_evict_first();
+    uint32_t pbase = 0, rpar = 0;
+    unsigned round = 0;
+    const int c = tid % RES_TILE, i = tid / RES_TILE;
+    const bool act = tid < RES_TILE * NV;
+    const uint32_t szD = RES_TILE * NB * sizeof(double);
+    /* all CTAs; false when one of them did not come in time.  The arrivals are
+     * spread over MEETS words, each watched by a lane of warp 0; warp 1 does
+     * `meanwhile` once the CTA has arrived */
+    auto meet = [&](auto &&meanwhile) {
+        __syncthreads();
+        if (warp == 0) {
+            ++round;
+            if (tid == 0) {
+                __threadfence();
+                atomicAdd(A.meet + MEET_STRIDE * (blockIdx.x % MEETS), 1u);
+            }
+            bool here = true;
+            if (tid < MEETS) {
+                const unsigned target = round * ((gridDim.x - tid + MEETS - 1) / MEETS);
+                const long long t0 = clock64();
+                while ((int)(ld_acquire(A.meet + MEET_STRIDE * tid) - target) < 0) {
+                    if (clock64() - t0 > (1LL << 31)) {
+                        here = false;
+                        break;
+                    }
+                }
+            }
+            here = __all_sync(FULL, here);
+            if (tid == 0) *s_ok = here ? 1 : 0;
+        } else if (warp == 1) {
+            meanwhile();
+        }
+        __syncthreads();
+        return *s_ok != 0;
+    };
+    auto tile_of = [&](int k) { return (int)blockIdx.x + k * (int)gridDim.x; };
+    auto blocks = [&](int k) { return reinterpret_cast<double *>(ring) + (size_t)(k % nbuf) * (1 + nx) * RES_TILE * NB; };
+    auto issue = [&](int k) { /* thread 0: the k-th tile's blocks */
+        const int p0 = tile_of(k) * RES_TILE;
+        if (tile_of(k) >= ntiles) return;
+        uint64_t *bar = &rbar[k % nbuf];
+        double *d = blocks(k);
+        mbar_arrive_expect_tx(bar, (1 + nx) * szD);
+        bulk_g2s_hint(d, A.Dinv + (size_t)p0 * NB, szD, bar, pol);
+        for (int s = 0; s < nx; ++s)
+            bulk_g2s_hint(d + (1 + s) * RES_TILE * NB, A.X + ((size_t)s * np16 + p0) * NB, szD, bar, pol);
+    };
+    /* the neighbours of this thread's cell of the k-th tile, and their dU */
+    auto neighbours = [&](int k, int (&nb)[4]) {
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+            nb[s] = (act && s < nx && tile_of(k) < ntiles) ? A.xnbr[(size_t)s * np16 + tile_of(k) * RES_TILE + c] : -1;
+    };
+    auto gather = [&](const int (&nb)[4], double (&g)[4]) {
+#pragma unroll
+        for (int s = 0; s < 4; ++s) g[s] = nb[s] >= 0 ? __ldcg(A.dU + (size_t)nb[s] * NV + i) : 0.0;
+    };
+    /* the sums of the partials that threads 32 v .. 32 v + 31 (and 32 v1 ..)
+     * of finalize_total would make, loads of both in flight together */
+    auto norm_part = [&](int v, int v1) {
+        constexpr int B = 6;
+        double acc[2] = {0.0, 0.0};
+        const int q0 = 32 * v + (tid & 31), d = 32 * (v1 - v);
+        for (int r = 0; r * SMALL_THREADS < ntiles; r += B) {
+            double x[2][B];
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                const int q = q0 + (r + k) * SMALL_THREADS;
+                x[0][k] = q < ntiles ? __ldcg(A.partials + q) : 0.0;
+                x[1][k] = d > 0 && q + d < ntiles ? __ldcg(A.partials + q + d) : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < B; ++k) { /* sums of squares: adding 0.0 changes none */
+                acc[0] += x[0][k];
+                acc[1] += x[1][k];
+            }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            acc[0] += __shfl_down_sync(FULL, acc[0], o);
+            acc[1] += __shfl_down_sync(FULL, acc[1], o);
+        }
+        if ((tid & 31) == 0) {
+            red[v] = acc[0];
+            if (d > 0) red[v1] = acc[1];
+        }
+    };
+    static_assert(SMALL_THREADS == 160, "the counts of barriers 2 and 3");
+    auto line = [&](auto phase) {
+        return thomas_line<double, THOMAS_P, true, true, decltype(phase)::value>(
+            SMALL_NS, 1, ls, ll, lt, A.G, A.Gam, A.b, A.y, A.dU, A.U, A.status, smem, pbase, pol, nullptr, true);
+    };
+    /* b, as the others stored it, for this warp's bulk copies */
+    auto start_vecs = [&]() {
+        if (tid == 32) fence_async_all();
+        line(std::integral_constant<int, PH_VECS>{});
+    };
+    int nb0[4], nb1[4]; /* the first two tiles' neighbours, the same in every sweep */
+    neighbours(0, nb0);
+    neighbours(1, nb1);
+    if (mine && warp == 1) {
+        line(std::integral_constant<int, PH_BLOCKS>{});
+        start_vecs();
+    }
+    for (;;) {
+        /* ---------------- line solves */
+        if (mine && warp < 2) ok = line(std::integral_constant<int, PH_RUN>{});
+        ok = __syncthreads_and(ok); /* the ring is free */
+        if (!ok) break;
+        if (tid == 0)
+            for (int k = 0; k < nbuf; ++k) issue(k);
+        const bool came = meet([]() {});
+        unsigned long long t0 = 0;
+        if (A.timer && blockIdx.x == 0 && tid == 0) t0 = globaltimer_ns();
+        /* ---------------- residual: R = sum X dU, b = -Dinv R; the next tile's
+         * neighbours' dU is read while a tile is worked on */
+        double g[4], gn[4];
+        int nn[4];
+        gather(nb0, g);
+        for (int k = 0; ok && tile_of(k) < ntiles; ++k) {
+            const int blk = tile_of(k), p0 = blk * RES_TILE;
+            if (act) {
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+                    if (s < nx) sg[(s * RES_TILE + c) * NV + i] = g[s];
+            }
+            if (k == 0)
+                gather(nb1, gn);
+            else
+                gather(nn, gn);
+            neighbours(k + 2, nn);
+            const bool landed = mbar_wait(&rbar[k % nbuf], (rpar >> (k % nbuf)) & 1u);
+            rpar ^= 1u << (k % nbuf);
+            if (__syncthreads_or(!landed)) {
+                if (tid == 0)
+                    for (int q = k; q < k + nbuf; ++q) /* let the copies land before the CTA retires */
+                        if (tile_of(q) < ntiles)
+                            mbar_wait(&rbar[q % nbuf], ((rpar >> (q % nbuf)) & 1u) ^ (q == k ? 1u : 0u), 1LL << 28);
+                ok = false;
+                break;
+            }
+            const double *sD = blocks(k), *sX = sD + RES_TILE * NB;
+            double r = 0.0;
+            if (act) {
+                double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+                for (int s = 0; s < nx; ++s) {
+                    const double *xr = sX + (s * RES_TILE + c) * NB + i;
+                    const double *q = sg + (s * RES_TILE + c) * NV;
+                    a0 += xr[0] * q[0];
+                    a1 += xr[9] * q[1];
+                    a2 += xr[18] * q[2];
+                    a0 += xr[27] * q[3];
+                    a1 += xr[36] * q[4];
+                    a2 += xr[45] * q[5];
+                    a0 += xr[54] * q[6];
+                    a1 += xr[63] * q[7];
+                    a2 += xr[72] * q[8];
+                }
+                r = a0 + (a1 + a2);
+                sr[c * NV + i] = r;
+            }
+            __syncthreads();
+            double sq = act ? r * r : 0.0;
+            if (act) sb[c * NV + i] = neg_dinv_row<double>(sD + c * NB + i, sr + c * NV);
+            for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(FULL, sq, o);
+            if ((tid & 31) == 0) red[warp] = sq;
+            __syncthreads();
+            if (act) A.b[(size_t)p0 * NV + tid] = sb[tid];
+            if (tid == 0) {
+                double tot = 0.0;
+                for (int w = 0; w < SMALL_THREADS / 32; ++w) tot += red[w];
+                A.partials[blk] = tot;
+                issue(k + nbuf); /* every thread is done with this buffer */
+            }
+            /* red, sg, sr and sb are next written behind another barrier */
+#pragma unroll
+            for (int s = 0; s < 4; ++s) g[s] = gn[s];
+        }
+        if (!ok) break;
+        /* the next solves' first blocks go into the ring, which is free again;
+         * their b follows the meeting and lands under the norm */
+        ok = meet([&]() {
+                 if (mine) line(std::integral_constant<int, PH_BLOCKS>{});
+             }) && came;
+        bool more = false;
+        if (ok) {
+            if (A.timer && blockIdx.x == 0 && tid == 0) {
+                atomicAdd(A.timer + 1, globaltimer_ns() - t0);
+                atomicAdd(A.timer + 2, 1ull);
+            }
+            /* ---------------- the norm, by every CTA: warp 1 starts the copies
+             * of b, the others add the partials in finalize_total's order
+             * (that of SMALL_THREADS threads, warp 0 taking warp 1's part too) */
+            if (warp == 1) {
+                if (mine) start_vecs();
+                asm volatile("bar.sync 3, 160;" ::: "memory");
+            } else {
+                norm_part(warp, warp == 0 ? 1 : warp);
+                asm volatile("bar.arrive 3, 160;" ::: "memory");
+                asm volatile("bar.sync 2, 128;" ::: "memory");
+            }
+            double tot = 0.0;
+            for (int w = 0; w < SMALL_THREADS / 32; ++w) tot += red[w];
+            nrm = sqrt(tot);
+            ++sw;
+            if (blockIdx.x == 0 && tid == 0 && sw < hist_cap) A.hist[sw] = nrm;
+            met = isfinite(nrm) && nrm <= tol * norm0;
+            more = isfinite(nrm) && !met && sw < max_sweeps;
+        }
+        if (!more) {
+            if (mine && warp == 1) {
+                if (!ok) start_vecs(); /* the copies that the barriers count on */
+                line(std::integral_constant<int, PH_DROP>{});
+            }
+            break;
+        }
+    }
+    if (!ok && tid == 0) atomicOr(A.status, ST_TIMEOUT);
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        if (atomicAdd(A.meet + MEET_STRIDE * MEETS, 1u) == gridDim.x - 1) {
+            /* every CTA has left the meetings */
+            for (int k = 0; k <= MEETS; ++k) A.meet[MEET_STRIDE * k] = 0u;
+            A.state->sweep = sw;
+            A.state->last = nrm;
+            cudaGraphSetConditional((cudaGraphConditionalHandle)A.loop, 0u);
+            if (A.use_check) cudaGraphSetConditional((cudaGraphConditionalHandle)A.check, ok && met ? 1u : 0u);
+        }
+    }
+}
+
+/* CTAs of a launch of all sweeps; 0: the system is not for it */
+int small_sweeps_grid(const FastLayout &L) {
+    if (L.nv != NV || L.nx < 1 || L.nx > 4) return 0;
+    const size_t smem = small_smem(L);
+    if ((long long)smem > smem_limit((const void *)small_sweeps_kernel)) return 0;
+    if (smem_raise((const void *)small_sweeps_kernel, smem)) return 0;
+    int per = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void *)small_sweeps_kernel, SMALL_THREADS,
+                                                      smem) != cudaSuccess)
+        return 0;
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const int cap = std::min(per, 2) * nsm;
+    if (L.nline > cap) return 0;
+    const int ntiles = L.np16 / RES_TILE;
+    return std::max(L.nline, std::min(ntiles, cap));
+}
+
+int launch_small_sweeps(cudaStream_t st, const FastLayout &L, const double *G, const double *Gam,
+                        const double *Dinv, const double *X, double *b, double *y, double *dU, double *U,
+                        const NormSink &ns, unsigned *meet, unsigned *status) {
+    const int grid = small_sweeps_grid(L);
+    if (grid < 1) return (int)cudaErrorInvalidValue;
+    SmallSweeps A{L.nline,  L.nx, L.np16, L.max_len, L.line_start, L.line_len, L.line_twist, L.xnbr,
+                  G,        Gam,  Dinv,   X,         b,            y,          dU,           U,
+                  ns.partials, ns.hist, ns.state, meet, status, ns.timer, ns.handle, ns.check_handle,
+                  ns.use_check,
+                  (long long)L.np16 * (3 + L.nx) * NB * (long long)sizeof(double) <= (96LL << 20)};
+    void *args[] = {&A};
+    return (int)cudaLaunchCooperativeKernel((const void *)small_sweeps_kernel, dim3(grid), dim3(SMALL_THREADS),
+                                            args, small_smem(L), st);
 }
 
 int fast_kernels_init() { return 0; }

@@ -210,6 +210,14 @@ template <typename T>
 int launch_fast_thomas(cudaStream_t st, const FastLayout &L, const T *G, const T *Gam,
                        const T *b, T *y, T *dU, T *U, unsigned *status, int accumulate,
                        int nacc = -1, const T *Uin = nullptr);
+/* all the sweeps of a solve of few lines as one cooperative launch: the grid
+ * it takes (0: not for this system), and the launch.  `ns` gives the norms'
+ * places and the graph's conditions; meet: SMALL_MEET_WORDS words, zero. */
+constexpr int SMALL_MEET_WORDS = 9 * 64;
+int small_sweeps_grid(const FastLayout &L);
+int launch_small_sweeps(cudaStream_t st, const FastLayout &L, const double *G, const double *Gam,
+                        const double *Dinv, const double *X, double *b, double *y, double *dU, double *U,
+                        const NormSink &ns, unsigned *meet, unsigned *status);
 int fast_kernels_init();
 /* Several lines' vectors packed into (or unpacked from) one contiguous
  * buffer by one launch: line k's span is [start[k]*9, start[k]*9 + len[k]*9)

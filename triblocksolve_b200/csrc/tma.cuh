@@ -170,6 +170,20 @@ __device__ __forceinline__ void bulk_add_s2g(void *dst, const void *src, uint32_
 __device__ __forceinline__ void bulk_s2g_commit() {
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
+/* all but the newest N of this thread's committed groups are complete: read,
+ * and written */
+template <int N>
+__device__ __forceinline__ void bulk_s2g_wait_but() {
+    asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
+}
+/* this thread's ordinary accesses (and those it has seen) before its bulk
+ * copies that follow, and the other way round */
+__device__ __forceinline__ void fence_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
+__device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 /* the shared memory of this thread's committed groups has been read */
 __device__ __forceinline__ void bulk_s2g_wait_read() {
     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
