@@ -737,7 +737,6 @@ static int check_residual(tbs_ctx *ctx, CondCtl cc) {
         RUN("permute", launch_permute_to_elem(st, nv, ne, L.pos_of_elem, ctx->d_Up, ctx->d_U));
         int rc = ref_residual(ctx, ctx->d_U, ctx->d_R, &np);
         if (rc) return rc;
-        RUN("permute", launch_permute_to_pos(st, nv, ne, L.pos_of_elem, ctx->d_R, ctx->d_Rp));
     }
     RUN("reduce_norm", launch_reduce_norm(st, ctx->d_partials2, np, ctx->d_state, ctx->d_hist,
                                           NORM_CHECK, cc.handle, cc.use_cond, cc.handle2, cc.use2));
@@ -746,6 +745,9 @@ static int check_residual(tbs_ctx *ctx, CondCtl cc) {
 
 /* b = -Dinv R of the true residual, for the sweeps after a failed check */
 static int check_restart(tbs_ctx *ctx) {
+    if (ctx->nvar != 9) /* the general residual is in element order */
+        RUN("permute", launch_permute_to_pos(ctx->stream, ctx->nvar, ctx->nelem, ctx->L.pos_of_elem, ctx->d_R,
+                                             ctx->d_Rp));
     RUN("fast_resid_check", resid64(ctx, 0, ctx->d_dUp, ctx->d_Rp, ctx->d_b, no_sink(), nullptr));
     return TBS_OK;
 }

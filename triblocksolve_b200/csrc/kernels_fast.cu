@@ -22,6 +22,7 @@
  */
 #include "device_common.cuh"
 #include "tbs_internal.hxx"
+#include "thomas.cuh"
 #include "tma.cuh"
 
 #include <cuda_runtime.h>
@@ -1376,620 +1377,11 @@ template int launch_fast_resid<float>(cudaStream_t, const FastLayout &, int, con
                                       const NormSink &, unsigned *, float *, int, const float *);
 
 /* =========================================================== line Thomas
- * One warp per line, twisted: lanes 0..8 run the top chain and lanes
- * 16..24 the bottom chain of the line with the same instruction stream, so
- * a line of n cells takes n+1 dependent steps instead of 2n.  Lane 0 (or a
- * copy warp) streams "jobs" through an NS-stage bulk-copy ring, each stage
- * holding one chunk of P cells per chain: jobs 0..nf-1 forward chunks (G
- * blocks and b), jobs nf..2nf-1 backward chunks in reverse (Gam blocks).
- * Chain forward:  y_s = b_s - G_s y_{s-1};  twist:  x_m = b_m - G_tw y_top
- * - Gam_tw y_bot;  chain backward:  x_s = y_s - Gam_s x_{s+1} (s+1 toward
- * the twist).
- *
- * What bounds it where few lines share an SM is the step: publish the
- * 9-vector in shared memory, read it back, a 9-term dot product.  On a warp
- * alone, rows held in registers, that is 86 cycles; so everything else is
- * kept off the chain.  Lane i owns row i; the row of the NEXT cell is read
- * into registers behind the current step's vector reads, across chunk
- * boundaries too: the next chunk's barrier is tested early in a chunk and
- * the result looked at a few steps later (testing it between chunks and
- * reading the row after it cost about 300 cycles per 8-cell chunk).  The
- * blocks are column-major, so that the nine lanes read a column of nine
- * neighbouring words: no bank conflicts and one copy of the vector (with
- * row-major blocks: two copies, lane-dependent offsets, 122 cycles a step
- * against 106; rows as aligned pairs of columns: 111).  Two partial sums,
- * since the vector's words arrive one after the other: the last one is two
- * operations from the result (three sums: 115 cycles).
- * YS: the line's y and x live in shared memory, and dU / U are written after
- * the line is solved: dU by one bulk copy, and in FP64 U += dU by one bulk
- * add (the L2 adds, so the warp does not wait for U); otherwise y goes to
- * global memory (read back one chunk ahead) and dU / U per step, U read
- * one chunk ahead with y (one-warp form) or staged behind the backward
- * chunk's Gam blocks by the copy warp (warp-specialised form).
- *   accumulate = 0:  U = dU
- *   accumulate = 1:  U += dU (the FP64 sweeps of a context; U read from a
- *                    second buffer Uin when one is given: line partitions)
- *   accumulate = 2:  U untouched (the residual kernel that follows adds
- *                    dU to U for its tile, with coalesced tile accesses:
- *                    the batch engine)
- */
+ * thomas.cuh holds the line solve; here are its launches at block size 9. */
 constexpr int THOMAS_P = 8;
 
 template <typename T>
-__host__ __device__ inline uint32_t thomas_half_bytes() {
-    return (uint32_t)(THOMAS_P * (NB + NV) * sizeof(T));
-}
-template <typename T>
-__host__ __device__ inline uint32_t thomas_stage_bytes() {
-    return 2 * thomas_half_bytes<T>();
-}
-
-/* The vector a step reads and the row it multiplies.
- * FP64: lane i's row in column order, and one copy of the vector read as
- * four pairs and a single (two partial sums, see above).
- * FP32: the vector in two copies (y_j at j and at 11 + j), so that a lane
- * whose row number and cell have different parity starts its pairs at
- * column 1; the order of the sum by lane is kept as it was first written,
- * since the outer refinement's history shows a change of FP32 rounding. */
-template <typename T> struct StepVec;
-
-template <>
-struct StepVec<double> {
-    static constexpr int BUF = 10; /* words of one buffer */
-    double2 p[4];
-    double s;
-    __device__ __forceinline__ void load(const double *v, int, int) {
-        const double2 *q = reinterpret_cast<const double2 *>(v);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) p[c] = q[c];
-        s = v[8];
-    }
-    static __device__ __forceinline__ void put(double *buf, int i, double y) { buf[i] = y; }
-};
-
-template <>
-struct StepVec<float> {
-    static constexpr int BUF = 20;
-    float2 p[4];
-    float s;
-    __device__ __forceinline__ void load(const float *v, int i, int odd) {
-        const int par = (i + odd) & 1;
-        const float2 *q = reinterpret_cast<const float2 *>(v + (par ? 12 : 0));
-#pragma unroll
-        for (int c = 0; c < 4; ++c) p[c] = q[c];
-        s = v[par ? 0 : 8];
-    }
-    static __device__ __forceinline__ void put(float *buf, int i, float y) {
-        buf[i] = y;
-        buf[11 + i] = y;
-    }
-};
-
-/* row i of a block, in the order StepVec gives the vector: FP64 columns
- * 0..8; FP32 the single's column, then the pairs' */
-template <typename T>
-struct Row {
-    T r[NV];
-};
-
-__device__ __forceinline__ void load_row(Row<double> &R, const double *blk, int i, int) {
-#pragma unroll
-    for (int j = 0; j < NV; ++j) R.r[j] = blk[NV * j + i];
-}
-
-__device__ __forceinline__ void load_row(Row<float> &R, const float *blk, int i, int odd) {
-    const int par = (i + odd) & 1;
-    const float *q = blk + i - (par ? 0 : NV);
-    R.r[0] = blk[par ? i : 8 * NV + i];
-#pragma unroll
-    for (int j = 1; j < NV; ++j) R.r[j] = q[NV * j];
-}
-
-/* init - row . vec */
-__device__ __forceinline__ double row_dot(const Row<double> &R, const StepVec<double> &V, double init) {
-    double a0 = init - R.r[0] * V.p[0].x;
-    double a1 = R.r[1] * V.p[0].y;
-#pragma unroll
-    for (int c = 1; c < 4; ++c) {
-        a0 -= R.r[2 * c] * V.p[c].x;
-        a1 += R.r[2 * c + 1] * V.p[c].y;
-    }
-    a0 -= R.r[8] * V.s;
-    return a0 - a1;
-}
-
-__device__ __forceinline__ float row_dot(const Row<float> &R, const StepVec<float> &V, float init) {
-    float a0 = init - R.r[0] * V.s;
-    float a1 = R.r[1] * V.p[0].x;
-    float a2 = R.r[2] * V.p[0].y;
-    a0 -= R.r[3] * V.p[1].x;
-    a1 += R.r[4] * V.p[1].y;
-    a2 += R.r[5] * V.p[2].x;
-    a0 -= R.r[6] * V.p[2].y;
-    a1 += R.r[7] * V.p[3].x;
-    a2 += R.r[8] * V.p[3].y;
-    return a0 - (a1 + a2);
-}
-
-/* words of the broadcast vectors: 2 halves x 2 alternating buffers */
-template <typename T>
-constexpr int BCAST = 4 * StepVec<T>::BUF;
-
-/* Forward steps kbase..kbase+P-1 of this half's chain (length len, first
- * position cpos relative to the line start), the chunk's blocks at sG and
- * its b behind them; `row` / `bi` hold the first cell's row and b, and are
- * left holding those of the next chunk, whose stage next() gives (null:
- * none; probe() has asked for it).  CHECK: some steps of the warp may lie
- * beyond one chain's end; those compute but write nothing. */
-template <typename T, int P, bool CHECK, bool YS, typename Probe, typename Next>
-__device__ __forceinline__ void fwd_chunk(const T *sG, Row<T> &row, T &bi, T *bc, T *ys, T *yg,
-                                          int kbase, int len, int cpos, int i, uint64_t ypol,
-                                          Probe &&probe, Next &&next) {
-    constexpr int VB = StepVec<T>::BUF;
-    const T *sB = sG + P * NB;
-    const T *sN = sG;
-#pragma unroll
-    for (int q = 0; q < P; ++q) {
-        Row<T> nrow;
-        StepVec<T> v;
-        T nb = T(0);
-        v.load(bc + (q & 1) * VB, i, q & 1);
-        if (q + 1 < P) {
-            load_row(nrow, sG + (q + 1) * NB, i, (q + 1) & 1);
-            nb = sB[(q + 1) * NV + i];
-        } else { /* no next chunk: some cell of this one, not used */
-            load_row(nrow, sN, i, 0);
-            nb = sN[P * NB + i];
-        }
-        if (q == 1) probe();
-        if (q == P - 3) {
-            const T *n = next();
-            if (n) sN = n;
-        }
-        const T yi = row_dot(row, v, bi);
-        /* lanes 9..15 of a half compute row 8 from the same inputs as lane
-         * 8 and store the same value to the same address: no divergence */
-        if (!CHECK || kbase + q < len) {
-            StepVec<T>::put(bc + ((q & 1) ^ 1) * VB, i, yi);
-            const int pos = cpos + kbase + q;
-            if (YS)
-                ys[pos * NV + i] = yi;
-            else /* kept in L2 for the backward chain (the blocks stream evict-first) */
-                st_hint(yg + (size_t)pos * NV + i, yi, ypol);
-        }
-        __syncwarp();
-        row = nrow;
-        bi = nb;
-    }
-}
-
-/* Backward steps kbase+P-1..kbase, `row` holding the row of the first of
- * them (and left holding the next chunk's).  YS: y and x in ys, `yk` the y
- * of the first step, left holding the next chunk's; otherwise the chunk's
- * y in yv.  uv: U of the chunk's cells read ahead in registers, or sU (when
- * set): the chunk's U staged behind its Gam blocks */
-template <typename T, int P, bool CHECK, bool YS, typename Probe, typename Next>
-__device__ __forceinline__ void bwd_chunk(const T *sG, Row<T> &row, T &yk, T *bc, T *ys, const T *yv,
-                                          const T *uv, T *dUl, T *Ul, int kbase, int len, int cpos,
-                                          int i, const T *sU, Probe &&probe, Next &&next) {
-    constexpr int VB = StepVec<T>::BUF;
-    const T *sN = sG;
-#pragma unroll
-    for (int q = P - 1; q >= 0; --q) {
-        const int f = (P - 1 - q) & 1; /* buffer alternates per step */
-        Row<T> nrow;
-        StepVec<T> v;
-        v.load(bc + f * VB, i, q & 1);
-        load_row(nrow, q > 0 ? sG + (q - 1) * NB : sN + (P - 1) * NB, i, (q + P - 1) & 1);
-        if (q == P - 2) probe();
-        if (q == 2) {
-            const T *n = next();
-            if (n) sN = n;
-        }
-        const int k = kbase + q;
-        const bool valid = !CHECK || (k >= 0 && k < len);
-        const int pos = cpos + k;
-        T nyk = T(0);
-        if (YS && ((CHECK || q == 0) ? (k >= 1 && k - 1 < len) : true)) nyk = ys[(pos - 1) * NV + i];
-        const T d = row_dot(row, v, YS ? yk : (valid ? yv[q] : T(0)));
-        if (valid) { /* lanes 9..15 repeat lane 8's row, value and address */
-            StepVec<T>::put(bc + (f ^ 1) * VB, i, d);
-            if (YS) {
-                ys[pos * NV + i] = d;
-            } else {
-                dUl[(size_t)pos * NV + i] = d;
-                if (Ul) Ul[(size_t)pos * NV + i] = (sU ? sU[q * NV + i] : uv[q]) + d;
-            }
-        }
-        __syncwarp();
-        row = nrow;
-        yk = nyk;
-    }
-}
-
-/* Solve one line (start ps, n cells, twist m) with the warp of the calling
- * CTA.  The staging barriers live at the start of `smem` and stay
- * initialised across the lines that a persistent CTA solves: bit s of
- * `pbase` is the parity with which barrier s completes its next phase.
- * Returns false when a staging wait ran out of time; the status bit is
- * then set and the copies in flight have landed. */
-/* bytes before the first staging buffer: the barriers (and, in the
- * warp-specialised form, the producer's counters) */
-template <bool WS>
-__host__ __device__ constexpr int thomas_hdr() { return WS ? 256 : 128; }
-
-/* the two warps of a warp-specialised line solve (the CTA may hold more) */
-__device__ __forceinline__ void ws_meet() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
-
-/* accumulate = 1 reads U from Uin when it is set (a second buffer: the
- * previous U stays intact), else from U itself.  drain (YS): dU has been
- * written when the call returns, not only read from shared memory (for kernels
- * that go on to read it), U before the next call writes it.  b and U are read
- * past the L1, which may hold an earlier sweep's. */
-/* PH 0: the whole line.  The other phases split it (WS; the copy warp's lane
- * 0 acts in all but the third): PH_BLOCKS starts the copies of the first jobs'
- * blocks, while others still write b; PH_VECS those of their b; PH_RUN is the
- * line after both; PH_DROP waits for the copies when no line follows. */
-enum { PH_ALL = 0, PH_BLOCKS, PH_VECS, PH_RUN, PH_DROP };
-
-template <typename T, int P, bool YS, bool WS = false, int PH = PH_ALL>
-__device__ __forceinline__ bool thomas_line(
-    int NS, int accumulate, int ps, int n, int m, const T *__restrict__ G,
-    const T *__restrict__ Gam, const T *__restrict__ b, T *__restrict__ y, T *__restrict__ dU,
-    T *__restrict__ U, unsigned *status, unsigned char *smem, uint32_t &pbase, uint64_t pol,
-    const T *__restrict__ Uin = nullptr, bool drain = false) {
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
-    /* WS (warp-specialised CTA of two warps): bars[0..NS) complete when a
-     * stage's copies have landed, bars[8..8+NS) when warp 0 has consumed
-     * it; warp 1 lane 0 issues the copies, warp 0 runs the chains */
-    uint64_t *empty = bars + 8;
-    volatile int *ws_issued = reinterpret_cast<volatile int *>(smem + 128);
-    volatile int *ws_abort = ws_issued + 1;
-    const uint32_t stage = 2 * P * (NB + NV) * sizeof(T);
-    const uint32_t half = P * (NB + NV) * sizeof(T);
-    unsigned char *st0 = smem + thomas_hdr<WS>();
-    T *bcall = reinterpret_cast<T *>(st0 + (size_t)NS * stage);
-    constexpr int VB = StepVec<T>::BUF;
-    T *ys = bcall + BCAST<T>;
-    const int lane = threadIdx.x & 31;
-    const int h = lane >> 4, li = lane & 15;
-    const int i = li < NV ? li : NV - 1;
-    const int nb = n - 1 - m;
-    const int len = h ? nb : m;      /* this half's chain length */
-    const int cpos = h ? m : 0;      /* its first position, relative to ps */
-    const int nchT = (m + P - 1) / P, nchB = (nb + P - 1) / P;
-    const int nch = h ? nchB : nchT;
-    const int nf = nchT > nchB ? nchT : nchB;
-    const int njobs = 2 * nf;
-    T *bc = bcall + h * 2 * VB;
-    T *yl = y + (size_t)ps * NV;
-    T *dUl = dU + (size_t)ps * NV;
-    T *Ul = U ? U + (size_t)ps * NV : nullptr;
-    const T *Uil = Uin ? Uin + (size_t)ps * NV : Ul;
-
-    const bool producer = WS && (threadIdx.x >> 5) == 1;
-    /* warp-specialised form: the copy warp also stages U behind the
-     * backward chunks' Gam blocks (where the forward stages hold b), so the
-     * chain warp reads it from shared memory */
-    const bool stage_u = WS && !YS && accumulate == 1 && Ul != nullptr;
-    __syncwarp(); /* the previous line's readers of the stages are done */
-    if (!producer && (PH == PH_ALL || PH == PH_RUN))
-        for (int t = lane; t < BCAST<T>; t += 32) bcall[t] = T(0);
-    __syncwarp();
-
-    /* copy size of chunk c of a chain of length ln, rounded up to 4 cells
-     * (16-byte multiple); the extra cells stay inside the line's range */
-    auto cells = [&](int ln, int c) { return ((min(P, ln - c * P) + 3) & ~3); };
-    auto issue = [&](int job, int s, bool blocks = true, bool vecs = true) {
-        unsigned char *base = st0 + (size_t)s * stage;
-        uint32_t bytes = 0;
-        if (job < nf) {
-            const int c = job;
-            if (c < nchT) bytes += cells(m, c) * (NB + NV) * sizeof(T);
-            if (c < nchB) bytes += cells(nb, c) * (NB + NV) * sizeof(T);
-        } else {
-            const int jb = job - nf, bw = NB + (stage_u ? NV : 0);
-            if (nchT - 1 - jb >= 0) bytes += cells(m, nchT - 1 - jb) * bw * sizeof(T);
-            if (nchB - 1 - jb >= 0) bytes += cells(nb, nchB - 1 - jb) * bw * sizeof(T);
-        }
-        if (blocks) mbar_arrive_expect_tx(&bars[s], bytes);
-        for (int hh = 0; hh < 2; ++hh) {
-            const int ln = hh ? nb : m, nc = hh ? nchB : nchT, cp = hh ? m : 0;
-            unsigned char *hb = base + hh * half;
-            if (job < nf) {
-                const int c = job;
-                if (c >= nc) continue;
-                const int cnt = cells(ln, c);
-                if (blocks)
-                    bulk_g2s_hint(hb, G + (size_t)(ps + cp + c * P) * NB, cnt * NB * sizeof(T), &bars[s], pol);
-                if (vecs)
-                    bulk_g2s(hb + P * NB * sizeof(T), b + (size_t)(ps + cp + c * P) * NV, cnt * NV * sizeof(T),
-                             &bars[s]);
-            } else if (blocks) {
-                const int c = nc - 1 - (job - nf);
-                if (c < 0) continue;
-                const int cnt = cells(ln, c);
-                bulk_g2s_hint(hb, Gam + (size_t)(ps + cp + c * P) * NB, cnt * NB * sizeof(T), &bars[s], pol);
-                if (stage_u)
-                    bulk_g2s(hb + P * NB * sizeof(T), Uil + (size_t)(cp + c * P) * NV, cnt * NV * sizeof(T),
-                             &bars[s]);
-            }
-        }
-    };
-    /* Each full barrier completes one phase per job landed in its stage,
-     * each empty barrier one per job consumed from it: `pbase` gives the
-     * parity of the first of them (carried across lines by a persistent
-     * CTA), RingPos the rest, without divisions */
-    struct RingPos {
-        int s = 0;
-        uint32_t wrap = 0;
-        __device__ void next(int NS) {
-            if (++s == NS) {
-                s = 0;
-                wrap ^= 1u;
-            }
-        }
-    };
-    auto parity = [&](const RingPos &r) { return ((pbase >> r.s) ^ r.wrap) & 1u; };
-    /* after the line, every job was waited for: barrier s completed one
-     * phase per job j = s, s+NS, ... below njobs */
-    auto close_phases = [&]() {
-        for (int s = 0; s < NS && s < njobs; ++s) {
-            const int cnt = (njobs - 1 - s) / NS + 1;
-            pbase ^= (uint32_t)(cnt & 1) << s;
-        }
-    };
-    if (producer) {
-        /* every job as soon as the consumer has released its stage: job
-         * j >= NS waits for the consumption of job j - NS */
-        if (PH == PH_BLOCKS || PH == PH_VECS || PH == PH_DROP) {
-            if (lane == 0)
-                for (int job = 0; job < NS && job < njobs; ++job) {
-                    if (PH == PH_DROP)
-                        mbar_wait(&bars[job], (pbase >> job) & 1u, 1LL << 28);
-                    else
-                        issue(job, job, PH == PH_BLOCKS, PH == PH_VECS);
-                }
-            return true;
-        }
-        if (lane == 0) {
-            RingPos r, e; /* e: the consumed job's place, NS jobs behind */
-            for (int job = 0; job < njobs; ++job) {
-                if (*ws_abort) break;
-                if (job >= NS) {
-                    if (!mbar_wait(&empty[e.s], parity(e))) {
-                        atomicOr(status, ST_TIMEOUT);
-                        break;
-                    }
-                    e.next(NS);
-                }
-                if (PH == PH_ALL || job >= NS) issue(job, r.s);
-                r.next(NS);
-                *ws_issued = job + 1;
-            }
-        }
-        __syncwarp();
-        ws_meet();
-        close_phases();
-        return true;
-    }
-    int issued = 0;
-    if (!WS && lane == 0) {
-        for (; issued < NS && issued < njobs; ++issued) issue(issued, issued);
-    }
-    int consumed = 0; /* jobs waited for */
-    bool timed_out = false;
-    const int both_full = (m < nb ? m : nb) / P; /* jobs where both chains run P steps */
-    /* y, written by the forward chains and read once by the backward ones */
-    const uint64_t ypol_last = YS ? 0ull : policy_evict_last();
-    const uint64_t ypol_first = YS ? 0ull : policy_evict_first();
-
-    RingPos rd; /* the next job to wait for */
-    bool landed = false;
-    auto probe = [&]() { landed = mbar_test(&bars[rd.s], parity(rd)); };
-    /* the next job's stage (this half's part of it), waited for when probe()
-     * did not find it landed; null when the wait ran out of time */
-    auto take = [&]() -> const T * {
-        const T *p = reinterpret_cast<const T *>(st0 + (size_t)rd.s * stage + h * half);
-        if (__any_sync(FULL, !landed)) {
-            if (__any_sync(FULL, !mbar_wait(&bars[rd.s], parity(rd)))) {
-                timed_out = true;
-                return nullptr;
-            }
-        }
-        ++consumed;
-        rd.next(NS);
-        return p;
-    };
-    /* the stage of the chunk just finished may be refilled */
-    int rel = 0;
-    auto release = [&]() {
-        if (WS) {
-            mbar_arrive_if(&empty[rel], lane == 0);
-        } else if (lane == 0 && issued < njobs) {
-            issue(issued, rel);
-            ++issued;
-        }
-        if (++rel == NS) rel = 0;
-    };
-
-    /* ---------------- forward */
-    const T *sG = nullptr, *sN = nullptr;
-    Row<T> row;
-    T bi = T(0);
-    if (nf > 0) {
-        sG = take();
-        if (sG) {
-            load_row(row, sG, i, 0);
-            bi = sG[P * NB + i];
-        }
-    }
-    for (int c = 0; c < nf && !timed_out; ++c) {
-        auto next = [&]() -> const T * { return sN = (c + 1 < nf ? take() : nullptr); };
-        if (c < both_full)
-            fwd_chunk<T, P, false, YS>(sG, row, bi, bc, ys, yl, c * P, len, cpos, i, ypol_last, probe,
-                                       next);
-        else
-            fwd_chunk<T, P, true, YS>(sG, row, bi, bc, ys, yl, c * P, len, cpos, i, ypol_last, probe,
-                                      next);
-        release();
-        sG = sN;
-    }
-
-    if (!timed_out) {
-        /* ---------------- twist: x_m = b_m - G_tw y_top - Gam_tw y_bot */
-        const int ptw = n - 1; /* relative to ps */
-        const T *ytop = bcall + (m & 1) * VB;
-        const T *ybot = bcall + (2 + (nb & 1)) * VB;
-        T xm = T(0);
-        if (lane < NV) {
-            const T *gr = G + (size_t)(ps + ptw) * NB + lane;
-            const T *cr = Gam + (size_t)(ps + ptw) * NB + lane;
-            T acc = __ldcg(b + (size_t)(ps + ptw) * NV + lane);
-#pragma unroll
-            for (int j = 0; j < NV; ++j) acc -= gr[NV * j] * ytop[j] + cr[NV * j] * ybot[j];
-            xm = acc;
-        }
-        __syncwarp();
-        if (lane < NV) {
-            for (int t = 0; t < 4; ++t) StepVec<T>::put(bcall + t * VB, lane, xm);
-            if (YS)
-                ys[ptw * NV + lane] = xm;
-            else {
-                dUl[(size_t)ptw * NV + lane] = xm;
-                if (accumulate < 2)
-                    Ul[(size_t)ptw * NV + lane] = (accumulate ? Uil[(size_t)ptw * NV + lane] : T(0)) + xm;
-            }
-        }
-        __syncwarp();
-
-        /* ---------------- backward */
-        T yv[P], uv[P], nyv[P], nuv[P];
-        auto load_chunk = [&](int c, T *yy, T *uu) {
-#pragma unroll
-            for (int q = 0; q < P; ++q) {
-                const int k = c * P + q;
-                yy[q] = T(0);
-                uu[q] = T(0);
-                if (!YS && c >= 0 && k < len) { /* lanes 9..15: lane 8's values */
-                    yy[q] = ld_hint(yl + (size_t)(cpos + k) * NV + i, ypol_first);
-                    if (accumulate == 1 && !stage_u) uu[q] = Uil[(size_t)(cpos + k) * NV + i];
-                }
-            }
-        };
-        if (!YS) load_chunk(nch - 1, yv, uv);
-        T yk = T(0);
-        if (nf > 0) {
-            probe();
-            sG = take();
-            if (sG) load_row(row, sG + (P - 1) * NB, i, (P - 1) & 1);
-            const int k = nch * P - 1;
-            if (YS && k >= 0 && k < len) yk = ys[(cpos + k) * NV + i];
-        }
-        for (int jb = 0; jb < nf && !timed_out; ++jb) {
-            const int c = nch - 1 - jb; /* this half's chunk (may be < 0) */
-            if (!YS) load_chunk(c - 1, nyv, nuv);
-            const bool full = (nchT - 1 - jb) * P + P <= m && (nchB - 1 - jb) * P + P <= nb &&
-                              nchT - 1 - jb >= 0 && nchB - 1 - jb >= 0;
-            const T *sU = stage_u ? sG + P * NB : nullptr;
-            T *Uw = accumulate < 2 ? Ul : nullptr;
-            auto next = [&]() -> const T * { return sN = (jb + 1 < nf ? take() : nullptr); };
-            if (full)
-                bwd_chunk<T, P, false, YS>(sG, row, yk, bc, ys, yv, uv, dUl, Uw, c * P, len, cpos, i, sU,
-                                           probe, next);
-            else
-                bwd_chunk<T, P, true, YS>(sG, row, yk, bc, ys, yv, uv, dUl, Uw, c * P, len, cpos, i, sU,
-                                          probe, next);
-            release();
-            sG = sN;
-            if (!YS) {
-#pragma unroll
-                for (int q = 0; q < P; ++q) {
-                    yv[q] = nyv[q];
-                    uv[q] = nuv[q];
-                }
-            }
-        }
-        if (YS && !timed_out) {
-            /* dU = x (and U = x or U += x) for the line's n cells.  The whole
-             * groups of 4 cells (16-byte multiples) of dU go by one bulk
-             * copy, and in FP64 those of U by one bulk add (U + x rounded
-             * once, as the loop would); what is left, and the forms that
-             * read another buffer, by the loop, whose U loads of a batch are
-             * issued together so that their latencies overlap */
-            const int nbulk = (n & ~3) * NV, nv = n * NV;
-            const bool ub = accumulate == 0 || (accumulate == 1 && sizeof(T) == 8 && !Uin);
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0 && nbulk > 0) {
-                bulk_s2g(dUl, ys, nbulk * sizeof(T));
-                if (drain) {
-                    bulk_s2g_commit();
-                    /* an earlier line's add to U is complete: the older group */
-                    bulk_s2g_wait_but<1>();
-                }
-                if (accumulate == 0) bulk_s2g(Ul, ys, nbulk * sizeof(T));
-                if (accumulate == 1 && ub) bulk_add_s2g(Ul, ys, nbulk * sizeof(T));
-                bulk_s2g_commit();
-            }
-            constexpr int B = 8;
-            for (int t0 = (accumulate < 2 && !ub ? 0 : nbulk) + lane; t0 < nv; t0 += 32 * B) {
-                T u[B];
-#pragma unroll
-                for (int k = 0; k < B; ++k) {
-                    const int t = t0 + 32 * k;
-                    u[k] = (accumulate == 1 && t < nv) ? __ldcg(Uil + t) : T(0);
-                }
-#pragma unroll
-                for (int k = 0; k < B; ++k) {
-                    const int t = t0 + 32 * k;
-                    if (t < nv) {
-                        const T x = ys[t];
-                        if (t >= nbulk) dUl[t] = x;
-                        if (accumulate < 2) Ul[t] = u[k] + x;
-                    }
-                }
-            }
-            if (lane == 0 && nbulk > 0) {
-                if (drain) bulk_s2g_wait_but<1>(); /* dU */
-                bulk_s2g_wait_read(); /* before the CTA's memory goes */
-            }
-            __syncwarp();
-        }
-    }
-    if (timed_out) {
-        if (WS) {
-            /* stop the producer (its own waits are bounded), then wait for
-             * the copies it issued */
-            if (lane == 0) *ws_abort = 1;
-            __syncwarp();
-            ws_meet();
-            issued = *ws_issued;
-        }
-        if (lane == 0) {
-            atomicOr(status, ST_TIMEOUT);
-            RingPos r = rd;
-            for (int job = consumed; job < issued; ++job) {
-                mbar_wait(&bars[r.s], parity(r), 1LL << 28);
-                r.next(NS);
-            }
-        }
-        __syncwarp();
-        return false;
-    }
-    if (WS) ws_meet();
-    close_phases();
-    return true;
-}
-
-__device__ __forceinline__ void thomas_init_bars(unsigned char *smem, int NS) {
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
-    if ((threadIdx.x & 31) == 0) {
-        for (int s = 0; s < NS; ++s) mbar_init(&bars[s], 1);
-        mbar_fence_init();
-    }
-    __syncwarp();
-}
+constexpr uint32_t thomas_stage() { return thomas_stage_bytes<T, NV, THOMAS_P>(); }
 
 /* one CTA (one warp) per line */
 /* lines from nacc on leave U alone (accumulate 2) */
@@ -2005,7 +1397,7 @@ __global__ void __launch_bounds__(32) fast_thomas_kernel(
     thomas_init_bars(smem, NS);
     const uint64_t pol = threadIdx.x == 0 ? policy_evict_first() : 0;
     uint32_t pbase = 0;
-    thomas_line<T, P, YS>(NS, l < nacc ? accumulate : 2, line_start[l], line_len[l], line_twist[l], G,
+    thomas_line<T, NV, P, YS>(NS, l < nacc ? accumulate : 2, line_start[l], line_len[l], line_twist[l], G,
                           Gam, b, y, dU, U, status, smem, pbase, pol, Uin);
 }
 
@@ -2022,21 +1414,11 @@ __global__ void __launch_bounds__(64) fast_thomas_ws_kernel(
     extern __shared__ __align__(128) unsigned char smem[];
     const int l = blockIdx.x;
     if (l >= nline) return;
-    if (threadIdx.x == 0) {
-        uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
-        for (int s = 0; s < NS; ++s) {
-            mbar_init(&bars[s], 1);
-            mbar_init(&bars[8 + s], 1);
-        }
-        int *cnt = reinterpret_cast<int *>(smem + 128);
-        cnt[0] = 0;
-        cnt[1] = 0;
-        mbar_fence_init();
-    }
+    if (threadIdx.x == 0) thomas_init_ws(smem, NS);
     __syncthreads();
     const uint64_t pol = threadIdx.x == 32 ? policy_evict_first() : 0;
     uint32_t pbase = 0;
-    thomas_line<T, P, YS, true>(NS, l < nacc ? accumulate : 2, line_start[l], line_len[l],
+    thomas_line<T, NV, P, YS, true>(NS, l < nacc ? accumulate : 2, line_start[l], line_len[l],
                                 line_twist[l], G, Gam, b, y, dU, U, status, smem, pbase, pol, Uin);
 }
 
@@ -2066,7 +1448,7 @@ __global__ void __launch_bounds__(32) fast_thomas_batch_kernel(
         if (active && !active[it.sys]) continue;
         const ThomasSys<T> S = sys[it.sys];
         const int l = it.unit;
-        if (!thomas_line<T, P, false>(NS, 2, S.line_start[l], S.line_len[l], S.line_twist[l], S.G,
+        if (!thomas_line<T, NV, P, false>(NS, 2, S.line_start[l], S.line_len[l], S.line_twist[l], S.G,
                                       S.Gam, S.b, S.y, S.dU, nullptr, status, smem, pbase, pol))
             break;
     }
@@ -2094,16 +1476,8 @@ __global__ void __launch_bounds__(64) fast_thomas_batch_ws_kernel(
     __shared__ int s_item, s_stop;
     const int nwork = *nwork_p;
     if (threadIdx.x == 0) {
-        uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
-        for (int s = 0; s < NS; ++s) {
-            mbar_init(&bars[s], 1);
-            mbar_init(&bars[8 + s], 1);
-        }
-        int *cnt = reinterpret_cast<int *>(smem + 128);
-        cnt[0] = 0;
-        cnt[1] = 0;
+        thomas_init_ws(smem, NS);
         s_stop = 0;
-        mbar_fence_init();
     }
     __syncthreads();
     const uint64_t pol = threadIdx.x == 32 ? policy_evict_first() : 0;
@@ -2118,7 +1492,7 @@ __global__ void __launch_bounds__(64) fast_thomas_batch_ws_kernel(
         if (active && !active[it.sys]) continue;
         const ThomasSys<T> S = sys[it.sys];
         const int l = it.unit;
-        const bool ok = thomas_line<T, P, false, true>(NS, 2, S.line_start[l], S.line_len[l],
+        const bool ok = thomas_line<T, NV, P, false, true>(NS, 2, S.line_start[l], S.line_len[l],
                                                        S.line_twist[l], S.G, S.Gam, S.b, S.y, S.dU,
                                                        nullptr, status, smem, pbase, pol);
         if (!ok && (threadIdx.x & 31) == 0) s_stop = 1;
@@ -2143,7 +1517,7 @@ struct ThomasCfg {
 
 template <typename T, bool WS = false>
 static ThomasCfg thomas_cfg(const FastLayout &L) {
-    const size_t sb = thomas_stage_bytes<T>();
+    const size_t sb = thomas_stage<T>();
     /* lines resident per SM in one wave, and the shared memory each may use
      * so that they all are: the SM's capacity over them, less the per-CTA
      * reservation.  The deeper the copy ring, the more of the DRAM latency
@@ -2157,7 +1531,7 @@ static ThomasCfg thomas_cfg(const FastLayout &L) {
     const int per_sm = (L.nline + nsm - 1) / nsm;
     const long long budget = (long long)smem_sm / (per_sm > 0 ? per_sm : 1) - reserved;
     const size_t ys_bytes = (size_t)((L.max_len + 3) & ~3) * NV * sizeof(T);
-    const size_t fixed = thomas_hdr<WS>() + BCAST<T> * sizeof(T);
+    const size_t fixed = thomas_hdr<WS>() + BCAST<T, NV> * sizeof(T);
     ThomasCfg c;
     c.ys = (long long)(fixed + ys_bytes + 3 * sb) <= budget;
     long long left = budget - (long long)fixed - (c.ys ? (long long)ys_bytes : 0);
@@ -2301,7 +1675,7 @@ struct SmallSweeps {
 };
 
 static size_t small_smem(const FastLayout &L) {
-    return SMALL_HDR + SMALL_NS * (size_t)thomas_stage_bytes<double>() + BCAST<double> * sizeof(double) +
+    return SMALL_HDR + SMALL_NS * (size_t)thomas_stage<double>() + BCAST<double, NV> * sizeof(double) +
            (size_t)((L.max_len + 3) & ~3) * NV * sizeof(double) +
            (size_t)(L.nx + 2) * RES_TILE * NV * sizeof(double);
 }
@@ -2320,20 +1694,13 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) small_sweeps_kernel(SmallSwe
     volatile int *s_ok = reinterpret_cast<volatile int *>(smem + 160);
     double *red = reinterpret_cast<double *>(smem + 168); /* one per warp, then the norm */
     unsigned char *ring = smem + SMALL_HDR;
-    double *aux = reinterpret_cast<double *>(ring + SMALL_NS * thomas_stage_bytes<double>()) + BCAST<double> +
+    double *aux = reinterpret_cast<double *>(ring + SMALL_NS * thomas_stage<double>()) + BCAST<double, NV> +
                   ((A.max_len + 3) & ~3) * NV;
     double *sg = aux, *sr = aux + nx * RES_TILE * NV, *sb = sr + RES_TILE * NV;
     if (tid == 0) {
-        for (int s = 0; s < SMALL_NS; ++s) {
-            mbar_init(&bars[s], 1);
-            mbar_init(&bars[8 + s], 1);
-        }
         mbar_init(&rbar[0], 1);
         mbar_init(&rbar[1], 1);
-        int *cnt = reinterpret_cast<int *>(smem + 128);
-        cnt[0] = 0;
-        cnt[1] = 0;
-        mbar_fence_init();
+        thomas_init_ws(smem, SMALL_NS);
     }
     __syncthreads();
     const SolveState *S = A.state;
@@ -2434,7 +1801,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) small_sweeps_kernel(SmallSwe
     };
     static_assert(SMALL_THREADS == 160, "the counts of barriers 2 and 3");
     auto line = [&](auto phase) {
-        return thomas_line<double, THOMAS_P, true, true, decltype(phase)::value>(
+        return thomas_line<double, NV, THOMAS_P, true, true, decltype(phase)::value>(
             SMALL_NS, 1, ls, ll, lt, A.G, A.Gam, A.b, A.y, A.dU, A.U, A.status, smem, pbase, pol, nullptr, true);
     };
     /* b, as the others stored it, for this warp's bulk copies */
@@ -3053,7 +2420,7 @@ static int sm_count() {
 template <typename T>
 size_t thomas_batch_smem(int stages, int warps) {
     return (warps == 2 ? thomas_hdr<true>() : thomas_hdr<false>()) +
-           (size_t)stages * 2 * THOMAS_P * (NB + NV) * sizeof(T) + BCAST<T> * sizeof(T);
+           (size_t)stages * 2 * THOMAS_P * (NB + NV) * sizeof(T) + BCAST<T, NV> * sizeof(T);
 }
 
 template <typename T>
@@ -3609,14 +2976,14 @@ template <int P, bool CHECK>
 __device__ __forceinline__ void fwd_chunk_m(const double *sG, const double *const *sB,
                                             double *const *bc, double *const *yg, int nown,
                                             int kbase, int len, int cpos, int i) {
-    Row<double> cur_row, next_row;
+    Row<double, NV> cur_row, next_row;
     load_row(cur_row, sG, i, 0);
     double cur_b[MULTI_RPW], next_b[MULTI_RPW];
 #pragma unroll
     for (int j = 0; j < MULTI_RPW; ++j) cur_b[j] = sB[j][i];
 #pragma unroll
     for (int q = 0; q < P; ++q) {
-        StepVec<double> v[MULTI_RPW];
+        StepVec<double, NV> v[MULTI_RPW];
 #pragma unroll
         for (int j = 0; j < MULTI_RPW; ++j) {
             v[j].load(bc[j] + (q & 1) * 10, i, 0);
@@ -3652,12 +3019,12 @@ template <int P, bool CHECK>
 __device__ __forceinline__ void bwd_chunk_m(const double *sG, double *const *bc,
                                             const double (*yv)[P], double *const *dUl, int nown,
                                             int kbase, int len, int cpos, int i) {
-    Row<double> cur_row, next_row;
+    Row<double, NV> cur_row, next_row;
     load_row(cur_row, sG + (P - 1) * NB, i, 0);
 #pragma unroll
     for (int q = P - 1; q >= 0; --q) {
         const int f = (P - 1 - q) & 1;
-        StepVec<double> v[MULTI_RPW];
+        StepVec<double, NV> v[MULTI_RPW];
 #pragma unroll
         for (int j = 0; j < MULTI_RPW; ++j) v[j].load(bc[j] + f * 10, i, 0);
         if (q > 0) load_row(next_row, sG + (q - 1) * NB, i, 0);
@@ -3732,7 +3099,7 @@ __device__ __forceinline__ void multi_thomas_line(const MultiLine &S, int l, int
     const uint32_t halfb = P * (NB + nr * NV) * sizeof(T);
     const uint32_t stage = 2 * halfb;
     unsigned char *st0 = smem + 128;
-    T *bcw = reinterpret_cast<T *>(st0 + (size_t)NS * stage) + w * MULTI_RPW * BCAST<T>;
+    T *bcw = reinterpret_cast<T *>(st0 + (size_t)NS * stage) + w * MULTI_RPW * BCAST<T, NV>;
     const int ps = line_start[l], n = line_len[l], m = line_twist[l];
     const int h = lane >> 4, li = lane & 15;
     const int i = li < NV ? li : NV - 1;
@@ -3753,13 +3120,13 @@ __device__ __forceinline__ void multi_thomas_line(const MultiLine &S, int l, int
         const int jj = j < nown ? j : 0;
         slot[j] = mine ? k0 + jj : 0;
         const int rr = mine ? rid[k0 + jj] : 0;
-        bc[j] = bcw + j * BCAST<T> + h * 20;
+        bc[j] = bcw + j * BCAST<T, NV> + h * 20;
         yl[j] = syp[rr] + (size_t)ps * NV;
         dUl[j] = sdp[rr] + (size_t)ps * NV;
         bg[j] = sbp[rr] + (size_t)ps * NV;
     }
     const uint64_t pol = tid == 0 ? policy_evict_first() : 0;
-    for (int t = lane; t < MULTI_RPW * BCAST<T>; t += 32) bcw[t] = T(0);
+    for (int t = lane; t < MULTI_RPW * BCAST<T, NV>; t += 32) bcw[t] = T(0);
     __syncwarp();
 
     auto cells = [&](int ln, int c) { return ((min(P, ln - c * P) + 3) & ~3); };
@@ -3841,7 +3208,7 @@ __device__ __forceinline__ void multi_thomas_line(const MultiLine &S, int l, int
             const T *cr = Gam + (size_t)(ps + ptw) * NB + lane;
 #pragma unroll
             for (int j = 0; j < MULTI_RPW; ++j) {
-                const T *base = bcw + j * BCAST<T>;
+                const T *base = bcw + j * BCAST<T, NV>;
                 const T *ytop = base + (m & 1) * 10;
                 const T *ybot = base + 20 + (nb & 1) * 10;
                 T acc = bg[j][(size_t)ptw * NV + lane];
@@ -3855,7 +3222,7 @@ __device__ __forceinline__ void multi_thomas_line(const MultiLine &S, int l, int
 #pragma unroll
             for (int j = 0; j < MULTI_RPW; ++j) {
                 if (j < nown) {
-                    T *base = bcw + j * BCAST<T>;
+                    T *base = bcw + j * BCAST<T, NV>;
                     for (int t = 0; t < 4; ++t) base[t * 10 + lane] = xm[j];
                     dUl[j][(size_t)ptw * NV + lane] = xm[j];
                 }
@@ -3941,7 +3308,7 @@ static size_t multi_thomas_stage(int nr) {
 
 static size_t multi_thomas_smem(int nr, int NS) {
     return 128 + (size_t)NS * multi_thomas_stage(nr) +
-           (size_t)multi_thomas_warps(nr) * MULTI_RPW * BCAST<double> * sizeof(double);
+           (size_t)multi_thomas_warps(nr) * MULTI_RPW * BCAST<double, NV> * sizeof(double);
 }
 
 /* ring depth: the shared memory each of the SM's resident lines may use,

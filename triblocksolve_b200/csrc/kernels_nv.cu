@@ -9,11 +9,7 @@
  *   nv_factor_kernel   one warp per chain, lane j < NV owns column j of
  *                      every block, Gauss-Jordan by columns with shuffles
  *   nv_twist_kernel    one CTA per line: the twist cell's pivot
- *   nv_thomas_kernel   one warp per line, the two half-warps on the two
- *                      chains, lane i < NV on row i; chunks of G (Gam)
- *                      and b stream through a ring of bulk copies in
- *                      shared memory and the previous vector arrives by
- *                      shuffles
+ *   nv_thomas_kernel   the line solve of thomas.cuh at block size NV
  *   nv_resid_kernel    persistent over 16-position tiles, Dinv and the
  *                      cross-line blocks staged by bulk copies, thread
  *                      (cell, row) = (t / NV, t % NV)
@@ -23,9 +19,12 @@
  */
 #include "device_common.cuh"
 #include "tbs_internal.hxx"
+#include "thomas.cuh"
 #include "tma.cuh"
 
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 namespace tbs {
 
@@ -285,29 +284,6 @@ __global__ void nv_xlayout_kernel(long long nslots, const int *__restrict__ xsrc
     }
 }
 
-/* init - row . v with the previous vector v held one component per lane of
- * this half-warp (lanes src0 .. src0+NV-1) */
-/* init - row . v, row i of the column-major block at blk (entry (i, j)
- * at i + NV j), with the previous vector v held one component per lane
- * of this half-warp (lanes src0 .. src0+NV-1) */
-template <int NV>
-__device__ __forceinline__ double nv_row_step(const double *blk, int i, double init, double vmine,
-                                              int src0) {
-    double a0 = init, a1 = 0.0, a2 = 0.0;
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        const double vj = __shfl_sync(NFULL, vmine, src0 + j);
-        const double g = blk[i + NV * j];
-        if (j % 3 == 0)
-            a0 -= g * vj;
-        else if (j % 3 == 1)
-            a1 += g * vj;
-        else
-            a2 += g * vj;
-    }
-    return a0 - (a1 + a2);
-}
-
 /* cells per chunk of a chain: 8, or 4 for blocks of 10..13 so that a
  * two-stage ring stays small enough for nine lines per SM (one wave at
  * 1,200 lines; measured: 10-25 % faster there, slower from 14 on, where
@@ -317,191 +293,30 @@ template <int NV>
 constexpr int nv_chunk() { return (NV >= 10 && NV <= 13) ? 4 : 8; }
 
 template <int NV>
-__host__ __device__ inline size_t nv_thomas_stage() {
-    return 2 * (size_t)nv_chunk<NV>() * (NV * NV + NV) * sizeof(double);
-}
+constexpr size_t nv_thomas_stage() { return thomas_stage_bytes<double, NV, nv_chunk<NV>()>(); }
 
-/* One warp per line: half-warp h runs chain h (top: positions 0..m-1 in
- * order, bottom: m..n-2 in elimination order), lane i < NV row i.  Lane 0
- * streams "jobs" through an NS-stage ring of bulk copies, each holding one
- * chunk of nv_chunk<NV>() cells of both chains: forward jobs the blocks of G and the
- * b vectors, backward jobs (in reverse) the blocks of Gam; y is read back
- * with plain loads one chunk ahead.  Forward y_s = b_s - G_s y_{s-1}, twist
- * x = b - G_tw y_top - Gam_tw y_bot, backward x_s = y_s - Gam_s x_{s+1};
- * accumulate 0: U = dU, 1: U += dU, 2: U untouched.  A staging wait that
- * runs out of time sets ST_TIMEOUT and the warp drains its copies. */
-template <int NV>
-__global__ void __launch_bounds__(32) nv_thomas_kernel(
+/* One line per CTA: thomas_line with the chain warp issuing its own copies,
+ * or (WS) a copy warp beside it; YS: y and x in shared memory. */
+template <int NV, bool WS, bool YS>
+__global__ void __launch_bounds__(WS ? 64 : 32) nv_thomas_kernel(
     int nline, int NS, const int *__restrict__ line_start, const int *__restrict__ line_len,
     const int *__restrict__ line_twist, const double *__restrict__ G, const double *__restrict__ Gam,
     const double *__restrict__ b, double *__restrict__ y, double *__restrict__ dU,
     double *__restrict__ U, int accumulate, unsigned *status) {
-    constexpr int NB = NV * NV, P = nv_chunk<NV>();
     extern __shared__ __align__(128) unsigned char smem[];
     const int l = blockIdx.x;
     if (l >= nline) return;
-    const int lane = threadIdx.x, h = lane >> 4, i = lane & 15;
-    const bool act = i < NV;
-    const int ii = act ? i : 0;
-    const int src0 = h << 4;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
-    const size_t half = (size_t)P * (NB + NV) * sizeof(double);
-    const size_t stage = 2 * half;
-    unsigned char *st0 = smem + 128;
-    if (lane == 0) {
-        for (int s = 0; s < NS; ++s) mbar_init(&bars[s], 1);
-        mbar_fence_init();
+    if (WS) {
+        if (threadIdx.x == 0) thomas_init_ws(smem, NS);
+        __syncthreads();
+    } else {
+        thomas_init_bars(smem, NS);
     }
-    __syncwarp();
-    const int ps = line_start[l], n = line_len[l], m = line_twist[l];
-    const int nb = n - 1 - m;
-    const int len = h ? nb : m;
-    const size_t base = (size_t)ps + (h ? m : 0);
-    const int nchT = (m + P - 1) / P, nchB = (nb + P - 1) / P;
-    const int nch = h ? nchB : nchT;
-    const int nf = nchT > nchB ? nchT : nchB;
-    const int njobs = 2 * nf;
-    const uint64_t pol = lane == 0 ? policy_evict_first() : 0;
-    auto cells = [&](int ln, int c) { return ((min(P, ln - c * P) + 3) & ~3); };
-    auto issue = [&](int job, int s) {
-        unsigned char *st = st0 + (size_t)s * stage;
-        uint32_t bytes = 0;
-        if (job < nf) {
-            if (job < nchT) bytes += cells(m, job) * (NB + NV) * sizeof(double);
-            if (job < nchB) bytes += cells(nb, job) * (NB + NV) * sizeof(double);
-        } else {
-            const int jb = job - nf;
-            if (nchT - 1 - jb >= 0) bytes += cells(m, nchT - 1 - jb) * NB * sizeof(double);
-            if (nchB - 1 - jb >= 0) bytes += cells(nb, nchB - 1 - jb) * NB * sizeof(double);
-        }
-        mbar_arrive_expect_tx(&bars[s], bytes);
-        for (int hh = 0; hh < 2; ++hh) {
-            const int ln = hh ? nb : m, nc = hh ? nchB : nchT, cp = hh ? m : 0;
-            unsigned char *hb = st + hh * half;
-            if (job < nf) {
-                const int c = job;
-                if (c >= nc) continue;
-                const int cnt = cells(ln, c);
-                const size_t p = (size_t)(ps + cp + c * P);
-                bulk_g2s_hint(hb, G + p * NB, cnt * NB * sizeof(double), &bars[s], pol);
-                bulk_g2s(hb + (size_t)P * NB * sizeof(double), b + p * NV, cnt * NV * sizeof(double), &bars[s]);
-            } else {
-                const int c = nc - 1 - (job - nf);
-                if (c < 0) continue;
-                const int cnt = cells(ln, c);
-                bulk_g2s_hint(hb, Gam + (size_t)(ps + cp + c * P) * NB, cnt * NB * sizeof(double),
-                              &bars[s], pol);
-            }
-        }
-    };
-    /* u: U at p, read ahead when accumulate == 1 */
-    auto put = [&](size_t p, double x, double u) {
-        dU[p * NV + i] = x;
-        if (accumulate == 0)
-            U[p * NV + i] = x;
-        else if (accumulate == 1)
-            U[p * NV + i] = u + x;
-    };
-    int issued = 0;
-    if (lane == 0)
-        for (; issued < NS && issued < njobs; ++issued) issue(issued, issued);
-    int consumed = 0;
-    bool timed_out = false;
-
-    /* ---------------- forward */
-    double yp = 0.0;
-    for (int c = 0; c < nf; ++c) {
-        const int s = c % NS;
-        if (!__all_sync(NFULL, mbar_wait(&bars[s], (uint32_t)(c / NS) & 1u))) {
-            timed_out = true;
-            break;
-        }
-        ++consumed;
-        const double *sG = reinterpret_cast<const double *>(st0 + (size_t)s * stage + h * half);
-        const double *sB = sG + P * NB;
-#pragma unroll
-        for (int q = 0; q < P; ++q) {
-            const int k = c * P + q;
-            const double yi = nv_row_step<NV>(sG + q * NB, ii, sB[q * NV + ii], yp, src0);
-            if (k < len) {
-                if (act) y[(base + k) * NV + i] = yi;
-                yp = yi;
-            }
-        }
-        __syncwarp();
-        if (lane == 0 && issued < njobs) {
-            issue(issued, s);
-            ++issued;
-        }
-    }
-    if (!timed_out) {
-        /* ---------------- twist (both halves compute the same values) */
-        const size_t ptw = (size_t)ps + n - 1;
-        double xm = b[ptw * NV + ii];
-        {
-            const double *gr = G + ptw * NB + ii;
-            const double *cr = Gam + ptw * NB + ii;
-#pragma unroll
-            for (int j = 0; j < NV; ++j) {
-                const double yt = __shfl_sync(NFULL, yp, j);
-                const double yb = __shfl_sync(NFULL, yp, 16 + j);
-                xm -= gr[NV * j] * yt + cr[NV * j] * yb;
-            }
-        }
-        if (h == 0 && act) put(ptw, xm, accumulate == 1 ? U[ptw * NV + i] : 0.0);
-        /* ---------------- backward */
-        /* y, and U when the solve adds dU to it, read one chunk ahead */
-        double yv[P], nyv[P], uv[P], nuv[P];
-        auto load_y = [&](int c, double *yy, double *uu) {
-#pragma unroll
-            for (int q = 0; q < P; ++q) {
-                const int k = c * P + q;
-                const bool ok = c >= 0 && k < len;
-                yy[q] = ok ? y[(base + k) * NV + ii] : 0.0;
-                uu[q] = (ok && accumulate == 1) ? U[(base + k) * NV + ii] : 0.0;
-            }
-        };
-        __syncwarp();
-        load_y(nch - 1, yv, uv);
-        double xp = xm;
-        for (int jb = 0; jb < nf; ++jb) {
-            const int job = nf + jb;
-            const int c = nch - 1 - jb; /* this half's chunk (may be < 0) */
-            load_y(c - 1, nyv, nuv);
-            const int s = job % NS;
-            if (!__all_sync(NFULL, mbar_wait(&bars[s], (uint32_t)(job / NS) & 1u))) {
-                timed_out = true;
-                break;
-            }
-            ++consumed;
-            const double *sG = reinterpret_cast<const double *>(st0 + (size_t)s * stage + h * half);
-#pragma unroll
-            for (int q = P - 1; q >= 0; --q) {
-                const int k = c * P + q;
-                const bool valid = c >= 0 && k < len;
-                const double xi = nv_row_step<NV>(sG + q * NB, ii, valid ? yv[q] : 0.0, xp, src0);
-                if (valid) {
-                    if (act) put(base + k, xi, uv[q]);
-                    xp = xi;
-                }
-            }
-            __syncwarp();
-            if (lane == 0 && issued < njobs) {
-                issue(issued, s);
-                ++issued;
-            }
-#pragma unroll
-            for (int q = 0; q < P; ++q) {
-                yv[q] = nyv[q];
-                uv[q] = nuv[q];
-            }
-        }
-    }
-    if (timed_out && lane == 0) {
-        atomicOr(status, ST_TIMEOUT);
-        for (int job = consumed; job < issued; ++job)
-            mbar_wait(&bars[job % NS], (uint32_t)(job / NS) & 1u, 1LL << 28);
-    }
+    const uint64_t pol = threadIdx.x == (WS ? 32 : 0) ? policy_evict_first() : 0;
+    uint32_t pbase = 0;
+    thomas_line<double, NV, nv_chunk<NV>(), YS, WS>(NS, accumulate, line_start[l], line_len[l],
+                                                    line_twist[l], G, Gam, b, y, dU, U, status, smem,
+                                                    pbase, pol);
 }
 
 /* positions per residual tile: 16 (the layout's granule), up to 64 for
@@ -702,32 +517,56 @@ struct NvOps {
         nv_xlayout_kernel<NV><<<grid_cap(nslots * 32, 256), 256, 0, st>>>(nslots, L.xsrc, O1, O2, X);
         return (int)cudaGetLastError();
     }
-    /* ring depth: the SM's shared memory over its resident lines, 2..6 */
-    static int thomas_ns(const FastLayout &L) {
+    /* The launch's form, from the lines resident per SM in one wave and the
+     * shared memory each may use so that they all are.  A copy warp beside the
+     * chain warp with y and x in shared memory is the fastest form wherever the
+     * line and a ring of three stages fit (us, with / without, nvar 5: 300x320
+     * 31 / 50, 600x640 62 / 102, 1200x320 51 / 63; nvar 2, 1200x1280: 114 /
+     * 189); without room for them the copy warp still pays while at most five
+     * lines share an SM (nvar 12, 600x640: 184 / 205), and costs beyond (nvar
+     * 4, 1200x1280: 317 / 224).  The rest of the share goes to the ring (2..8
+     * stages).  The form before, vectors passed by shuffles and barriers tested
+     * between chunks: nvar 5 60, 130 and 80 us, nvar 12 213 us at 600x640. */
+    struct Cfg {
+        bool ws, ys;
+        int ns;
+        size_t smem;
+        const void *fn;
+    };
+    static Cfg thomas_cfg(const FastLayout &L) {
         int dev = 0, nsm = 148, smem_sm = 228 * 1024, reserved = 1024;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
         cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
-        int per_sm = (L.nline + (nsm > 0 ? nsm : 148) - 1) / (nsm > 0 ? nsm : 148);
-        if (per_sm < 1) per_sm = 1;
-        long long ns = ((long long)smem_sm / per_sm - reserved - 128) / (long long)nv_thomas_stage<NV>();
-        if (ns > 6) ns = 6;
-        if (ns < 2) ns = 2;
-        return (int)ns;
+        if (nsm < 1) nsm = 148;
+        const int per_sm = std::max((L.nline + nsm - 1) / nsm, 1);
+        Cfg c{};
+        const long long sb = (long long)nv_thomas_stage<NV>();
+        const long long ys = (long long)((L.max_len + 3) & ~3) * NV * (long long)sizeof(double);
+        const long long bcast = (long long)(BCAST<double, NV> * sizeof(double));
+        const long long budget = std::min<long long>(smem_sm / per_sm, 227 * 1024) - reserved;
+        c.ys = thomas_hdr<true>() + bcast + ys + 3 * sb <= budget;
+        c.ws = c.ys || per_sm <= 5;
+        const long long fixed = (c.ws ? thomas_hdr<true>() : thomas_hdr<false>()) + bcast;
+        const long long left = budget - fixed - (c.ys ? ys : 0);
+        c.ns = (int)std::min<long long>(std::max<long long>(left / sb, 2), 8);
+        c.smem = (size_t)(fixed + c.ns * sb + (c.ys ? ys : 0));
+        c.fn = !c.ws  ? (const void *)nv_thomas_kernel<NV, false, false>
+               : c.ys ? (const void *)nv_thomas_kernel<NV, true, true>
+                      : (const void *)nv_thomas_kernel<NV, true, false>;
+        return c;
     }
-    static size_t thomas_smem(int ns) { return 128 + (size_t)ns * nv_thomas_stage<NV>(); }
     static int thomas(cudaStream_t st, const FastLayout &L, const double *G, const double *Gam,
                       const double *b, double *y, double *dU, double *U, int accumulate,
                       unsigned *status) {
-        const int ns = thomas_ns(L);
-        const size_t smem = thomas_smem(ns);
-        int rc = nv_set_smem((const void *)nv_thomas_kernel<NV>, smem);
+        const Cfg c = thomas_cfg(L);
+        int rc = nv_set_smem(c.fn, c.smem);
         if (rc) return rc;
-        nv_thomas_kernel<NV><<<L.nline, 32, smem, st>>>(L.nline, ns, L.line_start, L.line_len,
-                                                        L.line_twist, G, Gam, b, y, dU, U,
-                                                        accumulate, status);
-        return (int)cudaGetLastError();
+        int nline = L.nline, ns = c.ns;
+        const int *ls = L.line_start, *ll = L.line_len, *lt = L.line_twist;
+        void *args[] = {&nline, &ns, &ls, &ll, &lt, &G, &Gam, &b, &y, &dU, &U, &accumulate, &status};
+        return (int)cudaLaunchKernel(c.fn, dim3(L.nline), dim3(c.ws ? 64 : 32), args, c.smem, st);
     }
     static int resid(cudaStream_t st, const FastLayout &L, int mode, const double *Dinv,
                      const double *X, const double *dU, const double *Rsrc, double *b,
@@ -748,7 +587,8 @@ struct NvOps {
         return (int)cudaGetLastError();
     }
     static int prepare(const FastLayout &L) {
-        int rc = nv_set_smem((const void *)nv_thomas_kernel<NV>, thomas_smem(thomas_ns(L)));
+        const Cfg c = thomas_cfg(L);
+        int rc = nv_set_smem(c.fn, c.smem);
         if (!rc) rc = nv_set_smem((const void *)nv_resid_kernel<NV, 1>, nv_resid_smem<NV>(L.nx));
         if (!rc) rc = nv_set_smem((const void *)nv_resid_kernel<NV, 0>, nv_resid_smem<NV>(0));
         return rc;
