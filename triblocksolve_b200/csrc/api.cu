@@ -449,7 +449,7 @@ static int status_error(tbs_ctx *ctx, unsigned s) {
     if (s) {
         CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(unsigned), ctx->stream));
         if (ctx->d_counter) CK(cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned), ctx->stream));
-        if (ctx->d_meet) CK(cudaMemsetAsync(ctx->d_meet, 0, SMALL_MEET_WORDS * sizeof(unsigned), ctx->stream));
+        if (ctx->d_meet) CK(cudaMemsetAsync(ctx->d_meet, 0, GRID_MEET_WORDS * sizeof(unsigned), ctx->stream));
         if (s & ST_PIVOT)
             return ctx_fail(ctx, TBS_ERR_NUMERIC,
                             "zero or non-finite pivot in the no-pivot block factorization");
@@ -928,7 +928,7 @@ static int alloc_algo(tbs_ctx *ctx, int algo) {
     const int npmax = std::max({ref_line_res_partials(ctx->nelem) * 8, fast_resid_grid(ctx->L.np16),
                                 full_resid_blocks(ctx->nelem), 1024});
     DA(ctx->d_counter, 1);
-    DA(ctx->d_meet, SMALL_MEET_WORDS);
+    DA(ctx->d_meet, GRID_MEET_WORDS);
     if (ctx->npart_cap < npmax) {
         dfree(ctx, &ctx->d_partials);
         dfree(ctx, &ctx->d_partials2);

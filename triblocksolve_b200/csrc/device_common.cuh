@@ -7,6 +7,7 @@
 #define TBS_DEVICE_COMMON_CUH
 
 #include "tbs_internal.hxx"
+#include "tma.cuh"
 
 #include <cuda_runtime.h>
 
@@ -64,6 +65,53 @@ static __device__ __forceinline__ bool record_check(SolveState *S, double *hist,
         S->last = nrm;
     }
     return !pass && isfinite(nrm) && sw < S->max_sweeps;
+}
+
+/* ------------------------------------------------ CTAs of a cooperative launch
+ * meet[0 .. GRID_MEET_WORDS): zero when the launch starts (and again when
+ * grid_leave's last CTA has left).  The arrivals are spread over MEETS words,
+ * each watched by a lane of warp 0 (1.2 us a meeting of 148 CTAs).  `round`
+ * counts a CTA's meetings from 1; s_ok: a word of the CTA's shared memory.
+ * All threads call; false when the others did not come in about a second.
+ * Warp 1 does `meanwhile` once its CTA has arrived. */
+constexpr int MEETS = 8, MEET_STRIDE = GRID_MEET_WORDS / (MEETS + 1);
+
+template <typename F>
+static __device__ __forceinline__ bool grid_meet(unsigned *meet, unsigned round, volatile int *s_ok,
+                                                 F &&meanwhile) {
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicAdd(meet + MEET_STRIDE * (blockIdx.x % MEETS), 1u);
+        }
+        bool here = true;
+        if (threadIdx.x < MEETS) {
+            const unsigned target = round * ((gridDim.x - threadIdx.x + MEETS - 1) / MEETS);
+            const long long t0 = clock64();
+            while ((int)(ld_acquire(meet + MEET_STRIDE * threadIdx.x) - target) < 0) {
+                if (clock64() - t0 > (1LL << 31)) {
+                    here = false;
+                    break;
+                }
+            }
+        }
+        here = __all_sync(0xffffffffu, here);
+        if (threadIdx.x == 0) *s_ok = here ? 1 : 0;
+    } else if (threadIdx.x < 64) {
+        meanwhile();
+    }
+    __syncthreads();
+    return *s_ok != 0;
+}
+
+/* thread 0 of every CTA, after its last meeting: whether it is the last one;
+ * the words are then zero again */
+static __device__ __forceinline__ bool grid_leave(unsigned *meet) {
+    __threadfence();
+    if (atomicAdd(meet + MEET_STRIDE * MEETS, 1u) != gridDim.x - 1) return false;
+    for (int k = 0; k <= MEETS; ++k) meet[MEET_STRIDE * k] = 0u;
+    return true;
 }
 
 /* After a CTA's last tile: a ticket per CTA; the last CTA to finish adds

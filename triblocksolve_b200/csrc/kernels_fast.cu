@@ -1658,7 +1658,6 @@ int fast_prepare(const FastLayout &L) {
 constexpr int SMALL_THREADS = RES_THREADS_FAST;
 constexpr int SMALL_NS = 6;   /* ring stages of the line solve; two residual tiles lie in the ring */
 constexpr int SMALL_HDR = 256;
-constexpr int MEETS = 8, MEET_STRIDE = SMALL_MEET_WORDS / (MEETS + 1);
 
 struct SmallSweeps {
     int nline, nx, np16, max_len;
@@ -1666,7 +1665,7 @@ struct SmallSweeps {
     const double *G, *Gam, *Dinv, *X;
     double *b, *y, *dU, *U, *partials, *hist;
     SolveState *state;
-    unsigned *meet; /* MEETS counts of arrivals, one of CTAs that are done; zero between launches */
+    unsigned *meet; /* grid_meet's words */
     unsigned *status;
     unsigned long long *timer;
     unsigned long long loop, check; /* condition handles */
@@ -1718,36 +1717,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) small_sweeps_kernel(SmallSwe
     const int c = tid % RES_TILE, i = tid / RES_TILE;
     const bool act = tid < RES_TILE * NV;
     const uint32_t szD = RES_TILE * NB * sizeof(double);
-    /* all CTAs; false when one of them did not come in time.  The arrivals are
-     * spread over MEETS words, each watched by a lane of warp 0; warp 1 does
-     * `meanwhile` once the CTA has arrived */
-    auto meet = [&](auto &&meanwhile) {
-        __syncthreads();
-        if (warp == 0) {
-            ++round;
-            if (tid == 0) {
-                __threadfence();
-                atomicAdd(A.meet + MEET_STRIDE * (blockIdx.x % MEETS), 1u);
-            }
-            bool here = true;
-            if (tid < MEETS) {
-                const unsigned target = round * ((gridDim.x - tid + MEETS - 1) / MEETS);
-                const long long t0 = clock64();
-                while ((int)(ld_acquire(A.meet + MEET_STRIDE * tid) - target) < 0) {
-                    if (clock64() - t0 > (1LL << 31)) {
-                        here = false;
-                        break;
-                    }
-                }
-            }
-            here = __all_sync(FULL, here);
-            if (tid == 0) *s_ok = here ? 1 : 0;
-        } else if (warp == 1) {
-            meanwhile();
-        }
-        __syncthreads();
-        return *s_ok != 0;
-    };
+    auto meet = [&](auto &&meanwhile) { return grid_meet(A.meet, ++round, s_ok, meanwhile); };
     auto tile_of = [&](int k) { return (int)blockIdx.x + k * (int)gridDim.x; };
     auto blocks = [&](int k) { return reinterpret_cast<double *>(ring) + (size_t)(k % nbuf) * (1 + nx) * RES_TILE * NB; };
     auto issue = [&](int k) { /* thread 0: the k-th tile's blocks */
@@ -1932,10 +1902,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) small_sweeps_kernel(SmallSwe
     if (!ok && tid == 0) atomicOr(A.status, ST_TIMEOUT);
     __syncthreads();
     if (tid == 0) {
-        __threadfence();
-        if (atomicAdd(A.meet + MEET_STRIDE * MEETS, 1u) == gridDim.x - 1) {
-            /* every CTA has left the meetings */
-            for (int k = 0; k <= MEETS; ++k) A.meet[MEET_STRIDE * k] = 0u;
+        if (grid_leave(A.meet)) { /* every CTA has left the meetings */
             A.state->sweep = sw;
             A.state->last = nrm;
             cudaGraphSetConditional((cudaGraphConditionalHandle)A.loop, 0u);

@@ -18,6 +18,7 @@
  * Vectors are position ordered (np16 * 9 doubles, pads zero).
  */
 #include "ctx.hxx"
+#include "device_common.cuh"
 
 #include <cuda_runtime.h>
 
@@ -163,6 +164,164 @@ __global__ void __launch_bounds__(KR_THREADS) kr_scale_kernel(long long n, doubl
     for (; t < n; t += stride) dst[t] = a * src[t];
 }
 
+/* The sums of the partials of dot product c in kr_reduce_kernel's order, by
+ * one warp: the eight warps of that kernel one after the other. */
+__device__ __forceinline__ double kr_total(const double *__restrict__ partials, int c) {
+    const double *p = partials + (size_t)c * KR_BLOCKS;
+    const int lane = threadIdx.x & 31;
+    double v[KR_THREADS / 32];
+#pragma unroll
+    for (int q = 0; q < KR_THREADS / 32; ++q) {
+        const int t = 32 * q + lane;
+        v[q] = __ldcg(p + t);
+        if (t + KR_THREADS < KR_BLOCKS) v[q] += __ldcg(p + t + KR_THREADS);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < KR_THREADS / 32; ++q) v[q] += __shfl_down_sync(KFULL, v[q], o);
+    double tot = 0.0;
+#pragma unroll
+    for (int q = 0; q < KR_THREADS / 32; ++q) tot += v[q];
+    return tot; /* lane 0's */
+}
+static_assert(KR_BLOCKS <= 2 * KR_THREADS, "kr_total adds two partials a thread");
+
+/* One Arnoldi step's orthogonalization in one cooperative launch:
+ *   h = V^T w;  w -= V h;  h2 = V^T w, ww = w.w;  v_next = (w - V h2) / hn
+ * with hn = sqrt(ww - h2.h2), each sum in the order of kr_dots_kernel /
+ * kr_reduce_kernel / kr_combine_kernel, so the values are theirs.  Seven
+ * launches and two copies did this: at 301x257 67 us a step by themselves and
+ * the gaps between them; the vectors stay in the L2 there, so launches and
+ * the reductions' latency were what bound it.  The second product needs w -
+ * V h element by element only, so each thread goes on with its own elements.
+ * hout: h, then h2 and ww (host memory the device can write). */
+struct KrOrth {
+    long long n, ldv;
+    int count; /* basis vectors, 1 .. KRYLOV_MAX */
+    double *w, *V, *vnext, *partials, *hout;
+    unsigned *meet, *status;
+};
+
+__global__ void __launch_bounds__(KR_THREADS, 2) kr_orth_kernel(KrOrth A) {
+    __shared__ double red[KR_CHUNK][KR_THREADS / 32];
+    __shared__ double h[KRYLOV_MAX + 1], h2[KRYLOV_MAX + 2];
+    __shared__ int s_ok;
+    const int tid = threadIdx.x, warp = tid >> 5, count = A.count;
+    const long long t0 = blockIdx.x * (long long)KR_THREADS + tid;
+    const long long stride = (long long)gridDim.x * KR_THREADS;
+    const double *V = A.V;
+    /* partials of V_c . w for c < count (and w . w when self) */
+    auto dots = [&](int self) {
+        const int total = count + self;
+        for (int c0 = 0; c0 < total; c0 += KR_CHUNK) {
+            double acc[KR_CHUNK];
+#pragma unroll
+            for (int k = 0; k < KR_CHUNK; ++k) acc[k] = 0.0;
+            long long t = t0;
+            for (; t + (KR_UNROLL - 1) * stride < A.n; t += KR_UNROLL * stride) {
+                double wt[KR_UNROLL];
+#pragma unroll
+                for (int u = 0; u < KR_UNROLL; ++u) wt[u] = A.w[t + u * stride];
+#pragma unroll
+                for (int k = 0; k < KR_CHUNK; ++k) {
+                    const int c = c0 + k;
+                    if (c < count) {
+                        const double *vc = V + (size_t)c * A.ldv + t;
+                        double x[KR_UNROLL];
+#pragma unroll
+                        for (int u = 0; u < KR_UNROLL; ++u) x[u] = vc[u * stride];
+#pragma unroll
+                        for (int u = 0; u < KR_UNROLL; ++u) acc[k] += x[u] * wt[u];
+                    } else if (c == count && self) {
+#pragma unroll
+                        for (int u = 0; u < KR_UNROLL; ++u) acc[k] += wt[u] * wt[u];
+                    }
+                }
+            }
+            for (; t < A.n; t += stride) {
+                const double wt = A.w[t];
+#pragma unroll
+                for (int k = 0; k < KR_CHUNK; ++k) {
+                    const int c = c0 + k;
+                    if (c < count)
+                        acc[k] += V[(size_t)c * A.ldv + t] * wt;
+                    else if (c == count && self)
+                        acc[k] += wt * wt;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < KR_CHUNK; ++k) {
+                double v = acc[k];
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(KFULL, v, o);
+                if ((tid & 31) == 0) red[k][warp] = v;
+            }
+            __syncthreads();
+            if (tid < KR_CHUNK && c0 + tid < total) {
+                double tot = 0.0;
+                for (int q = 0; q < KR_THREADS / 32; ++q) tot += red[tid][q];
+                A.partials[(size_t)(c0 + tid) * KR_BLOCKS + blockIdx.x] = tot;
+            }
+            __syncthreads();
+        }
+    };
+    auto totals = [&](int total, double *out) {
+        for (int c = warp; c < total; c += KR_THREADS / 32) {
+            const double v = kr_total(A.partials, c);
+            if ((tid & 31) == 0) out[c] = v;
+        }
+        __syncthreads();
+    };
+    /* dst = scale * (w - sum_c coef[c] V_c), the scaling left out when 1 */
+    auto combine = [&](const double *coef, double *dst, double scale, bool scaled) {
+        long long t = t0;
+        for (; t + (KR_UNROLL - 1) * stride < A.n; t += KR_UNROLL * stride) {
+            double acc[KR_UNROLL];
+#pragma unroll
+            for (int u = 0; u < KR_UNROLL; ++u) acc[u] = A.w[t + u * stride];
+#pragma unroll 4
+            for (int c = 0; c < count; ++c) {
+                const double *vc = V + (size_t)c * A.ldv + t;
+#pragma unroll
+                for (int u = 0; u < KR_UNROLL; ++u) acc[u] += -coef[c] * vc[u * stride];
+            }
+#pragma unroll
+            for (int u = 0; u < KR_UNROLL; ++u) dst[t + u * stride] = scaled ? scale * acc[u] : acc[u];
+        }
+        for (; t < A.n; t += stride) {
+            double acc = A.w[t];
+            for (int c = 0; c < count; ++c) acc += -coef[c] * V[(size_t)c * A.ldv + t];
+            dst[t] = scaled ? scale * acc : acc;
+        }
+    };
+    dots(0);
+    bool ok = grid_meet(A.meet, 1, &s_ok, []() {});
+    if (ok) {
+        totals(count, h);
+        combine(h, A.w, 1.0, false);
+        /* the first partials are read by others until they come to the second
+         * meeting: the second ones lie behind them */
+        A.partials += (size_t)(KRYLOV_MAX + 2) * KR_BLOCKS;
+        dots(1);
+        ok = grid_meet(A.meet, 2, &s_ok, []() {});
+    }
+    if (ok) {
+        totals(count + 1, h2);
+        double s2 = 0.0; /* as the host's sum: no fused operations */
+        for (int c = 0; c < count; ++c) s2 = __dadd_rn(s2, __dmul_rn(h2[c], h2[c]));
+        const double hn = sqrt(fmax(__dsub_rn(h2[count], s2), 0.0));
+        combine(h2, A.vnext, 1.0 / hn, true);
+        if (blockIdx.x == 0) {
+            for (int c = tid; c < count; c += KR_THREADS) A.hout[c] = h[c];
+            for (int c = tid; c <= count; c += KR_THREADS) A.hout[KRYLOV_MAX + 2 + c] = h2[c];
+        }
+    } else if (tid == 0) {
+        atomicOr(A.status, ST_TIMEOUT);
+    }
+    __syncthreads();
+    if (tid == 0) grid_leave(A.meet);
+}
+
 }  // namespace
 
 struct KrylovBufs {
@@ -173,9 +332,11 @@ struct KrylovBufs {
     double *V = nullptr;    /* (m+1) x n */
     double *Z = nullptr;    /* m x n */
     double *w = nullptr;
-    double *partials = nullptr;  /* (KRYLOV_MAX + 2) x KR_BLOCKS */
-    double *h = nullptr, *h2 = nullptr, *y = nullptr;  /* KRYLOV_MAX + 2 each */
-    double *h_host = nullptr;    /* pinned: h and h2 read-backs */
+    double *partials = nullptr;  /* 2 x (KRYLOV_MAX + 2) x KR_BLOCKS */
+    double *h = nullptr, *y = nullptr;  /* KRYLOV_MAX + 2 each */
+    double *h_host = nullptr;    /* pinned, mapped: h and h2 of a step */
+    double *h_host_dev = nullptr;
+    unsigned *meet = nullptr;    /* kr_orth_kernel's meetings */
 };
 
 static int kfail(tbs_ctx *ctx, int code, const std::string &msg) {
@@ -205,7 +366,8 @@ static void krylov_free_vectors(KrylovBufs *k) {
     for (void *p : k->allocs) cudaFree(p);
     k->allocs.clear();
     k->bytes = 0;
-    k->V = k->Z = k->w = k->partials = k->h = k->h2 = k->y = nullptr;
+    k->V = k->Z = k->w = k->partials = k->h = k->y = nullptr;
+    k->meet = nullptr;
     k->m = 0;
     k->n = 0;
 }
@@ -244,8 +406,10 @@ static int kalloc(tbs_ctx *ctx, KrylovBufs *k, T **p, size_t count) {
 static int krylov_ensure(tbs_ctx *ctx, int m) {
     if (!ctx->krylov) {
         ctx->krylov = new KrylovBufs();
-        if (cudaMallocHost((void **)&ctx->krylov->h_host, 2 * (KRYLOV_MAX + 2) * sizeof(double)) !=
-            cudaSuccess) {
+        if (cudaHostAlloc((void **)&ctx->krylov->h_host, 2 * (KRYLOV_MAX + 2) * sizeof(double),
+                          cudaHostAllocMapped) != cudaSuccess ||
+            cudaHostGetDevicePointer((void **)&ctx->krylov->h_host_dev, ctx->krylov->h_host, 0) !=
+                cudaSuccess) {
             cudaGetLastError();
             krylov_free(ctx);
             return kfail(ctx, TBS_ERR_NOMEM, "pinned host allocation failed");
@@ -260,9 +424,9 @@ static int krylov_ensure(tbs_ctx *ctx, int m) {
     KA(k->V, (size_t)(m + 1) * n);
     KA(k->Z, (size_t)m * n);
     KA(k->w, (size_t)n);
-    KA(k->partials, (size_t)(KRYLOV_MAX + 2) * KR_BLOCKS);
+    KA(k->partials, 2 * (size_t)(KRYLOV_MAX + 2) * KR_BLOCKS);
+    KA(k->meet, (size_t)GRID_MEET_WORDS);
     KA(k->h, (size_t)KRYLOV_MAX + 2);
-    KA(k->h2, (size_t)KRYLOV_MAX + 2);
     KA(k->y, (size_t)KRYLOV_MAX + 2);
     k->m = m;
     k->n = n;
@@ -287,6 +451,17 @@ static int combine(tbs_ctx *ctx, double *x, const double *V, int count, const do
     KRUN("kr_combine", (kr_combine_kernel<<<148 * 8, KR_THREADS, 0, ctx->stream>>>(
                             k->n, x, V, k->n, count, coef, sign),
                         cudaGetLastError()));
+    return TBS_OK;
+}
+
+/* h and h2 of w against V_0 .. V_j into h_host, V_{j+1} */
+static int orth(tbs_ctx *ctx, int j) {
+    KrylovBufs *k = ctx->krylov;
+    KrOrth A{k->n, k->n, j + 1, k->w, k->V, k->V + (size_t)(j + 1) * k->n, k->partials, k->h_host_dev, k->meet,
+             ctx->d_status};
+    void *args[] = {&A};
+    KRUN("kr_orth", cudaLaunchCooperativeKernel((const void *)kr_orth_kernel, dim3(KR_BLOCKS), dim3(KR_THREADS),
+                                                args, 0, ctx->stream));
     return TBS_OK;
 }
 
@@ -372,18 +547,11 @@ static int gmres(tbs_ctx *ctx, int m, int psweeps, double tol, int max_iters, in
             double *Zj = k->Z + (size_t)j * n;
             rc = precond_product(ctx, Vj, Zj, k->w, psweeps);
             if (rc) return rc;
-            /* classical Gram-Schmidt, twice; the second pass also gives w.w */
-            rc = dots(ctx, k->w, k->V, j + 1, 0, k->h);
+            /* classical Gram-Schmidt, twice; the second pass also gives w.w; the
+             * next basis vector with it */
+            rc = orth(ctx, j);
             if (rc) return rc;
-            rc = combine(ctx, k->w, k->V, j + 1, k->h, -1.0);
-            if (rc) return rc;
-            rc = dots(ctx, k->w, k->V, j + 1, 1, k->h2);
-            if (rc) return rc;
-            rc = combine(ctx, k->w, k->V, j + 1, k->h2, -1.0);
-            if (rc) return rc;
-            KCK(cudaMemcpyAsync(hh, k->h, (j + 1) * sizeof(double), cudaMemcpyDeviceToHost, st));
-            rc = read_back(ctx, k->h2, j + 2, hh + KRYLOV_MAX + 2);
-            if (rc) return rc;
+            KCK(cudaStreamSynchronize(st));
             const double *h1 = hh, *h2 = hh + KRYLOV_MAX + 2;
             double ww = h2[j + 1], s2 = 0.0;
             for (int i = 0; i <= j; ++i) {
@@ -411,10 +579,6 @@ static int gmres(tbs_ctx *ctx, int m, int psweeps, double tol, int max_iters, in
             if (hist) hist[iters] = res;
             if (res <= tol * beta0 || iters >= max_iters || !(hn > 0.0) || !std::isfinite(res))
                 stop = true;
-            else if (j + 1 < m) {
-                rc = scale(ctx, k->V + (size_t)(j + 1) * n, k->w, 1.0 / hn);
-                if (rc) return rc;
-            }
         }
         /* y = R^-1 g (upper triangular, the rotated H), U += sum y_i z_i */
         for (int i = j - 1; i >= 0; --i) {

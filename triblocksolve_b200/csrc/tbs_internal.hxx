@@ -210,10 +210,11 @@ template <typename T>
 int launch_fast_thomas(cudaStream_t st, const FastLayout &L, const T *G, const T *Gam,
                        const T *b, T *y, T *dU, T *U, unsigned *status, int accumulate,
                        int nacc = -1, const T *Uin = nullptr);
+/* words in which the CTAs of a cooperative launch meet (grid_meet) */
+constexpr int GRID_MEET_WORDS = 9 * 64;
 /* all the sweeps of a solve of few lines as one cooperative launch: the grid
  * it takes (0: not for this system), and the launch.  `ns` gives the norms'
- * places and the graph's conditions; meet: SMALL_MEET_WORDS words, zero. */
-constexpr int SMALL_MEET_WORDS = 9 * 64;
+ * places and the graph's conditions; meet: GRID_MEET_WORDS words, zero. */
 int small_sweeps_grid(const FastLayout &L);
 int launch_small_sweeps(cudaStream_t st, const FastLayout &L, const double *G, const double *Gam,
                         const double *Dinv, const double *X, double *b, double *y, double *dU, double *U,
