@@ -250,10 +250,11 @@ int engine_init(Engine &e, int device, cudaStream_t stream, int algo) {
     ECK(cudaMemsetAsync(e.d_counter, 0, sizeof(unsigned), e.stream));
     ECK(cudaMemsetAsync(e.d_status, 0, sizeof(unsigned), e.stream));
     ECK(cudaMemsetAsync(e.d_ctl, 0, sizeof(BatchCtl), e.stream));
-    /* default schedule: 2 stages, as many CTAs per SM as fit, at most 8 */
+    /* schedule for members that come and go: 2 stages, as many CTAs per SM as
+     * fit, at most 8 (engine_fit_schedule: for a fixed set) */
     const int fit = algo == TBS_ALGO_FP64 ? thomas_batch_fit<double>(2, 1) : thomas_batch_fit<float>(2, 1);
     if (fit < 1) return efail(e, TBS_ERR_CUDA, "the batched Thomas kernel does not fit on an SM");
-    e.sched = BatchSched{std::min(fit, 8), 2, 1};
+    e.sched = e.sched_base = BatchSched{std::min(fit, 8), 2, 1};
     ECK(cudaStreamSynchronize(e.stream));
     return TBS_OK;
 }
@@ -505,6 +506,10 @@ int engine_set_members(Engine &e, const std::vector<Member> &members) {
     std::vector<MultiLine> mls;
     std::vector<WorkItem> mitems;
     if (!mixed) multi_items(members, mls, mitems);
+    if (!mitems.empty() && !e.grouped) {
+        e.grouped = true; /* and stays: members come and go, the graph is kept */
+        engine_drop_graph(e);
+    }
     int rc = ensure_capacity(e, std::max(n, 1), (int)std::max(nlines, 1LL), (int)mitems.size());
     if (rc) return rc;
 
@@ -610,7 +615,7 @@ int engine_set_members(Engine &e, const std::vector<Member> &members) {
          * blocks per tile */
         std::vector<std::vector<int>> g_solo, g_multi;
         for (const auto &grp : g_all) (grp.size() > 1 ? g_multi : g_solo).push_back(grp);
-        up.put(e.d_g_solo, group_index(g_solo, units(g_solo, 2)));
+        up.put(e.d_g_solo, group_index(g_solo, units(g_solo, 0)));
         up.put(e.d_g_units, group_index(g_multi, units(g_multi, 2), false));
     }
     up.put(e.d_g_prime, gi_prime);
@@ -682,7 +687,7 @@ static int engine_prime(Engine &e, Cond cc) {
     }
     BatchCtl *C = e.d_ctl;
     if (e.algo == TBS_ALGO_FP64) {
-        ERUN("fast_resid_rhs", launch_resid_batch<double>(st, 0, e.max_nx, e.d_rs_prime, e.d_g_prime, 1,
+        ERUN("fast_resid_rhs", launch_resid_batch<double>(st, 0, e.max_nx, e.d_rs_prime, e.d_g_prime,
                                                           nullptr, e.d_status));
         ERUN("reduce_norm", launch_reduce_batch(st, 160, e.d_red_prime, &C->nprime_sys, e.cap_mem, 1,
                                                 e.d_active, C, e.d_counter, cc.handle, cc.use,
@@ -702,14 +707,15 @@ static int engine_body(Engine &e, Cond cc, int inner) {
     if (e.algo == TBS_ALGO_FP64) {
         ERUN("fast_thomas", launch_thomas_batch<double>(st, e.sched, e.d_th64, e.d_lines, &C->nlines,
                                                         e.d_active, e.d_queue, e.d_status));
-        /* the line solves of several members of one system: their blocks
-         * read once per line for up to MULTI_MAX of them */
-        ERUN("multi_thomas", launch_multi_thomas_items(st, e.cap_mitems, e.d_ml, e.d_mitems, &C->nmitems,
-                                                       e.d_active, e.d_status));
-        ERUN("fast_resid", launch_resid_batch<double>(st, 1, e.max_nx, e.d_rs_body, e.d_g_solo,
-                                                      BATCH_CHUNK, e.d_active, e.d_status));
-        ERUN("fast_resid_group", launch_resid_group<double>(st, e.max_nx, e.d_rs_body, e.d_g_units,
-                                                            BATCH_CHUNK, e.d_active, e.d_status));
+        ERUN("fast_resid", launch_resid_solo(st, e.max_nx, e.d_rs_body, e.d_g_solo, e.d_active, e.d_status));
+        if (e.grouped) {
+            /* several members of one system: its blocks read once per line,
+             * and per tile, for up to MULTI_MAX of them */
+            ERUN("multi_thomas", launch_multi_thomas_items(st, e.cap_mitems, e.d_ml, e.d_mitems, &C->nmitems,
+                                                           e.d_active, e.d_status));
+            ERUN("fast_resid_group", launch_resid_group<double>(st, e.max_nx, e.d_rs_body, e.d_g_units,
+                                                                BATCH_CHUNK, e.d_active, e.d_status));
+        }
         ERUN("reduce_norm", launch_reduce_batch(st, 160, e.d_red_body, &C->nsys, e.cap_mem, 0,
                                                 e.d_active, C, e.d_counter, cc.handle, cc.use));
         return TBS_OK;
@@ -718,13 +724,13 @@ static int engine_body(Engine &e, Cond cc, int inner) {
      * launch, each inner residual adds its sweep's d to it, and the last d
      * goes to U with c (the order of the single-system sequence) */
     if (!e.fullpos)
-        ERUN("fast_resid32_rhs", launch_resid_batch<float>(st, 0, e.max_nx, e.d_rs32_rhs, e.d_g_tiles, 1,
+        ERUN("fast_resid32_rhs", launch_resid_batch<float>(st, 0, e.max_nx, e.d_rs32_rhs, e.d_g_tiles,
                                                            e.d_active, e.d_status));
     for (int m = 0; m < inner; ++m) {
         ERUN("fast_thomas32", launch_thomas_batch<float>(st, e.sched, e.d_th32, e.d_lines, &C->nlines,
                                                          e.d_active, e.d_queue, e.d_status));
         if (m + 1 < inner)
-            ERUN("fast_resid32", launch_resid_batch<float>(st, 3, e.max_nx, e.d_rs32_dx, e.d_g_tiles, 1,
+            ERUN("fast_resid32", launch_resid_batch<float>(st, 3, e.max_nx, e.d_rs32_dx, e.d_g_tiles,
                                                            e.d_active, e.d_status));
     }
     ERUN("axpy", launch_axpy2_batch(st, e.d_vec, e.d_g_tiles, e.d_active));
@@ -919,11 +925,39 @@ int engine_set_schedule(Engine &e, BatchSched s, int order) {
                                          " CTAs per SM with " + std::to_string(s.stages) +
                                          " stages and " + std::to_string(s.warps) + " warp(s) per line");
     const bool new_order = order != e.order;
-    e.sched = s;
+    e.sched_set = true;
+    e.sched = e.sched_base = s;
     e.order = order;
     engine_drop_graph(e);
     if (new_order && !e.members.empty()) return engine_upload_lines(e);
     return TBS_OK;
+}
+
+/* The lines a CTA solves one after another hide each other's latencies only if
+ * there are many: with q = cells per SM over the longest line's cells (at
+ * least how many lines an SM has to work on for all of them to end together),
+ * batch solves took, for 8 CTAs an SM of 2 stages and one warp a line / 4 of 3
+ * stages with a copy warp / 5 of the same (us):
+ *   q 1.1: 1179 / 1035 / 1104    q 2.5: 1417 / 1229 / 1285
+ *   q 3.8: 1645 / 1486 / 1510    q 9.7: 2997 / 2946 / 2794
+ *   q 13.5: 3091 / 3240 / 3140   q 26: 3152 / 3244 / 3183 */
+void engine_fit_schedule(Engine &e, const std::vector<tbs_ctx *> &systems) {
+    if (e.sched_set) return;
+    int nsm = 148, longest = 1;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e.device);
+    double cells = 0.0;
+    for (const tbs_ctx *c : systems) {
+        cells += c->nelem;
+        longest = std::max(longest, c->max_line);
+    }
+    const double q = cells / ((double)nsm * longest);
+    BatchSched s = q < 6.0 ? BatchSched{4, 3, 2} : q < 12.0 ? BatchSched{5, 3, 2} : BatchSched{8, 2, 1};
+    const int fit = e.algo == TBS_ALGO_FP64 ? thomas_batch_fit<double>(s.stages, s.warps)
+                                            : thomas_batch_fit<float>(s.stages, s.warps);
+    s.ctas_per_sm = std::max(1, std::min(s.ctas_per_sm, fit));
+    if (s.ctas_per_sm == e.sched.ctas_per_sm && s.stages == e.sched.stages && s.warps == e.sched.warps) return;
+    e.sched = s;
+    engine_drop_graph(e);
 }
 
 int engine_tune(Engine &e, BatchSched *best_s, int *best_o, double *best_ms) {
@@ -988,6 +1022,10 @@ int engine_tune(Engine &e, BatchSched *best_s, int *best_o, double *best_ms) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     e.sched = rc ? keep : bs;
+    if (!rc) {
+        e.sched_set = true;
+        e.sched_base = bs;
+    }
     e.order = rc ? keep_order : bo;
     engine_drop_graph(e);
     int rc2 = engine_upload_lines(e);
@@ -1070,6 +1108,7 @@ static int batch_ready(tbs_batch *b, double tol, int max_sweeps) {
     if (fp != b->fingerprint) {
         std::vector<Member> m;
         for (tbs_ctx *c : b->sys) m.push_back({c, ctx_vectors(c), true});
+        engine_fit_schedule(b->eng, b->sys);
         rc = engine_set_members(b->eng, m);
         if (rc) return rc;
         b->fingerprint = fp;
@@ -1144,6 +1183,7 @@ int tbs_batch_create(tbs_ctx *const *systems, int nsys, tbs_batch **out) {
         if (rc) return fail(rc);
         b->eng.inner = systems[0]->inner_sweeps;
         b->eng.inner_first = systems[0]->inner_first;
+        engine_fit_schedule(b->eng, b->sys);
     } catch (...) {
         return fail(bfail(b, TBS_ERR_NOMEM, "host allocation failed"));
     }
@@ -1188,7 +1228,7 @@ int tbs_batch_set_schedule(tbs_batch *b, int ctas_per_sm, int stages, int order)
     if (order != 0 && order != 1) return bfail(b, TBS_ERR_ARG, "bad line order");
     BGUARD_BEGIN
     if (cudaSetDevice(b->eng.device) != cudaSuccess) return bfail(b, TBS_ERR_CUDA, "cudaSetDevice failed");
-    return engine_set_schedule(b->eng, BatchSched{ctas_per_sm, stages, b->eng.sched.warps}, order);
+    return engine_set_schedule(b->eng, BatchSched{ctas_per_sm, stages, b->eng.sched_base.warps}, order);
     BGUARD_END
 }
 
@@ -1197,7 +1237,7 @@ int tbs_batch_set_warps_per_line(tbs_batch *b, int warps) {
     if (warps != 1 && warps != 2) return bfail(b, TBS_ERR_ARG, "warps per line must be 1 or 2");
     BGUARD_BEGIN
     if (cudaSetDevice(b->eng.device) != cudaSuccess) return bfail(b, TBS_ERR_CUDA, "cudaSetDevice failed");
-    BatchSched s = b->eng.sched;
+    BatchSched s = b->eng.sched_base;
     const int fit = b->eng.algo == TBS_ALGO_FP64 ? thomas_batch_fit<double>(s.stages, warps)
                                                  : thomas_batch_fit<float>(s.stages, warps);
     s.warps = warps;

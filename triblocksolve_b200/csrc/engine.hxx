@@ -52,6 +52,9 @@ struct Engine {
     int inner_first = 0;      /* > 0: the first outer step's (all members fresh together) */
     cudaStream_t stream = nullptr;
     BatchSched sched{8, 2, 1};
+    bool sched_set = false;   /* by the caller or by tuning; else by rule (engine_fit_schedule) */
+    BatchSched sched_base{8, 2, 1}; /* what a setter that leaves parts unsaid starts from */
+    bool grouped = false;     /* FP64: a system has had several members, so the graph has their launches */
     int order = 0;            /* Thomas items: 0 longest lines first, 1 mesh order */
     int max_nx = 0;           /* widest member (shared-memory size of the residual) */
     std::string err;
@@ -76,7 +79,7 @@ struct Engine {
     int cap_mitems = 0;
     int *d_g_tiles = nullptr, *d_g_prime = nullptr, *d_g_blocks = nullptr; /* group indices */
     int *d_g_chunks = nullptr; /* every member, units of BATCH_CHUNK tiles */
-    int *d_g_solo = nullptr;   /* members alone in their system, units of BATCH_CHUNK tiles */
+    int *d_g_solo = nullptr;   /* members alone in their system, units of single tiles */
     int *d_g_units = nullptr;  /* systems with several members, units of BATCH_CHUNK tiles */
     int *d_active = nullptr;
     unsigned *d_queue = nullptr, *d_counter = nullptr, *d_status = nullptr;
@@ -131,6 +134,8 @@ int engine_finish(Engine &e);
 /* times the persistent Thomas launch for each schedule that fits */
 int engine_tune(Engine &e, BatchSched *best, int *best_order, double *best_ms);
 int engine_set_schedule(Engine &e, BatchSched s, int order);
+/* the default schedule for a fixed set of systems, unless one was set */
+void engine_fit_schedule(Engine &e, const std::vector<tbs_ctx *> &systems);
 /* the active flags after the last run */
 int engine_read_active(Engine &e);
 

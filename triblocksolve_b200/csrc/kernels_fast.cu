@@ -2427,49 +2427,113 @@ __device__ __forceinline__ int chunk_end(int unit, int chunk, int ntiles) {
     return e < ntiles ? e : ntiles;
 }
 
-/* persistent residual over (member, tile or chunk) items: CTA k takes
- * items k, k + grid, ...; each tile completes one phase of the CTA's
- * barrier and writes its own partial */
-template <typename T, int CHUNK>
-__global__ void __launch_bounds__(RES_THREADS_FAST, CHUNK == 1 ? 8 : 6) fast_resid_batch_kernel(
+/* persistent residual over (member, tile) items: CTA k takes items k,
+ * k + grid, ...; each tile completes one phase of the CTA's barrier and writes
+ * its own partial */
+template <typename T>
+__global__ void __launch_bounds__(RES_THREADS_FAST, 8) fast_resid_batch_kernel(
     const ResidSys<T> *__restrict__ sys, const int *__restrict__ groups, int mode,
     const int *__restrict__ active, unsigned *status) {
-    constexpr int chunk = CHUNK;
     uint64_t *bar = resid_bar_init();
     const int nwork = group_items(groups);
     uint32_t parity = 0;
     GroupCursor gc;
-    bool ok = true;
-    for (int w = blockIdx.x; w < nwork && ok; w += gridDim.x) {
+    for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
         const WorkItem it = group_item_next(groups, w, gc);
         if (active && !active[it.sys]) continue;
         const ResidSys<T> S = sys[it.sys];
         NormSink ns{};
         ns.partials = (mode == 3) ? nullptr : S.partials; /* no counter: partials only */
-        const int t1 = chunk_end(it.unit, chunk, S.np16 / RES_TILE);
+        if (!fast_resid_body<T>(mode == 0 ? 0 : S.nx, S.np16, mode, S.Dinv, S.X, S.xnbr, S.dU, S.Rsrc, S.b,
+                                S.Uacc, ns, status, it.unit, bar, parity))
+            return;
+        parity ^= 1u;
+        __syncthreads(); /* the next tile's copies overwrite the stages */
+    }
+}
+
+/* A CTA's tiles of those of the active members of `groups` (one member a
+ * group, units of single tiles): run(member, first tile, tile behind the last)
+ * for each piece, until one returns false.  Full waves give each CTA
+ * BATCH_CHUNK consecutive tiles, the tiles left over are dealt equally to a
+ * tile.  (Equal consecutive shares of all tiles spread the CTAs' reads over
+ * the whole of memory: 8 systems of 600x640 took 15.4 ms, not 14.0.)  All
+ * threads take part; each warp makes the prefix sums for itself. */
+template <typename F>
+__device__ __forceinline__ void active_share(const int *__restrict__ groups, const int *__restrict__ active,
+                                             F &&run) {
+    const int ng = groups[0];
+    const int *base = groups + 1, *mlist = base + (ng + 1) + 2 * ng;
+    const int lane = threadIdx.x & 31;
+    auto tiles = [&](int g, int &m) {
+        m = g < ng ? mlist[g] : -1;
+        return m >= 0 && active[m] ? base[g + 1] - base[g] : 0;
+    };
+    int total = 0, m;
+    for (int g = lane; g - lane < ng; g += 32) total += tiles(g, m);
+    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(FULL, total, o);
+    const int wave = gridDim.x * BATCH_CHUNK;
+    for (int w0 = 0; w0 < total;) {
+        const int left = total - w0, deal = left < wave ? left : wave;
+        const int s = w0 + (int)((long long)deal * blockIdx.x / gridDim.x);
+        const int e = w0 + (int)((long long)deal * (blockIdx.x + 1) / gridDim.x);
+        w0 += deal;
+        int before = 0;
+        for (int g = lane; g - lane < ng && before < e; g += 32) {
+            const int n = tiles(g, m);
+            int pre = n;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int x = __shfl_up_sync(FULL, pre, o);
+                if (lane >= o) pre += x;
+            }
+            pre += before;
+            before = __shfl_sync(FULL, pre, 31);
+            pre -= n;
+            for (unsigned hit = __ballot_sync(FULL, pre < e && pre + n > s); hit; hit &= hit - 1) {
+                const int j = __ffs(hit) - 1;
+                const int p = __shfl_sync(FULL, pre, j), nj = __shfl_sync(FULL, n, j);
+                if (!run(__shfl_sync(FULL, m, j), max(s - p, 0), min(e - p, nj))) return;
+            }
+        }
+    }
+}
+
+/* The sweep residual (mode 1) of the members alone in their system.  HBM
+ * bounds it, as the single-system launch, when every CTA has the same work:
+ * dealt in chunks of 8 tiles, 12 systems of 117 000 cells together gave 37 of
+ * 888 CTAs a second chunk and took 66 us for 53 now. */
+template <typename T>
+__global__ void __launch_bounds__(RES_THREADS_FAST, 6) fast_resid_solo_kernel(
+    const ResidSys<T> *__restrict__ sys, const int *__restrict__ groups, const int *__restrict__ active,
+    unsigned *status) {
+    uint64_t *bar = resid_bar_init();
+    uint32_t parity = 0;
+    active_share(groups, active, [&](int member, int tb, int t1) {
+        const ResidSys<T> S = sys[member];
+        NormSink ns{};
+        ns.partials = S.partials; /* no counter: partials only */
         /* the next tile's neighbour indices load during the current tile */
-        const int nxm = mode == 0 ? 0 : S.nx;
-        const bool pre = CHUNK > 1 && nxm >= 1 && nxm <= 4 && threadIdx.x < RES_TILE * NV;
+        const bool pre = S.nx >= 1 && S.nx <= 4 && threadIdx.x < RES_TILE * NV;
         const int c = threadIdx.x % RES_TILE;
         int nbr[4], nxt[4];
-        const int tb = it.unit * chunk;
 #pragma unroll
         for (int s = 0; s < 4; ++s)
-            nbr[s] = (pre && s < nxm && tb < t1) ? S.xnbr[(size_t)s * S.np16 + tb * RES_TILE + c] : -1;
+            nbr[s] = (pre && s < S.nx) ? S.xnbr[(size_t)s * S.np16 + tb * RES_TILE + c] : -1;
         for (int t = tb; t < t1; ++t) {
 #pragma unroll
             for (int s = 0; s < 4; ++s)
-                nxt[s] = (pre && s < nxm && t + 1 < t1) ? S.xnbr[(size_t)s * S.np16 + (t + 1) * RES_TILE + c]
-                                                        : -1;
-            ok = fast_resid_body<T>(nxm, S.np16, mode, S.Dinv, S.X, S.xnbr, S.dU, S.Rsrc, S.b, S.Uacc, ns,
-                                    status, t, bar, parity, pre ? nbr : nullptr);
+                nxt[s] = (pre && s < S.nx && t + 1 < t1) ? S.xnbr[(size_t)s * S.np16 + (t + 1) * RES_TILE + c]
+                                                         : -1;
+            const bool ok = fast_resid_body<T>(S.nx, S.np16, 1, S.Dinv, S.X, S.xnbr, S.dU, S.Rsrc, S.b, S.Uacc,
+                                               ns, status, t, bar, parity, pre ? nbr : nullptr);
             parity ^= 1u;
-            if (!ok) break;
+            if (!ok) return false;
 #pragma unroll
             for (int s = 0; s < 4; ++s) nbr[s] = nxt[s];
             __syncthreads(); /* the next tile's copies overwrite the stages */
         }
-    }
+        return true;
+    });
 }
 
 /* Item w of a unit index (the group index layout with base[] the prefix
@@ -2665,19 +2729,19 @@ static int resid_batch_grid(size_t smem, const void *fn) {
 
 template <typename T>
 int launch_resid_batch(cudaStream_t st, int mode, int max_nx, const ResidSys<T> *sys,
-                       const int *groups, int chunk, const int *active, unsigned *status) {
-    if (mode != 0 && mode != 1 && mode != 3) return (int)cudaErrorInvalidValue;
-    if (chunk != 1 && chunk != BATCH_CHUNK) return (int)cudaErrorInvalidValue;
+                       const int *groups, const int *active, unsigned *status) {
+    if (mode != 0 && mode != 3) return (int)cudaErrorInvalidValue;
     const size_t smem = resid_smem_bytes<T>(mode == 0 ? 0 : max_nx);
-    if (chunk == 1) {
-        const int grid = resid_batch_grid(smem, (const void *)fast_resid_batch_kernel<T, 1>);
-        fast_resid_batch_kernel<T, 1><<<grid, RES_THREADS_FAST, smem, st>>>(sys, groups, mode, active,
-                                                                            status);
-    } else {
-        const int grid = resid_batch_grid(smem, (const void *)fast_resid_batch_kernel<T, BATCH_CHUNK>);
-        fast_resid_batch_kernel<T, BATCH_CHUNK><<<grid, RES_THREADS_FAST, smem, st>>>(sys, groups, mode,
-                                                                                      active, status);
-    }
+    const int grid = resid_batch_grid(smem, (const void *)fast_resid_batch_kernel<T>);
+    fast_resid_batch_kernel<T><<<grid, RES_THREADS_FAST, smem, st>>>(sys, groups, mode, active, status);
+    return (int)cudaGetLastError();
+}
+
+int launch_resid_solo(cudaStream_t st, int max_nx, const ResidSys<double> *sys, const int *groups,
+                      const int *active, unsigned *status) {
+    const size_t smem = resid_smem_bytes<double>(max_nx);
+    const int grid = resid_batch_grid(smem, (const void *)fast_resid_solo_kernel<double>);
+    fast_resid_solo_kernel<double><<<grid, RES_THREADS_FAST, smem, st>>>(sys, groups, active, status);
     return (int)cudaGetLastError();
 }
 
@@ -2884,15 +2948,9 @@ int launch_reduce_batch(cudaStream_t st, int threads, const ReduceSys *sys, cons
 /* opt the batched kernels into the shared memory of the widest member
  * (outside stream capture) */
 int batch_prepare(int max_nx) {
-    int rc = set_smem((const void *)fast_resid_batch_kernel<double, 1>, resid_smem_bytes<double>(max_nx));
-    if (!rc)
-        rc = set_smem((const void *)fast_resid_batch_kernel<double, BATCH_CHUNK>,
-                      resid_smem_bytes<double>(max_nx));
-    if (!rc)
-        rc = set_smem((const void *)fast_resid_batch_kernel<float, 1>, resid_smem_bytes<float>(max_nx));
-    if (!rc)
-        rc = set_smem((const void *)fast_resid_batch_kernel<float, BATCH_CHUNK>,
-                      resid_smem_bytes<float>(max_nx));
+    int rc = set_smem((const void *)fast_resid_batch_kernel<double>, resid_smem_bytes<double>(max_nx));
+    if (!rc) rc = set_smem((const void *)fast_resid_solo_kernel<double>, resid_smem_bytes<double>(max_nx));
+    if (!rc) rc = set_smem((const void *)fast_resid_batch_kernel<float>, resid_smem_bytes<float>(max_nx));
     if (!rc)
         rc = set_smem((const void *)fast_resid_group_kernel<double>, resid_smem_bytes<double>(max_nx));
 
@@ -2914,10 +2972,10 @@ template int launch_thomas_batch<double>(cudaStream_t, const BatchSched &, const
 template int launch_thomas_batch<float>(cudaStream_t, const BatchSched &, const ThomasSys<float> *,
                                         const WorkItem *, const int *, const int *, unsigned *,
                                         unsigned *);
-template int launch_resid_batch<double>(cudaStream_t, int, int, const ResidSys<double> *,
-                                        const int *, int, const int *, unsigned *);
-template int launch_resid_batch<float>(cudaStream_t, int, int, const ResidSys<float> *,
-                                       const int *, int, const int *, unsigned *);
+template int launch_resid_batch<double>(cudaStream_t, int, int, const ResidSys<double> *, const int *,
+                                        const int *, unsigned *);
+template int launch_resid_batch<float>(cudaStream_t, int, int, const ResidSys<float> *, const int *,
+                                        const int *, unsigned *);
 
 
 /* ============================================== several right-hand sides

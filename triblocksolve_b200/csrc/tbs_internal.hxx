@@ -440,11 +440,15 @@ inline int batch_chunks(int ntiles) { return (ntiles + BATCH_CHUNK - 1) / BATCH_
 inline size_t group_index_ints(int max_groups, int max_members) {
     return 1 + (size_t)(max_groups + 1) + 2 * (size_t)max_groups + (size_t)max_members;
 }
+/* mode 0 or 3 of every member; units of `groups`: single tiles */
 template <typename T>
-/* units of `groups`: single tiles (chunk 1) or chunks of BATCH_CHUNK tiles */
 int launch_resid_batch(cudaStream_t st, int mode, int max_nx, const ResidSys<T> *sys,
-                       const int *groups, int chunk, const int *active, unsigned *status);
-/* the sweep residual (mode 1) of every member, the members of one system
+                       const int *groups, const int *active, unsigned *status);
+/* the sweep residual (mode 1) of the members alone in their system; groups of
+ * one member, units single tiles */
+int launch_resid_solo(cudaStream_t st, int max_nx, const ResidSys<double> *sys, const int *groups,
+                      const int *active, unsigned *status);
+/* the sweep residual (mode 1) of systems with several members, the members of one system
  * together over one staging of its blocks per tile; gunits: the group
  * index of the members with base[] the prefix sums of units (chunks of
  * `chunk` tiles) per group */
