@@ -74,3 +74,32 @@ def test_default_schedule(nl, nk, n, want):
         batch.close()
         for s in solvers:
             s.close()
+
+
+@pytest.mark.parametrize("limit", [3, 60, 70000])
+def test_history_rows(limit):
+    """States and norms come back in one launch while the rows take at most
+    1 MiB (two rows of 70001 norms: 1.07 MiB, copied one by one); rows shorter
+    than the solve (3 sweeps) end at the limit."""
+    solvers = []
+    for i, (nl, nk, shift) in enumerate([(9, 31, 9.0), (4, 17, 4.0)]):
+        mesh = Mesh.structured(nl, nk)
+        s = Solver(0)
+        s.set_mesh(mesh)
+        s.set_jacobian(Jacobian.generate(mesh, shift, i))
+        s.factor(ALGO_FP64)
+        solvers.append(s)
+    batch = Batch(solvers)
+    try:
+        for _ in range(2):
+            sweeps, hist = batch.solve(1e-11, limit)
+            got = [s.solution() for s in solvers]
+            for k, s in enumerate(solvers):
+                n, h = s.solve(1e-11, limit)
+                assert n == sweeps[k]
+                np.testing.assert_array_equal(hist[k][: n + 1], h)
+                np.testing.assert_array_equal(got[k], s.solution())
+    finally:
+        batch.close()
+        for s in solvers:
+            s.close()

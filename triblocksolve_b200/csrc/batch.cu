@@ -1046,7 +1046,13 @@ struct tbs_batch {
     cudaStream_t own = nullptr;
     std::vector<tbs_ctx *> sys;
     std::vector<const void *> fingerprint;
+    char *h_out = nullptr; /* pinned: states, then rows of norms (batch_collect) */
+    size_t out_cap = 0;
 };
+
+/* bytes of norms a batch collects in one launch; longer histories are copied
+ * row by row */
+constexpr size_t COLLECT_MAX = size_t(1) << 20;
 
 static int bfail(tbs_batch *b, int code, const std::string &msg) {
     if (b) b->eng.err = msg;
@@ -1095,15 +1101,18 @@ static int batch_check_members(tbs_batch *b) {
 static int batch_ready(tbs_batch *b, double tol, int max_sweeps) {
     int rc = batch_check_members(b);
     if (rc) return rc;
+    /* the members' controls go out on their streams, behind what they still
+     * run, and are waited for together (one after the other: 8 us each) */
     for (tbs_ctx *c : b->sys) {
-        if (cudaStreamSynchronize(c->stream) != cudaSuccess)
+        if (max_sweeps + 1 > c->hist_cap && cudaStreamSynchronize(c->stream) != cudaSuccess)
             return bfail(b, TBS_ERR_CUDA, "member stream synchronisation failed");
         rc = ctx_ensure_hist(c, max_sweeps + 1);
         if (!rc) rc = ctx_set_state(c, tol, max_sweeps);
         if (rc) return bfail(b, rc, "batch member: " + c->err);
+    }
+    for (tbs_ctx *c : b->sys)
         if (cudaStreamSynchronize(c->stream) != cudaSuccess)
             return bfail(b, TBS_ERR_CUDA, "member stream synchronisation failed");
-    }
     std::vector<const void *> fp = batch_fingerprint(b);
     if (fp != b->fingerprint) {
         std::vector<Member> m;
@@ -1121,6 +1130,7 @@ static int batch_destroy_all(tbs_batch *b) {
     if (!b) return TBS_OK;
     cudaSetDevice(b->eng.device);
     engine_free(b->eng);
+    if (b->h_out) cudaFreeHost(b->h_out);
     if (b->own) cudaStreamDestroy(b->own);
     delete b;
     return TBS_OK;
@@ -1268,26 +1278,45 @@ int tbs_batch_solve(tbs_batch *b, double rel_tol, int max_sweeps, int *sweeps_ou
     if (cudaSetDevice(b->eng.device) != cudaSuccess) return bfail(b, TBS_ERR_CUDA, "cudaSetDevice failed");
     int rc = batch_ready(b, rel_tol, max_sweeps);
     if (rc) return rc;
-    rc = engine_run(b->eng, 0, 0);
-    if (rc) return rc;
-    cudaStream_t st = b->eng.stream;
     const int n = (int)b->sys.size();
-    for (int s = 0; s < n; ++s) {
-        tbs_ctx *c = b->sys[s];
-        if (xfer_to_host(st, c->h_state, c->d_state, sizeof(SolveState), 1) != 0)
-            return bfail(b, TBS_ERR_CUDA, "state read-back failed");
+    const size_t at = ((size_t)n * sizeof(SolveState) + 15) / 16 * 16;
+    const size_t row = (size_t)(hist_out ? max_sweeps + 1 : 0);
+    const size_t norms = n * row * sizeof(double);
+    const bool together = norms <= COLLECT_MAX;
+    const size_t need = at + (together ? norms : 0);
+    if (need > b->out_cap) {
+        if (b->h_out) cudaFreeHost(b->h_out);
+        b->h_out = nullptr;
+        b->out_cap = 0;
+        if (cudaMallocHost(&b->h_out, need) != cudaSuccess)
+            return bfail(b, TBS_ERR_NOMEM, "pinned allocation failed");
+        b->out_cap = need;
     }
-    if (cudaStreamSynchronize(st) != cudaSuccess) return bfail(b, TBS_ERR_CUDA, "synchronisation failed");
+    SolveState *states = reinterpret_cast<SolveState *>(b->h_out);
+    double *rows = reinterpret_cast<double *>(b->h_out + at);
+    rc = engine_launch(b->eng, 0, 0);
+    if (rc) return rc;
+    /* one launch behind the solve brings every member's state and norms, and
+     * one wait serves them and the status (copies member by member, the norms
+     * to pageable memory: 12 members 200 us) */
+    cudaStream_t st = b->eng.stream;
+    if (launch_batch_collect(st, b->eng.d_red_body, n, states, rows, together ? (int)row : 0) != 0)
+        return bfail(b, TBS_ERR_CUDA, "state read-back failed");
+    rc = engine_finish(b->eng);
+    if (rc) return rc;
     for (int s = 0; s < n; ++s) {
         tbs_ctx *c = b->sys[s];
-        const int sw = c->h_state->sweep;
+        *c->h_state = states[s];
+        const int sw = states[s].sweep;
         if (sweeps_out) sweeps_out[s] = sw;
-        if (hist_out &&
-            xfer_to_host(st, hist_out + (size_t)s * (max_sweeps + 1), c->d_hist,
-                         (size_t)(std::min(sw, max_sweeps) + 1) * sizeof(double), 1) != 0)
+        const size_t count = (size_t)(std::min(sw, max_sweeps) + 1);
+        if (hist_out && together)
+            std::memcpy(hist_out + s * row, rows + s * row, count * sizeof(double));
+        else if (hist_out && xfer_to_host(st, hist_out + s * row, c->d_hist, count * sizeof(double), 1) != 0)
             return bfail(b, TBS_ERR_CUDA, "history read-back failed");
     }
-    if (cudaStreamSynchronize(st) != cudaSuccess) return bfail(b, TBS_ERR_CUDA, "synchronisation failed");
+    if (!together && cudaStreamSynchronize(st) != cudaSuccess)
+        return bfail(b, TBS_ERR_CUDA, "synchronisation failed");
     return TBS_OK;
     BGUARD_END
 }

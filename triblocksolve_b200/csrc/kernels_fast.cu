@@ -2945,6 +2945,23 @@ int launch_reduce_batch(cudaStream_t st, int threads, const ReduceSys *sys, cons
     return (int)cudaGetLastError();
 }
 
+/* member blockIdx.x's state and the norms of its history to host rows of
+ * `stride` norms */
+__global__ void batch_collect_kernel(const ReduceSys *__restrict__ sys, SolveState *states, double *hist,
+                                     int stride) {
+    const ReduceSys R = sys[blockIdx.x];
+    const int n = min(R.state->sweep + 1, stride);
+    if (threadIdx.x == 0) states[blockIdx.x] = *R.state;
+    for (int k = threadIdx.x; k < n; k += blockDim.x) hist[(size_t)blockIdx.x * stride + k] = R.hist[k];
+}
+
+int launch_batch_collect(cudaStream_t st, const ReduceSys *sys, int n, SolveState *states, double *hist,
+                         int stride) {
+    if (n <= 0) return 0;
+    batch_collect_kernel<<<n, 64, 0, st>>>(sys, states, hist, stride);
+    return (int)cudaGetLastError();
+}
+
 /* opt the batched kernels into the shared memory of the widest member
  * (outside stream capture) */
 int batch_prepare(int max_nx) {

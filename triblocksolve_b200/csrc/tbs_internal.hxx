@@ -470,6 +470,10 @@ int launch_reduce_batch(cudaStream_t st, int threads, const ReduceSys *sys, cons
                         int cap, int is_start, int *active, BatchCtl *ctl, unsigned *counter,
                         unsigned long long cond_handle, int use_cond,
                         unsigned long long cond_handle2 = 0, int use2 = 0);
+/* states and norm histories (rows of `stride`) of n members to pinned host
+ * memory in one launch */
+int launch_batch_collect(cudaStream_t st, const ReduceSys *sys, int n, SolveState *states, double *hist,
+                         int stride);
 int batch_prepare(int max_nx);
 
 }  // namespace tbs
