@@ -3419,22 +3419,106 @@ int launch_multi_thomas_items(cudaStream_t st, int grid, const MultiLine *sys, c
 /* Residual of several right-hand sides per tile: Dinv and the cross-line
  * blocks are staged once, then for every active right-hand side r
  *   mode 0 (the start):  R = Rsrc_r (staged), U_r = 0
- *   mode 1 (a sweep):    R = sum X dU_r (gathers of all r issued together),
- *                        U_r += dU_r
+ *   mode 1 (a sweep):    R = sum X dU_r, U_r += dU_r
  * followed by b_r = -Dinv R and the tile's sum R^2 for r, each with the
  * expressions (and summation order) of fast_resid_body.  The last CTA to
  * finish adds every active r's partials in tile order (finalize_total's
  * order), records the norms, retires the right-hand sides whose solve has
- * ended and keeps the graph's loop running while any is active. */
+ * ended and keeps the graph's loop running while any is active.
+ *
+ * HBM would take 90 us for 8 right-hand sides at 360x384; shared memory is
+ * what bounds it.  A thread per (cell, row) that loads a block's row once and
+ * each right-hand side's vector for itself reads ten words for nine products
+ * and took 214 us at three quarters of the L1's throughput.  Here a thread has
+ * three rows (i0, i0 + 3, i0 + 6) of a cell for three right-hand sides, six
+ * words for nine products, without a branch for each; a cell's vectors arrive
+ * by asynchronous copies of adjacent words, the sums of squares of eight
+ * right-hand sides go down the lanes together (nine exchanges for forty), and
+ * R takes the place of the blocks it was made of, so that four CTAs fit an
+ * SM: 150 us. */
+constexpr int MULTI_KG = 3;                                    /* right-hand sides of a thread */
+static_assert(3 * MULTI_KG >= MULTI_MAX && RES_TILE * 9 <= RES_THREADS_FAST, "three groups of threads");
+
 static size_t multi_resid_smem(int nx, int nr) {
     const int nxa = nx > 0 ? nx : 1;
-    return 128 + (size_t)RES_TILE * NB * sizeof(double) * (1 + nx) +
-           (size_t)nr * nxa * RES_TILE * NV * sizeof(double) +
-           (size_t)nr * RES_TILE * NV * sizeof(double);
+    const size_t vec = (size_t)nr * RES_TILE * NV, blk = (size_t)RES_TILE * NB;
+    return 128 + (blk + std::max(nx * blk, vec) + nxa * vec) * sizeof(double);
+}
+
+/* rows i0, i0 + 3, i0 + 6 of a block times the vectors at v0 + off[k], in
+ * fast_resid_body's order */
+struct MultiAcc {
+    double a[MULTI_KG][3][3];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int k = 0; k < MULTI_KG; ++k)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) a[k][q][0] = a[k][q][1] = a[k][q][2] = 0.0;
+    }
+    __device__ __forceinline__ void add(const double *row, const double *v0, const int (&off)[MULTI_KG]) {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const double x0 = row[9 * j], x1 = row[9 * j + 3], x2 = row[9 * j + 6];
+#pragma unroll
+            for (int k = 0; k < MULTI_KG; ++k) {
+                const double v = v0[off[k] + j];
+                a[k][0][j % 3] += x0 * v;
+                a[k][1][j % 3] += x1 * v;
+                a[k][2][j % 3] += x2 * v;
+            }
+        }
+    }
+    /* the same in neg_dinv_row's order: products j and j + 3 open sum j, the
+     * latter rounded (what the compiler makes of the sum of two products) */
+    __device__ __forceinline__ void set(const double *row, const double *v0, const int (&off)[MULTI_KG]) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            double x[3][3];
+#pragma unroll
+            for (int m = 0; m < 3; ++m)
+#pragma unroll
+                for (int q = 0; q < 3; ++q) x[m][q] = row[9 * (j + 3 * m) + 3 * q];
+#pragma unroll
+            for (int k = 0; k < MULTI_KG; ++k) {
+                const double *v = v0 + off[k] + j;
+                const double u0 = v[0], u1 = v[3], u2 = v[6];
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+                    a[k][q][j] = __fma_rn(x[2][q], u2, __fma_rn(x[0][q], u0, __dmul_rn(x[1][q], u1)));
+            }
+        }
+    }
+    __device__ __forceinline__ double sum(int k, int q) const { return a[k][q][0] + (a[k][q][1] + a[k][q][2]); }
+};
+
+/* the warp's sums of v[0..8) (SQ: squared), each with the pairs of a shfl_down
+ * tree; lane 4 k has that of v[k] */
+template <bool SQ>
+__device__ __forceinline__ double warp_sums8(const double (&v)[8]) {
+    const int lane = threadIdx.x & 31;
+    double w[4], x[2], y;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const double keep = lane & 16 ? v[k + 4] : v[k], give = lane & 16 ? v[k] : v[k + 4];
+        const double got = __shfl_xor_sync(FULL, give, 16);
+        w[k] = SQ ? __dadd_rn(__dmul_rn(keep, keep), __dmul_rn(got, got)) : keep + got;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const double keep = lane & 8 ? w[k + 2] : w[k], give = lane & 8 ? w[k] : w[k + 2];
+        x[k] = keep + __shfl_xor_sync(FULL, give, 8);
+    }
+    {
+        const double keep = lane & 4 ? x[1] : x[0], give = lane & 4 ? x[0] : x[1];
+        y = keep + __shfl_xor_sync(FULL, give, 4);
+    }
+    y += __shfl_xor_sync(FULL, y, 2);
+    y += __shfl_xor_sync(FULL, y, 1);
+    return y;
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(RES_THREADS_FAST) multi_resid_kernel(
+__global__ void __launch_bounds__(RES_THREADS_FAST, 4) multi_resid_kernel(
     MultiSys M, const double *__restrict__ Dinv, const double *__restrict__ X,
     const int *__restrict__ xnbr, const double *__restrict__ Rsrc, unsigned long long handle,
     int use_cond, unsigned *status) {
@@ -3449,9 +3533,9 @@ __global__ void __launch_bounds__(RES_THREADS_FAST) multi_resid_kernel(
     const int ntiles = M.np16 / RES_TILE;
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem);
     double *sD = reinterpret_cast<double *>(smem + 128);
-    double *sX = sD + RES_TILE * NB;
-    double *sg = sX + nx * RES_TILE * NB; /* [k][s][c][i] gathers; mode 0: [k][c][i] R */
-    double *sr = sg + (size_t)nr * nxa * RES_TILE * NV; /* [k][c][i] R, then b */
+    double *sg = sD + RES_TILE * NB; /* [k][s][c][i] gathers, then b; mode 0: R */
+    double *sX = sg + (size_t)nr * nxa * RES_TILE * NV;
+    double *sr = sX; /* [k][c][i] R, in the place of the blocks it was made of; mode 0: b */
     __shared__ int rid[MULTI_MAX]; /* the k-th active right-hand side */
     if (tid == 0) {
         unsigned am = 0;
@@ -3468,8 +3552,23 @@ __global__ void __launch_bounds__(RES_THREADS_FAST) multi_resid_kernel(
     __syncthreads();
     const unsigned amask = amask_s;
     const int nact = __popc(amask);
-    const int c = tid % RES_TILE, i = tid / RES_TILE;
     const bool act = tid < RES_TILE * NV;
+    /* products: a cell, three of its rows, a group of right-hand sides */
+    const int c = tid % RES_TILE, i0 = (tid / RES_TILE) % 3;
+    const int k0 = tid / RES_TILE / 3 * MULTI_KG;
+    const int ng = act ? max(0, min(MULTI_KG, nact - k0)) : 0;
+    /* (a group that is not full repeats its last one and does not store it) */
+    int offg[MULTI_KG], offr[MULTI_KG];
+#pragma unroll
+    for (int k = 0; k < MULTI_KG; ++k) {
+        const int kk = max(0, min(k0 + k, nact - 1));
+        offg[k] = kk * nx * RES_TILE * NV;
+        offr[k] = kk * RES_TILE * NV;
+    }
+    /* loads: a word of a cell's vectors; the norm: (cell, row) as
+     * fast_resid_body deals them */
+    const int lc = tid / NV, li = tid % NV;
+    const int nat = c * NV + tid / RES_TILE;
     const uint32_t szD = RES_TILE * NB * sizeof(double), szR = RES_TILE * NV * sizeof(double);
     uint32_t parity = 0;
     bool failed = false;
@@ -3478,15 +3577,10 @@ __global__ void __launch_bounds__(RES_THREADS_FAST) multi_resid_kernel(
 #pragma unroll
     for (int s = 0; s < MULTI_NX; ++s)
         pnbr[s] = (MODE == 1 && act && s < nx && (int)blockIdx.x < ntiles)
-                      ? __ldg(xnbr + (size_t)s * M.np16 + blockIdx.x * RES_TILE + c) : -1;
+                      ? __ldg(xnbr + (size_t)s * M.np16 + blockIdx.x * RES_TILE + lc) : -1;
     for (int blk = blockIdx.x; blk < ntiles && nact > 0; blk += gridDim.x) {
         const int p0 = blk * RES_TILE;
         const int bn = blk + gridDim.x;
-        int pnxt[MULTI_NX];
-#pragma unroll
-        for (int s = 0; s < MULTI_NX; ++s)
-            pnxt[s] = (MODE == 1 && act && s < nx && bn < ntiles)
-                          ? __ldg(xnbr + (size_t)s * M.np16 + bn * RES_TILE + c) : -1;
         if (tid == 0) {
             const uint64_t pol = policy_evict_first();
             mbar_arrive_expect_tx(bar, szD + (MODE == 1 ? nx * szD : nact * szR));
@@ -3508,36 +3602,36 @@ __global__ void __launch_bounds__(RES_THREADS_FAST) multi_resid_kernel(
         if (act) {
             const size_t q = (size_t)p0 * NV + tid;
             if (MODE == 1) {
-                /* every load of the tile (the neighbour dU gathers, U and dU
-                 * of each active r) is issued before the first store, so
-                 * that their latencies overlap */
-                int nbr[MULTI_NX];
+                for (int k = 0; k < nact; ++k) {
+                    const double *d = M.dU + (size_t)rid[k] * vs + li;
 #pragma unroll
-                for (int s = 0; s < MULTI_NX; ++s) nbr[s] = pnbr[s];
-                double gv[MULTI_MAX][MULTI_NX], uv[MULTI_MAX], dv[MULTI_MAX];
+                    for (int s = 0; s < MULTI_NX; ++s)
+                        if (s < nx) {
+                            double *to = sg + (size_t)(k * nx + s) * RES_TILE * NV + tid;
+                            if (pnbr[s] >= 0) cp_async8(to, d + (size_t)pnbr[s] * NV);
+                            else *to = 0.0;
+                        }
+                }
+                cp_async_commit();
+                /* every load is issued before the first store */
+                double uv[MULTI_MAX], dv[MULTI_MAX];
 #pragma unroll
                 for (int k = 0; k < MULTI_MAX; ++k) {
                     uv[k] = dv[k] = 0.0;
-#pragma unroll
-                    for (int s = 0; s < MULTI_NX; ++s) gv[k][s] = 0.0;
                     if (k < nact) {
                         const size_t ro = (size_t)rid[k] * vs;
-#pragma unroll
-                        for (int s = 0; s < MULTI_NX; ++s)
-                            if (nbr[s] >= 0) gv[k][s] = __ldg(M.dU + ro + (size_t)nbr[s] * NV + i);
                         uv[k] = M.U[ro + q];
                         dv[k] = __ldg(M.dU + ro + q);
                     }
                 }
 #pragma unroll
-                for (int k = 0; k < MULTI_MAX; ++k) {
-                    if (k < nact) {
+                for (int s = 0; s < MULTI_NX; ++s)
+                    pnbr[s] = (s < nx && bn < ntiles)
+                                  ? __ldg(xnbr + (size_t)s * M.np16 + bn * RES_TILE + lc) : -1;
 #pragma unroll
-                        for (int s = 0; s < MULTI_NX; ++s)
-                            if (s < nx) sg[((size_t)(k * nx + s) * RES_TILE + c) * NV + i] = gv[k][s];
-                        M.U[(size_t)rid[k] * vs + q] = uv[k] + dv[k];
-                    }
-                }
+                for (int k = 0; k < MULTI_MAX; ++k)
+                    if (k < nact) M.U[(size_t)rid[k] * vs + q] = uv[k] + dv[k];
+                cp_async_wait<0>();
             } else {
                 for (int k = 0; k < nact; ++k) M.U[(size_t)rid[k] * vs + q] = 0.0;
             }
@@ -3552,112 +3646,50 @@ __global__ void __launch_bounds__(RES_THREADS_FAST) multi_resid_kernel(
             failed = true;
             break;
         }
-        /* R for every active r: the row of each slot's block is read once
-         * and feeds every r; per r the products are added in
-         * fast_resid_body's order (slots ascending, three accumulators) */
-        double sq[MULTI_MAX];
+        MultiAcc acc;
+        if (MODE == 1) {
+            acc.clear();
+            if (ng > 0)
+                for (int s = 0; s < nx; ++s)
+                    acc.add(sX + (s * RES_TILE + c) * NB + i0, sg + (s * RES_TILE + c) * NV, offg);
+            __syncthreads(); /* the blocks are read */
 #pragma unroll
-        for (int k = 0; k < MULTI_MAX; ++k) sq[k] = 0.0;
-        if (act) {
-            if (MODE == 1) {
-                double a0[MULTI_MAX], a1[MULTI_MAX], a2[MULTI_MAX];
+            for (int k = 0; k < MULTI_KG; ++k)
+                if (k < ng) {
 #pragma unroll
-                for (int k = 0; k < MULTI_MAX; ++k) a0[k] = a1[k] = a2[k] = 0.0;
-                for (int s = 0; s < nx; ++s) {
-                    const double *xr = sX + (s * RES_TILE + c) * NB + i;
-                    double x[NV];
-#pragma unroll
-                    for (int j = 0; j < NV; ++j) x[j] = xr[9 * j];
-#pragma unroll
-                    for (int k = 0; k < MULTI_MAX; ++k) {
-                        if (k < nact) {
-                            const double *g = sg + ((size_t)(k * nx + s) * RES_TILE + c) * NV;
-                            a0[k] += x[0] * g[0];
-                            a1[k] += x[1] * g[1];
-                            a2[k] += x[2] * g[2];
-                            a0[k] += x[3] * g[3];
-                            a1[k] += x[4] * g[4];
-                            a2[k] += x[5] * g[5];
-                            a0[k] += x[6] * g[6];
-                            a1[k] += x[7] * g[7];
-                            a2[k] += x[8] * g[8];
-                        }
-                    }
+                    for (int q = 0; q < 3; ++q)
+                        sr[(size_t)(k0 + k) * RES_TILE * NV + c * NV + i0 + 3 * q] = acc.sum(k, q);
                 }
-#pragma unroll
-                for (int k = 0; k < MULTI_MAX; ++k) {
-                    if (k < nact) {
-                        const double rr = a0[k] + (a1[k] + a2[k]);
-                        sr[(size_t)k * RES_TILE * NV + c * NV + i] = rr;
-                        sq[k] = rr * rr;
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int k = 0; k < MULTI_MAX; ++k) {
-                    if (k < nact) {
-                        const double rr = sg[(size_t)k * RES_TILE * NV + c * NV + i];
-                        sq[k] = rr * rr;
-                    }
-                }
-            }
+            __syncthreads();
         }
-        __syncthreads();
-        /* b = -Dinv R for every active r (into sg, free now); the row of
-         * Dinv is read once */
+        /* b = -Dinv R for every active r (into sg, free now), and R^2 */
         const double *rsrc = MODE == 1 ? sr : sg;
         double *sb = MODE == 1 ? sg : sr;
-        if (act) {
-            const double *drow = sD + c * NB + i;
-            double dr[NV];
+        if (ng > 0) acc.set(sD + c * NB + i0, rsrc + c * NV, offr);
 #pragma unroll
-            for (int j = 0; j < NV; ++j) dr[j] = drow[9 * j];
+        for (int k = 0; k < MULTI_KG; ++k)
+            if (k < ng) {
 #pragma unroll
-            for (int k = 0; k < MULTI_MAX; ++k) {
-                if (k < nact) {
-                    const double *rv = rsrc + (size_t)k * RES_TILE * NV + c * NV;
-                    double a0 = dr[0] * rv[0], a1 = dr[1] * rv[1], a2 = dr[2] * rv[2];
-                    a0 += dr[3] * rv[3];
-                    a1 += dr[4] * rv[4];
-                    a2 += dr[5] * rv[5];
-                    a0 += dr[6] * rv[6];
-                    a1 += dr[7] * rv[7];
-                    a2 += dr[8] * rv[8];
-                    sb[(size_t)k * RES_TILE * NV + c * NV + i] = -(a0 + (a1 + a2));
-                }
+                for (int q = 0; q < 3; ++q)
+                    sb[(size_t)(k0 + k) * RES_TILE * NV + c * NV + i0 + 3 * q] = -acc.sum(k, q);
             }
-        }
-        __syncthreads();
-        if (act) {
-            int k = 0;
-            for (int r = 0; r < nr; ++r) {
-                if (!((amask >> r) & 1u)) continue;
-                M.b[(size_t)r * vs + (size_t)p0 * NV + tid] = sb[(size_t)k * RES_TILE * NV + tid];
-                ++k;
-            }
-        }
         /* the tile's sum R^2 per r, in fast_resid_body's order */
+        double rr[MULTI_MAX];
 #pragma unroll
-        for (int k = 0; k < MULTI_MAX; ++k) {
-            if (k < nact) {
-                double v = sq[k];
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(FULL, v, o);
-                if ((tid & 31) == 0) red[k][tid >> 5] = v;
-            }
-        }
+        for (int k = 0; k < MULTI_MAX; ++k)
+            rr[k] = act && k < nact ? rsrc[(size_t)k * RES_TILE * NV + nat] : 0.0;
+        const double ws = warp_sums8<true>(rr);
+        if ((tid & 3) == 0) red[(tid & 31) >> 2][tid >> 5] = ws;
         __syncthreads();
-        if (tid == 0) {
-            int k = 0;
-            for (int r = 0; r < nr; ++r) {
-                if (!((amask >> r) & 1u)) continue;
-                double tot = 0.0;
-                for (int w = 0; w < RES_THREADS_FAST / 32; ++w) tot += red[k][w];
-                M.partials[(size_t)r * ntiles + blk] = tot;
-                ++k;
-            }
+        if (act)
+            for (int k = 0; k < nact; ++k)
+                M.b[(size_t)rid[k] * vs + (size_t)p0 * NV + tid] = sb[(size_t)k * RES_TILE * NV + tid];
+        if (tid < nact) {
+            double tot = 0.0;
+            for (int w = 0; w < RES_THREADS_FAST / 32; ++w) tot += red[tid][w];
+            M.partials[(size_t)rid[tid] * ntiles + blk] = tot;
         }
-#pragma unroll
-        for (int s = 0; s < MULTI_NX; ++s) pnbr[s] = pnxt[s];
+        if (MODE == 1) fence_async_smem(); /* R was stored where blocks are copied to */
         __syncthreads(); /* the next tile's copies overwrite the stages */
     }
     (void)failed;
@@ -3671,35 +3703,56 @@ __global__ void __launch_bounds__(RES_THREADS_FAST) multi_resid_kernel(
     __syncthreads();
     if (ticket != gridDim.x - 1) return;
     __threadfence();
-    __shared__ int any_go;
-    if (tid == 0) any_go = 0;
-    for (int r = 0; r < nr; ++r) {
-        if (!((amask >> r) & 1u)) continue;
-        double acc = strided_sum(M.partials + (size_t)r * ntiles, ntiles, (int)blockDim.x);
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(FULL, acc, o);
-        __syncthreads(); /* red[0] of the previous r is read */
-        if ((tid & 31) == 0) red[0][tid >> 5] = acc;
-        __syncthreads();
-        if (tid == 0) {
-            double tot = 0.0;
-            for (int w = 0; w < (int)((blockDim.x + 31) >> 5); ++w) tot += red[0][w];
-            const double nrm = sqrt(tot);
-            SolveState *S = M.state + r;
-            if (MODE == 0) {
-                S->sweep = 0;
-                S->norm0 = nrm;
-            } else {
-                S->sweep += 1;
-            }
-            const int sw = S->sweep;
-            if (sw < S->hist_cap) M.hist[(size_t)r * M.hist_stride + sw] = nrm;
-            S->last = nrm;
-            const bool go = isfinite(nrm) && nrm > S->tol * S->norm0 && sw < S->max_sweeps;
-            M.active[r] = go ? 1 : 0;
-            if (go) any_go = 1;
+    /* per r the order of strided_sum, all r side by side: one r after the other
+     * (each waits for its loads twelve times at 8640 tiles) a launch took 12 to
+     * 27 us longer */
+    double acc[MULTI_MAX];
+#pragma unroll
+    for (int r = 0; r < MULTI_MAX; ++r) acc[r] = 0.0;
+    {
+        constexpr int AHEAD = 3;
+        const double *p = M.partials + tid;
+        int t = tid;
+        for (; t + (AHEAD - 1) * RES_THREADS_FAST < ntiles; t += AHEAD * RES_THREADS_FAST, p += AHEAD * RES_THREADS_FAST) {
+            double v[AHEAD][MULTI_MAX];
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u)
+#pragma unroll
+                for (int r = 0; r < MULTI_MAX; ++r)
+                    v[u][r] = r < nr ? __ldcg(p + (size_t)r * ntiles + u * RES_THREADS_FAST) : 0.0;
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u)
+#pragma unroll
+                for (int r = 0; r < MULTI_MAX; ++r) acc[r] += v[u][r];
+        }
+        for (; t < ntiles; t += RES_THREADS_FAST, p += RES_THREADS_FAST) {
+#pragma unroll
+            for (int r = 0; r < MULTI_MAX; ++r)
+                if (r < nr) acc[r] += __ldcg(p + (size_t)r * ntiles);
         }
     }
+    const double ws = warp_sums8<false>(acc);
+    if ((tid & 3) == 0) red[(tid & 31) >> 2][tid >> 5] = ws;
     __syncthreads();
+    bool go = false;
+    if (tid < nr && ((amask >> tid) & 1u)) {
+        double tot = 0.0;
+        for (int w = 0; w < RES_THREADS_FAST / 32; ++w) tot += red[tid][w];
+        const double nrm = sqrt(tot);
+        SolveState *S = M.state + tid;
+        if (MODE == 0) {
+            S->sweep = 0;
+            S->norm0 = nrm;
+        } else {
+            S->sweep += 1;
+        }
+        const int sw = S->sweep;
+        if (sw < S->hist_cap) M.hist[(size_t)tid * M.hist_stride + sw] = nrm;
+        S->last = nrm;
+        go = isfinite(nrm) && nrm > S->tol * S->norm0 && sw < S->max_sweeps;
+        M.active[tid] = go ? 1 : 0;
+    }
+    const int any_go = __syncthreads_or(go);
     if (tid == 0) {
         if (use_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)handle, any_go ? 1u : 0u);
         *M.counter = 0u;
