@@ -142,39 +142,48 @@ int launch_reduce_norm(cudaStream_t st, const double *partials, int n, SolveStat
     return (int)cudaGetLastError();
 }
 
-template <typename T>
-__global__ void permute_to_pos_kernel(int nv, int nelem, const int *__restrict__ pos_of_elem,
-                                      const double *__restrict__ src, T *__restrict__ dst) {
-    long long n = (long long)nv * nelem;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
-         t += (long long)gridDim.x * blockDim.x) {
-        int e = (int)(t / nv), i = (int)(t - (long long)e * nv);
-        dst[(long long)pos_of_elem[e] * nv + i] = (T)src[t];
+/* Vectors between element and position order (src, dst by word; grid row r:
+ * vector r).  Bound by HBM once a word's element costs little: with a 64-bit
+ * division by nv a word 1200x1280 took 59 us, with 32-bit word numbers, nv a
+ * constant where it is 9, 55.  NVC 0: any nv.  Eight vectors of 360x384 in one
+ * launch: 40 us, 97 in eight. */
+template <int NVC, bool TO_POS, typename I>
+__global__ void permute_kernel(int nv_, long long n_, const int *__restrict__ pos_of_elem,
+                               const double *__restrict__ src, double *__restrict__ dst, long long src_stride,
+                               long long dst_stride) {
+    const I nv = NVC > 0 ? NVC : nv_, n = (I)n_;
+    src += blockIdx.y * src_stride;
+    dst += blockIdx.y * dst_stride;
+    for (I t = blockIdx.x * (I)blockDim.x + threadIdx.x; t < n; t += (I)gridDim.x * blockDim.x) {
+        const I e = t / nv;
+        const long long p = (long long)pos_of_elem[e] * nv + (t - e * nv);
+        if (TO_POS) dst[p] = src[t];
+        else dst[t] = src[p];
     }
 }
 
-__global__ void permute_to_elem_kernel(int nv, int nelem, const int *__restrict__ pos_of_elem,
-                                       const double *__restrict__ src, double *__restrict__ dst) {
-    long long n = (long long)nv * nelem;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
-         t += (long long)gridDim.x * blockDim.x) {
-        int e = (int)(t / nv), i = (int)(t - (long long)e * nv);
-        dst[t] = src[(long long)pos_of_elem[e] * nv + i];
-    }
-}
-
-int launch_permute_to_pos(cudaStream_t st, int nv, int nelem, const int *pos_of_elem,
-                          const double *src_elem, double *dst_pos) {
-    permute_to_pos_kernel<double>
-        <<<grid_for((long long)nv * nelem, 256), 256, 0, st>>>(nv, nelem, pos_of_elem, src_elem, dst_pos);
+template <bool TO_POS>
+static int launch_permute(cudaStream_t st, int nv, int nelem, const int *pos, const double *src, double *dst,
+                          int count, long long ss, long long ds) {
+    const long long n = (long long)nv * nelem;
+    const dim3 grid(grid_for(n, 256), count);
+    if (n >= (1LL << 31)) /* word numbers and strides past 32 bits */
+        permute_kernel<0, TO_POS, long long><<<grid, 256, 0, st>>>(nv, n, pos, src, dst, ss, ds);
+    else if (nv == 9)
+        permute_kernel<9, TO_POS, unsigned><<<grid, 256, 0, st>>>(nv, n, pos, src, dst, ss, ds);
+    else
+        permute_kernel<0, TO_POS, unsigned><<<grid, 256, 0, st>>>(nv, n, pos, src, dst, ss, ds);
     return (int)cudaGetLastError();
 }
 
-int launch_permute_to_elem(cudaStream_t st, int nv, int nelem, const int *pos_of_elem,
-                           const double *src_pos, double *dst_elem) {
-    permute_to_elem_kernel<<<grid_for((long long)nv * nelem, 256), 256, 0, st>>>(
-        nv, nelem, pos_of_elem, src_pos, dst_elem);
-    return (int)cudaGetLastError();
+int launch_permute_to_pos(cudaStream_t st, int nv, int nelem, const int *pos_of_elem, const double *src_elem,
+                          double *dst_pos, int count, long long src_stride, long long dst_stride) {
+    return launch_permute<true>(st, nv, nelem, pos_of_elem, src_elem, dst_pos, count, src_stride, dst_stride);
+}
+
+int launch_permute_to_elem(cudaStream_t st, int nv, int nelem, const int *pos_of_elem, const double *src_pos,
+                           double *dst_elem, int count, long long src_stride, long long dst_stride) {
+    return launch_permute<false>(st, nv, nelem, pos_of_elem, src_pos, dst_elem, count, src_stride, dst_stride);
 }
 
 __global__ void permute_f32_to_elem_kernel(int nv, int nelem, const int *__restrict__ pos_of_elem,

@@ -281,8 +281,7 @@ static int multi_group(tbs_ctx *ctx, int nr, const double *d_rhs, double *d_U, d
     cudaStream_t st = ctx->stream;
     const int ne = ctx->nelem;
     const size_t nv = (size_t)ne * 9, vs = (size_t)ctx->L.np16 * 9;
-    for (int r = 0; r < nr; ++r)
-        MRUN("permute", launch_permute_to_pos(st, 9, ne, ctx->L.pos_of_elem, d_rhs + r * nv, m->rhsp + r * vs));
+    MRUN("permute", launch_permute_to_pos(st, 9, ne, ctx->L.pos_of_elem, d_rhs, m->rhsp, nr, nv, vs));
     for (int r = 0; r < nr; ++r) {
         SolveState &S = m->h_state[r];
         std::memset(&S, 0, sizeof(S));
@@ -313,8 +312,7 @@ static int multi_group(tbs_ctx *ctx, int nr, const double *d_rhs, double *d_U, d
         }
         MCK(cudaGraphLaunch(m->gexec, st));
     }
-    for (int r = 0; r < nr; ++r)
-        MRUN("permute", launch_permute_to_elem(st, 9, ne, ctx->L.pos_of_elem, m->U + r * vs, d_U + r * nv));
+    MRUN("permute", launch_permute_to_elem(st, 9, ne, ctx->L.pos_of_elem, m->U, d_U, nr, vs, nv));
     MCK(cudaMemcpyAsync(m->h_state, m->state, nr * sizeof(SolveState), cudaMemcpyDeviceToHost, st));
     MCK(cudaStreamSynchronize(st));
     int rc = ctx_status(ctx);

@@ -151,10 +151,10 @@ int launch_reduce_norm(cudaStream_t st, const double *partials, int n, SolveStat
                        double *hist, int is_start, unsigned long long cond_handle, int use_cond,
                        unsigned long long cond_handle2 = 0, int use2 = 0);
 int launch_zero(cudaStream_t st, double *p, long long n);
-int launch_permute_to_pos(cudaStream_t st, int nv, int nelem, const int *pos_of_elem,
-                          const double *src_elem, double *dst_pos);
-int launch_permute_to_elem(cudaStream_t st, int nv, int nelem, const int *pos_of_elem,
-                           const double *src_pos, double *dst_elem);
+int launch_permute_to_pos(cudaStream_t st, int nv, int nelem, const int *pos_of_elem, const double *src_elem,
+                          double *dst_pos, int count = 1, long long src_stride = 0, long long dst_stride = 0);
+int launch_permute_to_elem(cudaStream_t st, int nv, int nelem, const int *pos_of_elem, const double *src_pos,
+                           double *dst_elem, int count = 1, long long src_stride = 0, long long dst_stride = 0);
 int launch_permute_f32_to_elem(cudaStream_t st, int nv, int nelem, const int *pos_of_elem,
                                const float *src_pos, double *dst_elem);
 
