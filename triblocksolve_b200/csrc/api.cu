@@ -1549,13 +1549,21 @@ static int get_vec(tbs_ctx *ctx, int which, double *out) {
     cudaStream_t st = ctx->stream;
     const size_t vb = (size_t)nvec(ctx) * sizeof(double);
     const double *src = nullptr;
+    /* pinned memory the device addresses: the reordering stores there itself */
+    double *pinned = static_cast<double *>(xfer_device_view(out));
+    if ((uintptr_t)pinned % sizeof(double) != 0) pinned = nullptr;
     if (ctx->algo == TBS_ALGO_REFERENCE) {
         src = which == 0 ? ctx->d_U : which == 1 ? ctx->d_R : ctx->d_dU;
     } else {
         const FastLayout &L = ctx->L;
         const int nv = ctx->nvar;
         if (which == 0) {
-            RUN("permute", launch_permute_to_elem(st, nv, ctx->nelem, L.pos_of_elem, ctx->d_Up, ctx->d_scratch));
+            RUN("permute", launch_permute_to_elem(st, nv, ctx->nelem, L.pos_of_elem, ctx->d_Up,
+                                                  pinned ? pinned : ctx->d_scratch));
+            if (pinned) {
+                CK(cudaStreamSynchronize(st));
+                return TBS_OK;
+            }
         } else if (which == 1 && nv != 9) {
             /* general block size: the reference-order residual of U */
             RUN("permute", launch_permute_to_elem(st, nv, ctx->nelem, L.pos_of_elem, ctx->d_Up, ctx->d_U));
