@@ -1555,13 +1555,13 @@ static ThomasCfg thomas_cfg(const FastLayout &L) {
 /* Which single-system line solve: the warp-specialised kernel (a copy
  * warp beside each chain warp) where few lines share an SM -- there the
  * launch is bound by the chain's step latency, and taking the copy issue
- * off the chain warp shortens every step (360 lines: 64 -> 51 us); the
+ * off the chain warp shortens every step (360 lines: 53 -> 45 us); the
  * one-warp kernel where many lines share an SM, whose warps hide each
  * other's latency and which holds more lines per SM in its registers
- * (1,200 lines: 409 us one-warp, 526 us warp-specialised).  At 600 lines
- * (5 per SM) the copy warp still pays: 117 -> 112 us (FP64), 87 -> 81 us
- * (FP32).  The
- * environment variable TBS_THOMAS_WS=0 / 1 forces one or the other. */
+ * (1,200 lines: 419 us one-warp, 569 us warp-specialised).  At 600 lines
+ * (5 per SM) the copy warp still pays: 128 -> 124 us (FP64), 91 -> 82 us
+ * (FP32).  The environment variable TBS_THOMAS_WS=0 / 1 forces one or the
+ * other. */
 static bool thomas_ws(const FastLayout &L) {
     static const int forced = [] {
         const char *e = getenv("TBS_THOMAS_WS");
