@@ -379,6 +379,32 @@ __device__ __forceinline__ bool thomas_line(
             pbase ^= (uint32_t)(cnt & 1) << s;
         }
     };
+    /* YS: U += x by the loads and stores of the warps (FP32, or U read from
+     * another buffer) waits for a round of loads after another: both warps of
+     * a line share it (600x640 FP32: a line solve of 82 us with the chain
+     * warp alone and 8 loads a lane in flight, 78) */
+    const bool share = WS && YS && PH == PH_ALL && accumulate == 1 && !(sizeof(T) == 8 && !Uin);
+    auto add_to_u = [&](int first, int w, int warps) {
+        constexpr int B = 16;
+        const int nv = n * NV, nbulk = (n & ~3) * NV;
+        for (int t0 = first + w * 32 + lane; t0 < nv; t0 += 32 * warps * B) {
+            T u[B];
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                const int t = t0 + 32 * warps * k;
+                u[k] = (accumulate == 1 && t < nv) ? __ldcg(Uil + t) : T(0);
+            }
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                const int t = t0 + 32 * warps * k;
+                if (t < nv) {
+                    const T x = ys[t];
+                    if (t >= nbulk) dUl[t] = x;
+                    if (accumulate < 2) Ul[t] = u[k] + x;
+                }
+            }
+        }
+    };
     if (producer) {
         /* every job as soon as the consumer has released its stage: job
          * j >= NS waits for the consumption of job j - NS */
@@ -409,6 +435,11 @@ __device__ __forceinline__ bool thomas_line(
             }
         }
         __syncwarp();
+        if (share) {
+            ws_meet(); /* x is in ys, or the chains have given up */
+            if (*ws_abort) return true;
+            add_to_u(0, 1, 2);
+        }
         ws_meet();
         close_phases();
         return true;
@@ -557,7 +588,7 @@ __device__ __forceinline__ bool thomas_line(
              * once, as the loop would); what is left, and the forms that
              * read another buffer, by the loop, whose U loads of a batch are
              * issued together so that their latencies overlap */
-            const int nbulk = (n & ~3) * NV, nv = n * NV;
+            const int nbulk = (n & ~3) * NV;
             const bool ub = accumulate == 0 || (accumulate == 1 && sizeof(T) == 8 && !Uin);
             fence_async_smem();
             __syncwarp();
@@ -572,24 +603,8 @@ __device__ __forceinline__ bool thomas_line(
                 if (accumulate == 1 && ub) bulk_add_s2g(Ul, ys, nbulk * sizeof(T));
                 bulk_s2g_commit();
             }
-            constexpr int B = 8;
-            for (int t0 = (accumulate < 2 && !ub ? 0 : nbulk) + lane; t0 < nv; t0 += 32 * B) {
-                T u[B];
-#pragma unroll
-                for (int k = 0; k < B; ++k) {
-                    const int t = t0 + 32 * k;
-                    u[k] = (accumulate == 1 && t < nv) ? __ldcg(Uil + t) : T(0);
-                }
-#pragma unroll
-                for (int k = 0; k < B; ++k) {
-                    const int t = t0 + 32 * k;
-                    if (t < nv) {
-                        const T x = ys[t];
-                        if (t >= nbulk) dUl[t] = x;
-                        if (accumulate < 2) Ul[t] = u[k] + x;
-                    }
-                }
-            }
+            if (share) ws_meet();
+            add_to_u(accumulate < 2 && !ub ? 0 : nbulk, 0, share ? 2 : 1);
             if (lane == 0 && nbulk > 0) {
                 if (drain) bulk_s2g_wait_but<1>(); /* dU */
                 bulk_s2g_wait_read(); /* before the CTA's memory goes */
