@@ -21,6 +21,7 @@
  * cp.async.bulk in FP64 and FP32 alike.
  */
 #include "device_common.cuh"
+#include "recip.cuh"
 #include "tbs_internal.hxx"
 #include "thomas.cuh"
 #include "tma.cuh"
@@ -363,18 +364,6 @@ __device__ __forceinline__ void gj_invert_cols(double (&w)[NV], int j, unsigned 
     }
 }
 
-/* 1 / d, correctly rounded, by Newton's iteration and Markstein's last step
- * (P. Markstein, IBM J. Res. Dev. 34 (1990) 111-119) from the hardware's
- * approximation: about 70 cycles, and no branch in the usual range. */
-__device__ __forceinline__ double rcp_chain(double d) {
-    double x;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
-    double e = fma(-d, x, 1.0);
-    x = fma(x, fma(e, e, e), x);
-    e = fma(-d, x, 1.0);
-    return fma(x, e, x);
-}
-
 /* Gauss-Jordan inverse of a 9x9 block held by 27 lanes: lane j + 9g
  * (column j, row group g) holds rows 3g..3g+2 of column j in w[0..2].  For
  * pivot p, the pivot column's entries of this lane's rows come from lane
@@ -383,9 +372,9 @@ __device__ __forceinline__ double rcp_chain(double d) {
  * then know the next pivot two operations after the reciprocal of this one.
  * Each entry is updated with the operations of gj_invert_cols (the pivot
  * column as 0 - column * r); no pivoting, as the reference's LU has none.
- * No branch stands in the chain: a pivot outside 2^-1000 .. 2^1000, where
- * rcp_chain does not hold, is noted, and the block is then done again with
- * the general reciprocal.  Returns whether a pivot was zero or not finite. */
+ * No branch stands in the chain: a pivot for which rcp_newton does not hold
+ * (rcp_exception) is noted, and the block is then done again with the general
+ * reciprocal.  Returns whether a pivot was zero or not finite. */
 template <bool GENERAL>
 __device__ __forceinline__ bool gj_pass_27(double (&w)[3], int j, int g) {
     bool bad = false;
@@ -409,8 +398,8 @@ __device__ __forceinline__ bool gj_pass_27(double (&w)[3], int j, int g) {
         if (GENERAL)
             bad |= !(fabs(piv) > 0.0 && isfinite(piv));
         else
-            bad |= (unsigned)((__double2hiint(piv) & 0x7fffffff) - 0x01700000) >= 0x7d000000u;
-        const double r = GENERAL ? __drcp_rn(piv) : rcp_chain(piv);
+            bad |= rcp_exception(piv);
+        const double r = GENERAL ? __drcp_rn(piv) : rcp_newton(piv);
         piv = dn - cn * (rn * r);
         t *= r;
 #pragma unroll
@@ -673,8 +662,8 @@ __global__ void __launch_bounds__(96) fast_factor_few_kernel(
  * and the pivot row's of its columns.  Each entry is updated with the
  * operations of gj_invert_cols (the pivot column as 0 - column * r); no
  * pivoting, as the reference's LU has none.  No branch stands in the chain: a
- * pivot outside 2^-1000 .. 2^1000, where rcp_chain does not hold, is noted,
- * and the blocks are then done again with the general reciprocal.  Returns
+ * pivot for which rcp_newton does not hold (rcp_exception) is noted, and the
+ * blocks are then done again with the general reciprocal.  Returns
  * whether a pivot of the lane's block was zero or not finite. */
 template <bool GENERAL>
 __device__ __forceinline__ bool gj_pass(double (&w)[3][3], int a, int b, int base) {
@@ -691,8 +680,8 @@ __device__ __forceinline__ bool gj_pass(double (&w)[3][3], int a, int b, int bas
         if (GENERAL)
             bad |= !(fabs(piv) > 0.0 && isfinite(piv));
         else
-            bad |= (unsigned)((__double2hiint(piv) & 0x7fffffff) - 0x01700000) >= 0x7d000000u;
-        const double r = GENERAL ? __drcp_rn(piv) : rcp_chain(piv);
+            bad |= rcp_exception(piv);
+        const double r = GENERAL ? __drcp_rn(piv) : rcp_newton(piv);
         if (b == pa) {
             t[pk] = 1.0;
 #pragma unroll

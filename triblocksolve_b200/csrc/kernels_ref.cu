@@ -17,6 +17,7 @@
  * nv columns of D'^-1 C are independent solves, and every dot product is
  * summed from 0.0 in ascending j as in the OKL loops.
  */
+#include "recip.cuh"
 #include "tbs_internal.hxx"
 #include "tma.cuh"
 
@@ -147,31 +148,14 @@ __global__ void __launch_bounds__(32) ref_line_lu_kernel(
  * inside a triangular solve), a second warp copying the coming cells' blocks
  * into shared memory. */
 
-/* RN(1 / d) by Newton's iteration and Markstein's last step (P. Markstein,
- * IBM J. Res. Dev. 34 (1990) 111-119); d within 2^-500 .. 2^500 and its
- * significand not all ones (the theorem's exception): ref_plain_divisor */
-__device__ __forceinline__ double ref_rcp(double d) {
-    double x;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
-    double e = fma(-d, x, 1.0);
-    x = fma(x, fma(e, e, e), x);
-    e = fma(-d, x, 1.0);
-    return fma(x, e, x);
-}
-
-/* |v| within 2^-e .. 2^e (not zero, not infinite, a number) */
-__device__ __forceinline__ bool ref_within(double v, int e) {
-    return (unsigned)((__double2hiint(v) & 0x7fffffff) - ((1023 - e) << 20)) < (unsigned)(2 * e) << 20;
-}
-
-/* a divisor left to the general division */
+/* a divisor left to the general division (rcp_newton, ref_div) */
 __device__ __forceinline__ bool ref_plain_divisor(double d) {
-    return !ref_within(d, 500) || ((__double2hiint(d) & 0xfffff) == 0xfffff && __double2loint(d) == -1);
+    return (int)!within_pow2(d, 500) | (int)ones_significand(d);
 }
 
 /* RN(n / d) from r = RN(1 / d) and rl, the rest of 1 / d to twice the
  * precision: q is within an ulp, the remainder exact and the last step
- * rounds correctly (Markstein, as above).  Holds for |d| within 2^-500 ..
+ * rounds correctly (Markstein, as for rcp_newton).  Holds for |d| within 2^-500 ..
  * 2^500 and |n| within 2^-400 .. 2^400; the caller checks both. */
 __device__ __forceinline__ double ref_div(double n, double d, double r, double rl) {
     const double q = fma(n, r, n * rl);
@@ -207,7 +191,7 @@ __device__ __forceinline__ bool ref_solve9(const double *D, const double *rc, co
 #pragma unroll
         for (int j = i + 1; j < 9; ++j) t = j == i + 1 ? p[i][j] : t + p[i][j];
         const double n = y[i] - t;
-        ok = ok && ref_within(n, 400);
+        ok = ok && within_pow2(n, 400);
         x[i] = ref_div(n, D[10 * i], rc[i], rc[9 + i]);
 #pragma unroll
         for (int k = 0; k < i; ++k) p[k][i] = k + 1 == i ? fma(D[k + 9 * i], x[i], 0.0) : D[k + 9 * i] * x[i];
@@ -239,7 +223,7 @@ __device__ __forceinline__ bool ref_lu27(double (&w)[3], int i, int g, bool firs
         for (int k = 0; k < 3; ++k) u[k] = __shfl_sync(0xffffffffu, w[k], j + 9 * g);
         if (PLAIN) bad |= !(fabs(a) > 0.0 && isfinite(a));
         odd |= ref_plain_divisor(a);
-        const double r = PLAIN ? 1.0 / a : ref_rcp(a);
+        const double r = PLAIN ? 1.0 / a : rcp_newton(a);
         if (first && i == j) {
             rc[j] = r;
             rc[9 + j] = fma(-a, r, 1.0) * r;
@@ -275,7 +259,7 @@ constexpr int LCELL = 3 * 81;        /* D, A, C */
  * the cells two steps ahead into shared memory and writing D', D'^-1 C and A
  * out.  ref_line_lu_kernel, which loads as it goes and divides 18 times a
  * cell, took 9,900 cycles a cell; 360x384: 1,960 us and 95 for the packing,
- * 720 together here. */
+ * 657 together here. */
 __global__ void __launch_bounds__(64) ref_line_lu9_kernel(
     int nline, const int *__restrict__ fc, const int *__restrict__ linesize,
     const int *__restrict__ linepoint, const int *__restrict__ lines,
@@ -508,7 +492,7 @@ __global__ void __launch_bounds__(64) ref_solve_du9_kernel(
             for (int t = lane; t < 9 * RC; t += 32) {
                 const int q = t / 9, i = t % 9;
                 double *d = stage[job % RS][q];
-                const double u = d[10 * i], r = ref_rcp(u);
+                const double u = d[10 * i], r = rcp_newton(u);
                 d[171 + i] = r;
                 d[180 + i] = fma(-u, r, 1.0) * r;
                 if (ref_plain_divisor(u)) d[189] = 1.0;
