@@ -36,9 +36,12 @@ namespace tbs {
  * blocks are column-major, so that the nine lanes read a column of nine
  * neighbouring words: no bank conflicts and one copy of the vector (with
  * row-major blocks: two copies, lane-dependent offsets, 122 cycles a step
- * against 106; rows as aligned pairs of columns: 111).  Two partial sums,
- * since the vector's words arrive one after the other: the last one is two
- * operations from the result (three sums: 115 cycles).
+ * against 106; rows as aligned pairs of columns: 111).  The dot product is
+ * three partial sums, so that no more than four roundings follow one another
+ * (two sums: six, and an error 3 to 4 % larger); the vector's words arrive
+ * one after the other, and the last of them joins the sum that starts from
+ * the right-hand side, two operations from the result: as fast as two sums
+ * to 1 % (45 us and 46 at 360x384, 32.9 and 32.8 at 181x301).
  * YS: the line's y and x live in shared memory, and dU / U are written after
  * the line is solved: dU by one bulk copy, and in FP64 U += dU by one bulk
  * add (the L2 adds, so the warp does not wait for U); otherwise y goes to
@@ -59,7 +62,7 @@ __host__ __device__ constexpr uint32_t thomas_stage_bytes() {
 
 /* The vector a step reads and the row it multiplies.
  * FP64: lane i's row in column order, and one copy of the vector read as
- * four pairs and a single (two partial sums, see above).
+ * four pairs and a single.
  * FP32: the vector in two copies (y_j at j and at 11 + j), so that a lane
  * whose row number and cell have different parity starts its pairs at
  * column 1; the order of the sum by lane is kept as it was first written,
@@ -122,19 +125,22 @@ __device__ __forceinline__ void load_row(Row<float, 9> &R, const float *blk, int
     for (int j = 1; j < 9; ++j) R.r[j] = q[9 * j];
 }
 
-/* init - row . vec */
+/* init - row . vec in three partial sums: the terms j with NV - 1 - j
+ * divisible by three go to the one that starts from init */
 template <int NV>
 __device__ __forceinline__ double row_dot(const Row<double, NV> &R, const StepVec<double, NV> &V, double init) {
-    double a0 = init - R.r[0] * V.v[0];
-    double a1 = R.r[1] * V.v[1];
+    double a0 = init, a1 = 0.0, a2 = 0.0;
 #pragma unroll
-    for (int j = 2; j < NV; ++j) {
-        if (j & 1)
-            a1 += R.r[j] * V.v[j];
-        else
+    for (int j = 0; j < NV; ++j) {
+        const int c = (NV - 1 - j) % 3;
+        if (c == 0)
             a0 -= R.r[j] * V.v[j];
+        else if (c == 1)
+            a1 = j < 3 ? R.r[j] * V.v[j] : a1 + R.r[j] * V.v[j];
+        else
+            a2 = j < 3 ? R.r[j] * V.v[j] : a2 + R.r[j] * V.v[j];
     }
-    return a0 - a1;
+    return a0 - (NV > 2 ? a1 + a2 : a1);
 }
 
 __device__ __forceinline__ float row_dot(const Row<float, 9> &R, const StepVec<float, 9> &V, float init) {
