@@ -13,6 +13,13 @@
 
 namespace tbs {
 
+/* x y and x y + z, rounded as written whatever the compiler would contract:
+ * for the sums that several kernels have to make alike, bit for bit */
+static __device__ __forceinline__ double mul_rn(double x, double y) { return __dmul_rn(x, y); }
+static __device__ __forceinline__ float mul_rn(float x, float y) { return __fmul_rn(x, y); }
+static __device__ __forceinline__ double fma_rn(double x, double y, double z) { return __fma_rn(x, y, z); }
+static __device__ __forceinline__ float fma_rn(float x, float y, float z) { return __fmaf_rn(x, y, z); }
+
 /* sum of p[t], p[t + stride], p[t + 2 stride], ... (t = threadIdx.x), added
  * in that order; eight loads are issued ahead of their adds so that their
  * latencies overlap without changing the sum */

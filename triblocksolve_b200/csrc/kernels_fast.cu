@@ -1098,19 +1098,32 @@ __device__ __forceinline__ uint64_t *resid_bar_init() {
     return bar;
 }
 
+/* the first six products of a row of a block (column-major, at its entry of
+ * column 0) with a vector, in the three sums a[0..2] that the others join:
+ * products j and j + 3 open sum j, the latter rounded by itself */
+template <typename T>
+__device__ __forceinline__ void open_sums(T (&a)[3], const T *row, const T *v) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) a[j] = fma_rn(row[9 * j], v[j], mul_rn(row[9 * j + 27], v[j + 3]));
+}
+
+/* a[j] += products j, j + 3, j + 6 (from product `first` on) */
+template <typename T>
+__device__ __forceinline__ void add_products(T (&a)[3], const T *row, const T *v, int first = 0) {
+#pragma unroll
+    for (int j = 0; j < 9; ++j)
+        if (j >= first) a[j % 3] = fma_rn(row[9 * j], v[j], a[j % 3]);
+}
+
 /* -(row of Dinv) . R for one (cell, row): dr points at entry (row, 0) of
  * the cell's column-major block, rv at the cell's R; three accumulators,
  * the order every b = -Dinv R of this file uses */
 template <typename T>
 __device__ __forceinline__ T neg_dinv_row(const T *dr, const T *rv) {
-    T a0 = dr[0] * rv[0], a1 = dr[9] * rv[1], a2 = dr[18] * rv[2];
-    a0 += dr[27] * rv[3];
-    a1 += dr[36] * rv[4];
-    a2 += dr[45] * rv[5];
-    a0 += dr[54] * rv[6];
-    a1 += dr[63] * rv[7];
-    a2 += dr[72] * rv[8];
-    return -(a0 + (a1 + a2));
+    T a[3];
+    open_sums(a, dr, rv);
+    add_products(a, dr, rv, 6);
+    return -(a[0] + (a[1] + a[2]));
 }
 
 /* One tile (positions blk*RES_TILE ..) with the staging barrier's phase of
@@ -1184,28 +1197,20 @@ __device__ __forceinline__ bool fast_resid_body(
     T r = T(0);
     if (mode >= 1) {
         if (act) {
-            T a0 = T(0), a1 = T(0), a2 = T(0);
+            T a[3] = {T(0), T(0), T(0)};
             for (int s = 0; s < nx; ++s) {
                 const T *xr = sX + (s * RES_TILE + c) * NB + i;
                 const T *g = sg + (s * RES_TILE + c) * NV;
-                a0 += xr[0] * g[0];
-                a1 += xr[9] * g[1];
-                a2 += xr[18] * g[2];
-                a0 += xr[27] * g[3];
-                a1 += xr[36] * g[4];
-                a2 += xr[45] * g[5];
-                a0 += xr[54] * g[6];
-                a1 += xr[63] * g[7];
-                a2 += xr[72] * g[8];
+                add_products(a, xr, g);
             }
-            r = a0 + (a1 + a2);
+            r = a[0] + (a[1] + a[2]);
             sr[c * NV + i] = r;
         }
         __syncthreads();
     } else if (act) {
         r = sr[c * NV + i];
     }
-    double sq = act ? (double)r * (double)r : 0.0;
+    double sq = act ? mul_rn((double)r, (double)r) : 0.0;
     if (mode == 3) {
         /* X held Dinv X: r is already Dinv R */
         if (act) sb[c * NV + i] = -r;
@@ -1824,25 +1829,17 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) small_sweeps_kernel(SmallSwe
             const double *sD = blocks(k), *sX = sD + RES_TILE * NB;
             double r = 0.0;
             if (act) {
-                double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+                double a[3] = {0.0, 0.0, 0.0};
                 for (int s = 0; s < nx; ++s) {
                     const double *xr = sX + (s * RES_TILE + c) * NB + i;
                     const double *q = sg + (s * RES_TILE + c) * NV;
-                    a0 += xr[0] * q[0];
-                    a1 += xr[9] * q[1];
-                    a2 += xr[18] * q[2];
-                    a0 += xr[27] * q[3];
-                    a1 += xr[36] * q[4];
-                    a2 += xr[45] * q[5];
-                    a0 += xr[54] * q[6];
-                    a1 += xr[63] * q[7];
-                    a2 += xr[72] * q[8];
+                    add_products(a, xr, q);
                 }
-                r = a0 + (a1 + a2);
+                r = a[0] + (a[1] + a[2]);
                 sr[c * NV + i] = r;
             }
             __syncthreads();
-            double sq = act ? r * r : 0.0;
+            double sq = act ? mul_rn(r, r) : 0.0;
             if (act) sb[c * NV + i] = neg_dinv_row<double>(sD + c * NB + i, sr + c * NV);
             for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(FULL, sq, o);
             if ((tid & 31) == 0) red[warp] = sq;
@@ -1991,33 +1988,21 @@ __device__ __forceinline__ void full_resid_body(
         const int pe = pos_of_elem[e];
         const double *u = Up + (size_t)pe * NV;
         const double *dr = D + (size_t)e * NB + i;
-        double a0 = dr[0] * u[0], a1 = dr[9] * u[1], a2 = dr[18] * u[2];
-        a0 += dr[27] * u[3];
-        a1 += dr[36] * u[4];
-        a2 += dr[45] * u[5];
-        a0 += dr[54] * u[6];
-        a1 += dr[63] * u[7];
-        a2 += dr[72] * u[8];
+        double a[3];
+        open_sums(a, dr, u);
+        add_products(a, dr, u, 6);
         for (int k2 = epoint[e]; k2 < epoint[e + 1]; ++k2) {
             const int f = ef[k2];
             if (f >= 0) {
                 const int e1 = fc[2 * f], e2 = fc[2 * f + 1];
                 const double *o = ((e == e1) ? O2 : O1) + (size_t)f * NB + i;
                 const double *un = Up + (size_t)pos_of_elem[(e == e1) ? e2 : e1] * NV;
-                a0 += o[0] * un[0];
-                a1 += o[9] * un[1];
-                a2 += o[18] * un[2];
-                a0 += o[27] * un[3];
-                a1 += o[36] * un[4];
-                a2 += o[45] * un[5];
-                a0 += o[54] * un[6];
-                a1 += o[63] * un[7];
-                a2 += o[72] * un[8];
+                add_products(a, o, un);
             }
         }
-        const double r = (rhs ? rhs[(size_t)e * NV + i] : 0.0) + (a0 + (a1 + a2));
+        const double r = (rhs ? rhs[(size_t)e * NV + i] : 0.0) + (a[0] + (a[1] + a[2]));
         Rp[(size_t)pe * NV + i] = (T)r;
-        sq = r * r;
+        sq = mul_rn(r, r);
     }
     __shared__ double red[FULLRES_THREADS / 32];
     for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(FULL, sq, o);
@@ -2171,29 +2156,17 @@ __device__ __forceinline__ bool full_resid_pos_body(
     if (act) {
         const double *dr = sD + c * NB + i;
         const double *u = sg + c * NV;
-        double a0 = dr[0] * u[0], a1 = dr[9] * u[1], a2 = dr[18] * u[2];
-        a0 += dr[27] * u[3];
-        a1 += dr[36] * u[4];
-        a2 += dr[45] * u[5];
-        a0 += dr[54] * u[6];
-        a1 += dr[63] * u[7];
-        a2 += dr[72] * u[8];
+        double a[3];
+        open_sums(a, dr, u);
+        add_products(a, dr, u, 6);
         for (int s = 0; s < nxf; ++s) {
             const double *o = sX + (s * RES_TILE + c) * NB + i;
             const double *un = sg + ((s + 1) * RES_TILE + c) * NV;
-            a0 += o[0] * un[0];
-            a1 += o[9] * un[1];
-            a2 += o[18] * un[2];
-            a0 += o[27] * un[3];
-            a1 += o[36] * un[4];
-            a2 += o[45] * un[5];
-            a0 += o[54] * un[6];
-            a1 += o[63] * un[7];
-            a2 += o[72] * un[8];
+            add_products(a, o, un);
         }
-        const double r = sr[c * NV + i] + (a0 + (a1 + a2));
+        const double r = sr[c * NV + i] + (a[0] + (a[1] + a[2]));
         so[c * NV + i] = (float)r;
-        sq = r * r;
+        sq = mul_rn(r, r);
     }
     __syncthreads();
     if (act) R32[(size_t)p0 * NV + tid] = so[tid]; /* contiguous tile store */
@@ -2291,7 +2264,7 @@ __device__ __forceinline__ void mixed_prime_body(const double *__restrict__ rhsp
         sR[tid] = (float)v;
         Up[q] = 0.0;
         if (c32) c32[q] = 0.0f;
-        sq = v * v;
+        sq = mul_rn(v, v);
     }
     if (Dinv32) {
         /* the first inner solve's right-hand side b32 = -Dinv32 R32 */
@@ -2672,25 +2645,17 @@ __global__ void __launch_bounds__(RES_THREADS_FAST) fast_resid_group_kernel(
                 }
                 T rr = T(0);
                 if (act) {
-                    T a0 = T(0), a1 = T(0), a2 = T(0);
+                    T a[3] = {T(0), T(0), T(0)};
                     for (int s = 0; s < nx; ++s) {
                         const T *xr = sX + (s * RES_TILE + c) * NB + i;
                         const T *g = sg + (s * RES_TILE + c) * NV;
-                        a0 += xr[0] * g[0];
-                        a1 += xr[9] * g[1];
-                        a2 += xr[18] * g[2];
-                        a0 += xr[27] * g[3];
-                        a1 += xr[36] * g[4];
-                        a2 += xr[45] * g[5];
-                        a0 += xr[54] * g[6];
-                        a1 += xr[63] * g[7];
-                        a2 += xr[72] * g[8];
+                        add_products(a, xr, g);
                     }
-                    rr = a0 + (a1 + a2);
+                    rr = a[0] + (a[1] + a[2]);
                     sr[c * NV + i] = rr;
                 }
                 __syncthreads();
-                double sq = act ? (double)rr * (double)rr : 0.0;
+                double sq = act ? mul_rn((double)rr, (double)rr) : 0.0;
                 if (act) sb[c * NV + i] = neg_dinv_row<T>(sD + c * NB + i, sr + c * NV);
                 __syncthreads();
                 if (act) Sc.b[(size_t)p0 * NV + tid] = sb[tid];
@@ -3264,7 +3229,7 @@ __device__ __forceinline__ void multi_thomas_line(const MultiLine &S, int l, int
                 const T *ybot = base + 20 + (nb & 1) * 10;
                 T acc = bg[j][(size_t)ptw * NV + lane];
 #pragma unroll
-                for (int jj = 0; jj < NV; ++jj) acc -= gr[NV * jj] * ytop[jj] + cr[NV * jj] * ybot[jj];
+                for (int jj = 0; jj < NV; ++jj) acc -= fma_rn(gr[NV * jj], ytop[jj], mul_rn(cr[NV * jj], ybot[jj]));
                 xm[j] = acc;
             }
         }
@@ -3477,8 +3442,7 @@ struct MultiAcc {
             }
         }
     }
-    /* the same in neg_dinv_row's order: products j and j + 3 open sum j, the
-     * latter rounded (what the compiler makes of the sum of two products) */
+    /* the same in neg_dinv_row's order */
     __device__ __forceinline__ void set(const double *row, const double *v0, const int (&off)[MULTI_KG]) {
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
@@ -3493,7 +3457,7 @@ struct MultiAcc {
                 const double u0 = v[0], u1 = v[3], u2 = v[6];
 #pragma unroll
                 for (int q = 0; q < 3; ++q)
-                    a[k][q][j] = __fma_rn(x[2][q], u2, __fma_rn(x[0][q], u0, __dmul_rn(x[1][q], u1)));
+                    a[k][q][j] = fma_rn(x[2][q], u2, fma_rn(x[0][q], u0, mul_rn(x[1][q], u1)));
             }
         }
     }
@@ -3510,7 +3474,7 @@ __device__ __forceinline__ double warp_sums8(const double (&v)[8]) {
     for (int k = 0; k < 4; ++k) {
         const double keep = lane & 16 ? v[k + 4] : v[k], give = lane & 16 ? v[k] : v[k + 4];
         const double got = __shfl_xor_sync(FULL, give, 16);
-        w[k] = SQ ? __dadd_rn(__dmul_rn(keep, keep), __dmul_rn(got, got)) : keep + got;
+        w[k] = SQ ? mul_rn(keep, keep) + mul_rn(got, got) : keep + got;
     }
 #pragma unroll
     for (int k = 0; k < 2; ++k) {

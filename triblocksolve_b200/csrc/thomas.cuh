@@ -7,6 +7,7 @@
 #ifndef TBS_THOMAS_CUH
 #define TBS_THOMAS_CUH
 
+#include "device_common.cuh"
 #include "tbs_internal.hxx"
 #include "tma.cuh"
 
@@ -126,33 +127,32 @@ __device__ __forceinline__ void load_row(Row<float, 9> &R, const float *blk, int
 }
 
 /* init - row . vec in three partial sums: the terms j with NV - 1 - j
- * divisible by three go to the one that starts from init */
+ * divisible by three go to the one that starts from init, each of the others
+ * opens with its second product, rounded, and the first */
 template <int NV>
 __device__ __forceinline__ double row_dot(const Row<double, NV> &R, const StepVec<double, NV> &V, double init) {
-    double a0 = init, a1 = 0.0, a2 = 0.0;
+    double a[3] = {init, 0.0, 0.0};
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
         const int c = (NV - 1 - j) % 3;
         if (c == 0)
-            a0 -= R.r[j] * V.v[j];
-        else if (c == 1)
-            a1 = j < 3 ? R.r[j] * V.v[j] : a1 + R.r[j] * V.v[j];
-        else
-            a2 = j < 3 ? R.r[j] * V.v[j] : a2 + R.r[j] * V.v[j];
+            a[0] = fma_rn(-R.r[j], V.v[j], a[0]);
+        else if (j < 3)
+            a[c] = j + 3 < NV ? fma_rn(R.r[j], V.v[j], mul_rn(R.r[j + 3], V.v[j + 3])) : mul_rn(R.r[j], V.v[j]);
+        else if (j >= 6)
+            a[c] = fma_rn(R.r[j], V.v[j], a[c]);
     }
-    return a0 - (NV > 2 ? a1 + a2 : a1);
+    return a[0] - (NV > 2 ? a[1] + a[2] : a[1]);
 }
 
 __device__ __forceinline__ float row_dot(const Row<float, 9> &R, const StepVec<float, 9> &V, float init) {
-    float a0 = init - R.r[0] * V.s;
-    float a1 = R.r[1] * V.p[0].x;
-    float a2 = R.r[2] * V.p[0].y;
-    a0 -= R.r[3] * V.p[1].x;
-    a1 += R.r[4] * V.p[1].y;
-    a2 += R.r[5] * V.p[2].x;
-    a0 -= R.r[6] * V.p[2].y;
-    a1 += R.r[7] * V.p[3].x;
-    a2 += R.r[8] * V.p[3].y;
+    float a0 = fma_rn(-R.r[0], V.s, init);
+    float a1 = fma_rn(R.r[1], V.p[0].x, mul_rn(R.r[4], V.p[1].y));
+    float a2 = fma_rn(R.r[2], V.p[0].y, mul_rn(R.r[5], V.p[2].x));
+    a0 = fma_rn(-R.r[3], V.p[1].x, a0);
+    a0 = fma_rn(-R.r[6], V.p[2].y, a0);
+    a1 = fma_rn(R.r[7], V.p[3].x, a1);
+    a2 = fma_rn(R.r[8], V.p[3].y, a2);
     return a0 - (a1 + a2);
 }
 
@@ -524,7 +524,7 @@ __device__ __forceinline__ bool thomas_line(
             const T *cr = Gam + (size_t)(ps + ptw) * NB + lane;
             T acc = __ldcg(b + (size_t)(ps + ptw) * NV + lane);
 #pragma unroll
-            for (int j = 0; j < NV; ++j) acc -= gr[NV * j] * ytop[j] + cr[NV * j] * ybot[j];
+            for (int j = 0; j < NV; ++j) acc -= fma_rn(gr[NV * j], ytop[j], mul_rn(cr[NV * j], ybot[j]));
             xm = acc;
         }
         __syncwarp();
