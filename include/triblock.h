@@ -459,6 +459,11 @@ int tbs_profile_read(tbs_ctx *ctx, int *n, const char **names,
  * second).  No copy is issued, so nothing is left in flight. */
 int tbs_selftest_timeout(tbs_ctx *ctx, long long budget_cycles);
 
+/* Self-test of tbs_gmres on a device that holds fewer CTAs at once: from here
+ * on its orthogonalization is launched with at most `ctas` (0: as many as
+ * fit).  The results do not depend on it. */
+int tbs_selftest_orth_ctas(tbs_ctx *ctx, int ctas);
+
 /* Algorithmic bytes one launch of each kernel moves (reads + writes of
  * every array it must touch once), for the roofline numerator.  The
  * multi-RHS kernels take the group size as a suffix: "multi_thomas/8",

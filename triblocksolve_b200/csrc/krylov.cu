@@ -39,84 +39,46 @@ constexpr int KR_CHUNK = 8;  /* vectors per pass of the dot kernel */
 constexpr int KRYLOV_MAX = 64;
 constexpr unsigned KFULL = 0xffffffffu;
 
-/* partials[c * KR_BLOCKS + block] = this block's part of V_c . w for
- * c < count, and of w . w for c == count when self != 0.  Each thread
- * keeps KR_UNROLL grid-stride elements' loads in flight at once. */
-constexpr int KR_UNROLL = 4;
+constexpr int KR_UNROLL = 4; /* elements whose loads a thread keeps in flight */
 
+/* partials[block] = this block's part of w . w */
 __global__ void __launch_bounds__(KR_THREADS) kr_dots_kernel(long long n, const double *__restrict__ w,
-                                                             const double *__restrict__ V, long long ldv,
-                                                             int count, int self, double *partials) {
-    __shared__ double red[KR_CHUNK][KR_THREADS / 32];
-    const int total = count + (self ? 1 : 0);
-    const long long t0 = blockIdx.x * (long long)KR_THREADS + threadIdx.x;
+                                                             double *partials) {
+    __shared__ double red[KR_THREADS / 32];
     const long long stride = (long long)gridDim.x * KR_THREADS;
-    for (int c0 = 0; c0 < total; c0 += KR_CHUNK) {
-        double acc[KR_CHUNK];
+    long long t = blockIdx.x * (long long)KR_THREADS + threadIdx.x;
+    double acc = 0.0;
+    for (; t + (KR_UNROLL - 1) * stride < n; t += KR_UNROLL * stride) {
+        double wt[KR_UNROLL];
 #pragma unroll
-        for (int k = 0; k < KR_CHUNK; ++k) acc[k] = 0.0;
-        long long t = t0;
-        for (; t + (KR_UNROLL - 1) * stride < n; t += KR_UNROLL * stride) {
-            double wt[KR_UNROLL];
+        for (int u = 0; u < KR_UNROLL; ++u) wt[u] = w[t + u * stride];
 #pragma unroll
-            for (int u = 0; u < KR_UNROLL; ++u) wt[u] = w[t + u * stride];
-#pragma unroll
-            for (int k = 0; k < KR_CHUNK; ++k) {
-                const int c = c0 + k;
-                if (c < count) {
-                    const double *vc = V + (size_t)c * ldv + t;
-                    double x[KR_UNROLL];
-#pragma unroll
-                    for (int u = 0; u < KR_UNROLL; ++u) x[u] = vc[u * stride];
-#pragma unroll
-                    for (int u = 0; u < KR_UNROLL; ++u) acc[k] += x[u] * wt[u];
-                } else if (c == count && self) {
-#pragma unroll
-                    for (int u = 0; u < KR_UNROLL; ++u) acc[k] += wt[u] * wt[u];
-                }
-            }
-        }
-        for (; t < n; t += stride) {
-            const double wt = w[t];
-#pragma unroll
-            for (int k = 0; k < KR_CHUNK; ++k) {
-                const int c = c0 + k;
-                if (c < count)
-                    acc[k] += V[(size_t)c * ldv + t] * wt;
-                else if (c == count && self)
-                    acc[k] += wt * wt;
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < KR_CHUNK; ++k) {
-            double v = acc[k];
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(KFULL, v, o);
-            if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = v;
-        }
-        __syncthreads();
-        if (threadIdx.x < KR_CHUNK && c0 + (int)threadIdx.x < total) {
-            double tot = 0.0;
-            for (int q = 0; q < KR_THREADS / 32; ++q) tot += red[threadIdx.x][q];
-            partials[(size_t)(c0 + threadIdx.x) * KR_BLOCKS + blockIdx.x] = tot;
-        }
-        __syncthreads();
+        for (int u = 0; u < KR_UNROLL; ++u) acc += wt[u] * wt[u];
+    }
+    for (; t < n; t += stride) acc += w[t] * w[t];
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(KFULL, acc, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double tot = 0.0;
+        for (int q = 0; q < KR_THREADS / 32; ++q) tot += red[q];
+        partials[blockIdx.x] = tot;
     }
 }
 
-/* out[c] = sum of the KR_BLOCKS partials of c, in a fixed order */
+/* *out = sum of the KR_BLOCKS partials, in a fixed order */
 __global__ void __launch_bounds__(KR_THREADS) kr_reduce_kernel(const double *__restrict__ partials,
                                                                double *out) {
     __shared__ double red[KR_THREADS / 32];
-    const double *p = partials + (size_t)blockIdx.x * KR_BLOCKS;
     double v = 0.0;
-    for (int t = threadIdx.x; t < KR_BLOCKS; t += KR_THREADS) v += p[t];
+    for (int t = threadIdx.x; t < KR_BLOCKS; t += KR_THREADS) v += partials[t];
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(KFULL, v, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
     if (threadIdx.x == 0) {
         double tot = 0.0;
         for (int q = 0; q < KR_THREADS / 32; ++q) tot += red[q];
-        out[blockIdx.x] = tot;
+        *out = tot;
     }
 }
 
@@ -189,12 +151,14 @@ static_assert(KR_BLOCKS <= 2 * KR_THREADS, "kr_total adds two partials a thread"
 
 /* One Arnoldi step's orthogonalization in one cooperative launch:
  *   h = V^T w;  w -= V h;  h2 = V^T w, ww = w.w;  v_next = (w - V h2) / hn
- * with hn = sqrt(ww - h2.h2), each sum in the order of kr_dots_kernel /
- * kr_reduce_kernel / kr_combine_kernel, so the values are theirs.  Seven
+ * with hn = sqrt(ww - h2.h2), the partials and their sums in the order of
+ * kr_dots_kernel and kr_reduce_kernel.  Seven
  * launches and two copies did this: at 301x257 67 us a step by themselves and
  * the gaps between them; the vectors stay in the L2 there, so launches and
  * the reductions' latency were what bound it.  The second product needs w -
  * V h element by element only, so each thread goes on with its own elements.
+ * The vectors are dealt to KR_BLOCKS blocks whatever the grid: all CTAs have
+ * to be resident, and as many as are take the blocks in turn.
  * hout: h, then h2 and ww (host memory the device can write). */
 struct KrOrth {
     long long n, ldv;
@@ -208,17 +172,17 @@ __global__ void __launch_bounds__(KR_THREADS, 2) kr_orth_kernel(KrOrth A) {
     __shared__ double h[KRYLOV_MAX + 1], h2[KRYLOV_MAX + 2];
     __shared__ int s_ok;
     const int tid = threadIdx.x, warp = tid >> 5, count = A.count;
-    const long long t0 = blockIdx.x * (long long)KR_THREADS + tid;
-    const long long stride = (long long)gridDim.x * KR_THREADS;
+    const long long stride = (long long)KR_BLOCKS * KR_THREADS;
     const double *V = A.V;
-    /* partials of V_c . w for c < count (and w . w when self) */
-    auto dots = [&](int self) {
+    /* partials of V_c . w for c < count (and w . w when self), of the elements
+     * of block lb */
+    auto dots = [&](int self, int lb) {
         const int total = count + self;
         for (int c0 = 0; c0 < total; c0 += KR_CHUNK) {
             double acc[KR_CHUNK];
 #pragma unroll
             for (int k = 0; k < KR_CHUNK; ++k) acc[k] = 0.0;
-            long long t = t0;
+            long long t = lb * (long long)KR_THREADS + tid;
             for (; t + (KR_UNROLL - 1) * stride < A.n; t += KR_UNROLL * stride) {
                 double wt[KR_UNROLL];
 #pragma unroll
@@ -260,7 +224,7 @@ __global__ void __launch_bounds__(KR_THREADS, 2) kr_orth_kernel(KrOrth A) {
             if (tid < KR_CHUNK && c0 + tid < total) {
                 double tot = 0.0;
                 for (int q = 0; q < KR_THREADS / 32; ++q) tot += red[tid][q];
-                A.partials[(size_t)(c0 + tid) * KR_BLOCKS + blockIdx.x] = tot;
+                A.partials[(size_t)(c0 + tid) * KR_BLOCKS + lb] = tot;
             }
             __syncthreads();
         }
@@ -273,8 +237,8 @@ __global__ void __launch_bounds__(KR_THREADS, 2) kr_orth_kernel(KrOrth A) {
         __syncthreads();
     };
     /* dst = scale * (w - sum_c coef[c] V_c), the scaling left out when 1 */
-    auto combine = [&](const double *coef, double *dst, double scale, bool scaled) {
-        long long t = t0;
+    auto combine = [&](const double *coef, double *dst, double scale, bool scaled, int lb) {
+        long long t = lb * (long long)KR_THREADS + tid;
         for (; t + (KR_UNROLL - 1) * stride < A.n; t += KR_UNROLL * stride) {
             double acc[KR_UNROLL];
 #pragma unroll
@@ -294,15 +258,18 @@ __global__ void __launch_bounds__(KR_THREADS, 2) kr_orth_kernel(KrOrth A) {
             dst[t] = scaled ? scale * acc : acc;
         }
     };
-    dots(0);
+    auto blocks = [&](auto &&work) {
+        for (int lb = blockIdx.x; lb < KR_BLOCKS; lb += gridDim.x) work(lb);
+    };
+    blocks([&](int lb) { dots(0, lb); });
     bool ok = grid_meet(A.meet, 1, &s_ok, []() {});
     if (ok) {
         totals(count, h);
-        combine(h, A.w, 1.0, false);
+        blocks([&](int lb) { combine(h, A.w, 1.0, false, lb); });
         /* the first partials are read by others until they come to the second
          * meeting: the second ones lie behind them */
         A.partials += (size_t)(KRYLOV_MAX + 2) * KR_BLOCKS;
-        dots(1);
+        blocks([&](int lb) { dots(1, lb); });
         ok = grid_meet(A.meet, 2, &s_ok, []() {});
     }
     if (ok) {
@@ -310,7 +277,7 @@ __global__ void __launch_bounds__(KR_THREADS, 2) kr_orth_kernel(KrOrth A) {
         double s2 = 0.0; /* as the host's sum: no fused operations */
         for (int c = 0; c < count; ++c) s2 = __dadd_rn(s2, __dmul_rn(h2[c], h2[c]));
         const double hn = sqrt(fmax(__dsub_rn(h2[count], s2), 0.0));
-        combine(h2, A.vnext, 1.0 / hn, true);
+        blocks([&](int lb) { combine(h2, A.vnext, 1.0 / hn, true, lb); });
         if (blockIdx.x == 0) {
             for (int c = tid; c < count; c += KR_THREADS) A.hout[c] = h[c];
             for (int c = tid; c <= count; c += KR_THREADS) A.hout[KRYLOV_MAX + 2 + c] = h2[c];
@@ -336,6 +303,7 @@ struct KrylovBufs {
     double *h = nullptr, *y = nullptr;  /* KRYLOV_MAX + 2 each */
     double *h_host = nullptr;    /* pinned, mapped: h and h2 of a step */
     double *h_host_dev = nullptr;
+    int orth_ctas = 0;           /* of kr_orth_kernel's launch */
     unsigned *meet = nullptr;    /* kr_orth_kernel's meetings */
 };
 
@@ -403,6 +371,18 @@ static int kalloc(tbs_ctx *ctx, KrylovBufs *k, T **p, size_t count) {
         if (s_) return s_;                           \
     } while (0)
 
+/* CTAs of kr_orth_kernel that are resident at once, at most `most` */
+static int orth_fit(const tbs_ctx *ctx, int most) {
+    int per = 0, nsm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void *)kr_orth_kernel, KR_THREADS, 0) !=
+            cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess) {
+        cudaGetLastError();
+        return 1;
+    }
+    return std::max(1, std::min(most, per * nsm));
+}
+
 static int krylov_ensure(tbs_ctx *ctx, int m) {
     if (!ctx->krylov) {
         ctx->krylov = new KrylovBufs();
@@ -416,6 +396,7 @@ static int krylov_ensure(tbs_ctx *ctx, int m) {
         }
     }
     KrylovBufs *k = ctx->krylov;
+    if (k->orth_ctas == 0) k->orth_ctas = orth_fit(ctx, KR_BLOCKS);
     const long long n = (long long)ctx->L.np16 * 9;
     if (k->m >= m && k->n == n) return TBS_OK;
     KCK(cudaStreamSynchronize(ctx->stream));
@@ -433,14 +414,12 @@ static int krylov_ensure(tbs_ctx *ctx, int m) {
     return TBS_OK;
 }
 
-/* out[0..count) (+ w.w at out[count] when self) on the device */
-static int dots(tbs_ctx *ctx, const double *w, const double *V, int count, int self, double *out) {
+/* *out = w . w on the device */
+static int square(tbs_ctx *ctx, const double *w, double *out) {
     KrylovBufs *k = ctx->krylov;
-    KRUN("kr_dots", (kr_dots_kernel<<<KR_BLOCKS, KR_THREADS, 0, ctx->stream>>>(
-                         k->n, w, V, k->n, count, self, k->partials),
+    KRUN("kr_dots", (kr_dots_kernel<<<KR_BLOCKS, KR_THREADS, 0, ctx->stream>>>(k->n, w, k->partials),
                      cudaGetLastError()));
-    KRUN("kr_dots", (kr_reduce_kernel<<<count + (self ? 1 : 0), KR_THREADS, 0, ctx->stream>>>(
-                         k->partials, out),
+    KRUN("kr_dots", (kr_reduce_kernel<<<1, KR_THREADS, 0, ctx->stream>>>(k->partials, out),
                      cudaGetLastError()));
     return TBS_OK;
 }
@@ -460,7 +439,7 @@ static int orth(tbs_ctx *ctx, int j) {
     KrOrth A{k->n, k->n, j + 1, k->w, k->V, k->V + (size_t)(j + 1) * k->n, k->partials, k->h_host_dev, k->meet,
              ctx->d_status};
     void *args[] = {&A};
-    KRUN("kr_orth", cudaLaunchCooperativeKernel((const void *)kr_orth_kernel, dim3(KR_BLOCKS), dim3(KR_THREADS),
+    KRUN("kr_orth", cudaLaunchCooperativeKernel((const void *)kr_orth_kernel, dim3(k->orth_ctas), dim3(KR_THREADS),
                                                 args, 0, ctx->stream));
     return TBS_OK;
 }
@@ -525,7 +504,7 @@ static int gmres(tbs_ctx *ctx, int m, int psweeps, double tol, int max_iters, in
     /* U = 0; R = rhs (position order) */
     KCK(cudaMemsetAsync(ctx->d_Up, 0, (size_t)n * sizeof(double), st));
     KCK((cudaError_t)xfer_copy(st, ctx->d_rhsp, k->w, (size_t)n * sizeof(double), 0));
-    rc = dots(ctx, k->w, nullptr, 0, 1, k->h);
+    rc = square(ctx, k->w, k->h);
     if (rc) return rc;
     rc = read_back(ctx, k->h, 1, hh);
     if (rc) return rc;
@@ -593,7 +572,7 @@ static int gmres(tbs_ctx *ctx, int m, int psweeps, double tol, int max_iters, in
         /* the true residual R = rhs + J U opens the next cycle */
         rc = matvec(ctx, ctx->d_Up, k->w, ctx->d_rhs);
         if (rc) return rc;
-        rc = dots(ctx, k->w, nullptr, 0, 1, k->h);
+        rc = square(ctx, k->w, k->h);
         if (rc) return rc;
         rc = read_back(ctx, k->h, 1, hh);
         if (rc) return rc;
@@ -614,6 +593,22 @@ static int gmres(tbs_ctx *ctx, int m, int psweeps, double tol, int max_iters, in
     KCK(cudaStreamSynchronize(st));
     if (ctx->prof) ctx_prof_resolve(ctx);
     return ctx_status(ctx);
+}
+
+extern "C" int tbs_selftest_orth_ctas(tbs_ctx *ctx, int ctas) {
+    if (!ctx) return kfail(nullptr, TBS_ERR_ARG, "null context");
+    try {
+        if (cudaSetDevice(ctx->device) != cudaSuccess)
+            return kfail(ctx, TBS_ERR_CUDA, "cudaSetDevice failed");
+        if (!ctx->factored) return kfail(ctx, TBS_ERR_STATE, "tbs_factor must come first");
+        if (ctas < 0) return kfail(ctx, TBS_ERR_ARG, "negative number of CTAs");
+        const int rc = krylov_ensure(ctx, 1);
+        if (rc) return rc;
+        ctx->krylov->orth_ctas = orth_fit(ctx, ctas > 0 ? std::min(ctas, KR_BLOCKS) : KR_BLOCKS);
+        return TBS_OK;
+    } catch (...) {
+        return kfail(ctx, TBS_ERR_NOMEM, "host allocation failed");
+    }
 }
 
 extern "C" int tbs_gmres(tbs_ctx *ctx, int restart, int precond_sweeps, double rel_tol,
