@@ -126,17 +126,18 @@ __global__ void __launch_bounds__(KR_THREADS) kr_scale_kernel(long long n, doubl
     for (; t < n; t += stride) dst[t] = a * src[t];
 }
 
-/* The sums of the partials of dot product c in kr_reduce_kernel's order, by
- * one warp: the eight warps of that kernel one after the other. */
-__device__ __forceinline__ double kr_total(const double *__restrict__ partials, int c) {
+/* The sums of the `blocks` partials of dot product c (the others are zero) in
+ * kr_reduce_kernel's order, by one warp: the eight warps of that kernel one
+ * after the other. */
+__device__ __forceinline__ double kr_total(const double *__restrict__ partials, int c, int blocks) {
     const double *p = partials + (size_t)c * KR_BLOCKS;
     const int lane = threadIdx.x & 31;
     double v[KR_THREADS / 32];
 #pragma unroll
     for (int q = 0; q < KR_THREADS / 32; ++q) {
         const int t = 32 * q + lane;
-        v[q] = __ldcg(p + t);
-        if (t + KR_THREADS < KR_BLOCKS) v[q] += __ldcg(p + t + KR_THREADS);
+        v[q] = t < blocks ? __ldcg(p + t) : 0.0;
+        if (t + KR_THREADS < blocks) v[q] += __ldcg(p + t + KR_THREADS);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
@@ -158,11 +159,16 @@ static_assert(KR_BLOCKS <= 2 * KR_THREADS, "kr_total adds two partials a thread"
  * the reductions' latency were what bound it.  The second product needs w -
  * V h element by element only, so each thread goes on with its own elements.
  * The vectors are dealt to KR_BLOCKS blocks whatever the grid: all CTAs have
- * to be resident, and as many as are take the blocks in turn.
+ * to be resident, and as many as are take the blocks in turn.  There are no
+ * CTAs for blocks without elements: they would meet for nothing, and keep the
+ * launches of other contexts off the SMs (60x64: 482 us a solve with 135
+ * CTAs, 488 with 296; eight threads with a system each 111 us a solve in all,
+ * 175 with 296, 147 with plain launches).
  * hout: h, then h2 and ww (host memory the device can write). */
 struct KrOrth {
     long long n, ldv;
-    int count; /* basis vectors, 1 .. KRYLOV_MAX */
+    int count;  /* basis vectors, 1 .. KRYLOV_MAX */
+    int blocks; /* of the KR_BLOCKS, those that have elements */
     double *w, *V, *vnext, *partials, *hout;
     unsigned *meet, *status;
 };
@@ -231,7 +237,7 @@ __global__ void __launch_bounds__(KR_THREADS, 2) kr_orth_kernel(KrOrth A) {
     };
     auto totals = [&](int total, double *out) {
         for (int c = warp; c < total; c += KR_THREADS / 32) {
-            const double v = kr_total(A.partials, c);
+            const double v = kr_total(A.partials, c, A.blocks);
             if ((tid & 31) == 0) out[c] = v;
         }
         __syncthreads();
@@ -259,7 +265,7 @@ __global__ void __launch_bounds__(KR_THREADS, 2) kr_orth_kernel(KrOrth A) {
         }
     };
     auto blocks = [&](auto &&work) {
-        for (int lb = blockIdx.x; lb < KR_BLOCKS; lb += gridDim.x) work(lb);
+        for (int lb = blockIdx.x; lb < A.blocks; lb += gridDim.x) work(lb);
     };
     blocks([&](int lb) { dots(0, lb); });
     bool ok = grid_meet(A.meet, 1, &s_ok, []() {});
@@ -436,11 +442,12 @@ static int combine(tbs_ctx *ctx, double *x, const double *V, int count, const do
 /* h and h2 of w against V_0 .. V_j into h_host, V_{j+1} */
 static int orth(tbs_ctx *ctx, int j) {
     KrylovBufs *k = ctx->krylov;
-    KrOrth A{k->n, k->n, j + 1, k->w, k->V, k->V + (size_t)(j + 1) * k->n, k->partials, k->h_host_dev, k->meet,
+    const int blocks = (int)std::min<long long>(KR_BLOCKS, (k->n + KR_THREADS - 1) / KR_THREADS);
+    KrOrth A{k->n, k->n, j + 1, blocks, k->w, k->V, k->V + (size_t)(j + 1) * k->n, k->partials, k->h_host_dev, k->meet,
              ctx->d_status};
     void *args[] = {&A};
-    KRUN("kr_orth", cudaLaunchCooperativeKernel((const void *)kr_orth_kernel, dim3(k->orth_ctas), dim3(KR_THREADS),
-                                                args, 0, ctx->stream));
+    KRUN("kr_orth", cudaLaunchCooperativeKernel((const void *)kr_orth_kernel, dim3(std::min(blocks, k->orth_ctas)),
+                                                dim3(KR_THREADS), args, 0, ctx->stream));
     return TBS_OK;
 }
 
