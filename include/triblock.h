@@ -459,6 +459,14 @@ int tbs_profile_read(tbs_ctx *ctx, int *n, const char **names,
  * second).  No copy is issued, so nothing is left in flight. */
 int tbs_selftest_timeout(tbs_ctx *ctx, long long budget_cycles);
 
+/* Self-test of the failure path of the launches whose CTAs wait for one
+ * another (tbs_solve of few lines, tbs_gmres): from here on CTA `absent` of
+ * each (-1: none) does not come, and the others give up after budget_cycles
+ * (0: the usual budget, about a second).  A solve or tbs_gmres then returns
+ * TBS_ERR_CUDA and leaves the context usable; the iterate is undefined until
+ * the next one succeeds. */
+int tbs_selftest_meetings(tbs_ctx *ctx, int absent, long long budget_cycles);
+
 /* Self-test of tbs_gmres on a device that holds fewer CTAs at once: from here
  * on its orthogonalization is launched with at most `ctas` (0: as many as
  * fit).  The results do not depend on it. */

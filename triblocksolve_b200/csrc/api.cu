@@ -844,7 +844,7 @@ static int body_small(tbs_ctx *ctx, CondCtl cc) {
     NormSink ns = sink(ctx, 0, cc);
     ns.timer = ctx->d_ktimer;
     CKL(launch_small_sweeps(ctx->stream, ctx->L, ctx->d_G, ctx->d_Gam, ctx->d_Dinv, ctx->d_X, ctx->d_b, ctx->d_y,
-                            ctx->d_dUp, ctx->d_Up, ns, ctx->d_meet, ctx->d_status));
+                            ctx->d_dUp, ctx->d_Up, ns, ctx->d_meet, ctx->d_status, ctx->meet_test));
     return TBS_OK;
 }
 
@@ -1729,6 +1729,14 @@ int tbs_selftest_timeout(tbs_ctx *ctx, long long budget_cycles) {
     CKL(launch_selftest_timeout(ctx->stream, budget_cycles, ctx->d_status));
     return status_check(ctx);
     GUARD_END
+}
+
+int tbs_selftest_meetings(tbs_ctx *ctx, int absent, long long budget_cycles) {
+    if (!ctx) return ctx_fail(nullptr, TBS_ERR_ARG, "null context");
+    if (budget_cycles < 0) return ctx_fail(ctx, TBS_ERR_ARG, "negative budget");
+    drop_graph(ctx); /* its launches have the values before */
+    ctx->meet_test = MeetTest{absent < 0 ? -1 : absent, budget_cycles};
+    return TBS_OK;
 }
 
 int tbs_memory_allocated(const tbs_ctx *ctx, size_t *bytes) {

@@ -98,6 +98,7 @@ struct tbs_ctx {
     unsigned *h_status_dev = nullptr;
     unsigned *d_counter = nullptr; /* last-CTA ticket of the fused norm */
     unsigned *d_meet = nullptr;    /* arrivals of the launch of all sweeps */
+    tbs::MeetTest meet_test;       /* tbs_selftest_meetings */
     int algo = -1;
 
     /* ---- graph cache ---- */

@@ -79,13 +79,16 @@ static __device__ __forceinline__ bool record_check(SolveState *S, double *hist,
  * grid_leave's last CTA has left).  The arrivals are spread over MEETS words,
  * each watched by a lane of warp 0 (1.2 us a meeting of 148 CTAs).  `round`
  * counts a CTA's meetings from 1; s_ok: a word of the CTA's shared memory.
- * All threads call; false when the others did not come in about a second.
+ * All threads call; false when the others did not come within `budget` cycles.
+ * A CTA that has given up leaves the launch and misses the later meetings, so
+ * that the others give up there.
  * Warp 1 does `meanwhile` once its CTA has arrived. */
 constexpr int MEETS = 8, MEET_STRIDE = GRID_MEET_WORDS / (MEETS + 1);
+constexpr long long MEET_BUDGET = 1LL << 31; /* about a second */
 
 template <typename F>
 static __device__ __forceinline__ bool grid_meet(unsigned *meet, unsigned round, volatile int *s_ok,
-                                                 F &&meanwhile) {
+                                                 long long budget, F &&meanwhile) {
     __syncthreads();
     if (threadIdx.x < 32) {
         if (threadIdx.x == 0) {
@@ -97,7 +100,7 @@ static __device__ __forceinline__ bool grid_meet(unsigned *meet, unsigned round,
             const unsigned target = round * ((gridDim.x - threadIdx.x + MEETS - 1) / MEETS);
             const long long t0 = clock64();
             while ((int)(ld_acquire(meet + MEET_STRIDE * threadIdx.x) - target) < 0) {
-                if (clock64() - t0 > (1LL << 31)) {
+                if (clock64() - t0 > budget) {
                     here = false;
                     break;
                 }

@@ -1674,6 +1674,7 @@ struct SmallSweeps {
     unsigned long long loop, check; /* condition handles */
     int use_check;
     int keep; /* the blocks fit in the L2 and are read to stay there */
+    MeetTest test;
 };
 
 static size_t small_smem(const FastLayout &L) {
@@ -1710,8 +1711,9 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) small_sweeps_kernel(SmallSwe
     const int max_sweeps = S->max_sweeps, hist_cap = S->hist_cap;
     int sw = S->sweep;
     double nrm = 0.0;
-    bool met = false, ok = true;
-    const bool mine = (int)blockIdx.x < A.nline;
+    const bool away = (int)blockIdx.x == A.test.absent;
+    bool met = false, ok = !away;
+    const bool mine = (int)blockIdx.x < A.nline && !away;
     const int ls = mine ? A.line_start[blockIdx.x] : 0, ll = mine ? A.line_len[blockIdx.x] : 0,
               lt = mine ? A.line_twist[blockIdx.x] : 0;
     const uint64_t pol = A.keep ? policy_evict_last() : policy_evict_first();
@@ -1720,7 +1722,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) small_sweeps_kernel(SmallSwe
     const int c = tid % RES_TILE, i = tid / RES_TILE;
     const bool act = tid < RES_TILE * NV;
     const uint32_t szD = RES_TILE * NB * sizeof(double);
-    auto meet = [&](auto &&meanwhile) { return grid_meet(A.meet, ++round, s_ok, meanwhile); };
+    auto meet = [&](auto &&meanwhile) { return grid_meet(A.meet, ++round, s_ok, A.test.budget, meanwhile); };
     auto tile_of = [&](int k) { return (int)blockIdx.x + k * (int)gridDim.x; };
     auto blocks = [&](int k) { return reinterpret_cast<double *>(ring) + (size_t)(k % nbuf) * (1 + nx) * RES_TILE * NB; };
     auto issue = [&](int k) { /* thread 0: the k-th tile's blocks */
@@ -1789,7 +1791,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) small_sweeps_kernel(SmallSwe
         line(std::integral_constant<int, PH_BLOCKS>{});
         start_vecs();
     }
-    for (;;) {
+    while (ok) {
         /* ---------------- line solves */
         if (mine && warp < 2) ok = line(std::integral_constant<int, PH_RUN>{});
         ok = __syncthreads_and(ok); /* the ring is free */
@@ -1894,7 +1896,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) small_sweeps_kernel(SmallSwe
             break;
         }
     }
-    if (!ok && tid == 0) atomicOr(A.status, ST_TIMEOUT);
+    if (!ok && !away && tid == 0) atomicOr(A.status, ST_TIMEOUT);
     __syncthreads();
     if (tid == 0) {
         if (grid_leave(A.meet)) { /* every CTA has left the meetings */
@@ -1927,14 +1929,15 @@ int small_sweeps_grid(const FastLayout &L) {
 
 int launch_small_sweeps(cudaStream_t st, const FastLayout &L, const double *G, const double *Gam,
                         const double *Dinv, const double *X, double *b, double *y, double *dU, double *U,
-                        const NormSink &ns, unsigned *meet, unsigned *status) {
+                        const NormSink &ns, unsigned *meet, unsigned *status, MeetTest test) {
     const int grid = small_sweeps_grid(L);
     if (grid < 1) return (int)cudaErrorInvalidValue;
     SmallSweeps A{L.nline,  L.nx, L.np16, L.max_len, L.line_start, L.line_len, L.line_twist, L.xnbr,
                   G,        Gam,  Dinv,   X,         b,            y,          dU,           U,
                   ns.partials, ns.hist, ns.state, meet, status, ns.timer, ns.handle, ns.check_handle,
                   ns.use_check,
-                  (long long)L.np16 * (3 + L.nx) * NB * (long long)sizeof(double) <= (96LL << 20)};
+                  (long long)L.np16 * (3 + L.nx) * NB * (long long)sizeof(double) <= (96LL << 20),
+                  MeetTest{test.absent, test.budget > 0 ? test.budget : MEET_BUDGET}};
     void *args[] = {&A};
     return (int)cudaLaunchCooperativeKernel((const void *)small_sweeps_kernel, dim3(grid), dim3(SMALL_THREADS),
                                             args, small_smem(L), st);

@@ -164,13 +164,15 @@ static_assert(KR_BLOCKS <= 2 * KR_THREADS, "kr_total adds two partials a thread"
  * launches of other contexts off the SMs (60x64: 482 us a solve with 135
  * CTAs, 488 with 296; eight threads with a system each 111 us a solve in all,
  * 175 with 296, 147 with plain launches).
- * hout: h, then h2 and ww (host memory the device can write). */
+ * hout: h, then h2 and ww, then whether the status of the stream's launches
+ * so far is set (host memory the device can write). */
 struct KrOrth {
     long long n, ldv;
     int count;  /* basis vectors, 1 .. KRYLOV_MAX */
     int blocks; /* of the KR_BLOCKS, those that have elements */
     double *w, *V, *vnext, *partials, *hout;
     unsigned *meet, *status;
+    MeetTest test;
 };
 
 __global__ void __launch_bounds__(KR_THREADS, 2) kr_orth_kernel(KrOrth A) {
@@ -267,8 +269,12 @@ __global__ void __launch_bounds__(KR_THREADS, 2) kr_orth_kernel(KrOrth A) {
     auto blocks = [&](auto &&work) {
         for (int lb = blockIdx.x; lb < A.blocks; lb += gridDim.x) work(lb);
     };
-    blocks([&](int lb) { dots(0, lb); });
-    bool ok = grid_meet(A.meet, 1, &s_ok, []() {});
+    const bool away = (int)blockIdx.x == A.test.absent;
+    bool ok = !away;
+    if (ok) {
+        blocks([&](int lb) { dots(0, lb); });
+        ok = grid_meet(A.meet, 1, &s_ok, A.test.budget, []() {});
+    }
     if (ok) {
         totals(count, h);
         blocks([&](int lb) { combine(h, A.w, 1.0, false, lb); });
@@ -276,7 +282,7 @@ __global__ void __launch_bounds__(KR_THREADS, 2) kr_orth_kernel(KrOrth A) {
          * meeting: the second ones lie behind them */
         A.partials += (size_t)(KRYLOV_MAX + 2) * KR_BLOCKS;
         blocks([&](int lb) { dots(1, lb); });
-        ok = grid_meet(A.meet, 2, &s_ok, []() {});
+        ok = grid_meet(A.meet, 2, &s_ok, A.test.budget, []() {});
     }
     if (ok) {
         totals(count + 1, h2);
@@ -288,11 +294,14 @@ __global__ void __launch_bounds__(KR_THREADS, 2) kr_orth_kernel(KrOrth A) {
             for (int c = tid; c < count; c += KR_THREADS) A.hout[c] = h[c];
             for (int c = tid; c <= count; c += KR_THREADS) A.hout[KRYLOV_MAX + 2 + c] = h2[c];
         }
-    } else if (tid == 0) {
+    } else if (tid == 0 && !away) {
         atomicOr(A.status, ST_TIMEOUT);
     }
     __syncthreads();
-    if (tid == 0) grid_leave(A.meet);
+    if (tid == 0 && grid_leave(A.meet)) {
+        __threadfence(); /* what the others did before they left */
+        A.hout[2 * (KRYLOV_MAX + 2)] = ld_acquire(A.status) ? 1.0 : 0.0;
+    }
 }
 
 }  // namespace
@@ -307,7 +316,7 @@ struct KrylovBufs {
     double *w = nullptr;
     double *partials = nullptr;  /* 2 x (KRYLOV_MAX + 2) x KR_BLOCKS */
     double *h = nullptr, *y = nullptr;  /* KRYLOV_MAX + 2 each */
-    double *h_host = nullptr;    /* pinned, mapped: h and h2 of a step */
+    double *h_host = nullptr;    /* pinned, mapped: h and h2 of a step, the status */
     double *h_host_dev = nullptr;
     int orth_ctas = 0;           /* of kr_orth_kernel's launch */
     unsigned *meet = nullptr;    /* kr_orth_kernel's meetings */
@@ -392,7 +401,7 @@ static int orth_fit(const tbs_ctx *ctx, int most) {
 static int krylov_ensure(tbs_ctx *ctx, int m) {
     if (!ctx->krylov) {
         ctx->krylov = new KrylovBufs();
-        if (cudaHostAlloc((void **)&ctx->krylov->h_host, 2 * (KRYLOV_MAX + 2) * sizeof(double),
+        if (cudaHostAlloc((void **)&ctx->krylov->h_host, (2 * (KRYLOV_MAX + 2) + 1) * sizeof(double),
                           cudaHostAllocMapped) != cudaSuccess ||
             cudaHostGetDevicePointer((void **)&ctx->krylov->h_host_dev, ctx->krylov->h_host, 0) !=
                 cudaSuccess) {
@@ -444,7 +453,7 @@ static int orth(tbs_ctx *ctx, int j) {
     KrylovBufs *k = ctx->krylov;
     const int blocks = (int)std::min<long long>(KR_BLOCKS, (k->n + KR_THREADS - 1) / KR_THREADS);
     KrOrth A{k->n, k->n, j + 1, blocks, k->w, k->V, k->V + (size_t)(j + 1) * k->n, k->partials, k->h_host_dev, k->meet,
-             ctx->d_status};
+             ctx->d_status, MeetTest{ctx->meet_test.absent, ctx->meet_test.budget > 0 ? ctx->meet_test.budget : MEET_BUDGET}};
     void *args[] = {&A};
     KRUN("kr_orth", cudaLaunchCooperativeKernel((const void *)kr_orth_kernel, dim3(std::min(blocks, k->orth_ctas)),
                                                 dim3(KR_THREADS), args, 0, ctx->stream));
@@ -538,6 +547,10 @@ static int gmres(tbs_ctx *ctx, int m, int psweeps, double tol, int max_iters, in
             rc = orth(ctx, j);
             if (rc) return rc;
             KCK(cudaStreamSynchronize(st));
+            if (hh[2 * (KRYLOV_MAX + 2)] != 0.0) { /* the coefficients may be an earlier step's */
+                rc = ctx_status(ctx);
+                if (rc) return rc;
+            }
             const double *h1 = hh, *h2 = hh + KRYLOV_MAX + 2;
             double ww = h2[j + 1], s2 = 0.0;
             for (int i = 0; i <= j; ++i) {

@@ -212,13 +212,19 @@ int launch_fast_thomas(cudaStream_t st, const FastLayout &L, const T *G, const T
                        int nacc = -1, const T *Uin = nullptr);
 /* words in which the CTAs of a cooperative launch meet (grid_meet) */
 constexpr int GRID_MEET_WORDS = 9 * 64;
+/* self-test of the meetings: CTA `absent` (-1: none) stays away from them,
+ * the others wait `budget` cycles (0: about a second) */
+struct MeetTest {
+    int absent = -1;
+    long long budget = 0;
+};
 /* all the sweeps of a solve of few lines as one cooperative launch: the grid
  * it takes (0: not for this system), and the launch.  `ns` gives the norms'
  * places and the graph's conditions; meet: GRID_MEET_WORDS words, zero. */
 int small_sweeps_grid(const FastLayout &L);
 int launch_small_sweeps(cudaStream_t st, const FastLayout &L, const double *G, const double *Gam,
                         const double *Dinv, const double *X, double *b, double *y, double *dU, double *U,
-                        const NormSink &ns, unsigned *meet, unsigned *status);
+                        const NormSink &ns, unsigned *meet, unsigned *status, MeetTest test = MeetTest{});
 int fast_kernels_init();
 /* Several lines' vectors packed into (or unpacked from) one contiguous
  * buffer by one launch: line k's span is [start[k]*9, start[k]*9 + len[k]*9)
