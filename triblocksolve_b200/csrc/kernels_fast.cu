@@ -1908,7 +1908,17 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) small_sweeps_kernel(SmallSwe
     }
 }
 
-/* CTAs of a launch of all sweeps; 0: the system is not for it */
+/* CTAs of a launch of all sweeps; 0: the system is not for it.
+ * Where a CTA's place is an SM (lines beyond 537 cells), a launch per kernel,
+ * with six CTAs an SM on the tiles, is faster from some 48 blocks of 16
+ * positions a CTA on (this / that, us a sweep: 60x600 72 / 74 at 46 blocks,
+ * 36x1000 104 / 104 at 46, 20x2000 180 / 179 at 51, 60x800 93 / 91 at 61, 100x600
+ * 85 / 83 at 76, 148x1000 162 / 139 at 187; three and four neighbours off the
+ * line: 10x2x1500 147 / 144 at 51, 5x5x1000 107 / 109 at 53, 7x7x700 92 / 90 at
+ * 72); with two CTAs an SM it is not, up to the 100 that their lines allow
+ * (296x530 103 / 109; 17x17x500 133 / 145 at 153). */
+constexpr int SMALL_BLOCKS = 48;
+
 int small_sweeps_grid(const FastLayout &L) {
     if (L.nv != NV || L.nx < 1 || L.nx > 4) return 0;
     const size_t smem = small_smem(L);
@@ -1924,6 +1934,7 @@ int small_sweeps_grid(const FastLayout &L) {
     const int cap = std::min(per, 2) * nsm;
     if (L.nline > cap) return 0;
     const int ntiles = L.np16 / RES_TILE;
+    if (per == 1 && (long long)ntiles * (1 + L.nx) > (long long)SMALL_BLOCKS * nsm) return 0;
     return std::max(L.nline, std::min(ntiles, cap));
 }
 
