@@ -1909,6 +1909,13 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) small_sweeps_kernel(SmallSwe
 }
 
 /* CTAs of a launch of all sweeps; 0: the system is not for it.
+ * One a line at least, and one a tile up to half an SM count of them, where
+ * several such launches fit beside each other in any case.  More tiles go
+ * nbuf to a CTA while there are places (the second tile's blocks are copied
+ * under the first), so that the launches of several threads' contexts fit:
+ * 60x64 takes 12.9 us a sweep with 120 CTAs and 12.3 with 240, and four
+ * threads with a system each 59 us a solve in all, 98 with 240, 66 with a
+ * launch per kernel.
  * Where a CTA's place is an SM (lines beyond 537 cells), a launch per kernel,
  * with six CTAs an SM on the tiles, is faster from some 48 blocks of 16
  * positions a CTA on (this / that, us a sweep: 60x600 72 / 74 at 46 blocks,
@@ -1933,9 +1940,10 @@ int small_sweeps_grid(const FastLayout &L) {
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const int cap = std::min(per, 2) * nsm;
     if (L.nline > cap) return 0;
-    const int ntiles = L.np16 / RES_TILE;
+    const int ntiles = L.np16 / RES_TILE, nbuf = small_bufs(L.nx);
     if (per == 1 && (long long)ntiles * (1 + L.nx) > (long long)SMALL_BLOCKS * nsm) return 0;
-    return std::max(L.nline, std::min(ntiles, cap));
+    const int share = std::max((ntiles + nbuf - 1) / nbuf, std::min(ntiles, nsm / 2));
+    return std::max(L.nline, std::min(share, cap));
 }
 
 int launch_small_sweeps(cudaStream_t st, const FastLayout &L, const double *G, const double *Gam,
