@@ -1532,7 +1532,7 @@ static ThomasCfg thomas_cfg(const FastLayout &L) {
     cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
     if (nsm < 1) nsm = 148;
     const int per_sm = (L.nline + nsm - 1) / nsm;
-    const long long budget = (long long)smem_sm / (per_sm > 0 ? per_sm : 1) - reserved;
+    const long long budget = smem_share(smem_sm, per_sm, reserved);
     const size_t ys_bytes = (size_t)((L.max_len + 3) & ~3) * NV * sizeof(T);
     const size_t fixed = thomas_hdr<WS>() + BCAST<T, NV> * sizeof(T);
     ThomasCfg c;
@@ -3349,8 +3349,8 @@ static size_t multi_thomas_smem(int nr, int NS) {
            (size_t)multi_thomas_warps(nr) * MULTI_RPW * BCAST<double, NV> * sizeof(double);
 }
 
-/* ring depth: the shared memory each of the SM's resident lines may use,
- * at least 3 and at most 8 stages */
+/* ring depth: the shared memory each of the SM's resident lines may use (the
+ * kernel's static arrays come out of it), at least 3 and at most 8 stages */
 static int multi_thomas_ns(const FastLayout &L, int nr) {
     int dev = 0, nsm = 148, smem_sm = 228 * 1024, reserved = 1024;
     cudaGetDevice(&dev);
@@ -3362,8 +3362,10 @@ static int multi_thomas_ns(const FastLayout &L, int nr) {
     const int by_threads = 2048 / (32 * multi_thomas_warps(nr));
     if (per_sm > by_threads) per_sm = by_threads;
     if (per_sm < 1) per_sm = 1;
-    const long long budget = (long long)smem_sm / per_sm - reserved - (long long)multi_thomas_smem(nr, 0);
-    long long ns = budget / (long long)multi_thomas_stage(nr);
+    cudaFuncAttributes fa{};
+    cudaFuncGetAttributes(&fa, (const void *)multi_thomas_kernel<THOMAS_P>);
+    const long long budget = smem_share(smem_sm, per_sm, reserved) - (long long)fa.sharedSizeBytes;
+    long long ns = (budget - (long long)multi_thomas_smem(nr, 0)) / (long long)multi_thomas_stage(nr);
     if (ns > 8) ns = 8;
     if (ns < 3) ns = 3;
     return (int)ns;

@@ -545,7 +545,7 @@ struct NvOps {
         const long long sb = (long long)nv_thomas_stage<NV>();
         const long long ys = (long long)((L.max_len + 3) & ~3) * NV * (long long)sizeof(double);
         const long long bcast = (long long)(BCAST<double, NV> * sizeof(double));
-        const long long budget = std::min<long long>(smem_sm / per_sm, 227 * 1024) - reserved;
+        const long long budget = std::min<long long>(smem_share(smem_sm, per_sm, reserved), 227 * 1024 - reserved);
         c.ys = thomas_hdr<true>() + bcast + ys + 3 * sb <= budget;
         c.ws = c.ys || per_sm <= 5;
         const long long fixed = (c.ws ? thomas_hdr<true>() : thomas_hdr<false>()) + bcast;

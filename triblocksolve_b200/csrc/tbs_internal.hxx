@@ -124,6 +124,12 @@ struct FastLayout {
  * a context with a smaller mesh must not lower it under a larger one.
  * Returns a cudaError_t as an int. */
 int smem_raise(const void *fn, size_t need);
+/* shared memory of each of `per_sm` CTAs of which all are to be resident on an
+ * SM that has smem_sm bytes, `reserved` of them per CTA for the system; it is
+ * allocated in units of 128 bytes */
+inline long long smem_share(int smem_sm, int per_sm, int reserved) {
+    return (smem_sm / (per_sm > 0 ? per_sm : 1)) / 128 * 128 - reserved;
+}
 
 /* ------------------------------------------------------ kernel launchers
  * All launches go on `st`; they return cudaGetLastError() as an int. */
