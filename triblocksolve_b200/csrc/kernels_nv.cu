@@ -292,12 +292,16 @@ __global__ void nv_xlayout_kernel(long long nslots, const int *__restrict__ xsrc
 template <int NV>
 constexpr int nv_chunk() { return (NV >= 10 && NV <= 13) ? 4 : 8; }
 
+/* and where a line's y and x do not fit in shared memory beside the ring: at
+ * block size 16 half chunks, twice as many of them and a copy warp, since only
+ * three lines an SM are resident with either (us, 8 and 4 cells: 600x640 359 /
+ * 350, 1200x640 615 / 603, 740x300 168 / 168; block sizes 14 and 15 lose) */
 template <int NV>
-constexpr size_t nv_thomas_stage() { return thomas_stage_bytes<double, NV, nv_chunk<NV>()>(); }
+constexpr int nv_chunk_far() { return NV == 16 ? 4 : nv_chunk<NV>(); }
 
 /* One line per CTA: thomas_line with the chain warp issuing its own copies,
  * or (WS) a copy warp beside it; YS: y and x in shared memory. */
-template <int NV, bool WS, bool YS>
+template <int NV, int P, bool WS, bool YS>
 __global__ void __launch_bounds__(WS ? 64 : 32) nv_thomas_kernel(
     int nline, int NS, const int *__restrict__ line_start, const int *__restrict__ line_len,
     const int *__restrict__ line_twist, const double *__restrict__ G, const double *__restrict__ Gam,
@@ -314,9 +318,8 @@ __global__ void __launch_bounds__(WS ? 64 : 32) nv_thomas_kernel(
     }
     const uint64_t pol = threadIdx.x == (WS ? 32 : 0) ? policy_evict_first() : 0;
     uint32_t pbase = 0;
-    thomas_line<double, NV, nv_chunk<NV>(), YS, WS>(NS, accumulate, line_start[l], line_len[l],
-                                                    line_twist[l], G, Gam, b, y, dU, U, status, smem,
-                                                    pbase, pol);
+    thomas_line<double, NV, P, YS, WS>(NS, accumulate, line_start[l], line_len[l], line_twist[l], G, Gam, b,
+                                       y, dU, U, status, smem, pbase, pol);
 }
 
 /* positions per residual tile: 16 (the layout's granule), up to 64 for
@@ -526,7 +529,8 @@ struct NvOps {
      * lines share an SM (nvar 12, 600x640: 184 / 205), and costs beyond (nvar
      * 4, 1200x1280: 317 / 224).  The rest of the share goes to the ring (2..8
      * stages).  The form before, vectors passed by shuffles and barriers tested
-     * between chunks: nvar 5 60, 130 and 80 us, nvar 12 213 us at 600x640. */
+     * between chunks: nvar 5 60, 130 and 80 us, nvar 12 213, nvar 16 366 and now
+     * 350 us at 600x640. */
     struct Cfg {
         bool ws, ys;
         int ns;
@@ -542,19 +546,23 @@ struct NvOps {
         if (nsm < 1) nsm = 148;
         const int per_sm = std::max((L.nline + nsm - 1) / nsm, 1);
         Cfg c{};
-        const long long sb = (long long)nv_thomas_stage<NV>();
+        constexpr int PN = nv_chunk<NV>(), PF = nv_chunk_far<NV>();
+        constexpr long long near_stage = thomas_stage_bytes<double, NV, PN>(),
+                            far_stage = thomas_stage_bytes<double, NV, PF>();
         const long long ys = (long long)((L.max_len + 3) & ~3) * NV * (long long)sizeof(double);
         const long long bcast = (long long)(BCAST<double, NV> * sizeof(double));
         const long long budget = std::min<long long>(smem_share(smem_sm, per_sm, reserved), 227 * 1024 - reserved);
-        c.ys = thomas_hdr<true>() + bcast + ys + 3 * sb <= budget;
-        c.ws = c.ys || per_sm <= 5;
+        c.ys = thomas_hdr<true>() + bcast + ys + 3 * near_stage <= budget;
+        c.ws = c.ys || per_sm <= 5 || PF != PN;
+        const long long sb = c.ys ? near_stage : far_stage;
         const long long fixed = (c.ws ? thomas_hdr<true>() : thomas_hdr<false>()) + bcast;
         const long long left = budget - fixed - (c.ys ? ys : 0);
-        c.ns = (int)std::min<long long>(std::max<long long>(left / sb, 2), 8);
+        c.ns = (int)std::min<long long>(std::max<long long>(left / sb, 2 * near_stage / sb), 8);
         c.smem = (size_t)(fixed + c.ns * sb + (c.ys ? ys : 0));
-        c.fn = !c.ws  ? (const void *)nv_thomas_kernel<NV, false, false>
-               : c.ys ? (const void *)nv_thomas_kernel<NV, true, true>
-                      : (const void *)nv_thomas_kernel<NV, true, false>;
+        c.fn = c.ys ? (const void *)nv_thomas_kernel<NV, PN, true, true>
+                    : (const void *)nv_thomas_kernel<NV, PF, true, false>;
+        if constexpr (PF == PN)
+            if (!c.ws) c.fn = (const void *)nv_thomas_kernel<NV, PN, false, false>;
         return c;
     }
     static int thomas(cudaStream_t st, const FastLayout &L, const double *G, const double *Gam,
