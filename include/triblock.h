@@ -358,7 +358,9 @@ int tbs_part_check(tbs_ctx *ctx, double *owned_norm);
  * (block size 9; every launch, graph-launched ones included): the sum of
  * their durations in microseconds, each from its earliest CTA start to the
  * finish of its last CTA on the GPU's global nanosecond clock, and their
- * number.  reset != 0 starts a new record.  Waits for the context's
+ * number.  Where all the sweeps of a solve are one launch (few lines), a
+ * sweep's residual is a part of it, recorded from the first copy of the CTA
+ * that ends its line solve last to the end of the last tile.  reset != 0 starts a new record.  Waits for the context's
  * stream.  No counterpart in the reference (its timing is host-side,
  * src/main.cxx:233-252). */
 int tbs_resid_timer(tbs_ctx *ctx, double *total_us, long long *launches, int reset);

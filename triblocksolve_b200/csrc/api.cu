@@ -410,6 +410,7 @@ static int build_layout(tbs_ctx *ctx) {
     L.nxf = nxf;
     L.nline = nline;
     L.max_len = ctx->max_line;
+    L.longest = (int)(std::max_element(len.begin(), len.end()) - len.begin());
     ctx->n_xslots_real = nreal;
     ctx->n_fslots_real = nfreal;
     DA(L.line_start, nline);

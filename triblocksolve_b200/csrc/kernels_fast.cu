@@ -1663,7 +1663,7 @@ constexpr int SMALL_NS = 6;   /* ring stages of the line solve; two residual til
 constexpr int SMALL_HDR = 256;
 
 struct SmallSweeps {
-    int nline, nx, np16, max_len;
+    int nline, nx, np16, max_len, longest;
     const int *line_start, *line_len, *line_twist, *xnbr;
     const double *G, *Gam, *Dinv, *X;
     double *b, *y, *dU, *U, *partials, *hist;
@@ -1796,11 +1796,11 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) small_sweeps_kernel(SmallSwe
         if (mine && warp < 2) ok = line(std::integral_constant<int, PH_RUN>{});
         ok = __syncthreads_and(ok); /* the ring is free */
         if (!ok) break;
+        unsigned long long t0 = 0;
+        if (A.timer && (int)blockIdx.x == A.longest && tid == 0) t0 = globaltimer_ns();
         if (tid == 0)
             for (int k = 0; k < nbuf; ++k) issue(k);
         const bool came = meet([]() {});
-        unsigned long long t0 = 0;
-        if (A.timer && blockIdx.x == 0 && tid == 0) t0 = globaltimer_ns();
         /* ---------------- residual: R = sum X dU, b = -Dinv R; the next tile's
          * neighbours' dU is read while a tile is worked on */
         double g[4], gn[4];
@@ -1865,7 +1865,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) small_sweeps_kernel(SmallSwe
              }) && came;
         bool more = false;
         if (ok) {
-            if (A.timer && blockIdx.x == 0 && tid == 0) {
+            if (A.timer && (int)blockIdx.x == A.longest && tid == 0) {
                 atomicAdd(A.timer + 1, globaltimer_ns() - t0);
                 atomicAdd(A.timer + 2, 1ull);
             }
@@ -1951,7 +1951,7 @@ int launch_small_sweeps(cudaStream_t st, const FastLayout &L, const double *G, c
                         const NormSink &ns, unsigned *meet, unsigned *status, MeetTest test) {
     const int grid = small_sweeps_grid(L);
     if (grid < 1) return (int)cudaErrorInvalidValue;
-    SmallSweeps A{L.nline,  L.nx, L.np16, L.max_len, L.line_start, L.line_len, L.line_twist, L.xnbr,
+    SmallSweeps A{L.nline,  L.nx, L.np16, L.max_len, L.longest, L.line_start, L.line_len, L.line_twist, L.xnbr,
                   G,        Gam,  Dinv,   X,         b,            y,          dU,           U,
                   ns.partials, ns.hist, ns.state, meet, status, ns.timer, ns.handle, ns.check_handle,
                   ns.use_check,

@@ -100,6 +100,7 @@ struct FastLayout {
     int nx;        /* cross-line coupling slots per position */
     int nline;
     int max_len;   /* longest line */
+    int longest;   /* a line of that length */
     /* device arrays */
     int *line_start;   /* [nline] multiple of 4 */
     int *line_len;     /* [nline] */
@@ -192,7 +193,11 @@ struct NormSink {
     unsigned long long check_handle;
     unsigned long long *timer;   /* null, or the launch's device-clock record: [0] the
                                   * earliest CTA start (all ones between launches),
-                                  * [1] += last finish - [0] in ns, [2] += 1 launch */
+                                  * [1] += last finish - [0] in ns, [2] += 1 launch; of
+                                  * the launch of all sweeps, a sweep's residual: from
+                                  * the first copy of the CTA whose line is the longest
+                                  * (the last to end its line solve, as a launch would
+                                  * start) to the meeting behind the tiles */
 };
 /* NormSink::is_start of the check of a converged solve: a norm at or below
  * the tolerance ends the solve with the history unchanged; a larger one
