@@ -1926,8 +1926,9 @@ int tbs_kernel_bytes(tbs_ctx *ctx, const char *kernel, double *bytes) {
         b = N * 2 * vec + X * (blk + 4.0 + vec);
     else if (k == "pij_sweep") /* Dinv, face blocks + index + neighbour dU, own dU, U in/out, b out */
         b = N * (blk + 4 * vec) + (double)ctx->n_fslots_real * (blk + 4.0 + vec);
-    else if (k == "fast_factor") /* D, A, C in; Dinv, G, Gam out */
-        b = N * blk + 2 * (N - ctx->nline) * blk + 3 * N * blk;
+    else if (k == "fast_factor") /* D, A, C in; Dinv, G, Gam out; FP64: X in and out */
+        b = N * blk + 2 * (N - ctx->nline) * blk + 3 * N * blk +
+            (ctx->algo == TBS_ALGO_FP64 && ctx->nvar == 9 ? 2 * X * blk : 0.0);
     if (b < 0) return ctx_fail(ctx, TBS_ERR_ARG, "unknown kernel name " + k);
     *bytes = b;
     return TBS_OK;

@@ -282,8 +282,7 @@ int launch_mixed_prime(cudaStream_t st, const FastLayout &L, const double *rhsp,
                        double *Up, double *partials, const float *Dinv32, float *b32, float *c32);
 
 /* TBS_ALGO_FP64 for the block sizes other than 9 (kernels_nv.cu): the
- * same launch sequence with kernels templated on nv (2..16); G and Gam are
- * column-major here (the size-9 kernels keep them row-major). */
+ * same launch sequence with kernels templated on nv (2..16), the same layout */
 bool nv_supported(int nv);
 int nv_prepare(int nv, const FastLayout &L);
 int launch_nv_factor(cudaStream_t st, int nv, const FastLayout &L, const double *jacD,

@@ -47,12 +47,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
     return ok != 0;
 }
 
-/* plain arrival (count 1) on `bar` */
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-/* the same by the lanes with `on` set, without a branch */
+/* arrival (count 1) on `bar` by the lanes with `on` set, without a branch */
 __device__ __forceinline__ void mbar_arrive_if(uint64_t *bar, bool on) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
