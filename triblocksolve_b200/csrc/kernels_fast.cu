@@ -281,13 +281,14 @@ int launch_axpy2_f32_f64(cudaStream_t st, const float *c, const float *d, double
  * warp that copies the coming cells' blocks into shared memory, forms G (no
  * step waits for it) and writes the results, so that the chain warps run
  * nothing but the chain.
- * Few lines (at most two per SM) leave the SM's pipes idle and the step's
- * latency counts alone; there 27 lanes per chain are faster (27 multiply-adds
- * a product, 98 cycles a pivot against 122), one CTA per line:
- * fast_factor_few_kernel.  Measured (us; few / this / a warp per chain doing
- * everything, the form before): 100 lines of 256 cells 157 / 204 / 218, 290 of
- * 256 195 / 201 / 229, 440 of 256 239 / 201 / 261, 600 of 640 876 / 758 / 789,
- * 1200 of 1280 3,060 / 2,260 / 2,810.
+ * Few lines (at most seven for four SMs) leave the SM's pipes idle and the
+ * step's latency counts alone; there 27 lanes per chain are faster (27
+ * multiply-adds a product, a pivot's chain shorter by a fifth), one CTA per
+ * line: fast_factor_few_kernel.  Measured with the cross-line copy (us; few /
+ * this / a warp per chain doing everything and the copy behind it, the form
+ * before): 100 lines of 256 cells 160 / 215 / 240, 255 of 256 199 / 219, 290 of
+ * 256 234 / 216 / 279, 440 of 256 273 / 218 / 332, 600 of 640 920 / 777 / 1,020,
+ * 1200 of 1280 4,210 / 2,840 / 3,750.
  */
 
 struct FactorOut {
@@ -460,7 +461,7 @@ __device__ __forceinline__ void put_27(const double (&c)[3], double *x, int j, i
 constexpr int FEW_STAGES = 6;
 constexpr int FEW_WORDS = (3 * FEW_STAGES + 5) * NB;
 
-/* The factorization of few lines (at most two per SM): one CTA per line,
+/* The factorization of few lines (launch_fast_factor): one CTA per line,
  * warps 0 / 1 on its top / bottom chain, warp 2 helping both; the three meet
  * once per cell.  In step s a chain warp eliminates cell s (Gam_{s-1},
  * Dinv_s), the helper starts the copies of cell s + 4, forms and writes
@@ -993,12 +994,12 @@ int launch_fast_factor(cudaStream_t st, const FastLayout &L, const double *jacD,
     if (nsm < 1) nsm = 148;
     /* CTAs that copy, each with at least a few blocks.  While the
      * factorization's CTAs are at most one per SM: one per SM, so that all are
-     * resident at once and the chains stay spread over the SMs (360x384: 307
-     * us with 148, 329 with 74, 458 with 296, which fills the SMs and puts two
-     * factorizing CTAs on one; 120x128: 88, 89, 105).  Else four per SM, which
-     * take their places as they come free (600x640: 758 us with 592, 864 with
-     * 148; 1200x640: 1,420 and 1,890). */
-    const bool few = L.nline <= 2 * nsm;
+     * resident at once and the chains stay spread over the SMs (360x384: 1.07
+     * of the time with half as many, 1.5 with twice as many, which fill the SMs
+     * and put two factorizing CTAs on one; 120x128: 1.01 and 1.2).  Else four
+     * per SM, which take their places as they come free (600x640: 0.88 of the
+     * time with one per SM, 1200x640: 0.75). */
+    const bool few = 4 * (long long)L.nline <= 7 * (long long)nsm;
     const int nfac = (L.nline + 2) / 3;
     const int most = few || nfac <= nsm ? nsm : 4 * nsm;
     const int copiers = X ? (int)std::min<long long>(most, (xc.nslots + 63) / 64) : 0;
