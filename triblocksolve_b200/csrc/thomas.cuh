@@ -156,6 +156,14 @@ __device__ __forceinline__ float row_dot(const Row<float, 9> &R, const StepVec<f
     return a0 - (a1 + a2);
 }
 
+/* The next chunk's stage is taken two steps before its first row is read, so
+ * that the barrier's answer is there; where blocks of 13 and more leave the
+ * ring two stages, at that step: a stage is refilled when its chunk is done,
+ * and what is taken early was asked for late (900x1100, nvar 13 529 / 520 us, 15
+ * 830 / 817, 16 878 / 867; smaller blocks and deeper rings lose up to 3 %). */
+template <int NV, bool YS>
+constexpr bool LATE = NV >= 13 && !YS;
+
 /* words of the broadcast vectors: 2 halves x 2 alternating buffers */
 template <typename T, int NV>
 constexpr int BCAST = 4 * StepVec<T, NV>::BUF;
@@ -178,6 +186,10 @@ __device__ __forceinline__ void fwd_chunk(const T *sG, Row<T, NV> &row, T &bi, T
         Row<T, NV> nrow;
         StepVec<T, NV> v;
         T nb = T(0);
+        if (LATE<NV, YS> && q == P - 1) {
+            const T *n = next();
+            if (n) sN = n;
+        }
         v.load(bc + (q & 1) * VB, i, q & 1);
         if (q + 1 < P) {
             load_row(nrow, sG + (q + 1) * NB, i, (q + 1) & 1);
@@ -187,7 +199,7 @@ __device__ __forceinline__ void fwd_chunk(const T *sG, Row<T, NV> &row, T &bi, T
             nb = sN[P * NB + i];
         }
         if (q == 1) probe();
-        if (q == P - 3) {
+        if (!LATE<NV, YS> && q == P - 3) {
             const T *n = next();
             if (n) sN = n;
         }
@@ -224,10 +236,14 @@ __device__ __forceinline__ void bwd_chunk(const T *sG, Row<T, NV> &row, T &yk, T
         const int f = (P - 1 - q) & 1; /* buffer alternates per step */
         Row<T, NV> nrow;
         StepVec<T, NV> v;
+        if (LATE<NV, YS> && q == 0) {
+            const T *n = next();
+            if (n) sN = n;
+        }
         v.load(bc + f * VB, i, q & 1);
         load_row(nrow, q > 0 ? sG + (q - 1) * NB : sN + (P - 1) * NB, i, (q + P - 1) & 1);
         if (q == P - 2) probe();
-        if (q == 2) {
+        if (!LATE<NV, YS> && q == 2) {
             const T *n = next();
             if (n) sN = n;
         }
