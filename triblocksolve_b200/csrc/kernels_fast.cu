@@ -1099,21 +1099,35 @@ __device__ __forceinline__ uint64_t *resid_bar_init() {
     return bar;
 }
 
-/* the first six products of a row of a block (column-major, at its entry of
- * column 0) with a vector, in the three sums a[0..2] that the others join:
- * products j and j + 3 open sum j, the latter rounded by itself */
+/* The products of a row of a block (column-major, at its entry of column 0)
+ * with a vector, in three sums: a_j takes products j, j + 3, j + 6.
+ * open_sums: the first six, products j and j + 3 opening a_j, the latter
+ * rounded by itself.  (The sums as an array: the batch residual spilled.) */
 template <typename T>
-__device__ __forceinline__ void open_sums(T (&a)[3], const T *row, const T *v) {
-#pragma unroll
-    for (int j = 0; j < 3; ++j) a[j] = fma_rn(row[9 * j], v[j], mul_rn(row[9 * j + 27], v[j + 3]));
+__device__ __forceinline__ void open_sums(T &a0, T &a1, T &a2, const T *row, const T *v) {
+    a0 = fma_rn(row[0], v[0], mul_rn(row[27], v[3]));
+    a1 = fma_rn(row[9], v[1], mul_rn(row[36], v[4]));
+    a2 = fma_rn(row[18], v[2], mul_rn(row[45], v[5]));
 }
 
-/* a[j] += products j, j + 3, j + 6 (from product `first` on) */
+/* the last three products */
 template <typename T>
-__device__ __forceinline__ void add_products(T (&a)[3], const T *row, const T *v, int first = 0) {
-#pragma unroll
-    for (int j = 0; j < 9; ++j)
-        if (j >= first) a[j % 3] = fma_rn(row[9 * j], v[j], a[j % 3]);
+__device__ __forceinline__ void close_sums(T &a0, T &a1, T &a2, const T *row, const T *v) {
+    a0 = fma_rn(row[54], v[6], a0);
+    a1 = fma_rn(row[63], v[7], a1);
+    a2 = fma_rn(row[72], v[8], a2);
+}
+
+/* all nine */
+template <typename T>
+__device__ __forceinline__ void add_products(T &a0, T &a1, T &a2, const T *row, const T *v) {
+    a0 = fma_rn(row[0], v[0], a0);
+    a1 = fma_rn(row[9], v[1], a1);
+    a2 = fma_rn(row[18], v[2], a2);
+    a0 = fma_rn(row[27], v[3], a0);
+    a1 = fma_rn(row[36], v[4], a1);
+    a2 = fma_rn(row[45], v[5], a2);
+    close_sums(a0, a1, a2, row, v);
 }
 
 /* -(row of Dinv) . R for one (cell, row): dr points at entry (row, 0) of
@@ -1121,10 +1135,10 @@ __device__ __forceinline__ void add_products(T (&a)[3], const T *row, const T *v
  * the order every b = -Dinv R of this file uses */
 template <typename T>
 __device__ __forceinline__ T neg_dinv_row(const T *dr, const T *rv) {
-    T a[3];
-    open_sums(a, dr, rv);
-    add_products(a, dr, rv, 6);
-    return -(a[0] + (a[1] + a[2]));
+    T a0, a1, a2;
+    open_sums(a0, a1, a2, dr, rv);
+    close_sums(a0, a1, a2, dr, rv);
+    return -(a0 + (a1 + a2));
 }
 
 /* One tile (positions blk*RES_TILE ..) with the staging barrier's phase of
@@ -1198,13 +1212,13 @@ __device__ __forceinline__ bool fast_resid_body(
     T r = T(0);
     if (mode >= 1) {
         if (act) {
-            T a[3] = {T(0), T(0), T(0)};
+            T a0 = T(0), a1 = T(0), a2 = T(0);
             for (int s = 0; s < nx; ++s) {
                 const T *xr = sX + (s * RES_TILE + c) * NB + i;
                 const T *g = sg + (s * RES_TILE + c) * NV;
-                add_products(a, xr, g);
+                add_products(a0, a1, a2, xr, g);
             }
-            r = a[0] + (a[1] + a[2]);
+            r = a0 + (a1 + a2);
             sr[c * NV + i] = r;
         }
         __syncthreads();
@@ -1832,13 +1846,13 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) small_sweeps_kernel(SmallSwe
             const double *sD = blocks(k), *sX = sD + RES_TILE * NB;
             double r = 0.0;
             if (act) {
-                double a[3] = {0.0, 0.0, 0.0};
+                double a0 = 0.0, a1 = 0.0, a2 = 0.0;
                 for (int s = 0; s < nx; ++s) {
                     const double *xr = sX + (s * RES_TILE + c) * NB + i;
                     const double *q = sg + (s * RES_TILE + c) * NV;
-                    add_products(a, xr, q);
+                    add_products(a0, a1, a2, xr, q);
                 }
-                r = a[0] + (a[1] + a[2]);
+                r = a0 + (a1 + a2);
                 sr[c * NV + i] = r;
             }
             __syncthreads();
@@ -2011,19 +2025,19 @@ __device__ __forceinline__ void full_resid_body(
         const int pe = pos_of_elem[e];
         const double *u = Up + (size_t)pe * NV;
         const double *dr = D + (size_t)e * NB + i;
-        double a[3];
-        open_sums(a, dr, u);
-        add_products(a, dr, u, 6);
+        double a0, a1, a2;
+        open_sums(a0, a1, a2, dr, u);
+        close_sums(a0, a1, a2, dr, u);
         for (int k2 = epoint[e]; k2 < epoint[e + 1]; ++k2) {
             const int f = ef[k2];
             if (f >= 0) {
                 const int e1 = fc[2 * f], e2 = fc[2 * f + 1];
                 const double *o = ((e == e1) ? O2 : O1) + (size_t)f * NB + i;
                 const double *un = Up + (size_t)pos_of_elem[(e == e1) ? e2 : e1] * NV;
-                add_products(a, o, un);
+                add_products(a0, a1, a2, o, un);
             }
         }
-        const double r = (rhs ? rhs[(size_t)e * NV + i] : 0.0) + (a[0] + (a[1] + a[2]));
+        const double r = (rhs ? rhs[(size_t)e * NV + i] : 0.0) + (a0 + (a1 + a2));
         Rp[(size_t)pe * NV + i] = (T)r;
         sq = mul_rn(r, r);
     }
@@ -2179,15 +2193,15 @@ __device__ __forceinline__ bool full_resid_pos_body(
     if (act) {
         const double *dr = sD + c * NB + i;
         const double *u = sg + c * NV;
-        double a[3];
-        open_sums(a, dr, u);
-        add_products(a, dr, u, 6);
+        double a0, a1, a2;
+        open_sums(a0, a1, a2, dr, u);
+        close_sums(a0, a1, a2, dr, u);
         for (int s = 0; s < nxf; ++s) {
             const double *o = sX + (s * RES_TILE + c) * NB + i;
             const double *un = sg + ((s + 1) * RES_TILE + c) * NV;
-            add_products(a, o, un);
+            add_products(a0, a1, a2, o, un);
         }
-        const double r = sr[c * NV + i] + (a[0] + (a[1] + a[2]));
+        const double r = sr[c * NV + i] + (a0 + (a1 + a2));
         so[c * NV + i] = (float)r;
         sq = mul_rn(r, r);
     }
@@ -2668,13 +2682,13 @@ __global__ void __launch_bounds__(RES_THREADS_FAST) fast_resid_group_kernel(
                 }
                 T rr = T(0);
                 if (act) {
-                    T a[3] = {T(0), T(0), T(0)};
+                    T a0 = T(0), a1 = T(0), a2 = T(0);
                     for (int s = 0; s < nx; ++s) {
                         const T *xr = sX + (s * RES_TILE + c) * NB + i;
                         const T *g = sg + (s * RES_TILE + c) * NV;
-                        add_products(a, xr, g);
+                        add_products(a0, a1, a2, xr, g);
                     }
-                    rr = a[0] + (a[1] + a[2]);
+                    rr = a0 + (a1 + a2);
                     sr[c * NV + i] = rr;
                 }
                 __syncthreads();
