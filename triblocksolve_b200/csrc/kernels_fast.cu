@@ -3025,7 +3025,12 @@ template int launch_resid_batch<float>(cudaStream_t, int, int, const ResidSys<fl
  * first `nown` of them write. */
 constexpr int MULTI_RPW = 2;
 
-template <int P, bool CHECK>
+/* AHEAD: the vectors of both right-hand sides of a warp are read before either
+ * product; else each before its own, which takes 36 registers fewer.  The
+ * kernel of one system has room for them (8 right-hand sides at 360x384: 155 us
+ * for 161); the one that reads its lines' addresses from memory has not (it
+ * spilled: 2 right-hand sides 111 us, 83 without). */
+template <int P, bool CHECK, bool AHEAD>
 __device__ __forceinline__ void fwd_chunk_m(const double *sG, const double *const *sB,
                                             double *const *bc, double *const *yg, int nown,
                                             int kbase, int len, int cpos, int i) {
@@ -3039,7 +3044,7 @@ __device__ __forceinline__ void fwd_chunk_m(const double *sG, const double *cons
         StepVec<double, NV> v[MULTI_RPW];
 #pragma unroll
         for (int j = 0; j < MULTI_RPW; ++j) {
-            v[j].load(bc[j] + (q & 1) * 10, i, 0);
+            if (AHEAD) v[j].load(bc[j] + (q & 1) * 10, i, 0);
             next_b[j] = 0.0;
         }
         if (q + 1 < P) {
@@ -3049,7 +3054,10 @@ __device__ __forceinline__ void fwd_chunk_m(const double *sG, const double *cons
         }
         double yi[MULTI_RPW];
 #pragma unroll
-        for (int j = 0; j < MULTI_RPW; ++j) yi[j] = row_dot(cur_row, v[j], cur_b[j]);
+        for (int j = 0; j < MULTI_RPW; ++j) {
+            if (!AHEAD) v[j].load(bc[j] + (q & 1) * 10, i, 0);
+            yi[j] = row_dot(cur_row, v[j], cur_b[j]);
+        }
         /* lanes 9..15 repeat lane 8's row, value and address: no divergence */
         if (!CHECK || kbase + q < len) {
             const int pos = cpos + kbase + q;
@@ -3068,7 +3076,7 @@ __device__ __forceinline__ void fwd_chunk_m(const double *sG, const double *cons
     }
 }
 
-template <int P, bool CHECK>
+template <int P, bool CHECK, bool AHEAD>
 __device__ __forceinline__ void bwd_chunk_m(const double *sG, double *const *bc,
                                             const double (*yv)[P], double *const *dUl, int nown,
                                             int kbase, int len, int cpos, int i) {
@@ -3079,13 +3087,17 @@ __device__ __forceinline__ void bwd_chunk_m(const double *sG, double *const *bc,
         const int f = (P - 1 - q) & 1;
         StepVec<double, NV> v[MULTI_RPW];
 #pragma unroll
-        for (int j = 0; j < MULTI_RPW; ++j) v[j].load(bc[j] + f * 10, i, 0);
+        for (int j = 0; j < MULTI_RPW; ++j)
+            if (AHEAD) v[j].load(bc[j] + f * 10, i, 0);
         if (q > 0) load_row(next_row, sG + (q - 1) * NB, i, 0);
         const bool valid = !CHECK || (kbase + q >= 0 && kbase + q < len);
         const int pos = cpos + kbase + q;
         double d[MULTI_RPW];
 #pragma unroll
-        for (int j = 0; j < MULTI_RPW; ++j) d[j] = row_dot(cur_row, v[j], valid ? yv[j][q] : 0.0);
+        for (int j = 0; j < MULTI_RPW; ++j) {
+            if (!AHEAD) v[j].load(bc[j] + f * 10, i, 0);
+            d[j] = row_dot(cur_row, v[j], valid ? yv[j][q] : 0.0);
+        }
         if (valid) { /* lanes 9..15 repeat lane 8's row, value and address */
 #pragma unroll
             for (int j = 0; j < MULTI_RPW; ++j) {
@@ -3107,7 +3119,7 @@ __device__ __forceinline__ void bwd_chunk_m(const double *sG, double *const *bc,
  * chunks of b of the active right-hand sides, a backward stage a chunk of
  * Gam rows.  All warps have consumed a stage before it is refilled (one
  * CTA barrier per chunk). */
-template <int P>
+template <int P, bool AHEAD>
 __device__ __forceinline__ void multi_thomas_line(const MultiLine &S, int l, int NS,
                                                   const int *__restrict__ active, unsigned *status) {
     using T = double;
@@ -3234,9 +3246,9 @@ __device__ __forceinline__ void multi_thomas_line(const MultiLine &S, int l, int
 #pragma unroll
             for (int j = 0; j < MULTI_RPW; ++j) sB[j] = sG + P * NB + slot[j] * P * NV;
             if (c < both_full)
-                fwd_chunk_m<P, false>(sG, sB, bc, yl, nown, c * P, len, cpos, i);
+                fwd_chunk_m<P, false, AHEAD>(sG, sB, bc, yl, nown, c * P, len, cpos, i);
             else
-                fwd_chunk_m<P, true>(sG, sB, bc, yl, nown, c * P, len, cpos, i);
+                fwd_chunk_m<P, true, AHEAD>(sG, sB, bc, yl, nown, c * P, len, cpos, i);
             __syncwarp();
         }
         if (__syncthreads_or(!ok)) {
@@ -3308,9 +3320,9 @@ __device__ __forceinline__ void multi_thomas_line(const MultiLine &S, int l, int
                 const bool full = (nchT - 1 - jb) * P + P <= m && (nchB - 1 - jb) * P + P <= nb &&
                                   nchT - 1 - jb >= 0 && nchB - 1 - jb >= 0;
                 if (full)
-                    bwd_chunk_m<P, false>(sG, bc, yv, dUl, nown, c * P, len, cpos, i);
+                    bwd_chunk_m<P, false, AHEAD>(sG, bc, yv, dUl, nown, c * P, len, cpos, i);
                 else
-                    bwd_chunk_m<P, true>(sG, bc, yv, dUl, nown, c * P, len, cpos, i);
+                    bwd_chunk_m<P, true, AHEAD>(sG, bc, yv, dUl, nown, c * P, len, cpos, i);
                 __syncwarp();
             }
             if (__syncthreads_or(!ok)) {
@@ -3340,7 +3352,7 @@ template <int P>
 __global__ void __launch_bounds__(32 * MULTI_MAX / MULTI_RPW) multi_thomas_kernel(
     int nline, int NS, MultiLine S, const int *__restrict__ active, unsigned *status) {
     if ((int)blockIdx.x >= nline) return;
-    multi_thomas_line<P>(S, blockIdx.x, NS, active, status);
+    multi_thomas_line<P, true>(S, blockIdx.x, NS, active, status);
 }
 
 /* the batch engine: item k = (group of one system's members, line) */
@@ -3350,7 +3362,7 @@ __global__ void __launch_bounds__(32 * MULTI_MAX / MULTI_RPW) multi_thomas_items
     int NS, const int *__restrict__ active, unsigned *status) {
     if ((int)blockIdx.x >= *nitems) return;
     const WorkItem it = items[blockIdx.x];
-    multi_thomas_line<P>(sys[it.sys], it.unit, NS, active, status);
+    multi_thomas_line<P, false>(sys[it.sys], it.unit, NS, active, status);
 }
 
 static int multi_thomas_warps(int nr) { return (nr + MULTI_RPW - 1) / MULTI_RPW; }
