@@ -164,8 +164,8 @@ static_assert(KR_BLOCKS <= 2 * KR_THREADS, "kr_total adds two partials a thread"
  * launches of other contexts off the SMs (60x64: 482 us a solve with 135
  * CTAs, 488 with 296; eight threads with a system each 111 us a solve in all,
  * 175 with 296, 147 with plain launches).
- * hout: h, then h2 and ww, then whether the status of the stream's launches
- * so far is set (host memory the device can write). */
+ * hout: h, then h2 and ww, then a word set to 1 when the status of the
+ * stream's launches so far is set (host memory the device can write). */
 struct KrOrth {
     long long n, ldv;
     int count;  /* basis vectors, 1 .. KRYLOV_MAX */
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(KR_THREADS, 2) kr_orth_kernel(KrOrth A) {
     __syncthreads();
     if (tid == 0 && grid_leave(A.meet)) {
         __threadfence(); /* what the others did before they left */
-        A.hout[2 * (KRYLOV_MAX + 2)] = ld_acquire(A.status) ? 1.0 : 0.0;
+        if (ld_acquire(A.status)) A.hout[2 * (KRYLOV_MAX + 2)] = 1.0;
     }
 }
 
@@ -454,6 +454,7 @@ static int orth(tbs_ctx *ctx, int j) {
     const int blocks = (int)std::min<long long>(KR_BLOCKS, (k->n + KR_THREADS - 1) / KR_THREADS);
     KrOrth A{k->n, k->n, j + 1, blocks, k->w, k->V, k->V + (size_t)(j + 1) * k->n, k->partials, k->h_host_dev, k->meet,
              ctx->d_status, MeetTest{ctx->meet_test.absent, ctx->meet_test.budget > 0 ? ctx->meet_test.budget : MEET_BUDGET}};
+    k->h_host[2 * (KRYLOV_MAX + 2)] = 0.0;
     void *args[] = {&A};
     KRUN("kr_orth", cudaLaunchCooperativeKernel((const void *)kr_orth_kernel, dim3(std::min(blocks, k->orth_ctas)),
                                                 dim3(KR_THREADS), args, 0, ctx->stream));
