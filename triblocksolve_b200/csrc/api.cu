@@ -646,7 +646,7 @@ static int body(tbs_ctx *ctx, CondCtl cc, int inner) {
     cudaStream_t st = ctx->stream;
     const int nv = ctx->nvar, ne = ctx->nelem;
     if (ctx->algo == TBS_ALGO_REFERENCE) {
-        RUN("ref_solve_du", launch_ref_solve_du(st, nv, ctx->nline, ctx->d_linesize, ctx->d_linepoint,
+        RUN("ref_solve_du", launch_ref_solve_du(st, nv, ctx->nline, ctx->nlineelem, ctx->max_line, ctx->d_linesize, ctx->d_linepoint,
                                                 ctx->d_lines, ctx->d_DLU, ctx->d_DinvC, ctx->d_A,
                                                 ctx->d_dU, ctx->d_R));
         RUN("ref_add_copy", launch_ref_add_copy(st, nvec(ctx), ctx->d_dU, ctx->d_U, ctx->d_rhs, ctx->d_R));
@@ -992,8 +992,8 @@ static int run_factor(tbs_ctx *ctx, int algo) {
         CKL(copy_words(st, ctx->d_jacD, ctx->d_DLU, nb * sizeof(double)));
         CK(cudaMemsetAsync(ctx->d_DinvC, 0, nb * sizeof(double), st));
         CK(cudaMemsetAsync(ctx->d_A, 0, nb * sizeof(double), st));
-        RUN("ref_line_lu", launch_ref_line_lu(st, nv, ctx->nline, ctx->d_fc, ctx->d_linesize,
-                                              ctx->d_linepoint, ctx->d_lines, ctx->d_lineface,
+        RUN("ref_line_lu", launch_ref_line_lu(st, nv, ctx->nline, ctx->nlineelem, ctx->max_line, ctx->d_fc,
+                                              ctx->d_linesize, ctx->d_linepoint, ctx->d_lines, ctx->d_lineface,
                                               ctx->d_DLU, ctx->d_O1, ctx->d_O2, ctx->d_DinvC,
                                               ctx->d_A, ctx->d_status));
         return TBS_OK;

@@ -23,6 +23,8 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 namespace tbs {
 
 constexpr int REF_MAXNV = 32;
@@ -55,7 +57,9 @@ __device__ __forceinline__ void solve_lu_lane(const double *A, const double *b, 
 /* In-place no-pivot Doolittle on a shared-memory block, rows over lanes.
  * Row j is final when step j starts and only rows i > j change in it, so
  * lane i applying its own row's updates reproduces lineLU_v2.okl:17-27. */
-__device__ __forceinline__ void lu_rows(double *A, int lane, int nv, unsigned *status) {
+template <int NV>
+__device__ __forceinline__ void lu_rows(double *A, int lane, int nv_rt, unsigned *status) {
+    const int nv = NV ? NV : nv_rt;
     for (int j = 0; j < nv; ++j) {
         __syncwarp();
         const double ajj = A[MIDX(j, j, nv)];
@@ -70,11 +74,13 @@ __device__ __forceinline__ void lu_rows(double *A, int lane, int nv, unsigned *s
     __syncwarp();
 }
 
+template <int NV>
 __global__ void __launch_bounds__(32) ref_line_lu_kernel(
-    int nv, int nline, const int *__restrict__ fc, const int *__restrict__ linesize,
+    int nv_rt, int nline, const int *__restrict__ fc, const int *__restrict__ linesize,
     const int *__restrict__ linepoint, const int *__restrict__ lines,
     const int *__restrict__ lineface, double *__restrict__ Dia, const double *__restrict__ O1,
     const double *__restrict__ O2, double *__restrict__ DinvC, unsigned *status) {
+    const int nv = NV ? NV : nv_rt;
     const int l = blockIdx.x;
     if (l >= nline) return;
     const int lane = threadIdx.x;
@@ -91,7 +97,7 @@ __global__ void __launch_bounds__(32) ref_line_lu_kernel(
     int e = lines[m0];
     if (lane < nv)
         for (int j = 0; j < nv; ++j) sDe[MIDX(lane, j, nv)] = Dia[MIDX(lane, j, nv) + bs * e];
-    lu_rows(sDe, lane, nv, status);
+    lu_rows<NV>(sDe, lane, nv, status);
     if (lane < nv)
         for (int j = 0; j < nv; ++j) Dia[MIDX(lane, j, nv) + bs * e] = sDe[MIDX(lane, j, nv)];
 
@@ -121,7 +127,7 @@ __global__ void __launch_bounds__(32) ref_line_lu_kernel(
         }
         __syncwarp();
         /* Gamma(:,i) = D'_{k-1}^-1 C(:,i)  (lineLU_v2.okl:142-144) */
-        if (lane < nv) solve_lu_lane<0>(sDl, &sC[MIDX(0, lane, nv)], &sGamma[MIDX(0, lane, nv)], nv);
+        if (lane < nv) solve_lu_lane<NV>(sDl, &sC[MIDX(0, lane, nv)], &sGamma[MIDX(0, lane, nv)], nv);
         __syncwarp();
         /* D_k - A_k Gamma  (lineLU_v2.okl:147-161) */
         if (lane < nv) {
@@ -131,7 +137,7 @@ __global__ void __launch_bounds__(32) ref_line_lu_kernel(
                 sDe[MIDX(lane, kk, nv)] -= tot;
             }
         }
-        lu_rows(sDe, lane, nv, status);
+        lu_rows<NV>(sDe, lane, nv, status);
         if (lane < nv) {
             for (int j = 0; j < nv; ++j) {
                 Dia[MIDX(lane, j, nv) + bs * e] = sDe[MIDX(lane, j, nv)];
@@ -417,25 +423,58 @@ __global__ void ref_assemble_A_kernel(int nv, int nline, const int *__restrict__
     }
 }
 
+/* Block size 9: whether the kernels of two warps a line are the faster ones.
+ * They are where the longest line's chain sets the time or four lines an SM
+ * (their registers allow no more) take them all in a few rounds; the kernels
+ * of one warp a line, slower along a chain, hold all of an SM's lines at once
+ * and have nothing to fill before the first cell.  Estimates, in us: two
+ * warps, `step` a cell and line and two cells' worth (the factorization) or
+ * three to start a line, in rounds of four lines an SM; one warp, a cell
+ * `alone` and `more` for each line that shares the SM, or `flow` a cell and SM.
+ * Measured (two warps / one, us): solve 592x16 23 / 38, 1200x100 288 / 299,
+ * 1800x100 384 / 317, 700x8 24 / 22, 592x3 11 / 11, 20000x16 588 / 364, 20000x1
+ * 82 / 23; factorization 592x16 37 / 87, 1200x16 84 / 105,
+ * 1800x100 682 / 714, 2500x16 148 / 138, 20000x3 221 / 154. */
+struct RefRate {
+    double step, start, alone, more, flow;
+};
+constexpr RefRate REF_LU{1.74, 2.0, 5.2, 0.16, 0.385}, REF_DU{1.0, 3.0, 2.6, 0.05, 0.17};
+
+static bool ref_two_warps(const RefRate &r, int nline, long long cells, int longest) {
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (nsm < 1) nsm = 148;
+    const double rounds = (nline + 4 * nsm - 1) / (4 * nsm), mean = (double)cells / nline;
+    const double two = r.step * std::max(longest + r.start, rounds * (mean + r.start));
+    const double one = std::max(longest * (r.alone + r.more * nline / nsm), r.flow * (double)cells / nsm);
+    return two < one;
+}
+
+
 /* the line factorization (DLU in place, DinvC) and the packed lower blocks */
-int launch_ref_line_lu(cudaStream_t st, int nv, int nline, const int *fc, const int *linesize,
-                       const int *linepoint, const int *lines, const int *lineface, double *DLU,
+int launch_ref_line_lu(cudaStream_t st, int nv, int nline, long long cells, int longest, const int *fc,
+                       const int *linesize, const int *linepoint, const int *lines, const int *lineface, double *DLU,
                        const double *O1, const double *O2, double *DinvC, double *A, unsigned *status) {
     if (nv < 1 || nv > REF_MAXNV) return (int)cudaErrorInvalidValue;
-    if (nv == 9) {
+    if (nv == 9 && ref_two_warps(REF_LU, nline, cells, longest)) {
         ref_line_lu9_kernel<<<nline, 64, 0, st>>>(nline, fc, linesize, linepoint, lines, lineface, DLU, O1,
                                                   O2, DinvC, A, status);
         return (int)cudaGetLastError();
     }
     const size_t smem = 5 * (size_t)nv * nv * sizeof(double);
     if (smem > 48 * 1024) {
-        const int e = smem_raise((const void *)ref_line_lu_kernel, smem);
+        const int e = smem_raise((const void *)ref_line_lu_kernel<0>, smem);
         if (e != 0) return e;
     }
     ref_assemble_A_kernel<<<nline, dim3(32, 8), 0, st>>>(nv, nline, fc, linesize, linepoint, lines,
                                                          lineface, O1, O2, A);
-    ref_line_lu_kernel<<<nline, 32, smem, st>>>(nv, nline, fc, linesize, linepoint, lines, lineface, DLU,
-                                                O1, O2, DinvC, status);
+    if (nv == 9)
+        ref_line_lu_kernel<9><<<nline, 32, smem, st>>>(nv, nline, fc, linesize, linepoint, lines, lineface,
+                                                       DLU, O1, O2, DinvC, status);
+    else
+        ref_line_lu_kernel<0><<<nline, 32, smem, st>>>(nv, nline, fc, linesize, linepoint, lines, lineface,
+                                                       DLU, O1, O2, DinvC, status);
     return (int)cudaGetLastError();
 }
 
@@ -602,11 +641,13 @@ __global__ void __launch_bounds__(64) ref_solve_du9_kernel(
 /* linesmoothLU_TriBlock_v3.okl:92-226, any block size.  Lane 0 runs solveLU as the
  * reference does (its `if(i==0)` guard, :154/:192); the other lanes do the
  * row-parallel matvecs and prefetch the next cell's blocks meanwhile. */
+template <int NV>
 __global__ void __launch_bounds__(32) ref_solve_du_kernel(
-    int nv, int nline, const int *__restrict__ linesize, const int *__restrict__ linepoint,
+    int nv_rt, int nline, const int *__restrict__ linesize, const int *__restrict__ linepoint,
     const int *__restrict__ lines, const double *__restrict__ Dia,
     const double *__restrict__ DinvC, const double *__restrict__ A, double *__restrict__ dU,
     const double *__restrict__ R) {
+    const int nv = NV ? NV : nv_rt;
     const int l = blockIdx.x;
     if (l >= nline) return;
     const int lane = threadIdx.x;
@@ -625,7 +666,7 @@ __global__ void __launch_bounds__(32) ref_solve_du_kernel(
         for (int j = 0; j < nv; ++j) sDia[MIDX(lane, j, nv)] = Dia[MIDX(lane, j, nv) + bs * e];
     }
     __syncwarp();
-    if (lane == 0) solve_lu_lane<0>(sDia, sS, sdU, nv);
+    if (lane == 0) solve_lu_lane<NV>(sDia, sS, sdU, nv);
     __syncwarp();
     if (lane < nv) dU[lane + (size_t)nv * e] = sdU[lane];
 
@@ -645,7 +686,7 @@ __global__ void __launch_bounds__(32) ref_solve_du_kernel(
             sS[lane] = -R[lane + (size_t)nv * e] - tot;
         }
         __syncwarp();
-        if (lane == 0) solve_lu_lane<0>(sDia, sS, sdU, nv);
+        if (lane == 0) solve_lu_lane<NV>(sDia, sS, sdU, nv);
         __syncwarp();
         if (lane < nv) dU[lane + (size_t)nv * e] = sdU[lane];
     }
@@ -666,17 +707,19 @@ __global__ void __launch_bounds__(32) ref_solve_du_kernel(
     }
 }
 
-int launch_ref_solve_du(cudaStream_t st, int nv, int nline, const int *linesize,
-                        const int *linepoint, const int *lines, const double *DLU,
+int launch_ref_solve_du(cudaStream_t st, int nv, int nline, long long cells, int longest,
+                        const int *linesize, const int *linepoint, const int *lines, const double *DLU,
                         const double *DinvC, const double *A, double *dU, const double *R) {
     if (nv < 1 || nv > REF_MAXNV) return (int)cudaErrorInvalidValue;
     const size_t smem = (2 * (size_t)nv * nv + 2 * REF_MAXNV) * sizeof(double);
-    if (nv == 9) {
+    if (nv == 9 && ref_two_warps(REF_DU, nline, cells, longest))
         ref_solve_du9_kernel<<<nline, 64, 0, st>>>(nline, linesize, linepoint, lines, DLU, DinvC, A, dU, R);
-    } else {
-        ref_solve_du_kernel<<<nline, 32, smem, st>>>(nv, nline, linesize, linepoint, lines, DLU,
-                                                        DinvC, A, dU, R);
-    }
+    else if (nv == 9)
+        ref_solve_du_kernel<9><<<nline, 32, smem, st>>>(nv, nline, linesize, linepoint, lines, DLU, DinvC, A,
+                                                        dU, R);
+    else
+        ref_solve_du_kernel<0><<<nline, 32, smem, st>>>(nv, nline, linesize, linepoint, lines, DLU, DinvC, A,
+                                                        dU, R);
     return (int)cudaGetLastError();
 }
 

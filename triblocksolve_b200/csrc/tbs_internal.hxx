@@ -135,13 +135,14 @@ inline long long smem_share(int smem_sm, int per_sm, int reserved) {
 /* ------------------------------------------------------ kernel launchers
  * All launches go on `st`; they return cudaGetLastError() as an int. */
 
-/* reference-order kernels (kernels_ref.cu, built with -fmad=false) */
-int launch_ref_line_lu(cudaStream_t st, int nv, int nline, const int *fc, const int *linesize,
-                       const int *linepoint, const int *lines, const int *lineface, double *DLU,
+/* reference-order kernels (kernels_ref.cu, built with -fmad=false); cells,
+ * longest: of all lines together, of the longest line */
+int launch_ref_line_lu(cudaStream_t st, int nv, int nline, long long cells, int longest, const int *fc,
+                       const int *linesize, const int *linepoint, const int *lines, const int *lineface, double *DLU,
                        const double *O1, const double *O2, double *DinvC, double *A,
                        unsigned *status);
-int launch_ref_solve_du(cudaStream_t st, int nv, int nline, const int *linesize,
-                        const int *linepoint, const int *lines, const double *DLU,
+int launch_ref_solve_du(cudaStream_t st, int nv, int nline, long long cells, int longest,
+                        const int *linesize, const int *linepoint, const int *lines, const double *DLU,
                         const double *DinvC, const double *A, double *dU, const double *R);
 int launch_ref_add_copy(cudaStream_t st, long long n, const double *dU, double *U,
                         const double *rhs, double *R);
