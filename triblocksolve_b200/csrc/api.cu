@@ -409,6 +409,7 @@ static int build_layout(tbs_ctx *ctx) {
     L.nx = nx;
     L.nxf = nxf;
     L.nline = nline;
+    L.cells = ctx->nlineelem;
     L.max_len = ctx->max_line;
     L.longest = (int)(std::max_element(len.begin(), len.end()) - len.begin());
     ctx->n_xslots_real = nreal;
@@ -646,9 +647,9 @@ static int body(tbs_ctx *ctx, CondCtl cc, int inner) {
     cudaStream_t st = ctx->stream;
     const int nv = ctx->nvar, ne = ctx->nelem;
     if (ctx->algo == TBS_ALGO_REFERENCE) {
-        RUN("ref_solve_du", launch_ref_solve_du(st, nv, ctx->nline, ctx->nlineelem, ctx->max_line, ctx->d_linesize, ctx->d_linepoint,
-                                                ctx->d_lines, ctx->d_DLU, ctx->d_DinvC, ctx->d_A,
-                                                ctx->d_dU, ctx->d_R));
+        RUN("ref_solve_du", launch_ref_solve_du(st, nv, ctx->nline, ctx->nlineelem, ctx->max_line,
+                                                ctx->d_linesize, ctx->d_linepoint, ctx->d_lines, ctx->d_DLU,
+                                                ctx->d_DinvC, ctx->d_A, ctx->d_dU, ctx->d_R));
         RUN("ref_add_copy", launch_ref_add_copy(st, nvec(ctx), ctx->d_dU, ctx->d_U, ctx->d_rhs, ctx->d_R));
         int np = 0;
         RUN("ref_line_res", launch_ref_line_res(st, nv, ctx->nline, ne, ctx->d_epoint, ctx->d_ef,

@@ -977,10 +977,138 @@ __global__ void __launch_bounds__(128, 3) fast_factor_kernel(
     if (bad && act) atomicOr(status, ST_PIVOT);
 }
 
+/* The factorization of many short lines: one warp per line, its top chain, its
+ * bottom chain and its twist cell one after the other, the blocks in registers
+ * a cell ahead.  Nothing has to be filled or drained, and 20 lines an SM hide
+ * each other's latencies, where the pairs of warps above spend three steps a
+ * line at the ends of their chains and hold nine. */
+__global__ void __launch_bounds__(32) fast_factor_short_kernel(
+    int nline, const int *__restrict__ line_start, const int *__restrict__ line_len,
+    const int *__restrict__ line_twist, const int *__restrict__ fsrc,
+    const double *__restrict__ jacD, const double *__restrict__ O1, const double *__restrict__ O2,
+    FactorOut out, XCopy xc, unsigned *status) {
+    __shared__ double sM[NB], sA[NB], sC[NB], sGm[2][NB];
+    const int line = blockIdx.x;
+    if (line >= nline) {
+        xcopy_part(xc, O1, O2);
+        return;
+    }
+    const int lane = threadIdx.x;
+    /* lanes 27..31 repeat lanes 18..22 and store nothing */
+    const bool act = lane < 27;
+    const int j = act ? lane % 9 : lane - 27;
+    const int g = act ? lane / 9 : 2, r0 = 3 * g;
+    const int ps = line_start[line], n = line_len[line], m = line_twist[line];
+    const int ptw = ps + n - 1;
+    double an[3], cn[3], dn[3];
+    auto load = [&](double (&v)[3], const double *x) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) v[k] = x[r0 + k + NV * j];
+    };
+    auto clear = [&](double (&v)[3]) { v[0] = v[1] = v[2] = 0.0; };
+    /* the blocks of step s of a chain: A, C and D of its cell, C alone (the
+     * coupling to the twist) behind the last cell */
+    auto fetch = [&](int chain, int cs, int len, int s) {
+        const int *q = fsrc + 5 * (s < len ? cs + s : ptw);
+        const int at = s < len || !chain ? 1 : 3;
+        const size_t f = (size_t)q[at] * NB;
+        const bool second = q[at + 1] != 0;
+        load(cn, (second ? O1 : O2) + f);
+        if (s < len) {
+            load(an, (second ? O2 : O1) + f);
+            load(dn, jacD + (size_t)q[0] * NB);
+        }
+    };
+    auto put = [&](const double (&v)[3], size_t p, auto &&store) {
+        if (act) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) store(p * NB + r0 + k + NV * j, v[k]);
+        }
+    };
+    auto dinv = [&](size_t q, double v) { out.put_dinv(q, v); };
+    auto gq = [&](size_t q, double v) { out.put_g(q, v); };
+    auto gamq = [&](size_t q, double v) { out.put_gam(q, v); };
+    bool bad = false;
+    for (int chain = 0; chain < 2; ++chain) {
+        const int len = chain ? n - 1 - m : m, cs = ps + (chain ? m : 0);
+        if (len == 0) continue;
+        double w[3], x[3];
+        load(w, jacD + (size_t)fsrc[5 * cs] * NB);
+        fetch(chain, cs, len, 1);
+        for (int s = 0;; ++s) {
+            if (s > 0) {
+                const double d[3] = {dn[0], dn[1], dn[2]};
+                if (act) {
+                    put_27(cn, sC, j, r0);
+                    put_27(an, sA, j, r0);
+                }
+                if (s < len) fetch(chain, cs, len, s + 1);
+                __syncwarp();
+                clear(x);
+                product_27<false>(x, sM, sC, j, r0);
+                put(x, cs + s - 1, gamq);
+                if (act) put_27(x, sGm[chain], j, r0);
+                __syncwarp();
+                if (s == len) break;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) w[k] = d[k];
+                product_27<true>(w, sA, sGm[chain], j, r0);
+            }
+            bad = gj_invert_27(w, j, g) || bad;
+            if (act) put_27(w, sM, j, r0);
+            put(w, cs + s, dinv);
+            __syncwarp();
+            clear(x);
+            if (s > 0) product_27<false>(x, sM, sA, j, r0);
+            put(x, cs + s, gq);
+            __syncwarp(); /* sA and sC are written again */
+        }
+        __syncwarp(); /* and sM */
+    }
+    /* ---------------- the twist cell */
+    const int *q = fsrc + 5 * ptw;
+    double w[3];
+    load(w, jacD + (size_t)q[0] * NB);
+    clear(an);
+    clear(cn);
+    if (q[1] >= 0) load(an, (q[2] ? O2 : O1) + (size_t)q[1] * NB);
+    if (q[3] >= 0) load(cn, (q[4] ? O2 : O1) + (size_t)q[3] * NB);
+    if (act) {
+        put_27(an, sA, j, r0);
+        put_27(cn, sC, j, r0);
+    }
+    __syncwarp();
+    if (m > 0) product_27<true>(w, sA, sGm[0], j, r0);
+    if (n - 1 - m > 0) product_27<true>(w, sC, sGm[1], j, r0);
+    bad = gj_invert_27(w, j, g) || bad;
+    if (act) put_27(w, sM, j, r0);
+    __syncwarp();
+    double ga[3] = {0.0, 0.0, 0.0}, gc[3] = {0.0, 0.0, 0.0};
+    product_27<false>(ga, sM, sA, j, r0);
+    product_27<false>(gc, sM, sC, j, r0);
+    put(w, ptw, dinv);
+    put(ga, ptw, gq);
+    put(gc, ptw, gamq);
+    if (bad && lane == 0) atomicOr(status, ST_PIVOT);
+}
+
 /* cells in shared memory per pair of warps: six (copies four steps ahead)
  * where the CTAs of three lines are at most two per SM, else four, which
  * keeps three CTAs resident */
 static int fac_stages(const FastLayout &L, int nsm) { return (L.nline + 2) / 3 <= 2 * nsm ? 6 : 4; }
+
+/* Whether the lines are short: sixteen cells on average, and the longest, at
+ * 1.65 us a cell on its one warp, done while the others are (0.3 us a cell and
+ * SM) or before a chain of half as many cells and its ends would be.  Measured
+ * (us, with the cross-line copy; this / three lines a CTA / a warp per chain, a
+ * launch for the twists and one for the copy, the form before): 30000x1 99 /
+ * 212 / 206, 50000x3 300 / 552 / 474, 600x3 12 / 16 / 25, 20000x8 320 / 401 /
+ * 377, 3000x13 92 / 99 / 123, 9000 lines of 1 to 11 117 / 181 / 164; 3000x50
+ * 328 / 307 / 364, one line of 500 and 9000 of 3 824 / 425 / 462. */
+static bool fac_short(const FastLayout &L, int nsm) {
+    const double longest = L.max_len, cells = L.cells;
+    return cells <= 16.0 * L.nline && 1.65 * longest <= std::max(0.3 * cells / nsm, 1.7 * (0.5 * longest + 3.0));
+}
 
 int launch_fast_factor(cudaStream_t st, const FastLayout &L, const double *jacD, const double *O1,
                        const double *O2, double *Dinv, double *G, double *Gam, float *Dinv32,
@@ -1003,6 +1131,13 @@ int launch_fast_factor(cudaStream_t st, const FastLayout &L, const double *jacD,
     const int nfac = (L.nline + 2) / 3;
     const int most = few || nfac <= nsm ? nsm : 4 * nsm;
     const int copiers = X ? (int)std::min<long long>(most, (xc.nslots + 63) / 64) : 0;
+    if (fac_short(L, nsm)) {
+        xc.first = L.nline;
+        const int warps = X ? (int)std::min<long long>(32LL * nsm, (xc.nslots + 15) / 16) : 0;
+        fast_factor_short_kernel<<<L.nline + warps, 32, 0, st>>>(L.nline, L.line_start, L.line_len, L.line_twist,
+                                                                 L.fsrc, jacD, O1, O2, out, xc, status);
+        return (int)cudaGetLastError();
+    }
     if (few) {
         xc.first = L.nline;
         fast_factor_few_kernel<<<L.nline + copiers, 96, 2 * FEW_WORDS * sizeof(double), st>>>(

@@ -99,6 +99,7 @@ struct FastLayout {
     int ntile_own; /* tiles of the owned lines (all tiles unless the mesh ends in halo lines) */
     int nx;        /* cross-line coupling slots per position */
     int nline;
+    int cells;     /* of all lines */
     int max_len;   /* longest line */
     int longest;   /* a line of that length */
     /* device arrays */
